@@ -94,6 +94,18 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "cacheir_b200_rms_norm": (c_int, [c_void_p] * 5 + [c_int, c_int, c_float, c_int, c_void_p]),
     "cacheir_b200_rope_inplace": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int, c_longlong, c_void_p]),
     "cacheir_b200_rope_append": (c_int, [c_void_p] * 5 + [c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_longlong, c_void_p]),
+    "cacheir_b200_rms_norm_quantize_rows": (
+        c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int, c_float, c_void_p, c_size_t, c_void_p]),
+    "cacheir_b200_qgemm_rows": (
+        c_int,
+        [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,  # x packed scales zero_points residual y
+         c_int, c_void_p, c_int, c_int, c_int, c_int,                  # M n_rows N K bits scale_dtype
+         c_longlong, c_int, c_int, c_void_p, c_size_t, c_void_p]),     # x_stride epilogue layout ws bytes stream
+    "cacheir_b200_rope_append_rows": (
+        c_int, [c_void_p] * 5 + [c_int, c_void_p, c_void_p] + [c_int] * 6 + [c_void_p]),
+    "cacheir_b200_paged_attention_prompt": (
+        c_int,
+        [c_void_p] * 7 + [c_int] * 7 + [c_longlong, c_longlong, c_float, c_int, c_void_p]),
     "cacheir_b200_kv_append": (
         c_int, [c_void_p] * 6 + [c_int, c_int, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_void_p]),
     "cacheir_b200_kv_append_q8": (

@@ -198,6 +198,45 @@ __global__ void rope_append_kernel(T* __restrict__ qkv, const int32_t* __restric
   pool[dst + 1] = e1;
 }
 
+// ---- the same for the rows of a prompt: q and k heads rotate by a table of (cos, sin), the new k and v rows go to the
+// pool (only q is read from the row afterwards). Bound by memory: 16-byte pieces, four pairs per thread; the row's place in
+// the pool is (pages[row], position % page). Rows from *n_rows on are left alone.
+__global__ void __launch_bounds__(256)
+rope_append_rows_kernel(__half* __restrict__ qkv, const int32_t* __restrict__ positions, const int32_t* __restrict__ pages,
+                        const int* __restrict__ n_rows, const float2* __restrict__ table, int table_positions,
+                        __half* __restrict__ k_cache, __half* __restrict__ v_cache, int q_dim, int k_dim, int head_dim, int num_slots,
+                        int page_size) {
+  const int row = blockIdx.x;
+  if (n_rows && row >= *n_rows) return;
+  const int pos = positions[row], page = pages[row];
+  if (pos < 0 || pos >= table_positions) return;
+  const int n = q_dim + 2 * k_dim;
+  const float4* angles = reinterpret_cast<const float4*>(table + static_cast<size_t>(pos) * (head_dim / 2));
+  for (int col = 8 * threadIdx.x; col < n; col += 8 * blockDim.x) {
+    uint4* p = reinterpret_cast<uint4*>(qkv + static_cast<size_t>(row) * n + col);
+    uint4 raw = *p;
+    if (col < q_dim + k_dim) {
+      __half2* h = reinterpret_cast<__half2*>(&raw);
+      const float4 a = angles[col % head_dim / 4], b = angles[col % head_dim / 4 + 1];      // (cos, sin) of two pairs each
+      const float c[4] = {a.x, a.z, b.x, b.z}, s[4] = {a.y, a.w, b.y, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 v = __half22float2(h[i]);
+        float re, ro;
+        rope_rotate(v.x, v.y, c[i], s[i], &re, &ro);
+        h[i] = __halves2half2(__float2half_rn(re), __float2half_rn(ro));
+      }
+      if (col < q_dim) *p = raw;
+    }
+    if (col >= q_dim && page >= 0 && page < num_slots) {
+      const int kv_col = (col - q_dim) % k_dim;
+      const size_t dst = ((static_cast<size_t>(page) * (k_dim / head_dim) + kv_col / head_dim) * page_size + pos % page_size) *
+                             static_cast<size_t>(head_dim) + kv_col % head_dim;
+      *reinterpret_cast<uint4*>((col < q_dim + k_dim ? k_cache : v_cache) + dst) = raw;
+    }
+  }
+}
+
 // ---- KV append into 8-bit pools: each new row is quantised with its own scale --------------------
 // scale = fp16(max|row| / 127) (1 for an all-zero row), byte = clamp(rint(value / scale), -127, 127) + 128.
 // One CTA per (kv head, request); k and v rows of head_dim values each.
@@ -383,6 +422,21 @@ extern "C" int cacheir_b200_rope_table(float* table, int positions, int head_dim
   const size_t total = static_cast<size_t>(positions) * (head_dim / 2);
   rope_table_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, as_stream(stream)>>>(
       reinterpret_cast<float2*>(table), positions, head_dim, theta);
+  return launch_status();
+}
+
+extern "C" int cacheir_b200_rope_append_rows(void* qkv, const int32_t* positions, const int32_t* pages, const int32_t* n_rows,
+                                             const float* rope_table, int rope_table_positions, void* k_cache, void* v_cache, int M,
+                                             int q_dim, int k_dim, int head_dim, int num_slots, int page_size, void* stream) {
+  if (M <= 0) return 0;
+  if (!qkv || !positions || !pages || !rope_table || !k_cache || !v_cache || rope_table_positions <= 0 || num_slots <= 0 || page_size <= 0)
+    return CACHEIR_B200_EINVAL;
+  if (head_dim <= 0 || head_dim % 8 != 0 || q_dim <= 0 || k_dim <= 0 || q_dim % head_dim != 0 || k_dim % head_dim != 0) return CACHEIR_B200_EINVAL;
+  if (!aligned_to(qkv, 16) || !aligned_to(rope_table, 16) || !aligned_to(k_cache, 16) || !aligned_to(v_cache, 16)) return CACHEIR_B200_EALIGN;
+  rope_append_rows_kernel<<<M, 256, 0, as_stream(stream)>>>(static_cast<__half*>(qkv), positions, pages, n_rows,
+                                                            reinterpret_cast<const float2*>(rope_table), rope_table_positions,
+                                                            static_cast<__half*>(k_cache), static_cast<__half*>(v_cache), q_dim, k_dim, head_dim,
+                                                            num_slots, page_size);
   return launch_status();
 }
 

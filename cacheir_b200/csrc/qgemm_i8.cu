@@ -27,6 +27,7 @@
 #include "qgemv_common.cuh"
 #include "tc_ptx.cuh"
 #include "fixed_point.cuh"
+#include "i8_recombine.cuh"
 
 namespace cb200 {
 namespace {
@@ -261,6 +262,62 @@ rms_norm_quantize_kernel(const __half* __restrict__ x, const __half* __restrict_
   quantize_row_from_registers<PT>(vals, nvec, planes, mp, m, sx + m, qsum + m, scratch);
 }
 
+// ---- the same pre-pass for the rows of a prompt (qgemm_i8_rows.cu) ----------------------
+// Blocks of 128 rows, each laid out like a pass of 128: block t starts at byte t * 256 * K of the planes. Only the
+// first *n_rows rows are real (n_rows null: all); what the others hold is never stored by the GEMM.
+template <int PT>
+__global__ void __launch_bounds__(512)
+quantize_tall_kernel(const __half* __restrict__ x, long long x_stride, int M, const int* __restrict__ n_rows, int K,
+                     int8_t* __restrict__ planes, float* __restrict__ sx, int* __restrict__ qsum) {
+  __shared__ float scratch[32];
+  const int m = blockIdx.x;
+  if (m >= (n_rows ? min(M, *n_rows) : M)) return;
+  const int nvec = K / 8;
+  float vals[PT][8];
+#pragma unroll
+  for (int i = 0; i < PT; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) vals[i][j] = 0.f;
+    if (c < nvec) VecIO<__half, 8>::ld(x + static_cast<size_t>(m) * x_stride + c * 8, vals[i]);
+  }
+  quantize_row_from_registers<PT>(vals, nvec, planes + static_cast<size_t>(m >> 7) * 256 * K, 128, m & 127, sx + m, qsum + m, scratch);
+}
+
+template <int PT>
+__global__ void __launch_bounds__(512)
+rms_norm_quantize_tall_kernel(const __half* __restrict__ x, const __half* __restrict__ weight, int M, const int* __restrict__ n_rows,
+                              int hidden, float eps, int8_t* __restrict__ planes, float* __restrict__ sx, int* __restrict__ qsum) {
+  __shared__ float scratch[32];
+  const int m = blockIdx.x;
+  if (m >= (n_rows ? min(M, *n_rows) : M)) return;
+  const int nvec = hidden / 8;
+  float vals[PT][8], w[PT][8];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < PT; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) vals[i][j] = 0.f;
+    if (c < nvec) {
+      VecIO<__half, 8>::ld(x + static_cast<size_t>(m) * hidden + c * 8, vals[i]);
+      VecIO<__half, 8>::ld(weight + c * 8, w[i]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < PT; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss = fmaf(vals[i][j], vals[i][j], ss);
+  const float inv = rsqrtf(block_sum(ss, scratch) / static_cast<float>(hidden) + eps);
+#pragma unroll
+  for (int i = 0; i < PT; ++i)
+    if (static_cast<int>(threadIdx.x + i * blockDim.x) < nvec) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) vals[i][j] = __half2float(__float2half_rn(vals[i][j] * inv * w[i][j]));
+    }
+  quantize_row_from_registers<PT>(vals, nvec, planes + static_cast<size_t>(m >> 7) * 256 * hidden, 128, m & 127, sx + m, qsum + m, scratch);
+}
+
 struct I8Params {
   const void* scales;
   const float* zero_points;
@@ -283,27 +340,6 @@ struct I8Params {
 // 64 up rows of the same output columns (tile rows 64..127, weight rows N/2+64t..): one pass, one
 // accumulator, and twice as many CTAs as whole-half tiles would give.
 constexpr int kPairRows = 64;
-
-// y value from the exact integer sums: (256*hi + lo - zero*qsum) as float. Integer zero points in
-// [-255, 255] (what the reference packer produces) are handled in integers, anything else in double precision.
-// (The double-precision form is rare and kept out of line so that the epilogues stay short.)
-__device__ __noinline__ float recombine_fractional(int32_t hi, int32_t lo, float zero, int qsum) {
-  return static_cast<float>(256.0 * hi + static_cast<double>(lo) - static_cast<double>(zero) * qsum);
-}
-// `zero_int` is the zero point as an integer and `zero_is_int` says whether that is exact; both are
-// per-thread constants worked out once, outside the loops over the batch rows.
-__device__ __forceinline__ float recombine(int32_t hi, int32_t lo, float zero, int zero_int, bool zero_is_int, int qsum) {
-  if (zero_is_int) {
-    // 32-bit arithmetic only (64-bit integer math and its conversion cost several times more issue
-    // slots): with qsum = 256*qh + ql, v = 256*(hi - z*qh) + (lo - z*ql); both brackets fit in 32 bits
-    // for |z| <= 255. The float of v is exact-rounded while the first bracket is below 2^24
-    // (|v| < 2^32, far above what cancelled sums reach), and within 1.5 units in the last place beyond.
-    const int a = hi - zero_int * (qsum >> 8);
-    const int b = lo - zero_int * (qsum & 255);
-    return fmaf(static_cast<float>(a), 256.f, static_cast<float>(b));
-  }
-  return recombine_fractional(hi, lo, zero, qsum);
-}
 
 constexpr int kTailBytes = 1024;   // scratch behind the ring and the exchange buffer: barriers, TMEM base, per-row constants
 
@@ -850,7 +886,43 @@ int launch_i8(const QGemvParams& q, void* workspace, cudaStream_t stream) {
 
 size_t qgemm_i8_workspace_bytes(int M, int K) {
   if (M <= 0 || K <= 0) return 0;
+  if (M > 64) {   // two planes of whole 128-row blocks, then scales and sums of their rows (qgemm_i8_rows.cu)
+    const size_t rows = (static_cast<size_t>(M) + 127) / 128 * 128;
+    return rows * 2 * K + rows * 8 + 1024;
+  }
   return static_cast<size_t>(128) * K + 1024;   // two planes of up to 64 rows, then scales and sums
+}
+
+TallPlanes tall_planes(void* workspace, int M, int K) {
+  const size_t rows = (static_cast<size_t>(M) + 127) / 128 * 128;
+  TallPlanes t;
+  t.planes = static_cast<int8_t*>(workspace);
+  t.sx = reinterpret_cast<float*>(t.planes + rows * 2 * K);
+  t.qsum = reinterpret_cast<int*>(t.sx + rows);
+  return t;
+}
+
+int qgemm_i8_quantize_tall(const void* x, long long x_stride, int M, const int* n_rows, int K, void* workspace, cudaStream_t stream) {
+  const TallPlanes t = tall_planes(workspace, M, K);
+  const __half* xp = static_cast<const __half*>(x);
+  if (K <= 2048) quantize_tall_kernel<1><<<M, 256, 0, stream>>>(xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);
+  else if (K <= 4096) quantize_tall_kernel<1><<<M, 512, 0, stream>>>(xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);
+  else if (K <= 8192) quantize_tall_kernel<2><<<M, 512, 0, stream>>>(xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);
+  else if (K <= 16384) quantize_tall_kernel<4><<<M, 512, 0, stream>>>(xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);
+  else quantize_tall_kernel<8><<<M, 512, 0, stream>>>(xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);   // K <= 32768
+  return launch_status();
+}
+
+int qgemm_i8_rms_norm_quantize_tall(const void* x, const void* weight, int M, const int* n_rows, int hidden, float eps, void* workspace,
+                                    cudaStream_t stream) {
+  const TallPlanes t = tall_planes(workspace, M, hidden);
+  const __half* xp = static_cast<const __half*>(x);
+  const __half* wp = static_cast<const __half*>(weight);
+  if (hidden <= 2048) rms_norm_quantize_tall_kernel<1><<<M, 256, 0, stream>>>(xp, wp, M, n_rows, hidden, eps, t.planes, t.sx, t.qsum);
+  else if (hidden <= 4096) rms_norm_quantize_tall_kernel<1><<<M, 512, 0, stream>>>(xp, wp, M, n_rows, hidden, eps, t.planes, t.sx, t.qsum);
+  else if (hidden <= 8192) rms_norm_quantize_tall_kernel<2><<<M, 512, 0, stream>>>(xp, wp, M, n_rows, hidden, eps, t.planes, t.sx, t.qsum);
+  else return CACHEIR_B200_EUNSUPPORTED;
+  return launch_status();
 }
 
 bool qgemm_i8_supported(const QGemvParams& q, const void* workspace, size_t workspace_bytes) {

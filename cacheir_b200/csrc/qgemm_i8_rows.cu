@@ -1,0 +1,346 @@
+// Integer dequant-GEMM for prompts: more than 64 activation rows against tile-ordered int8 or int4 codes, sm_100a.
+//
+//   y[M, N] = x[M, K] . ((code[N, K] - zero[N]) * scale[N])^T      M > 64, fp16 x/y
+//
+// The arithmetic is that of qgemm_i8.cu (16-bit fixed-point activations split into two planes of signed bytes, exact int32
+// sums, the same recombination), so the results are the same bits. What differs is the shape of the work: a pass of 64 rows is
+// bound by streaming the weights, hundreds of rows are bound by the tensor cores and by what an SM can take in from L2.
+//
+// A pair of CTAs (cta_group::2) owns 256 weight rows x 128 activation rows: each CTA brings its 128 weight rows (16 KB per
+// 128-column k block) and one of the two planes (128 rows, 16 KB), and one MMA of M 256, N 256 (128 high, 128 low columns)
+// serves both. That is 32 KB per CTA and 512 tensor-core cycles; a CTA by itself would need 48 KB for the same cycles (both planes), more
+// than L2 delivers. The accumulator takes 256 of the 512 tensor-memory columns, so the epilogue of one tile runs under the main
+// loop of the next. Persistent: pairs walk the tiles with the row blocks innermost, so that the weights of the few tiles
+// in flight are read from HBM once and the activation planes stay in L2.
+//
+// Warps: 0 copies, 1 issues MMAs (even CTA only), 2-5 epilogue, with int4 codes 6-9 widen nibble tiles to byte tiles.
+#include "common.cuh"
+#include "qgemv_common.cuh"
+#include "tc_ptx.cuh"
+#include "i8_recombine.cuh"
+
+namespace cb200 {
+namespace {
+
+using namespace ptx;
+
+constexpr int kRows = 128;            // weight rows per CTA, activation rows per tile, bytes of k per stage
+constexpr int kTile = kRows * kRows;  // 16 KB: a weight tile, or one plane of an activation tile
+constexpr int kAccCols = 256;         // [128 high | 128 low]
+constexpr int kPairHalf = 64;         // SwiGLU: 64 gate and 64 up rows per weight tile
+constexpr int kChunk = 16;            // activation rows an epilogue thread handles at a time
+
+__device__ int g_i8_rows_status = 0;
+
+__host__ __device__ constexpr int stage_bytes(int bits) { return 2 * kTile + (bits == 4 ? kTile / 2 : 0); }
+__host__ __device__ constexpr int num_stages(int bits) { return bits == 4 ? 5 : 6; }
+__host__ __device__ constexpr int num_threads(int bits) { return bits == 4 ? 320 : 192; }
+constexpr int kExchangeBytes = 2 * kChunk * kPairHalf * 4;
+constexpr int kTailBytes = kExchangeBytes + 4 * kRows * 4 + 512;     // SwiGLU exchange, row scales and sums of two tiles, barriers
+
+struct RowsParams {
+  const void* scales;
+  const float* zero_points;
+  const __half* residual;
+  __half* y;
+  const float* sx;
+  const int* qsum;
+  const int* n_rows;
+  const uint8_t* w_tiled;
+  int M, N, K, n_out;
+  int scale_f16;
+  int bands;          // weight tiles of 128 rows
+};
+
+template <int BITS, bool SWIGLU>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(num_threads(BITS), 1)
+qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const RowsParams p) {
+  constexpr int S = num_stages(BITS);
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* s_w = smem;                       // [S] byte tiles of this CTA's weight rows
+  uint8_t* s_x = s_w + S * kTile;            // [S] this CTA's plane
+  uint8_t* s_raw = s_x + S * kTile;          // [S] int4: nibble tiles
+  float* s_up = reinterpret_cast<float*>(s_raw + (BITS == 4 ? S * kTile / 2 : 0));    // [2][kChunk][64]
+  float* s_sx = s_up + 2 * kChunk * kPairHalf;                                       // [2][128]
+  int* s_qsum = reinterpret_cast<int*>(s_sx + 2 * kRows);                             // [2][128]
+  uint64_t* full = reinterpret_cast<uint64_t*>(s_qsum + 2 * kRows);   // [S] (even CTA) operands of both CTAs have landed
+  uint64_t* empty = full + S;                // [S] the MMAs that read the stage have retired
+  uint64_t* raw_full = empty + S;            // [S] int4: this CTA's nibble tile has landed
+  uint64_t* ready = raw_full + S;            // [S] int4 (even CTA): the byte tiles of both CTAs are written
+  uint64_t* acc_full = ready + S;            // [2]
+  uint64_t* acc_empty = acc_full + 2;        // [2] (even CTA) both CTAs' epilogues have read the accumulator
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int rows = p.n_rows ? min(p.M, *p.n_rows) : p.M;
+  const int row_blocks = (rows + kRows - 1) / kRows;
+  const int kblocks = p.K / kRows;
+  const int tiles = (p.bands + 1) / 2 * row_blocks;
+  const int pairs = gridDim.x >> 1;
+  const int pair = blockIdx.x >> 1;
+
+  if (warp == 0 && lane == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(smem_u32(&full[s]), 1);
+      mbar_init(smem_u32(&empty[s]), 1);
+      mbar_init(smem_u32(&raw_full[s]), 1);
+      mbar_init(smem_u32(&ready[s]), 8);          // four converter warps of each CTA
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(smem_u32(&acc_full[a]), 1);
+      mbar_init(smem_u32(&acc_empty[a]), 8);      // four epilogue warps of each CTA
+    }
+    mbar_fence_init();
+  }
+  if (warp == 1) tc_alloc_pair(smem_u32(tmem_slot), 2 * kAccCols);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_release();                         // both CTAs' barriers exist before either is signalled
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // ---------------- copies ----------------
+      int it = 0;
+      bool ok = true;
+      for (int t = pair; t < tiles && ok; t += pairs) {
+        const int band = t / row_blocks * 2 + static_cast<int>(rank), block = t % row_blocks;
+        for (int kb = 0; kb < kblocks; ++kb, ++it) {
+          const int s = it % S;
+          if (it >= S && !mbar_wait(smem_u32(&empty[s]), ((it / S) & 1) ^ 1, &g_i8_rows_status, (6 << 8) | 1)) { ok = false; break; }
+          const uint32_t bar = map_to_rank(smem_u32(&full[s]), 0);
+          if (rank == 0) mbar_expect_tx(smem_u32(&full[s]), BITS == 8 ? 4 * kTile : 2 * kTile);
+          // (a band beyond the last one, where their number is odd, reads as zero)
+          if constexpr (BITS == 8) {
+            tma_load_2d_pair(smem_u32(s_w + s * kTile), &tmap_w, bar, 0, (band * kblocks + kb) * kRows);
+          } else {
+            const int b = min(band, p.bands - 1);
+            mbar_expect_tx(smem_u32(&raw_full[s]), kTile / 2);
+            bulk_load(smem_u32(s_raw + s * (kTile / 2)), p.w_tiled + (static_cast<size_t>(b) * kblocks + kb) * (kTile / 2), kTile / 2,
+                      smem_u32(&raw_full[s]));
+          }
+          tma_load_2d_pair(smem_u32(s_x + s * kTile), &tmap_x, bar, 0, ((block * kblocks + kb) * 2 + static_cast<int>(rank)) * kRows);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {
+      // ---------------- MMAs of the pair ----------------
+      // D = s32, A (codes) unsigned 8 bit, B (activation bytes) signed 8 bit, both K-major, N = 256, M = 256
+      constexpr uint32_t idesc = (2u << 4) | (0u << 7) | (1u << 10) | (static_cast<uint32_t>(kAccCols >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);
+      int it = 0, n = 0;
+      bool ok = true;
+      for (int t = pair; t < tiles && ok; t += pairs, ++n) {
+        const int a = n & 1;
+        if (n >= 2 && !mbar_wait_cluster(smem_u32(&acc_empty[a]), ((n >> 1) & 1) ^ 1, &g_i8_rows_status, (6 << 8) | 2)) break;
+        tc_fence_after();
+        const uint32_t d = tmem_base + a * kAccCols;
+        for (int kb = 0; kb < kblocks; ++kb, ++it) {
+          const int s = it % S;
+          if (!mbar_wait_cluster(smem_u32(&full[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 3)) { ok = false; break; }
+          if (BITS == 4 && !mbar_wait_cluster(smem_u32(&ready[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 4)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t w = smem_u32(s_w + s * kTile), x = smem_u32(s_x + s * kTile);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            tc_mma_i8_ss_pair(d, smem_desc_sw128(w + j * 32), smem_desc_sw128(x + j * 32), idesc, (kb > 0 || j > 0) ? 1u : 0u);
+          tc_commit_pair(smem_u32(&empty[s]));
+        }
+        tc_commit_pair(smem_u32(&acc_full[a]));
+      }
+    }
+  } else if (warp < 6) {
+    // ---------------- epilogue: lane quarter = warp % 4, a thread owns one weight row ----------------
+    const int q = warp & 3;
+    const int r = q * 32 + lane;
+    const int tid = threadIdx.x - 64;
+    const bool is_up = SWIGLU && r >= kPairHalf;
+    int n = 0;
+    bool ok = true;       // (a wait that gave up leaves the loops and their barriers as they are, without stores)
+    for (int t = pair; t < tiles; t += pairs, ++n) {
+      const int a = n & 1;
+      const int band = t / row_blocks * 2 + static_cast<int>(rank), m0 = t % row_blocks * kRows;
+      const int col = SWIGLU ? band * kPairHalf + (r & (kPairHalf - 1)) : band * kRows + r;      // output column
+      bool col_ok = col < p.n_out;
+      const int w_row = is_up ? p.N / 2 + col : col;
+      s_sx[a * kRows + tid] = p.sx[m0 + tid];              // (the arrays cover whole blocks of 128 rows)
+      s_qsum[a * kRows + tid] = p.qsum[m0 + tid];
+      float scale = 0.f, zero = 128.f;
+      if (col_ok) {
+        scale = p.scale_f16 ? __half2float(static_cast<const __half*>(p.scales)[w_row]) : static_cast<const float*>(p.scales)[w_row];
+        if (p.zero_points) zero = p.zero_points[w_row];
+      }
+      const bool zero_is_int = zero == rintf(zero) && fabsf(zero) <= 255.f;
+      const int zero_int = zero_is_int ? __float2int_rn(zero) : 0;
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      ok = ok && mbar_wait(smem_u32(&acc_full[a]), (n >> 1) & 1, &g_i8_rows_status, (6 << 8) | 5);
+      col_ok = col_ok && ok;
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t acc = tmem_base + a * kAccCols + (static_cast<uint32_t>(q * 32) << 16);
+      const int real = min(kRows, rows - m0);
+      __half* y = p.y + static_cast<size_t>(m0) * p.n_out + col;
+      const __half* res = p.residual ? p.residual + static_cast<size_t>(m0) * p.n_out + col : nullptr;
+#pragma unroll 1
+      for (int c0 = 0; c0 < kRows; c0 += kChunk) {
+        uint32_t hi[kChunk], lo[kChunk];
+        tc_ld_x16(acc + c0, hi);
+        tc_ld_x16(acc + kRows + c0, lo);
+        float add[kChunk];
+        if constexpr (!SWIGLU) {
+#pragma unroll
+          for (int j = 0; j < kChunk; ++j)
+            add[j] = res && col_ok && c0 + j < real ? __half2float(res[static_cast<size_t>(c0 + j) * p.n_out]) : 0.f;
+        }
+        tc_wait_ld();
+        if (c0 + kChunk >= kRows) {                        // the accumulator is in registers: the next tile may have it
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&acc_empty[a]), 0));
+        }
+        float v[kChunk];
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j) {
+          const int m = a * kRows + c0 + j;
+          v[j] = recombine(static_cast<int32_t>(hi[j]), static_cast<int32_t>(lo[j]), zero, zero_int, zero_is_int, s_qsum[m]) * (scale * s_sx[m]);
+        }
+        if constexpr (SWIGLU) {
+          // gate and up of a column sit 64 lanes apart: the up side hands over the first half of the chunk and finishes
+          // the second, the gate side the other way round
+          constexpr int H = kChunk / 2;
+          float* buf = s_up + ((c0 / kChunk) & 1) * kChunk * kPairHalf + (r & (kPairHalf - 1));
+#pragma unroll
+          for (int j = 0; j < H; ++j) {
+            if (is_up) buf[j * kPairHalf] = v[j];
+            else buf[(H + j) * kPairHalf] = v[H + j];
+          }
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < H; ++j) {
+            const float other = buf[(is_up ? H + j : j) * kPairHalf];
+            const float g = is_up ? other : v[j], u = is_up ? v[H + j] : other;
+            const int m = c0 + (is_up ? H + j : j);
+            if (col_ok && m < real) y[static_cast<size_t>(m) * p.n_out] = __float2half_rn(silu_fast(g) * u);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < kChunk; ++j)
+            if (col_ok && c0 + j < real) y[static_cast<size_t>(c0 + j) * p.n_out] = __float2half_rn(__fadd_rn(v[j], add[j]));
+        }
+      }
+    }
+  } else if constexpr (BITS == 4) {
+    // ---------------- int4: nibble tile -> byte tile ----------------
+    // Thread r owns tile row r: 64 bytes of nibbles (16-byte chunk c at c ^ ((r >> 1) & 3)) become 128 bytes of codes in the
+    // 128-byte swizzle order (chunk c at c ^ (r & 7)); even columns sit in the low nibbles.
+    const int r = threadIdx.x - 192;
+    int it = 0;
+    bool ok = true;
+    for (int t = pair; t < tiles && ok; t += pairs)
+      for (int kb = 0; kb < kblocks; ++kb, ++it) {
+        const int s = it % S;
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&raw_full[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 6));
+        if (!ok) break;
+        const uint8_t* raw_row = s_raw + s * (kTile / 2) + r * (kRows / 2);
+        uint8_t* out_row = s_w + s * kTile + r * kRows;
+        uint4 raw[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) raw[c] = *reinterpret_cast<const uint4*>(raw_row + ((c ^ ((r >> 1) & 3)) * 16));
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint32_t w[4] = {raw[c].x, raw[c].y, raw[c].z, raw[c].w};
+          uint32_t o[8];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint32_t even = w[j] & 0x0F0F0F0Fu;
+            const uint32_t odd = (w[j] >> 4) & 0x0F0F0F0Fu;
+            o[2 * j] = __byte_perm(even, odd, 0x5140);
+            o[2 * j + 1] = __byte_perm(even, odd, 0x7362);
+          }
+          *reinterpret_cast<uint4*>(out_row + (((2 * c) ^ (r & 7)) * 16)) = make_uint4(o[0], o[1], o[2], o[3]);
+          *reinterpret_cast<uint4*>(out_row + (((2 * c + 1) ^ (r & 7)) * 16)) = make_uint4(o[4], o[5], o[6], o[7]);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor core reads these bytes through the async proxy
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&ready[s]), 0));
+      }
+  }
+  // Nobody leaves while the other CTA may still signal its barriers, read its operands or use the pair's tensor memory.
+  __syncwarp();
+  tc_fence_before();
+  cluster_sync_release();
+  if (warp == 1) {
+    tc_fence_after();
+    tc_dealloc_pair(tmem_base, 2 * kAccCols);
+  }
+}
+
+template <int BITS, bool SWIGLU>
+int launch_rows(const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, const RowsParams& p, cudaStream_t stream) {
+  constexpr int kSmem = 1024 + num_stages(BITS) * stage_bytes(BITS) + kTailBytes;
+  static_assert((4 * num_stages(BITS) + 4) * 8 + 8 <= 512, "barriers and the tensor-memory base fit in the tail");
+  auto kern = qgemm_i8_rows_kernel<BITS, SWIGLU>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  const int tiles = (p.bands + 1) / 2 * ((p.M + kRows - 1) / kRows);
+  const int pairs = tiles < kNumSMs / 2 ? tiles : kNumSMs / 2;
+  kern<<<2 * pairs, num_threads(BITS), kSmem, stream>>>(tmap_w, tmap_x, p);
+  return launch_status();
+}
+
+}  // namespace
+
+// Tile-ordered per-row codes, fp16 activations, more than 64 rows; the 64-row kernel takes what is left.
+bool qgemm_i8_rows_supported(const QGemvParams& q, const void* workspace, size_t workspace_bytes) {
+  if (q.x_dtype != CACHEIR_B200_F16 || (q.bits != 8 && q.bits != 4) || q.group_size != 0 || !q.tiled || q.norm_weight) return false;
+  if (q.M <= 64 || q.K % kRows != 0 || q.K < kRows || q.K > 32768) return false;
+  const bool swiglu = q.epilogue == CACHEIR_B200_EPI_SWIGLU;
+  if (q.epilogue != CACHEIR_B200_EPI_NONE && q.epilogue != CACHEIR_B200_EPI_RESIDUAL && !swiglu) return false;
+  if (swiglu != q.paired || (swiglu && (q.N / 2) % kPairHalf != 0)) return false;
+  if (!workspace || workspace_bytes < qgemm_i8_workspace_bytes(q.M, q.K) || !aligned_to(workspace, 128)) return false;
+  if (!aligned_to(q.packed, 16) || !aligned_to(q.x, 16) || (q.x_stride * 2) % 16 != 0) return false;
+  return tensor_map_encoder() != nullptr;
+}
+
+int launch_qgemm_i8_rows(const QGemvParams& q, const int* n_rows, void* workspace, cudaStream_t stream) {
+  const TallPlanes planes = tall_planes(workspace, q.M, q.K);
+  if (!q.x_prequantized) {
+    const int rc = qgemm_i8_quantize_tall(q.x, q.x_stride, q.M, n_rows, q.K, workspace, stream);
+    if (rc != 0) return rc;
+  }
+  const bool swiglu = q.epilogue == CACHEIR_B200_EPI_SWIGLU;
+  RowsParams p{};
+  p.scales = q.scales; p.zero_points = q.zero_points;
+  p.residual = q.epilogue == CACHEIR_B200_EPI_RESIDUAL ? static_cast<const __half*>(q.residual) : nullptr;
+  p.y = static_cast<__half*>(q.y);
+  p.sx = planes.sx; p.qsum = planes.qsum; p.n_rows = n_rows;
+  p.w_tiled = static_cast<const uint8_t*>(q.packed);
+  p.M = q.M; p.N = q.N; p.K = q.K;
+  p.n_out = swiglu ? q.N / 2 : q.N;
+  p.scale_f16 = q.scale_dtype == CACHEIR_B200_F16 ? 1 : 0;
+  p.bands = swiglu ? (p.n_out + kPairHalf - 1) / kPairHalf : (p.n_out + kRows - 1) / kRows;
+  const uint64_t kblocks = static_cast<uint64_t>(q.K / kRows), blocks = static_cast<uint64_t>((q.M + kRows - 1) / kRows);
+  CUtensorMap tmap_w, tmap_x;
+  // (nibble tiles travel by plain bulk copies: their map is only a valid placeholder)
+  if (!encode_u8_tiles_plain(&tmap_w, q.packed, static_cast<uint64_t>(p.bands) * kblocks * (q.bits == 4 ? kRows / 2 : kRows)) ||
+      !encode_u8_tiles_plain(&tmap_x, planes.planes, blocks * kblocks * 2 * kRows))
+    return CACHEIR_B200_EUNSUPPORTED;
+  if (q.bits == 4) return swiglu ? launch_rows<4, true>(tmap_w, tmap_x, p, stream) : launch_rows<4, false>(tmap_w, tmap_x, p, stream);
+  return swiglu ? launch_rows<8, true>(tmap_w, tmap_x, p, stream) : launch_rows<8, false>(tmap_w, tmap_x, p, stream);
+}
+
+int qgemm_i8_rows_device_status(bool reset) {
+  int status = 0;
+  if (cudaMemcpyFromSymbol(&status, g_i8_rows_status, sizeof(int)) != cudaSuccess) return -1;
+  if (reset && status != 0) {
+    const int zero = 0;
+    cudaMemcpyToSymbol(g_i8_rows_status, &zero, sizeof(int));
+  }
+  return status;
+}
+
+}  // namespace cb200

@@ -237,6 +237,10 @@ int qgemv_dispatch(const void* x, const void* norm_weight, float norm_eps, const
   p.vector_ok = aligned_to(packed, 16) && row_bytes % 16 == 0 && aligned_to(x, 16) &&
                 (p.x_stride * esize) % 16 == 0;
   cudaStream_t st = as_stream(stream);
+  // More than 64 rows of per-row codes in tile order, with scratch for all of them: one launch over blocks of 128 rows (the same
+  // bits as the 64-row passes below, which stream the weights once per 64 rows: K 4096, N 14336, 128 rows 15 us against 56).
+  if (M > 64 && qgemm_i8_rows_supported(p, workspace, workspace_bytes))
+    return plan_only ? (1 << 8) | 1 : launch_qgemm_i8_rows(p, nullptr, workspace, st);
   if (M > 64 && !p.x_prequantized && !norm_weight) {
     // The integer tensor-core kernel takes up to 64 batch rows per launch, the fp16 one up to 128. A taller
     // batch runs as chunks of that height (the weights stream once per chunk, still far cheaper than the
@@ -319,6 +323,7 @@ extern "C" int cacheir_b200_qgemv(const void* x, const void* packed, const void*
 
 namespace cb200 {
 int peer_collectives_device_status(bool reset);
+int paged_prompt_device_status(bool reset);
 }
 
 extern "C" int cacheir_b200_device_status(int reset) {
@@ -327,7 +332,11 @@ extern "C" int cacheir_b200_device_status(int reset) {
   const int i8 = qgemm_i8_device_status(reset != 0);
   const int peer = peer_collectives_device_status(reset != 0);
   const int gemv = qgemv_mma_device_status(reset != 0);
-  return gemm != 0 ? gemm : (attn != 0 ? attn : (i8 != 0 ? i8 : (peer != 0 ? peer : gemv)));
+  const int rows = qgemm_i8_rows_device_status(reset != 0);
+  const int prompt = paged_prompt_device_status(reset != 0);
+  for (const int status : {gemm, attn, i8, peer, gemv, rows, prompt})
+    if (status != 0) return status;
+  return 0;
 }
 
 extern "C" int cacheir_b200_quantize_activations(const void* x, int M, int K, long long x_stride, int x_dtype,
@@ -351,6 +360,38 @@ extern "C" int cacheir_b200_rms_norm_quantize(const void* x, const void* residua
       (out && !aligned_to(out, 16)))
     return CACHEIR_B200_EALIGN;
   return qgemm_i8_rms_norm_quantize(x, residual, weight, sum_out, out, rows, hidden, eps, workspace, as_stream(stream));
+}
+
+extern "C" int cacheir_b200_rms_norm_quantize_rows(const void* x, const void* weight, int M, const int32_t* n_rows, int hidden, float eps,
+                                                   void* workspace, size_t workspace_bytes, void* stream) {
+  if (M <= 0 || hidden <= 0) return 0;
+  if (!x || !weight) return CACHEIR_B200_EINVAL;
+  if (M <= 64 || hidden % 128 != 0 || hidden > 8192) return CACHEIR_B200_EUNSUPPORTED;
+  if (!workspace || workspace_bytes < qgemm_i8_workspace_bytes(M, hidden) || !aligned_to(workspace, 128)) return CACHEIR_B200_EWORKSPACE;
+  if (!aligned_to(x, 16) || !aligned_to(weight, 16)) return CACHEIR_B200_EALIGN;
+  return qgemm_i8_rms_norm_quantize_tall(x, weight, M, n_rows, hidden, eps, workspace, as_stream(stream));
+}
+
+extern "C" int cacheir_b200_qgemm_rows(const void* x, const void* packed, const void* scales, const float* zero_points,
+                                       const void* residual, void* y, int M, const int32_t* n_rows, int N, int K, int bits,
+                                       int scale_dtype, long long x_stride, int epilogue, int weight_layout, void* workspace,
+                                       size_t workspace_bytes, void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  constexpr int kAllFlags = CACHEIR_B200_LAYOUT_TILED | CACHEIR_B200_X_PREQUANTIZED | CACHEIR_B200_LAYOUT_PAIRED;
+  if (!packed || !scales || !y || (weight_layout & ~kAllFlags) != 0) return CACHEIR_B200_EINVAL;
+  if (scale_dtype != CACHEIR_B200_F32 && scale_dtype != CACHEIR_B200_F16) return CACHEIR_B200_EINVAL;
+  if (epilogue == CACHEIR_B200_EPI_RESIDUAL && !residual) return CACHEIR_B200_EINVAL;
+  QGemvParams p{};
+  p.x = x; p.packed = packed; p.scales = scales; p.zero_points = zero_points; p.residual = residual; p.y = y;
+  p.M = M; p.N = N; p.K = K; p.bits = bits; p.x_dtype = CACHEIR_B200_F16; p.scale_dtype = scale_dtype;
+  p.x_stride = x_stride > 0 ? x_stride : K;
+  p.epilogue = epilogue;
+  p.tiled = (weight_layout & CACHEIR_B200_LAYOUT_TILED) != 0;
+  p.paired = (weight_layout & CACHEIR_B200_LAYOUT_PAIRED) != 0;
+  p.x_prequantized = (weight_layout & CACHEIR_B200_X_PREQUANTIZED) != 0;
+  if (!p.x_prequantized && !x) return CACHEIR_B200_EINVAL;
+  if (!qgemm_i8_rows_supported(p, workspace, workspace_bytes)) return CACHEIR_B200_EUNSUPPORTED;
+  return launch_qgemm_i8_rows(p, n_rows, workspace, as_stream(stream));
 }
 
 static int qkv_rope_append_dispatch(const void* x, const void* norm_weight, float norm_eps, const void* packed, const void* scales,

@@ -60,6 +60,20 @@ int qgemv_mma_device_status(bool reset);
 int qgemm_i8_quantize_activations(const void* x, long long x_stride, int M, int K, void* workspace, cudaStream_t stream);
 int qgemm_i8_rms_norm_quantize(const void* x, const void* residual, const void* weight, void* sum_out, void* out, int M,
                                int hidden, float eps, void* workspace, cudaStream_t stream);
+// Prompts and other batches of more than 64 rows on the integer tensor cores (qgemm_i8_rows.cu): blocks of 128 rows.
+// `n_rows` (device, may be null): only the first *n_rows of the M rows are real.
+struct TallPlanes {
+  int8_t* planes;   // [row block][k block][128 high, 128 low rows][128 bytes]
+  float* sx;
+  int* qsum;
+};
+TallPlanes tall_planes(void* workspace, int M, int K);
+int qgemm_i8_quantize_tall(const void* x, long long x_stride, int M, const int* n_rows, int K, void* workspace, cudaStream_t stream);
+int qgemm_i8_rms_norm_quantize_tall(const void* x, const void* weight, int M, const int* n_rows, int hidden, float eps, void* workspace,
+                                    cudaStream_t stream);
+bool qgemm_i8_rows_supported(const QGemvParams& p, const void* workspace, size_t workspace_bytes);
+int launch_qgemm_i8_rows(const QGemvParams& p, const int* n_rows, void* workspace, cudaStream_t stream);
+int qgemm_i8_rows_device_status(bool reset);
 // Device-side status word of the tensor-core kernel (0 = no bounded wait ever gave up).
 int qgemm_tc_device_status(bool reset);
 

@@ -371,6 +371,91 @@ def rope_append(qkv: torch.Tensor, positions: torch.Tensor, page_table: torch.Te
                                                qkv.stride(0), _stream()), "rope_append")
 
 
+# ---- the rows of prompts (the runtime's own buffers: shapes are checked when its plan is made) -----------------------
+def _count(n_rows: torch.Tensor | None) -> None:
+    if n_rows is not None and (n_rows.dtype != torch.int32 or not n_rows.is_cuda):
+        raise TypeError("n_rows must be an int32 CUDA tensor")
+
+
+def rms_norm_quantize_rows(x: torch.Tensor, weight: torch.Tensor, eps: float, workspace: torch.Tensor, n_rows: torch.Tensor | None = None) -> None:
+    """RMSNorm and fixed-point form of more than 64 fp16 rows; `qgemm_rows(prequantized=True)` consumes it."""
+    _require_cuda(x, weight, workspace)
+    _count(n_rows)
+    if x.dim() != 2 or not x.is_contiguous() or x.dtype != torch.float16 or weight.dtype != torch.float16 or weight.numel() != x.shape[1]:
+        raise ValueError("rms_norm_quantize_rows expects contiguous fp16 x [M, K] and an fp16 weight [K]")
+    check(_lib.load().cacheir_b200_rms_norm_quantize_rows(x.data_ptr(), weight.data_ptr(), int(x.shape[0]), _ptr(n_rows), int(x.shape[1]), float(eps),
+                                                          workspace.data_ptr(), workspace.numel() * workspace.element_size(), _stream()),
+          "rms_norm_quantize_rows")
+
+
+def qgemm_rows(x: torch.Tensor | None, packed: torch.Tensor, scales: torch.Tensor, zero_points: torch.Tensor | None, *, bits: int, n: int, k: int,
+               out: torch.Tensor, workspace: torch.Tensor, epilogue: int = EPI_NONE, residual: torch.Tensor | None = None, paired: bool = False,
+               n_rows: torch.Tensor | None = None) -> torch.Tensor:
+    """`qgemv` for more than 64 rows and tile-ordered per-row codes; without x the workspace holds its fixed-point form already."""
+    _require_cuda(x, packed, scales, zero_points, residual, out, workspace)
+    _count(n_rows)
+    m = int(out.shape[0])
+    n_out = n // 2 if epilogue == EPI_SWIGLU else n
+    if out.dtype != torch.float16 or tuple(out.shape) != (m, n_out) or not out.is_contiguous():
+        raise ValueError("out must be a contiguous fp16 [M, N_out] tensor")
+    if x is not None and (x.dtype != torch.float16 or tuple(x.shape) != (m, k) or x.stride(1) != 1):
+        raise ValueError("x must be fp16 [M, K] with dense rows")
+    if residual is not None and (residual.shape != out.shape or residual.dtype != out.dtype or not residual.is_contiguous()):
+        raise ValueError("residual must match out")
+    if packed.dtype != torch.uint8 or packed.numel() != pack_tiled_bytes(n, k, bits) or not packed.is_contiguous():
+        raise ValueError("packed must be the uint8 buffer produced by pack_relayout")
+    if scales.dtype not in (torch.float32, torch.float16) or scales.numel() != n or not scales.is_contiguous():
+        raise ValueError("scales must be a contiguous float32 or float16 tensor [N]")
+    if zero_points is not None and (zero_points.dtype != torch.float32 or zero_points.numel() != n):
+        raise ValueError("zero_points must be float32 [N]")
+    layout = 1 | (2 if x is None else 0) | (4 if paired else 0)
+    check(_lib.load().cacheir_b200_qgemm_rows(
+        _ptr(x), packed.data_ptr(), scales.data_ptr(), _ptr(zero_points), _ptr(residual), out.data_ptr(), m, _ptr(n_rows), n, k, bits,
+        F16 if scales.dtype == torch.float16 else F32, 0 if x is None else x.stride(0), epilogue, layout, workspace.data_ptr(),
+        workspace.numel() * workspace.element_size(), _stream()), "qgemm_rows")
+    return out
+
+
+def rope_append_rows(qkv: torch.Tensor, positions: torch.Tensor, pages: torch.Tensor, table: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, *,
+                     q_dim: int, k_dim: int, head_dim: int, n_rows: torch.Tensor | None = None) -> None:
+    """RoPE on q and k of dense rows qkv [M, q_dim + 2*k_dim] by `rope_table`; k and v go to row positions % page of page `pages`."""
+    _require_cuda(qkv, positions, pages, table, k_cache, v_cache)
+    _count(n_rows)
+    slots, kv_heads, page_size, pool_dim = (int(s) for s in k_cache.shape)
+    m = int(qkv.shape[0])
+    if qkv.dtype != torch.float16 or tuple(qkv.shape) != (m, q_dim + 2 * k_dim) or not qkv.is_contiguous():
+        raise ValueError("qkv must be contiguous fp16 [M, q_dim + 2*k_dim]")
+    if pool_dim != head_dim or kv_heads * head_dim != k_dim or v_cache.shape != k_cache.shape or k_cache.dtype != torch.float16 or v_cache.dtype != torch.float16:
+        raise ValueError("the pools must be fp16 and hold k_dim / head_dim heads of head_dim values")
+    if any(t.dtype != torch.int32 or t.numel() < m or not t.is_contiguous() for t in (positions, pages)):
+        raise ValueError("positions and pages must be contiguous int32 [M]")
+    if table.dtype != torch.float32 or not table.is_contiguous() or tuple(table.shape[1:]) != (head_dim // 2, 2):
+        raise ValueError("rope table must be float32 [positions, head_dim/2, 2]")
+    check(_lib.load().cacheir_b200_rope_append_rows(
+        qkv.data_ptr(), positions.data_ptr(), pages.data_ptr(), _ptr(n_rows), table.data_ptr(), int(table.shape[0]), k_cache.data_ptr(),
+        v_cache.data_ptr(), m, q_dim, k_dim, head_dim, slots, page_size, _stream()), "rope_append_rows")
+
+
+def paged_attention_prompt(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, page_table: torch.Tensor, tiles: torch.Tensor,
+                           n_tiles: torch.Tensor, out: torch.Tensor, *, softmax_scale: float | None = None) -> torch.Tensor:
+    """Causal attention of prompt rows q, out [M, H, D] (dense heads). `tiles` int32 [*, 4]: (sequence, first row, first position,
+    tokens) with tokens * H / KVH <= 64, of which n_tiles (device) are real; page_table [sequences, max_pages]."""
+    _require_cuda(q, k_cache, v_cache, page_table, tiles, n_tiles, out)
+    m, heads, head_dim = (int(s) for s in q.shape)
+    slots, kv_heads, page_size, pool_dim = (int(s) for s in k_cache.shape)
+    if any(t.dtype != torch.float16 for t in (q, k_cache, v_cache, out)) or pool_dim != head_dim or v_cache.shape != k_cache.shape or out.shape != q.shape:
+        raise ValueError("q, out [M, H, D] and the pools must be fp16 with one head_dim")
+    if any(t.stride(2) != 1 or t.stride(1) != head_dim for t in (q, out)) or not k_cache.is_contiguous() or not v_cache.is_contiguous():
+        raise ValueError("heads and pools must be dense")
+    if any(t.dtype != torch.int32 or not t.is_contiguous() for t in (page_table, tiles, n_tiles)) or tiles.dim() != 2 or tiles.shape[1] != 4:
+        raise ValueError("page_table, tiles [*, 4] and n_tiles must be contiguous int32")
+    check(_lib.load().cacheir_b200_paged_attention_prompt(
+        q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), page_table.data_ptr(), tiles.data_ptr(), n_tiles.data_ptr(), out.data_ptr(),
+        int(tiles.shape[0]), int(page_table.shape[0]), heads, kv_heads, int(page_table.shape[1]), page_size, head_dim, q.stride(0), out.stride(0),
+        float(softmax_scale or 0.0), slots, _stream()), "paged_attention_prompt")
+    return out
+
+
 def kv_append_q8(k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, kv_scales: torch.Tensor,
                  page_table: torch.Tensor, positions: torch.Tensor) -> None:
     """`kv_append` into uint8 pools: each new row is quantised with its own fp16 scale (kv_scales [slots, KVH, 2, page])."""

@@ -173,6 +173,7 @@ class _Engine:
         self.validated_sessions: list[Any] = []
         # prompt tokens per pass of the chunked prefill (0: one token per step)
         self.prefill_chunk = 2048 if self.ragged else 64
+        self.prompt_rows = 0 if self.ragged else self._prompt_rows(kv_dtype)
         self._rope_tables: dict[tuple[int, float], torch.Tensor] = {}
         self.attention_splits = int(attention_splits)
         self.max_plans = max(1, int(max_plans)) * (4 if self.ragged else 1)     # (ragged plans share their buffers)
@@ -180,6 +181,7 @@ class _Engine:
         self._derived: dict[tuple, torch.Tensor] = {}
         self._largest: dict[str, float] = {}
         self.plans: OrderedDict[tuple, "_DecodePlan"] = OrderedDict()
+        self.prompt_plans: OrderedDict[tuple, "_DecodePlan"] = OrderedDict()      # one per bucket of rows, on shared buffers
         self.plans_lowered = 0          # decode graphs lowered to launch lists so far
         self.graph_captures = 0         # CUDA graphs captured so far
         self.kernel_counts: OrderedDict[str, int] = OrderedDict()
@@ -187,6 +189,25 @@ class _Engine:
         self.fused_weights: dict[tuple[str, ...], B200PackedWeight | torch.Tensor] = {}
         self.prefix_cache = B200PrefixCache(self.allocator, int(self.config.num_layers))
         self.tokenizer = ByteTokenizer(int(self.config.vocab_size))
+
+    def _prompt_rows(self, kv_dtype: str) -> int:
+        """Rows of the widest prompt pass (`_PromptPlan`), 0 where prompts go through 64-row passes of the decode plan: it
+        takes packed fp16 graphs of fused ops with 16-token fp16 pages. Bounded so that the logits of a pass stay under 256 MB."""
+        ops_taken = {"token_embedding", "quantized_fused_rmsnorm_qkv_rope", "paged_attention_decode", "quantized_matmul", "add", "rms_norm",
+                     "quantized_fused_swiglu"}
+        c = self.config
+        if (self.dtype != torch.float16 or not self.quant or self.tp.enabled or kv_dtype != "same" or self.page_size != 16
+                or int(c.head_dim) not in (64, 128) or int(c.num_attention_heads) // int(c.num_key_value_heads) > 16
+                or int(c.hidden_size) % 128 or int(c.hidden_size) > 8192 or int(c.intermediate_size) % 128
+                or any(node.op not in ops_taken for node in self.graph.nodes)):
+            return 0
+        rows = min(2048, (1 << 27) // int(c.vocab_size) // 128 * 128)
+        return rows if rows >= 128 else 0
+
+    @property
+    def pass_rows(self) -> int:
+        """Prompt tokens that one pass takes."""
+        return self.prompt_rows if self.prompt_rows and self.prefill_chunk else self.prefill_chunk
 
     def count(self, name: str, n: int = 1) -> None:
         self.kernel_counts[name] = self.kernel_counts.get(name, 0) + n
@@ -337,20 +358,27 @@ class _Engine:
                           lambda width: self.plan_class(self, bucket(rows), width, segments=bucket(segments),
                                                         logit_rows=bucket(max(1, logit_rows))))
 
-    def _plan(self, key: tuple, needed_pages: int, make: Callable[[int], "_DecodePlan"]) -> "_DecodePlan":
-        plan = self.plans.get(key)
+    def _plan(self, key: tuple, needed_pages: int, make: Callable[[int], "_DecodePlan"],
+              plans: "OrderedDict[tuple, _DecodePlan] | None" = None) -> "_DecodePlan":
+        plans = self.plans if plans is None else plans
+        plan = plans.get(key)
         if plan is not None and (plan.pool_generation != self.allocator.generation or plan.width < needed_pages):
-            self.plans.pop(key)
+            plans.pop(key)
             plan = None
         if plan is None:
             plan = make(max(needed_pages, (self.max_seq_len + self.page_size - 1) // self.page_size))
             self.plans_lowered += 1
-            self.plans[key] = plan
-            while len(self.plans) > self.max_plans:
-                self.plans.popitem(last=False)
+            plans[key] = plan
+            while len(plans) > self.max_plans:
+                plans.popitem(last=False)
         else:
-            self.plans.move_to_end(key)
+            plans.move_to_end(key)
         return plan
+
+    def prompt_plan(self, rows: int, needed_pages: int) -> "_PromptPlan":
+        """The plan for up to `rows` prompt rows of any sequences (more than 64 of them)."""
+        size = min(bucket(rows), self.prompt_rows)
+        return self._plan(("prompt", size), needed_pages, lambda width: _PromptPlan(self, size, width), self.prompt_plans)
 
     def prefill_plan(self, rows: int, needed_pages: int) -> "_DecodePlan":
         """The plan that pushes `rows` prompt tokens through the decode graph at once: row i is one (sequence,
@@ -370,19 +398,14 @@ class _DecodePlan:
     """Static device buffers and the flat launch list of one decode step for a
     fixed batch size; optionally a CUDA graph of that list."""
 
+    decodes = True       # one row per sequence, lengths advance on the device
+
     def __init__(self, engine: _Engine, batch: int, width: int):
         self.engine = engine
         self.batch = batch
         self.width = width
         self.pool_generation = engine.allocator.generation
-        dev = engine.device
-        self.ids = torch.zeros((batch,), device=dev, dtype=torch.int64)
-        self.positions = torch.zeros((batch,), device=dev, dtype=torch.int32)
-        self.seq_lens = torch.zeros((batch,), device=dev, dtype=torch.int32)
-        self.page_table = torch.zeros((batch, width), device=dev, dtype=torch.int32)
-        self.host_ids = torch.zeros((batch,), dtype=torch.int64).pin_memory()
-        self.host_lens = torch.zeros((batch,), dtype=torch.int32).pin_memory()
-        self.host_table = torch.zeros((batch, width), dtype=torch.int32).pin_memory()
+        self._make_buffers()
         self.synced_owner_state: list[tuple[str, int, int, int]] | None = None
         self.repeat_key: tuple | None = None     # the session list whose next steps need only new token ids (see _repeat_step)
         self.repeat_tokens: list[int] = []
@@ -396,6 +419,16 @@ class _DecodePlan:
         self.steps_run = 0
         self.logits: torch.Tensor | None = None
         self._lower()
+
+    def _make_buffers(self) -> None:
+        dev, batch, width = self.engine.device, self.batch, self.width
+        self.ids = torch.zeros((batch,), device=dev, dtype=torch.int64)
+        self.positions = torch.zeros((batch,), device=dev, dtype=torch.int32)
+        self.seq_lens = torch.zeros((batch,), device=dev, dtype=torch.int32)
+        self.page_table = torch.zeros((batch, width), device=dev, dtype=torch.int32)
+        self.host_ids = torch.zeros((batch,), dtype=torch.int64).pin_memory()
+        self.host_lens = torch.zeros((batch,), dtype=torch.int32).pin_memory()
+        self.host_table = torch.zeros((batch, width), dtype=torch.int32).pin_memory()
 
     # -- graph lowering --------------------------------------------------------------
     def _emit(self, fn: Callable[[], None], count_key: str, launches: int = 1) -> None:
@@ -423,10 +456,11 @@ class _DecodePlan:
         for name in eng.graph.outputs:
             uses[name] = uses.get(name, 0) + 1
 
-        if eng.dtype == torch.float16 and eng.quant:
+        if eng.dtype == torch.float16 and eng.quant and self.decodes:
             widest = max(int(eng.config.hidden_size), int(eng.config.intermediate_size))
             self._gemm_ws = torch.zeros((ops.qgemv_workspace_bytes(self.batch, widest),), device=eng.device, dtype=torch.uint8)
-        self._emit(lambda: ops.advance_positions(self.positions, self.seq_lens), "b200.advance_positions")
+        if self.decodes:
+            self._emit(lambda: ops.advance_positions(self.positions, self.seq_lens), "b200.advance_positions")
         skip: set[int] = set()
         for idx, node in enumerate(nodes):
             if idx in skip:
@@ -448,7 +482,7 @@ class _DecodePlan:
                     names = (nxt.inputs[1],) if nxt.op == "quantized_matmul" else tuple(nxt.inputs[1:3])
                     if self._i8_eligible(eng.matmul_weight(names, True, self.batch), int(x.shape[1]), swiglu=len(names) == 2):
                         ws = self._gemm_workspace(int(x.shape[1]))
-                        self._emit(lambda x=x, w=w, eps=eps, ws=ws: ops.rms_norm_quantize(x, w, eps, ws), "b200.rms_norm_quantize")
+                        self._norm_quantize(x, w, eps, ws)
                         env[node.outputs[0]] = x            # placeholder: the consumer reads the workspace, not this tensor
                         self._prequantized.add(node.outputs[0])
                         fused = True
@@ -518,9 +552,9 @@ class _DecodePlan:
                 consumer = self._attention_consumer(nodes, idx, node)
                 if self._i8_eligible(weight, int(x.shape[1])):
                     ws = self._gemm_workspace(int(x.shape[1]))
-                    self._emit(lambda x=x, w=norm_w, eps=eps, ws=ws: ops.rms_norm_quantize(x, w, eps, ws), "b200.rms_norm_quantize")
+                    self._norm_quantize(x, norm_w, eps, ws)
                     pool = eng.allocator.pool_for_layer(int(consumer.attrs.get("layer", 0))) if consumer is not None else None
-                    if (pool is not None and weight.bits == 8 and self._rows_of(node.inputs[4]) // eng.tp.world == k_dim and pool["keys"].dtype == torch.float16
+                    if (self.decodes and pool is not None and weight.bits == 8 and self._rows_of(node.inputs[4]) // eng.tp.world == k_dim and pool["keys"].dtype == torch.float16
                             and int(pool["keys"].shape[3]) == head_dim and int(pool["keys"].shape[1]) * head_dim == k_dim):
                         # projection + RoPE + append of the new k/v rows in one kernel
                         n, k = weight.shape
@@ -547,11 +581,7 @@ class _DecodePlan:
                 pool = eng.allocator.pool_for_layer(int(consumer.attrs.get("layer", 0))) if consumer is not None else None
                 if (pool is not None and "scales" not in pool and pool["keys"].dtype == qkv.dtype and int(pool["keys"].shape[3]) == head_dim
                         and int(pool["keys"].shape[1]) * head_dim == k_dim and int(qkv.shape[1]) == q_dim + 2 * k_dim):
-                    # RoPE on q|k and the append of the new k / v rows in one launch
-                    k_pool, v_pool = pool["keys"], pool["values"]
-                    self._emit(lambda qkv=qkv, k_pool=k_pool, v_pool=v_pool, hd=head_dim, theta=theta:
-                               ops.rope_append(qkv, self.positions, self.page_table, k_pool, v_pool, q_dim=q_dim, k_dim=k_dim,
-                                               head_dim=hd, theta=theta), "b200.rope_append")
+                    self._rope_append(qkv, pool, q_dim, k_dim, head_dim, theta)
                     self._kv_appended.add(node.outputs[1])
                 else:
                     qk = qkv[:, : q_dim + k_dim]   # q and k heads are adjacent: one RoPE launch covers both
@@ -581,7 +611,7 @@ class _DecodePlan:
                 nxt = nodes[idx + 1] if idx + 1 < len(nodes) else None
                 quant_ws = None
                 if (nxt is not None and nxt.op == "quantized_matmul" and nxt.inputs[0] == node.outputs[0]
-                        and uses.get(node.outputs[0], 0) == 1 and eng.fuse_attention_prepass and not eng.tp.enabled):
+                        and uses.get(node.outputs[0], 0) == 1 and eng.fuse_attention_prepass and not eng.tp.enabled and self.decodes):
                     # (single GPU only: under tensor parallelism the o projection keeps its own pre-pass)
                     k_total = int(attrs["num_heads"]) * int(attrs["head_dim"])
                     if (self._i8_eligible(eng.matmul_weight((nxt.inputs[1],), True, self.batch, "replicated"), k_total)
@@ -622,6 +652,15 @@ class _DecodePlan:
         # Greedy feedback variant: the row argmax overwrites `ids` (already consumed by the
         # embedding gather of this step), so the next replay needs nothing from the host.
         self.feedback_tail = lambda: ops.argmax_rows(logits, self.ids)
+
+    def _norm_quantize(self, x: torch.Tensor, w: torch.Tensor, eps: float, ws: torch.Tensor) -> None:
+        self._emit(lambda: ops.rms_norm_quantize(x, w, eps, ws), "b200.rms_norm_quantize")
+
+    def _rope_append(self, qkv: torch.Tensor, pool: dict[str, torch.Tensor], q_dim: int, k_dim: int, head_dim: int, theta: float) -> None:
+        """RoPE on q|k and the append of the new k / v rows in one launch."""
+        k_pool, v_pool = pool["keys"], pool["values"]
+        self._emit(lambda: ops.rope_append(qkv, self.positions, self.page_table, k_pool, v_pool, q_dim=q_dim, k_dim=k_dim, head_dim=head_dim,
+                                           theta=theta), "b200.rope_append")
 
     def _rows_of(self, weight_name: str) -> int:
         spec = self.engine.graph.weights[weight_name]
@@ -811,6 +850,119 @@ class _DecodePlan:
             self.run_program(feedback=True)
             out[i].copy_(self.ids, non_blocking=True)
         return out
+
+
+class _PromptPlan(_DecodePlan):
+    """The decode graph over the rows of prompts: up to `batch` (sequence, position) rows of any sequences in one pass.
+
+    What a row needs travels in one copy: its id, position and page, and the attention's tiles of neighbouring tokens. The
+    number of rows lives on the device, so that a plan serves every step of its bucket. Products run on the integer tensor
+    cores in blocks of 128 rows (group-wise int4: fp16 ones), attention reads a tile's keys once for its tokens and heads.
+    Activations live in buffers that all prompt plans share."""
+
+    decodes = False
+    SEQUENCES = 256      # of one pass: the page tables' room
+
+    def __init__(self, engine: _Engine, batch: int, width: int):
+        config = engine.config
+        self.group = int(config.num_attention_heads) // int(config.num_key_value_heads)
+        self.tile_tokens = 64 // self.group
+        self.sequences = min(batch, self.SEQUENCES)
+        self.max_tiles = batch // self.tile_tokens + self.sequences
+        size = 4 + 4 * batch + 4 * self.max_tiles
+        self.host_meta = torch.zeros((size,), dtype=torch.int32).pin_memory()
+        self.meta = torch.zeros((size,), device=engine.device, dtype=torch.int32)
+        self.n_rows, self.n_tiles = self.meta[0:1], self.meta[1:2]
+        self.row_pages = self.meta[4 + 3 * batch:4 + 4 * batch]
+        self.tiles = self.meta[4 + 4 * batch:].view(-1, 4)
+        self._turn: dict[int, int] = {}
+        super().__init__(engine, batch, width)
+
+    def _make_buffers(self) -> None:
+        dev, n = self.engine.device, self.batch
+        self.ids = self.meta[4:4 + 2 * n].view(torch.int64)
+        self.positions = self.meta[4 + 2 * n:4 + 3 * n]
+        self.page_table = torch.zeros((self.sequences, self.width), device=dev, dtype=torch.int32)
+        self.host_table = torch.zeros((self.sequences, self.width), dtype=torch.int32).pin_memory()
+
+    def _buf(self, cols: int) -> torch.Tensor:
+        """Shared by all plans and layers. Of the residual's width five take turns (an operand is at most four products old),
+        of the other widths one value is alive at a time."""
+        turn = self._turn.get(cols, 0)
+        self._turn[cols] = (turn + 1) % (5 if cols == int(self.engine.config.hidden_size) else 1)
+        storage = self.engine.scratch(f"prompt{cols}.{turn}", self.engine.prompt_rows * cols * 2)
+        return storage[: self.batch * cols * 2].view(torch.float16).view(self.batch, cols)
+
+    def _gemm_workspace(self, k: int) -> torch.Tensor:
+        widest = max(int(self.engine.config.hidden_size), int(self.engine.config.intermediate_size))
+        return self.engine.scratch("prompt.planes", ops.qgemv_workspace_bytes(self.engine.prompt_rows, widest))
+
+    def _i8_eligible(self, weight: Any, k: int, swiglu: bool = False) -> bool:
+        return (isinstance(weight, B200PackedWeight) and weight.bits in (4, 8) and not weight.group_size and weight.tiled
+                and weight.paired == swiglu and k % 128 == 0 and k <= 8192)
+
+    def _norm_quantize(self, x: torch.Tensor, w: torch.Tensor, eps: float, ws: torch.Tensor) -> None:
+        self._emit(lambda: ops.rms_norm_quantize_rows(x, w, eps, ws, self.n_rows), "b200.rms_norm_quantize")
+
+    def _matmul(self, x: torch.Tensor, weight: B200PackedWeight | torch.Tensor, *, epilogue: int = ops.EPI_NONE,
+                residual: torch.Tensor | None = None, prequantized: bool = False, out: torch.Tensor | None = None) -> torch.Tensor:
+        if not (isinstance(weight, B200PackedWeight) and weight.tiled and not weight.group_size
+                and weight.paired == (epilogue == ops.EPI_SWIGLU)):
+            return super()._matmul(x, weight, epilogue=epilogue, residual=residual, prequantized=prequantized, out=out)
+        n, k, bits = weight.shape[0], weight.shape[1], weight.bits
+        epilogue = ops.EPI_RESIDUAL if residual is not None else epilogue
+        out = out if out is not None else self._buf(n // 2 if epilogue == ops.EPI_SWIGLU else n)
+        ws = self._gemm_workspace(k)
+        key = f"b200.qgemm_rows.int{bits}" + (".swiglu" if epilogue == ops.EPI_SWIGLU else ".residual" if residual is not None else "")
+        self.engine.gemm_plans[f"q{bits}:{(self.batch, 1, k)}x{weight.shape}"] = key
+        self._emit(lambda: ops.qgemm_rows(None if prequantized else x, weight.packed_values, weight.scales, weight.zero_points, bits=bits, n=n, k=k,
+                                          out=out, workspace=ws, epilogue=epilogue, residual=residual, paired=weight.paired, n_rows=self.n_rows),
+                   key, launches=1 if prequantized else 2)
+        return out
+
+    def _rope_append(self, qkv: torch.Tensor, pool: dict[str, torch.Tensor], q_dim: int, k_dim: int, head_dim: int, theta: float) -> None:
+        table = self.engine.rope_table(head_dim, theta)
+        self._emit(lambda: ops.rope_append_rows(qkv, self.positions, self.row_pages, table, pool["keys"], pool["values"], q_dim=q_dim, k_dim=k_dim,
+                                                head_dim=head_dim, n_rows=self.n_rows), "b200.rope_append")
+
+    def _attention(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, attrs: dict[str, Any], *,
+                   appended: bool = False, quant_ws: torch.Tensor | None = None) -> tuple[torch.Tensor, bool]:
+        if not appended:
+            raise NotImplementedError("a prompt pass appends its rows with the rotation")
+        heads, head_dim = int(attrs["num_heads"]), int(attrs["head_dim"])
+        pool = self.engine.allocator.pool_for_layer(int(attrs.get("layer", 0)))
+        out = self._buf(heads * head_dim)
+        q3 = q.as_strided((self.batch, heads, head_dim), (q.stride(0), head_dim, 1), q.storage_offset())
+        out3 = out.view(self.batch, heads, head_dim)
+        self._emit(lambda: ops.paged_attention_prompt(q3, pool["keys"], pool["values"], self.page_table, self.tiles, self.n_tiles, out3),
+                   "b200.paged_attention_prompt")
+        return out, False
+
+    def sync_parts(self, parts: list[tuple[B200PagedKVCache, int, list[int]]]) -> None:
+        """The rows of this pass: tokens of each (cache, position of the first one, tokens), whose pages are reserved."""
+        self.h2d_done.synchronize()      # the pinned staging buffers must not change under a pending copy
+        n, step = self.batch, self.tile_tokens
+        meta, table = self.host_meta.numpy(), self.host_table.numpy()
+        ids, positions, pages = meta[4:4 + 2 * n].view(np.int64), meta[4 + 2 * n:4 + 3 * n], meta[4 + 3 * n:4 + 4 * n]
+        row, tiles = 0, []
+        for i, (cache, start, tokens) in enumerate(parts):
+            count = len(tokens)
+            at = np.arange(start, start + count, dtype=np.int32)
+            table[i] = cache.page_table_row(self.width)
+            ids[row:row + count] = tokens
+            positions[row:row + count] = at
+            pages[row:row + count] = table[i][at // self.engine.page_size]
+            first = np.arange(0, count, step, dtype=np.int32)
+            tiles.append(np.stack([np.full_like(first, i), row + first, start + first, np.minimum(step, count - first)], axis=1))
+            row += count
+        listed = np.concatenate(tiles)
+        listed = listed[np.argsort(-(listed[:, 2] + listed[:, 3]), kind="stable")]      # most keys first
+        meta[0], meta[1] = row, len(listed)
+        end = 4 + 4 * n + 4 * len(listed)
+        meta[4 + 4 * n:end] = listed.reshape(-1)
+        self.meta[:end].copy_(self.host_meta[:end], non_blocking=True)
+        self.page_table[:len(parts)].copy_(self.host_table[:len(parts)], non_blocking=True)
+        self.h2d_done.record()
 
 
 RaggedPlan = make_plan_class(_DecodePlan)
@@ -1059,7 +1211,7 @@ class B200DecodeRuntime:
         if mode == "prefill" and chunk > 1 and len(tokens) > chunk // 4:
             self._enforce_memory_limit()
             try:
-                return self._prefill_chunked(tokens, chunk)
+                return self._prefill_chunked(tokens, self._engine.pass_rows)
             except (torch.cuda.OutOfMemoryError, KVPoolExhausted) as exc:
                 self._recover_from_oom()
                 raise RuntimeError("CacheIR CUDA runtime recovered from an out-of-memory condition; "
@@ -1105,7 +1257,7 @@ class B200DecodeRuntime:
             session.kv_cache.extend(len(tokens))
         results = []
         with torch.cuda.device(self.device):
-            passes = cut_passes(token_batches, eng.prefill_chunk or 64)
+            passes = cut_passes(token_batches, eng.pass_rows or 64, None if eng.ragged else _PromptPlan.SEQUENCES)
             for part in passes:                                   # (session, first token, last token + 1)
                 want = [(i, int(p)) for i, lo, hi in part for p in wanted[i] if lo <= int(p) < hi]
                 logits = self._run_rows(sessions, token_batches, starts, part, want)
@@ -1133,11 +1285,24 @@ class B200DecodeRuntime:
             plan.sync_portions([(sessions[i].kv_cache, starts[i] + lo, [int(t) for t in token_batches[i][lo:hi]]) for i, lo, hi in part], rows)
             plan.run_program()
             return plan.logits[: len(rows)]
-        needed = max(len(s.kv_cache.pages) for s in sessions)
-        plan = eng.prefill_plan(eng.prefill_chunk or 64, needed)
-        plan.sync_prefill_rows([(sessions[i].kv_cache, starts[i] + p, int(token_batches[i][p])) for i, lo, hi in part for p in range(lo, hi)])
+        logits = self._run_prompt_rows([(sessions[i].kv_cache, starts[i] + lo, token_batches[i][lo:hi]) for i, lo, hi in part])
+        return logits[rows]
+
+    def _run_prompt_rows(self, parts: list[tuple[B200PagedKVCache, int, list[int]]]) -> torch.Tensor:
+        """One pass over tokens of several sequences, (cache, position of the first one, tokens) each, whose pages are
+        reserved. Returns the logits of all rows in order (valid until the next pass)."""
+        eng = self._engine
+        rows = sum(len(tokens) for _, _, tokens in parts)
+        needed = max(len(cache.pages) for cache, _, _ in parts)
+        # up to 64 rows the weights are the bottleneck and the decode plan's kernels stream them best
+        if rows > 64 and eng.prompt_rows and eng.prefill_chunk:
+            plan = eng.prompt_plan(rows, needed)
+            plan.sync_parts(parts)
+        else:
+            plan = eng.prefill_plan(eng.prefill_chunk or 64, needed)
+            plan.sync_prefill_rows([(cache, start + i, int(t)) for cache, start, tokens in parts for i, t in enumerate(tokens)])
         plan.run_program()
-        return plan.logits[rows]
+        return plan.logits[:rows]
 
     def _check_room(self, sessions, lengths: list[int]) -> None:
         """Raise before anything is reserved when a step cannot get its pages, state slots or positions."""
@@ -1172,41 +1337,27 @@ class B200DecodeRuntime:
                 start = cache.tokens
                 cache.extend(len(part))
                 self._check_positions([self])
-                needed = (cache.tokens + eng.page_size - 1) // eng.page_size
-                plan = eng.prefill_plan(chunk, needed)
-                plan.sync_prefill_chunk(cache, start, part)
-                plan.run_program()
-                out[0, c0:c0 + len(part)] = plan.logits[: len(part)]
+                out[0, c0:c0 + len(part)] = self._run_prompt_rows([(cache, start, part)])
         eng.count("cacheir.b200_prefill_chunk", (len(tokens) + chunk - 1) // chunk)
         return out
 
     def _prefill_packed(self, sessions: list["B200DecodeRuntime"], token_id_batches: list[list[int]], out: torch.Tensor) -> None:
         """Prefill of several sequences through shared passes (cuda.py:584-629 pads every prompt to the longest and
         masks; here nothing is padded): the (sequence, position) pairs are laid out in order and cut into passes of
-        `prefill_chunk` rows; a pass appends all its K/V rows, then every row attends to the tokens up to itself
+        `pass_rows` rows; a pass appends all its K/V rows, then every row attends to the tokens up to itself
         through its own sequence's page table. `out[i, t]` receives the logits of token t of sequence i."""
         eng = self._engine
-        chunk = eng.prefill_chunk
-        work: list[tuple[int, int]] = []                       # (sequence index, position)
-        for i, (session, ids) in enumerate(zip(sessions, token_id_batches)):
-            start = session.kv_cache.tokens
+        starts = [session.kv_cache.tokens for session in sessions]
+        for session, ids in zip(sessions, token_id_batches):
             session.kv_cache.extend(len(ids))                  # reserves the pages of the whole prompt
-            work.extend((i, start + t) for t in range(len(ids)))
         self._check_positions(sessions)
-        needed = max((s.kv_cache.tokens + eng.page_size - 1) // eng.page_size for s in sessions)
-        starts = [s.kv_cache.tokens - len(ids) for s, ids in zip(sessions, token_id_batches)]
-        passes = 0
         with torch.cuda.device(self.device):
-            for w0 in range(0, len(work), chunk):
-                part = work[w0:w0 + chunk]
-                plan = eng.prefill_plan(chunk, needed)
-                plan.sync_prefill_rows([(sessions[i].kv_cache, pos, int(token_id_batches[i][pos - starts[i]])) for i, pos in part])
-                plan.run_program()
-                seq = torch.tensor([i for i, _ in part], device=self.device, dtype=torch.long)
-                tok = torch.tensor([pos - starts[i] for i, pos in part], device=self.device, dtype=torch.long)
-                out[seq, tok] = plan.logits[: len(part)]
-                passes += 1
-        eng.count("cacheir.b200_prefill_chunk", passes)
+            passes = cut_passes(token_id_batches, eng.pass_rows, _PromptPlan.SEQUENCES)
+            for part in passes:                                # (sequence, first token, last token + 1)
+                logits = self._run_prompt_rows([(sessions[i].kv_cache, starts[i] + lo, token_id_batches[i][lo:hi]) for i, lo, hi in part])
+                for (i, lo, hi), rows in zip(part, logits.split([hi - lo for _, lo, hi in part])):
+                    out[i, lo:hi] = rows
+        eng.count("cacheir.b200_prefill_chunk", len(passes))
 
     def run_prefill_batch(self, sessions: list["B200DecodeRuntime"], token_id_batches: list[list[int]]) -> torch.Tensor:
         """Variable-length batched prefill (cuda.py:584-629): returns zero-padded logits [N, max_len, vocab]."""
@@ -1323,15 +1474,15 @@ class B200DecodeRuntime:
                                f"(kernel class {status >> 8}, wait {status & 0xFF}); the last results are undefined")
 
 
-def cut_passes(token_batches: list[list[int]], rows: int) -> list[list[tuple[int, int, int]]]:
-    """Cut a step into passes of at most `rows` rows: lists of (sequence, first token, last token + 1). A sequence's
-    tokens stay in order across passes."""
+def cut_passes(token_batches: list[list[int]], rows: int, sequences: int | None = None) -> list[list[tuple[int, int, int]]]:
+    """Cut a step into passes of at most `rows` rows (of at most `sequences` sequences): lists of (sequence, first token,
+    last token + 1). A sequence's tokens stay in order across passes."""
     passes: list[list[tuple[int, int, int]]] = [[]]
     room = rows
     for i, tokens in enumerate(token_batches):
         lo = 0
         while lo < len(tokens):
-            if room == 0:
+            if room == 0 or len(passes[-1]) == sequences:
                 passes.append([])
                 room = rows
             hi = min(len(tokens), lo + room)

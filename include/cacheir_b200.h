@@ -429,6 +429,34 @@ int cacheir_b200_rope_append(void* qkv, const int32_t* positions, const int32_t*
                              int max_pages_per_seq, int page_size, int dtype, long long qkv_batch_stride,
                              void* stream);
 
+/* ---- the rows of prompts: more than 64 rows of several sequences in one pass --------------------------------------
+ * M is the room of the buffers; `n_rows` (device, may be NULL: all) says how many of the M rows are real, so that one
+ * captured launch serves every smaller step. Replaces the padded prefill of cacheir/runtime/cuda.py:584-629.
+ *
+ * RMSNorm of fp16 rows and their 16-bit fixed-point form in `workspace` (cacheir_b200_qgemv_workspace_bytes(M, hidden)),
+ * hidden a multiple of 128 and at most 8192, M > 64. */
+int cacheir_b200_rms_norm_quantize_rows(const void* x, const void* weight, int M, const int32_t* n_rows, int hidden,
+                                        float eps, void* workspace, size_t workspace_bytes, void* stream);
+/* cacheir_b200_qgemv_ex for M > 64 fp16 rows and per-row int8 / int4 codes in tile order (paired tiles with the SwiGLU
+ * epilogue); x may be NULL with CACHEIR_B200_X_PREQUANTIZED. The same bits as passes of 64 rows. */
+int cacheir_b200_qgemm_rows(const void* x, const void* packed, const void* scales, const float* zero_points,
+                            const void* residual, void* y, int M, const int32_t* n_rows, int N, int K, int bits,
+                            int scale_dtype, long long x_stride, int epilogue, int weight_layout, void* workspace,
+                            size_t workspace_bytes, void* stream);
+/* RoPE on q and k of dense fp16 rows [M][q_dim + 2*k_dim] by the table of cacheir_b200_rope_table; the rotated k and the v
+ * go to pool slot pages[row] at positions[row] % page_size. Afterwards only the q columns of the rows are defined. */
+int cacheir_b200_rope_append_rows(void* qkv, const int32_t* positions, const int32_t* pages, const int32_t* n_rows,
+                                  const float* rope_table, int rope_table_positions, void* k_cache, void* v_cache, int M,
+                                  int q_dim, int k_dim, int head_dim, int num_slots, int page_size, void* stream);
+/* Causal attention of prompt rows over fp16 pools (head_dim 64 or 128, 16-token pages, at most 64 heads per KV head).
+ * tiles: [max_tiles][4] int32 (sequence, first row, first position, tokens), tokens * heads / kv_heads <= 64, of which the
+ * first *n_tiles are real; token i of a tile attends to the first_position + i + 1 tokens of page_table[sequence]. */
+int cacheir_b200_paged_attention_prompt(const void* q, const void* k_cache, const void* v_cache, const int32_t* page_table,
+                                        const int32_t* tiles, const int32_t* n_tiles, void* out, int max_tiles,
+                                        int num_sequences, int heads, int kv_heads, int max_pages, int page_size,
+                                        int head_dim, long long q_stride, long long out_stride, float softmax_scale,
+                                        int num_slots, void* stream);
+
 /* The same into 8-bit pools (see cacheir_b200_paged_attention_decode_batch_ex): every new row is quantised with its
  * own scale, scale = fp16(max|row| / 127) (1 for an all-zero row), byte = clamp(rint(value / scale), -127, 127) + 128;
  * the scale goes to kv_scales[slot][kv_head][0 (K) | 1 (V)][pos % page_size] (fp16). head_dim <= 256.

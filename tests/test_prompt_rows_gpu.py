@@ -1,0 +1,132 @@
+"""The kernels of prompt passes (more than 64 rows of several sequences) against the 64-row kernels they extend."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _status():
+    from cacheir_b200 import _lib
+    return int(_lib.load().cacheir_b200_device_status(1))
+
+
+# edges: one row past the 64-row kernels, whole and ragged blocks of 128, an odd number of weight tiles (half a pair), a last tile
+# that is not full, a single k block, more tiles than CTA pairs
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("m, n, k, epilogue", [(65, 128, 128, 0), (128, 384, 256, 1), (129, 320, 1024, 0), (300, 1280, 2048, 1), (192, 256, 640, 2),
+                                               (257, 640, 1152, 2), (1024, 4096, 512, 0)])
+def test_rows_equal_passes_of_64(bits, m, n, k, epilogue):
+    from cacheir_b200 import ops
+    from cacheir_b200.quantization import pack_weight_device, to_tiled
+
+    g = torch.Generator(device="cuda").manual_seed(m * 7 + n + k)
+    w = to_tiled(pack_weight_device(torch.randn((n, k), device="cuda", generator=g) * 0.02, "int8" if bits == 8 else "int4_awq"), paired=epilogue == 2)
+    x = torch.randn((m, k), device="cuda", generator=g).half()
+    x[m // 2] = 0.0
+    n_out = n // 2 if epilogue == 2 else n
+    res = torch.randn((m, n_out), device="cuda", generator=g).half() if epilogue == 1 else None
+    kw = dict(bits=bits, n=n, k=k, epilogue=epilogue, paired=w.paired)
+    ws = torch.zeros(ops.qgemv_workspace_bytes(64, k), device="cuda", dtype=torch.uint8)
+    want = torch.cat([ops.qgemv(x[i:i + 64], w.packed_values, w.scales, w.zero_points, residual=None if res is None else res[i:i + 64], workspace=ws,
+                                tiled=True, **kw) for i in range(0, m, 64)])
+    big = torch.full((ops.qgemv_workspace_bytes(m, k),), 255, device="cuda", dtype=torch.uint8)
+
+    def same(a, b):      # the residual may join in one fused rounding or two: a float32 rounding apart, so at most neighbours in fp16
+        return torch.equal(a, b) if epilogue != 1 else bool(((a.float() - b.float()).abs() <= 2.0 ** -10 * b.float().abs().clamp_min(2.0 ** -14)).all())
+    assert same(ops.qgemv(x, w.packed_values, w.scales, w.zero_points, residual=res, workspace=big, tiled=True, **kw), want)
+    real = m - 31                        # only some of the rows are real: the others stay as they were
+    out = torch.full((m, n_out), 7.0, device="cuda", dtype=torch.float16)
+    ops.qgemm_rows(x, w.packed_values, w.scales, w.zero_points, residual=res, out=out, workspace=big,
+                   n_rows=torch.tensor([real], device="cuda", dtype=torch.int32), **kw)
+    assert same(out[:real], want[:real]) and bool((out[real:] == 7.0).all())
+    assert _status() == 0
+
+
+@pytest.mark.parametrize("heads, kv_heads, dim", [(32, 8, 128), (6, 2, 64), (16, 1, 128), (3, 3, 128)])
+def test_prompt_attention_equals_the_rows_one_by_one(heads, kv_heads, dim):
+    """Several sequences, some with tokens in the cache already; each row's output against the decode kernel's, which sees the
+    same keys. Both round probabilities to fp16 (2^-11 each, averaged over the keys) and the output once more: rel-L2 5e-4."""
+    from cacheir_b200 import ops
+
+    rng = np.random.default_rng(heads)
+    parts = [(0, 1), (0, 64), (15, 17), (200, 130), (63, 2), (0, 333)]            # (tokens before, rows)
+    group, page = heads // kv_heads, 16
+    step = 64 // group
+    pages = [(a + n + page - 1) // page for a, n in parts]
+    perm = rng.permutation(sum(pages) + 3)
+    table = np.zeros((len(parts), max(pages)), dtype=np.int32)
+    tiles, row_table, lens, at, row = [], [], [], 0, 0
+    for i, (a, n) in enumerate(parts):
+        table[i, :pages[i]] = perm[at:at + pages[i]]
+        at += pages[i]
+        tiles += [(i, row + t, a + t, min(step, n - t)) for t in range(0, n, step)]
+        row_table += [i] * n
+        lens += range(a + 1, a + n + 1)
+        row += n
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    k, v = (torch.randn((sum(pages) + 3, kv_heads, page, dim), device="cuda", generator=g).half() for _ in range(2))
+    wide = torch.randn((row + 5, heads * dim + 64), device="cuda", generator=g).half()      # rows of a wider buffer
+    q = wide[:, :heads * dim].as_strided((row + 5, heads, dim), (wide.stride(0), dim, 1))
+    listed = torch.zeros((len(tiles) + 9, 4), dtype=torch.int32)
+    listed[:len(tiles)] = torch.tensor(tiles, dtype=torch.int32)
+    out = torch.full((row + 5, heads, dim), 7.0, device="cuda", dtype=torch.float16)
+    ops.paged_attention_prompt(q, k, v, torch.from_numpy(table).cuda(), listed.cuda(), torch.tensor([len(tiles)], dtype=torch.int32, device="cuda"), out)
+    want = ops.paged_attention_decode_batch(q[:row], k, v, torch.from_numpy(table[row_table]).cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda"))
+    err = (out[:row].float() - want.float()).norm() / want.float().norm()
+    assert float(err) <= 5e-4, float(err)
+    assert bool((out[row:] == 7.0).all()) and _status() == 0
+
+
+def test_rope_append_rows_equals_rope_append():
+    from cacheir_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q_dim, k_dim, dim, rows = 512, 256, 128, 70
+    qkv = torch.randn((rows, q_dim + 2 * k_dim), device="cuda", generator=g).half()
+    positions = torch.arange(rows, device="cuda", dtype=torch.int32) + 11
+    slots = torch.randperm(8, device="cuda", generator=g).int()
+    table = slots.repeat(rows, 1).contiguous()
+    pools = [torch.zeros((8, 2, 16, dim), device="cuda", dtype=torch.float16) for _ in range(4)]
+    a, b = qkv.clone(), qkv.clone()
+    ops.rope_append(a, positions, table, pools[0], pools[1], q_dim=q_dim, k_dim=k_dim, head_dim=dim, theta=10000.0)
+    ops.rope_append_rows(b, positions, slots[positions.long() // 16].contiguous(), ops.rope_table(128, dim, 10000.0, torch.device("cuda")), pools[2], pools[3],
+                         q_dim=q_dim, k_dim=k_dim, head_dim=dim, n_rows=torch.tensor([rows], device="cuda", dtype=torch.int32))
+    assert torch.equal(a[:, :q_dim], b[:, :q_dim]) and torch.equal(pools[0], pools[2]) and torch.equal(pools[1], pools[3])
+
+
+@pytest.mark.parametrize("quant", ["int8", "int4_awq", "int4_g128"])
+def test_prompt_pass_equals_passes_of_64_rows(quant):
+    """Prompts through one pass against 64-row passes of the decode plan: logits and the cached rows that later steps read. The
+    products are the same integers (int4_g128: the same fp16 products), only the attention adds in another order."""
+    import cacheir_b200 as C
+
+    gen = torch.Generator(device="cuda")
+
+    def source(key, shape):
+        gen.manual_seed(len(key) * 131 + sum(map(ord, key)))
+        return torch.ones(shape, device="cuda") if len(shape) == 1 else torch.randn(shape, device="cuda", generator=gen) * 0.05
+
+    art = C.build_decoder_artifact(C.ModelConfig(architecture="LlamaForCausalLM", hidden_size=512, intermediate_size=768, num_layers=2, num_attention_heads=4,
+                                                 num_key_value_heads=2, vocab_size=640, max_position_embeddings=512, rope_theta=10000.0, dtype="float16"),
+                                   quant=quant, modes=("decode",))
+    rt = C.B200DecodeRuntime(art, dtype="float16", tensor_source=source, max_seq_len=512)
+    assert rt._engine.prompt_rows == 2048
+    rng = np.random.default_rng(5)
+    prompts = [[int(t) for t in rng.integers(0, 640, n)] for n in (5, 200, 1, 70)]
+    fast, slow = [rt.fork() for _ in prompts], [rt.fork() for _ in prompts]
+    got = [rt.run_prefill_batch(fast, prompts), rt.run_prefill_batch(fast, [p[::-1] for p in prompts]), rt.run_prefill_batch(fast, prompts)][2]   # third: a replay
+    follow = rt.run_step_batch(fast, [[3] * n for n in (40, 1, 66, 2)])          # portions behind cached tokens
+    assert rt.kernel_counts["b200.paged_attention_prompt"] > 0
+    rt._engine.prompt_rows = 0
+    want = rt.run_prefill_batch(slow, prompts)
+    want_follow = rt.run_step_batch(slow, [[3] * n for n in (40, 1, 66, 2)])
+    for a, b in ((got, want), (follow, want_follow)):
+        assert float((a.float() - b.float()).norm() / b.float().norm()) <= 2e-3
+    for layer in range(2):
+        pool = rt.kv_allocator.pool_for_layer(layer)
+        for f, s in zip(fast, slow):
+            for name in ("keys", "values"):
+                a, b = (torch.cat([pool[name][p.page_id][:, :p.length] for p in x.kv_cache.pages], dim=1).float() for x in (f, s))
+                assert float((a - b).norm() / b.norm()) <= 2e-3
+    rt.check_device_status()
