@@ -13,7 +13,8 @@
 // loop of the next. Persistent: pairs walk the tiles with the row blocks innermost, so that the weights of the few tiles
 // in flight are read from HBM once and the activation planes stay in L2.
 //
-// Warps: 0 copies, 1 issues MMAs (even CTA only), 2-5 epilogue, with int4 codes 6-9 widen nibble tiles to byte tiles.
+// Warps: 0 copies, 1 issues MMAs (even CTA only), 2-9 epilogue (four per half of the activation rows), with int4 codes 10-21
+// widen nibble tiles to byte tiles in three groups that take every third stage.
 #include "common.cuh"
 #include "qgemv_common.cuh"
 #include "tc_ptx.cuh"
@@ -34,9 +35,11 @@ __device__ int g_i8_rows_status = 0;
 
 __host__ __device__ constexpr int stage_bytes(int bits) { return 2 * kTile + (bits == 4 ? kTile / 2 : 0); }
 __host__ __device__ constexpr int num_stages(int bits) { return bits == 4 ? 5 : 6; }
-__host__ __device__ constexpr int num_threads(int bits) { return bits == 4 ? 320 : 192; }
-constexpr int kExchangeBytes = 2 * kChunk * kPairHalf * 4;
-constexpr int kTailBytes = kExchangeBytes + 4 * kRows * 4 + 512;     // SwiGLU exchange, row scales and sums of two tiles, barriers
+constexpr int kEpilogueThreads = 256;
+constexpr int kConverterGroups = 3;     // one group needs 1770 cycles from barrier to barrier for a stage of 512 tensor-core cycles
+__host__ __device__ constexpr int num_threads(int bits) { return 64 + kEpilogueThreads + (bits == 4 ? kConverterGroups * 128 : 0); }
+constexpr int kExchangeBytes = 2 * 2 * kChunk * kPairHalf * 4;
+constexpr int kTailBytes = kExchangeBytes + 2 * kRows * 16 + 512;     // SwiGLU exchange, row scales and sums of two tiles, barriers
 
 struct RowsParams {
   const void* scales;
@@ -61,10 +64,9 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   uint8_t* s_w = smem;                       // [S] byte tiles of this CTA's weight rows
   uint8_t* s_x = s_w + S * kTile;            // [S] this CTA's plane
   uint8_t* s_raw = s_x + S * kTile;          // [S] int4: nibble tiles
-  float* s_up = reinterpret_cast<float*>(s_raw + (BITS == 4 ? S * kTile / 2 : 0));    // [2][kChunk][64]
-  float* s_sx = s_up + 2 * kChunk * kPairHalf;                                       // [2][128]
-  int* s_qsum = reinterpret_cast<int*>(s_sx + 2 * kRows);                             // [2][128]
-  uint64_t* full = reinterpret_cast<uint64_t*>(s_qsum + 2 * kRows);   // [S] (even CTA) operands of both CTAs have landed
+  float* s_up = reinterpret_cast<float*>(s_raw + (BITS == 4 ? S * kTile / 2 : 0));    // [half][2][kChunk][64]
+  int4* s_row = reinterpret_cast<int4*>(s_up + 4 * kChunk * kPairHalf);               // [2][128] (scale, sum >> 8, sum & 255, sum)
+  uint64_t* full = reinterpret_cast<uint64_t*>(s_row + 2 * kRows);   // [S] (even CTA) operands of both CTAs have landed
   uint64_t* empty = full + S;                // [S] the MMAs that read the stage have retired
   uint64_t* raw_full = empty + S;            // [S] int4: this CTA's nibble tile has landed
   uint64_t* ready = raw_full + S;            // [S] int4 (even CTA): the byte tiles of both CTAs are written
@@ -91,7 +93,7 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&acc_full[a]), 1);
-      mbar_init(smem_u32(&acc_empty[a]), 8);      // four epilogue warps of each CTA
+      mbar_init(smem_u32(&acc_empty[a]), 16);     // eight epilogue warps of each CTA
     }
     mbar_fence_init();
   }
@@ -136,13 +138,13 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       bool ok = true;
       for (int t = pair; t < tiles && ok; t += pairs, ++n) {
         const int a = n & 1;
-        if (n >= 2 && !mbar_wait_cluster(smem_u32(&acc_empty[a]), ((n >> 1) & 1) ^ 1, &g_i8_rows_status, (6 << 8) | 2)) break;
+        if (n >= 2 && !mbar_wait(smem_u32(&acc_empty[a]), ((n >> 1) & 1) ^ 1, &g_i8_rows_status, (6 << 8) | 2)) break;
         tc_fence_after();
         const uint32_t d = tmem_base + a * kAccCols;
         for (int kb = 0; kb < kblocks; ++kb, ++it) {
           const int s = it % S;
-          if (!mbar_wait_cluster(smem_u32(&full[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 3)) { ok = false; break; }
-          if (BITS == 4 && !mbar_wait_cluster(smem_u32(&ready[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 4)) { ok = false; break; }
+          if (!mbar_wait(smem_u32(&full[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 3)) { ok = false; break; }
+          if (BITS == 4 && !mbar_wait(smem_u32(&ready[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 4)) { ok = false; break; }
           tc_fence_after();
           const uint32_t w = smem_u32(s_w + s * kTile), x = smem_u32(s_x + s * kTile);
 #pragma unroll
@@ -153,10 +155,12 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         tc_commit_pair(smem_u32(&acc_full[a]));
       }
     }
-  } else if (warp < 6) {
-    // ---------------- epilogue: lane quarter = warp % 4, a thread owns one weight row ----------------
+  } else if (warp < 10) {
+    // ---------------- epilogue: lane quarter = warp % 4, a thread owns one weight row and 64 of the activation rows ----------------
+    // About ten instructions per output; a scheduler has two of these warps, so the loops keep 16 independent outputs going.
     const int q = warp & 3;
     const int r = q * 32 + lane;
+    const int half = (warp - 2) >> 2;
     const int tid = threadIdx.x - 64;
     const bool is_up = SWIGLU && r >= kPairHalf;
     int n = 0;
@@ -167,8 +171,10 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       const int col = SWIGLU ? band * kPairHalf + (r & (kPairHalf - 1)) : band * kRows + r;      // output column
       bool col_ok = col < p.n_out;
       const int w_row = is_up ? p.N / 2 + col : col;
-      s_sx[a * kRows + tid] = p.sx[m0 + tid];              // (the arrays cover whole blocks of 128 rows)
-      s_qsum[a * kRows + tid] = p.qsum[m0 + tid];
+      if (tid < kRows) {                                   // (the arrays cover whole blocks of 128 rows)
+        const int sum = p.qsum[m0 + tid];
+        s_row[a * kRows + tid] = make_int4(__float_as_int(p.sx[m0 + tid]), sum >> 8, sum & 255, sum);
+      }
       float scale = 0.f, zero = 128.f;
       if (col_ok) {
         scale = p.scale_f16 ? __half2float(static_cast<const __half*>(p.scales)[w_row]) : static_cast<const float*>(p.scales)[w_row];
@@ -176,60 +182,78 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       }
       const bool zero_is_int = zero == rintf(zero) && fabsf(zero) <= 255.f;
       const int zero_int = zero_is_int ? __float2int_rn(zero) : 0;
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+      const bool all_int = __all_sync(0xffffffffu, zero_is_int);
+      asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueThreads) : "memory");
       ok = ok && mbar_wait(smem_u32(&acc_full[a]), (n >> 1) & 1, &g_i8_rows_status, (6 << 8) | 5);
       col_ok = col_ok && ok;
       __syncwarp();
       tc_fence_after();
-      const uint32_t acc = tmem_base + a * kAccCols + (static_cast<uint32_t>(q * 32) << 16);
+      const uint32_t acc = tmem_base + a * kAccCols + half * (kRows / 2) + (static_cast<uint32_t>(q * 32) << 16);
       const int real = min(kRows, rows - m0);
       __half* y = p.y + static_cast<size_t>(m0) * p.n_out + col;
       const __half* res = p.residual ? p.residual + static_cast<size_t>(m0) * p.n_out + col : nullptr;
 #pragma unroll 1
-      for (int c0 = 0; c0 < kRows; c0 += kChunk) {
+      for (int c0 = 0; c0 < kRows / 2; c0 += kChunk) {
         uint32_t hi[kChunk], lo[kChunk];
         tc_ld_x16(acc + c0, hi);
         tc_ld_x16(acc + kRows + c0, lo);
+        const int first = half * (kRows / 2) + c0;          // activation row of the tile
         float add[kChunk];
         if constexpr (!SWIGLU) {
 #pragma unroll
           for (int j = 0; j < kChunk; ++j)
-            add[j] = res && col_ok && c0 + j < real ? __half2float(res[static_cast<size_t>(c0 + j) * p.n_out]) : 0.f;
+            add[j] = res && col_ok && first + j < real ? __half2float(res[static_cast<size_t>(first + j) * p.n_out]) : 0.f;
         }
         tc_wait_ld();
-        if (c0 + kChunk >= kRows) {                        // the accumulator is in registers: the next tile may have it
+        if (c0 + kChunk >= kRows / 2) {                     // the accumulator is in registers: the next tile may have it
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&acc_empty[a]), 0));
         }
+        const int4* row = s_row + a * kRows + first;
         float v[kChunk];
+        if (all_int) {
 #pragma unroll
-        for (int j = 0; j < kChunk; ++j) {
-          const int m = a * kRows + c0 + j;
-          v[j] = recombine(static_cast<int32_t>(hi[j]), static_cast<int32_t>(lo[j]), zero, zero_int, zero_is_int, s_qsum[m]) * (scale * s_sx[m]);
+          for (int j = 0; j < kChunk; ++j) {
+            const int4 at = row[j];
+            v[j] = fmaf(static_cast<float>(static_cast<int>(hi[j]) - zero_int * at.y), 256.f, static_cast<float>(static_cast<int>(lo[j]) - zero_int * at.z)) *
+                   (scale * __int_as_float(at.x));
+          }
+        } else {
+#pragma unroll 1
+          for (int j = 0; j < kChunk; ++j) {                // (rolled, on registers picked by comparison: rare)
+            int h = 0, l = 0;
+#pragma unroll
+            for (int i = 0; i < kChunk; ++i)
+              if (i == j) { h = static_cast<int>(hi[i]); l = static_cast<int>(lo[i]); }
+            const float f = recombine(h, l, zero, zero_int, zero_is_int, row[j].w) * (scale * __int_as_float(row[j].x));
+#pragma unroll
+            for (int i = 0; i < kChunk; ++i)
+              if (i == j) v[i] = f;
+          }
         }
         if constexpr (SWIGLU) {
           // gate and up of a column sit 64 lanes apart: the up side hands over the first half of the chunk and finishes
           // the second, the gate side the other way round
           constexpr int H = kChunk / 2;
-          float* buf = s_up + ((c0 / kChunk) & 1) * kChunk * kPairHalf + (r & (kPairHalf - 1));
+          float* buf = s_up + (half * 2 + ((c0 / kChunk) & 1)) * kChunk * kPairHalf + (r & (kPairHalf - 1));
 #pragma unroll
           for (int j = 0; j < H; ++j) {
             if (is_up) buf[j * kPairHalf] = v[j];
             else buf[(H + j) * kPairHalf] = v[H + j];
           }
-          asm volatile("bar.sync 1, 128;" ::: "memory");
+          asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
 #pragma unroll
           for (int j = 0; j < H; ++j) {
             const float other = buf[(is_up ? H + j : j) * kPairHalf];
             const float g = is_up ? other : v[j], u = is_up ? v[H + j] : other;
-            const int m = c0 + (is_up ? H + j : j);
+            const int m = first + (is_up ? H + j : j);
             if (col_ok && m < real) y[static_cast<size_t>(m) * p.n_out] = __float2half_rn(silu_fast(g) * u);
           }
         } else {
 #pragma unroll
           for (int j = 0; j < kChunk; ++j)
-            if (col_ok && c0 + j < real) y[static_cast<size_t>(c0 + j) * p.n_out] = __float2half_rn(__fadd_rn(v[j], add[j]));
+            if (col_ok && first + j < real) y[static_cast<size_t>(first + j) * p.n_out] = __float2half_rn(__fadd_rn(v[j], add[j]));
         }
       }
     }
@@ -237,37 +261,39 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     // ---------------- int4: nibble tile -> byte tile ----------------
     // Thread r owns tile row r: 64 bytes of nibbles (16-byte chunk c at c ^ ((r >> 1) & 3)) become 128 bytes of codes in the
     // 128-byte swizzle order (chunk c at c ^ (r & 7)); even columns sit in the low nibbles.
-    const int r = threadIdx.x - 192;
-    int it = 0;
+    const int r = threadIdx.x & 127;
+    static_assert((64 + kEpilogueThreads) % 128 == 64, "converter warps start at a multiple of two warps");
+    const int steps = tiles > pair ? ((tiles - pair - 1) / pairs + 1) * kblocks : 0;
     bool ok = true;
-    for (int t = pair; t < tiles && ok; t += pairs)
-      for (int kb = 0; kb < kblocks; ++kb, ++it) {
-        const int s = it % S;
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&raw_full[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 6));
-        if (!ok) break;
-        const uint8_t* raw_row = s_raw + s * (kTile / 2) + r * (kRows / 2);
-        uint8_t* out_row = s_w + s * kTile + r * kRows;
-        uint4 raw[4];
+    const int group = (warp - 10) >> 2;
+    for (int it = 0; it < steps; ++it) {         // (waits for every stage: a barrier's parity only tells neighbouring phases apart)
+      const int s = it % S;
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&raw_full[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 6));
+      if (!ok) break;
+      if (it % kConverterGroups != group) continue;
+      const uint8_t* raw_row = s_raw + s * (kTile / 2) + r * (kRows / 2);
+      uint8_t* out_row = s_w + s * kTile + r * kRows;
+      uint4 raw[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) raw[c] = *reinterpret_cast<const uint4*>(raw_row + ((c ^ ((r >> 1) & 3)) * 16));
+      for (int c = 0; c < 4; ++c) raw[c] = *reinterpret_cast<const uint4*>(raw_row + ((c ^ ((r >> 1) & 3)) * 16));
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const uint32_t w[4] = {raw[c].x, raw[c].y, raw[c].z, raw[c].w};
-          uint32_t o[8];
+      for (int c = 0; c < 4; ++c) {
+        const uint32_t w[4] = {raw[c].x, raw[c].y, raw[c].z, raw[c].w};
+        uint32_t o[8];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint32_t even = w[j] & 0x0F0F0F0Fu;
-            const uint32_t odd = (w[j] >> 4) & 0x0F0F0F0Fu;
-            o[2 * j] = __byte_perm(even, odd, 0x5140);
-            o[2 * j + 1] = __byte_perm(even, odd, 0x7362);
-          }
-          *reinterpret_cast<uint4*>(out_row + (((2 * c) ^ (r & 7)) * 16)) = make_uint4(o[0], o[1], o[2], o[3]);
-          *reinterpret_cast<uint4*>(out_row + (((2 * c + 1) ^ (r & 7)) * 16)) = make_uint4(o[4], o[5], o[6], o[7]);
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t even = w[j] & 0x0F0F0F0Fu;
+          const uint32_t odd = (w[j] >> 4) & 0x0F0F0F0Fu;
+          o[2 * j] = __byte_perm(even, odd, 0x5140);
+          o[2 * j + 1] = __byte_perm(even, odd, 0x7362);
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor core reads these bytes through the async proxy
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&ready[s]), 0));
+        *reinterpret_cast<uint4*>(out_row + (((2 * c) ^ (r & 7)) * 16)) = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4*>(out_row + (((2 * c + 1) ^ (r & 7)) * 16)) = make_uint4(o[4], o[5], o[6], o[7]);
       }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor core reads these bytes through the async proxy
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&ready[s]), 0));
+    }
   }
   // Nobody leaves while the other CTA may still signal its barriers, read its operands or use the pair's tensor memory.
   __syncwarp();

@@ -257,12 +257,13 @@ int qgemv_dispatch(const void* x, const void* norm_weight, float norm_eps, const
         c.x = static_cast<const char*>(x) + static_cast<size_t>(m0) * p.x_stride * esize;
         c.y = static_cast<char*>(y) + static_cast<size_t>(m0) * n_out * esize;
         c.residual = residual ? static_cast<const char*>(residual) + static_cast<size_t>(m0) * n_out * esize : nullptr;
-        const int rc = i8_ok ? launch_qgemm_i8(c, workspace, st) : launch_qgemm_tc(c, st);
+        const int rc = i8_ok ? launch_qgemm_i8(c, workspace, st) : qgemv_stream_supported(c) ? launch_qgemv_stream(c, st) : launch_qgemm_tc(c, st);
         if (rc != 0) return rc;
       }
       return 0;
     }
   }
+  if (qgemv_stream_supported(p)) return plan_only ? (4 << 8) : launch_qgemv_stream(p, st);
   // up to 8 batch rows of int4 codes in row order: the streaming GEMV reads every code once and needs no pre-pass
   if (qgemv_mma_supported(p)) return plan_only ? (4 << 8) : launch_qgemv_mma(p, st);
   if (qgemm_i8_supported(p, workspace, workspace_bytes))

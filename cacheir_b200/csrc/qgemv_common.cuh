@@ -46,6 +46,10 @@ int launch_qgemv_cuda_core(const QGemvParams& p, cudaStream_t stream);
 bool qgemv_mma_supported(const QGemvParams& p);
 int launch_qgemv_mma(const QGemvParams& p, cudaStream_t stream);
 
+// Streaming dequant-GEMV for up to 32 rows (warp MMAs on codes unpacked in registers; both code layouts).
+bool qgemv_stream_supported(const QGemvParams& p);
+int launch_qgemv_stream(const QGemvParams& p, cudaStream_t stream);
+
 // Tensor-core (tcgen05) small-M GEMM: weights are the 128-row MMA operand.
 bool qgemm_tc_supported(const QGemvParams& p);
 int launch_qgemm_tc(const QGemvParams& p, cudaStream_t stream);

@@ -22,6 +22,7 @@ cacheir/runtime/scheduler.py:508-577): `run`, `fork`, `run_decode_batch`,
 """
 from __future__ import annotations
 
+import gc
 import os
 
 from collections import OrderedDict
@@ -671,6 +672,8 @@ class _DecodePlan:
         """Will this projection run on the integer tensor cores (and so accept pre-quantized activations)?"""
         if swiglu and isinstance(weight, B200PackedWeight) and ((weight.shape[0] // 2) % 64 != 0 or (weight.tiled and not weight.paired)):
             return False
+        if isinstance(weight, B200PackedWeight) and weight.bits == 4 and self.batch <= 8:
+            return False                 # the streaming kernel takes fp16 rows as they are
         return (isinstance(weight, B200PackedWeight) and weight.bits in (4, 8) and not weight.group_size
                 and self.engine.dtype == torch.float16 and self.batch <= 64 and k % 128 == 0 and k <= 8192
                 and hasattr(self, "_gemm_ws"))
@@ -689,7 +692,7 @@ class _DecodePlan:
                                    workspace=ws, tiled=weight.tiled, prequantized=prequantized, paired=weight.paired)
             key = f"b200.qgemv.int{bits}" + (".swiglu" if epilogue == ops.EPI_SWIGLU else ".residual" if residual is not None else "")
             eng.gemm_plans[f"q{bits}:{(self.batch, 1, k)}x{weight.shape}"] = key
-            if ws is not None and k % 128 == 0 and k <= 32768 and not prequantized:   # activation pre-pass + integer GEMM per 64-row chunk
+            if ws is not None and k % 128 == 0 and k <= 32768 and not prequantized and self.batch > 8:   # activation pre-pass + integer GEMM per 64-row chunk
                 self._emit(fn, key, launches=2 * ((self.batch + 63) // 64))
                 return out
         else:
@@ -818,11 +821,17 @@ class _DecodePlan:
             graph = getattr(self, attr)
             if graph is None:
                 graph = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(graph):
-                    for fn in self.program:
-                        fn()
-                    if feedback:
-                        self.feedback_tail()
+                collecting = gc.isenabled()
+                gc.disable()          # a collection that frees another plan's graph, event or pinned buffer would end the capture
+                try:
+                    with torch.cuda.graph(graph):
+                        for fn in self.program:
+                            fn()
+                        if feedback:
+                            self.feedback_tail()
+                finally:
+                    if collecting:
+                        gc.enable()
                 setattr(self, attr, graph)
                 eng.graph_captures += 1
             graph.replay()

@@ -28,8 +28,9 @@ def test_rows_equal_passes_of_64(bits, m, n, k, epilogue):
     res = torch.randn((m, n_out), device="cuda", generator=g).half() if epilogue == 1 else None
     kw = dict(bits=bits, n=n, k=k, epilogue=epilogue, paired=w.paired)
     ws = torch.zeros(ops.qgemv_workspace_bytes(64, k), device="cuda", dtype=torch.uint8)
-    want = torch.cat([ops.qgemv(x[i:i + 64], w.packed_values, w.scales, w.zero_points, residual=None if res is None else res[i:i + 64], workspace=ws,
-                                tiled=True, **kw) for i in range(0, m, 64)])
+    whole = [torch.cat([t, torch.zeros((-m % 64, t.shape[1]), device="cuda", dtype=t.dtype)]) if t is not None else None for t in (x, res)]
+    want = torch.cat([ops.qgemv(whole[0][i:i + 64], w.packed_values, w.scales, w.zero_points, residual=None if res is None else whole[1][i:i + 64],
+                                workspace=ws, tiled=True, **kw) for i in range(0, m, 64)])[:m]
     big = torch.full((ops.qgemv_workspace_bytes(m, k),), 255, device="cuda", dtype=torch.uint8)
 
     def same(a, b):      # the residual may join in one fused rounding or two: a float32 rounding apart, so at most neighbours in fp16
