@@ -286,6 +286,12 @@ void resolve_attention_splits(int batch, int heads, int kv_heads, int max_pages,
     if (s < want) s = static_cast<int>(want);
     const int cap = static_cast<int>((max_ctx + 255) / 256);
     if (s > cap) s = cap;
+    // Up to eight splits that fit the GPU at once merge inside a thread-block cluster without a launch of their own, so
+    // that chunks down to one stage (64 tokens) pay. (Tables of up to 256 tokens keep one split, which can leave activation planes.)
+    long long near = (max_ctx + 63) / 64;
+    if (near > want) near = want;
+    if (near > kMaxClusterSplits) near = kMaxClusterSplits;
+    if (s > 1 && near > s && near * units <= 2 * kNumSMs) s = static_cast<int>(near);
   }
   if (s > kMaxAttentionSplits) s = kMaxAttentionSplits;
   if (s < 1) s = 1;
@@ -388,7 +394,10 @@ int attention_dispatch(
                          (static_cast<long long>(head_dim) * kv_esize) % 8 == 0;
   int rc;
   if (paged_attention_fast_supported(p, dtype)) {
+    // (all CTAs at once: a cluster's short members would otherwise hold SMs that other sequences wait for)
+    p.cluster = p.splits > 1 && p.splits <= kMaxClusterSplits && static_cast<long long>(p.splits) * p.kv_heads * p.batch <= 2 * kNumSMs ? 1 : 0;
     rc = launch_paged_attention_fast(p, dtype, st);
+    if (p.cluster) return rc;
   } else if (kv8) {
     switch (dtype) {
       case CACHEIR_B200_F32: rc = launch_general<float, 4, true>(p, vector_ok, st); break;

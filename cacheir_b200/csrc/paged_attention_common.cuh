@@ -7,6 +7,7 @@
 namespace cb200 {
 
 constexpr int kMaxAttentionSplits = 64;
+constexpr int kMaxClusterSplits = 8;      // the portable cluster size
 constexpr float kLog2e = 1.4426950408889634f;
 
 // Kernel arguments of one paged decode attention launch. Split partials live in
@@ -34,6 +35,7 @@ struct AttnParams {
   int group;         // heads / kv_heads
   int head_chunks;   // CTAs along the query heads of one KV head
   int splits, chunk_tokens;
+  int cluster;       // the splits of a (sequence, kv head) are one thread-block cluster and merge in it: no combine launch
   long long q_stride, out_stride;  // elements between consecutive sequences
   float scale_log2;                // softmax_scale * log2(e)
 };

@@ -109,10 +109,47 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// The splits of one (sequence, kv head) as a cluster: every CTA has left its merged state in its shared memory (s_out
+// [group][D] unnormalised, s_max and s_den per head); each finishes a share of the outputs, the splits in order.
+template <typename T, int D>
+__device__ __forceinline__ void combine_in_cluster(const AttnParams& p, const float* s_out, const float* s_max, const float* s_den, int b, int kvh,
+                                                   int split, int threads) {
+  auto remote = [](const float* local, uint32_t rank) {
+    uint32_t addr;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+  };
+  cluster_sync_all();
+  for (int idx = split * threads + threadIdx.x; idx < p.group * D; idx += p.splits * threads) {
+    const int row = idx / D;
+    float m[8], l[8], part[8], m_tot = -INFINITY;        // all of them are requested before the first is used
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      m[s] = s < p.splits ? remote(s_max + row, s) : -INFINITY;
+      l[s] = s < p.splits ? remote(s_den + row, s) : 0.f;
+      part[s] = s < p.splits ? remote(s_out + idx, s) : 0.f;
+    }
+#pragma unroll
+    for (int s = 0; s < 8; ++s) m_tot = fmaxf(m_tot, m[s]);
+    float l_tot = 0.f, o = 0.f;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const float w = m[s] == -INFINITY ? 0.f : exp2f(m[s] - m_tot);
+      l_tot = fmaf(l[s], w, l_tot);
+      o = fmaf(part[s], w, o);
+    }
+    T* ob = static_cast<T*>(p.out) + static_cast<size_t>(b) * p.out_stride + static_cast<size_t>(kvh * p.group) * D;
+    Elem<T>::st(ob + idx, l_tot > 0.f ? o / l_tot : 0.f);
+  }
+  cluster_sync_all();                                    // nobody's state is read any more
+}
+
 // QUANT: single split, launched as clusters of the kv heads of one sequence (grid z = padded row count of the
 // planes); the epilogue also writes the output row as the integer GEMM's fixed-point planes, bit for bit what the
 // stand-alone pre-pass makes of the stored fp16 output.
-template <typename T, int D, bool QUANT>
+template <typename T, int D, bool QUANT, bool CLUSTER>
 __global__ void __launch_bounds__(kFastThreads)
 paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                         const AttnParams p, const int stages) {
@@ -145,7 +182,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   }
   const int seq_len = p.seq_lens[b];
   const int t_begin = split * p.chunk_tokens;
-  if (p.splits > 1 && t_begin >= seq_len) return;      // combine never reads this split
+  if (!CLUSTER && p.splits > 1 && t_begin >= seq_len) return;      // combine never reads this split
   const int t_end = min(seq_len, t_begin + p.chunk_tokens);
   const int page_begin = t_begin / kPage;              // chunk_tokens is a multiple of the page size
   const int n_pages = t_end > t_begin ? (t_end - t_begin + kPage - 1) / kPage : 0;
@@ -391,6 +428,9 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       p.quant_sx[b] = amax > 0.f ? amax / kQMax : 0.f;
     }
   } else {
+  [[maybe_unused]] float* s_fin = s_o + kConsumerWarps * 16 * D;                     // cluster form: [group][D], then maxima and denominators
+  [[maybe_unused]] float* s_fin_m = s_fin + 16 * D;
+  [[maybe_unused]] float* s_fin_l = s_fin_m + 16;
   for (int idx = threadIdx.x; idx < p.group * D; idx += kFastThreads) {
     const int row = idx / D;
     const int d = idx % D;
@@ -406,7 +446,10 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       acc = fmaf(s_o[(w * 16 + row) * D + d], wgt, acc);
     }
     const int h = kvh * p.group + row;
-    if (p.splits == 1) {
+    if constexpr (CLUSTER) {
+      s_fin[idx] = acc;
+      if (d == 0) { s_fin_m[row] = m_tot; s_fin_l[row] = l_tot; }
+    } else if (p.splits == 1) {
       T* ob = static_cast<T*>(p.out) + static_cast<size_t>(b) * p.out_stride;
       Elem<T>::st(ob + static_cast<size_t>(h) * D + d, l_tot > 0.f ? acc / l_tot : 0.f);
     } else {
@@ -418,6 +461,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       }
     }
   }
+  if constexpr (CLUSTER) combine_in_cluster<T, D>(p, s_fin, s_fin_m, s_fin_l, b, kvh, split, kFastThreads);
   }
 }
 
@@ -453,6 +497,7 @@ constexpr float kByteBias = 1152.f;     // 1024 + 128: what every operand built 
 constexpr int kQ8Warps = 6;
 constexpr int kQ8Threads = (kQ8Warps + 1) * 32;
 
+template <bool CLUSTER>
 __global__ void __launch_bounds__(kQ8Threads, 2)
 paged_decode_mma_q8_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                            const AttnParams p, const int stages) {
@@ -475,7 +520,7 @@ paged_decode_mma_q8_kernel(const __grid_constant__ CUtensorMap tmap_k, const __g
   const int lane = threadIdx.x & 31;
   const int seq_len = p.seq_lens[b];
   const int t_begin = split * p.chunk_tokens;
-  if (p.splits > 1 && t_begin >= seq_len) return;      // combine never reads this split
+  if (!CLUSTER && p.splits > 1 && t_begin >= seq_len) return;      // combine never reads this split
   const int t_end = min(seq_len, t_begin + p.chunk_tokens);
   const int page_begin = t_begin / kPage;
   const int n_pages = t_end > t_begin ? (t_end - t_begin + kPage - 1) / kPage : 0;
@@ -692,6 +737,9 @@ paged_decode_mma_q8_kernel(const __grid_constant__ CUtensorMap tmap_k, const __g
     }
   }
   __syncthreads();
+  [[maybe_unused]] float* s_fin = s_o + kQ8Warps * 16 * D;                     // cluster form: [group][D], then maxima and denominators
+  [[maybe_unused]] float* s_fin_m = s_fin + 16 * D;
+  [[maybe_unused]] float* s_fin_l = s_fin_m + 16;
   for (int idx = threadIdx.x; idx < p.group * D; idx += kQ8Threads) {
     const int row = idx / D;
     const int d = idx % D;
@@ -707,7 +755,10 @@ paged_decode_mma_q8_kernel(const __grid_constant__ CUtensorMap tmap_k, const __g
       acc = fmaf(s_o[(w * 16 + row) * D + d], wgt, acc);
     }
     const int h = kvh * p.group + row;
-    if (p.splits == 1) {
+    if constexpr (CLUSTER) {
+      s_fin[idx] = acc;
+      if (d == 0) { s_fin_m[row] = m_tot; s_fin_l[row] = l_tot; }
+    } else if (p.splits == 1) {
       __half* ob = static_cast<__half*>(p.out) + static_cast<size_t>(b) * p.out_stride;
       ob[static_cast<size_t>(h) * D + d] = __float2half_rn(l_tot > 0.f ? acc / l_tot : 0.f);
     } else {
@@ -719,6 +770,7 @@ paged_decode_mma_q8_kernel(const __grid_constant__ CUtensorMap tmap_k, const __g
       }
     }
   }
+  if constexpr (CLUSTER) combine_in_cluster<__half, D>(p, s_fin, s_fin_m, s_fin_l, b, kvh, split, kQ8Threads);
 }
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -753,6 +805,26 @@ bool encode_pool(CUtensorMap* map, const void* base, int dtype, uint64_t rows, i
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <typename Kernel>
+int launch_splits(Kernel kern, int threads, size_t smem, const CUtensorMap& tmap_k, const CUtensorMap& tmap_v, const AttnParams& p, int stages,
+                  cudaStream_t stream) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(p.splits, p.kv_heads, p.batch);
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.splits;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.cluster ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmap_k, tmap_v, p, stages);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  return launch_status();
+}
+
 template <typename T, int D>
 int launch_fast(const AttnParams& p, int dtype, uint64_t pool_rows, cudaStream_t stream) {
   CUtensorMap tmap_k, tmap_v;
@@ -761,11 +833,11 @@ int launch_fast(const AttnParams& p, int dtype, uint64_t pool_rows, cudaStream_t
   constexpr int kStageBytes = kPagesPerStage * 2 * kPage * D * 2;
   const int stages = D == 128 ? 3 : 4;
   size_t smem = 1024 + static_cast<size_t>(stages) * kStageBytes + 256;
-  const size_t merge = static_cast<size_t>(kConsumerWarps) * 16 * (D + 2) * sizeof(float) + 1024;
+  const size_t merge = (static_cast<size_t>(kConsumerWarps) * 16 * (D + 2) + 16 * (D + 2)) * sizeof(float) + 1024;
   if (smem < merge) smem = merge;
   if constexpr (std::is_same<T, __half>::value && D == 128) {
     if (p.quant_planes) {      // the kv heads of a sequence form a cluster; grid z covers the padding rows of the planes too
-      auto kern = paged_decode_mma_kernel<T, D, true>;
+      auto kern = paged_decode_mma_kernel<T, D, true, false>;
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
       if (e != cudaSuccess) return static_cast<int>(e);
       cudaLaunchConfig_t cfg{};
@@ -785,12 +857,10 @@ int launch_fast(const AttnParams& p, int dtype, uint64_t pool_rows, cudaStream_t
       return launch_status();
     }
   }
-  auto kern = paged_decode_mma_kernel<T, D, false>;
+  auto kern = p.cluster ? paged_decode_mma_kernel<T, D, false, true> : paged_decode_mma_kernel<T, D, false, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  const dim3 grid(p.splits, p.kv_heads, p.batch);
-  kern<<<grid, kFastThreads, smem, stream>>>(tmap_k, tmap_v, p, stages);
-  return launch_status();
+  return launch_splits(kern, kFastThreads, smem, tmap_k, tmap_v, p, stages, stream);
 }
 
 
@@ -812,13 +882,12 @@ int launch_fast_q8(const AttnParams& p, uint64_t pool_rows, cudaStream_t stream)
   constexpr int kStageBytes = kQ8Warps * 2 * kPage * 128 + 1024;
   const int stages = 4;
   size_t smem = 1024 + static_cast<size_t>(stages) * kStageBytes + 256;
-  const size_t merge = static_cast<size_t>(kQ8Warps) * 16 * (128 + 2) * sizeof(float) + 1024;
+  const size_t merge = (static_cast<size_t>(kQ8Warps) * 16 * (128 + 2) + 16 * (128 + 2)) * sizeof(float) + 1024;
   if (smem < merge) smem = merge;
-  cudaError_t e = cudaFuncSetAttribute(paged_decode_mma_q8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  auto kern = p.cluster ? paged_decode_mma_q8_kernel<true> : paged_decode_mma_q8_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  const dim3 grid(p.splits, p.kv_heads, p.batch);
-  paged_decode_mma_q8_kernel<<<grid, kQ8Threads, smem, stream>>>(tmap_k, tmap_v, p, stages);
-  return launch_status();
+  return launch_splits(kern, kQ8Threads, smem, tmap_k, tmap_v, p, stages, stream);
 }
 
 }  // namespace
