@@ -17,8 +17,25 @@ Shape choose_shape(int T, int N, int K, int batch) {
   return {mt, split};
 }
 
+// Tokens per tile of a CTA pair, 0: single CTAs.
+int choose_pair(int T, int N, int K, int batch) {
+  if (T < 192 || (batch > 1 && N % (2 * kTileN) != 0)) return 0;
+  auto cost = [&](int tt) {          // turns of the busiest pair, in tiles of 128 tokens (a narrow tile asks more of L2)
+    const long long tiles = static_cast<long long>((T + tt - 1) / tt) * ((N + 2 * kTileN - 1) / (2 * kTileN)) * batch;
+    return (tiles + kNumSMs / 2 - 1) / (kNumSMs / 2) * (tt == 256 ? 16 : 10);
+  };
+  const long long tiles = static_cast<long long>((T + 127) / 128) * ((N + 2 * kTileN - 1) / (2 * kTileN)) * batch;
+  if (tiles < kNumSMs / 4) return 0;          // few tiles: single CTAs that split K
+  return cost(256) <= cost(128) ? 256 : 128;
+}
+
 template <int EPI>
 int launch_mt(const cacheir_b200_dense_args& p, cudaStream_t stream) {
+  switch (choose_pair(p.T, p.N, p.K, p.batch)) {
+    case 256: return launch_pair<EPI, 256>(p, stream);
+    case 128: return launch_pair<EPI, 128>(p, stream);
+    default: break;
+  }
   const Shape s = choose_shape(p.T, p.N, p.K, p.batch);
   switch (s.mt) {
     case 16: return launch<EPI, 16, false>(p, s.split, stream, {});

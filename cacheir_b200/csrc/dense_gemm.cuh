@@ -93,6 +93,105 @@ constexpr bool is_paired(int epi) {
   return epi == CACHEIR_B200_DENSE_GEGLU || epi == CACHEIR_B200_DENSE_SWIGLU || epi == CACHEIR_B200_DENSE_CLAMPED_GLU;
 }
 
+// What an epilogue thread needs of its output column.
+struct Column {
+  int n, r;                  // column, and its row of the weight tile
+  bool n_ok;
+  long long ycol;
+  float bias, w1, b1, w2, b2;
+};
+
+// v[j] = column c.n of token t + j -> what is stored. Called by whole warps; row_of gives the output row of a token, -1: none.
+template <int EPI, bool GROUPED, int G, typename RowOf>
+__device__ __forceinline__ void finish_columns(const cacheir_b200_dense_args& p, const Column& c, float (&v)[G], int t, int t_end, RowOf row_of) {
+  const int n = c.n, r = c.r;
+  const bool n_ok = c.n_ok;
+  const long long ycol = c.ycol;
+  const float w1 = c.w1, b1 = c.b1, w2 = c.w2, b2 = c.b2;
+#pragma unroll
+  for (int j = 0; j < G; ++j) v[j] += c.bias;
+  if constexpr (is_paired(EPI)) {
+    // W rows alternate gate, up: neighbouring lanes trade, the even lane finishes token j and the odd one j + 1
+    const bool odd = (r & 1) != 0, tail = n >= p.N - p.tail_cols;      // (tail: plain float32 columns behind the pairs)
+#pragma unroll
+    for (int j = 0; j < G; j += 2) {
+      const float got = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+      const float y = odd ? paired<EPI>(got, v[j + 1], p.limit) : paired<EPI>(v[j], got, p.limit);
+      const int row = row_of(t + j + (odd ? 1 : 0));
+      if (n_ok && !tail && row >= 0)
+        static_cast<__nv_bfloat16*>(p.y)[static_cast<long long>(row) * p.y_stride + (n >> 1)] = __float2bfloat16_rn(y);
+      if (n_ok && tail) {
+        float* dst = p.tail + static_cast<long long>(t + j) * p.tail_stride + (n - (p.N - p.tail_cols));
+        if (t + j < t_end) dst[0] = v[j];
+        if (t + j + 1 < t_end) dst[p.tail_stride] = v[j + 1];
+      }
+    }
+  } else if constexpr (EPI == CACHEIR_B200_DENSE_RESIDUAL) {
+    float x[G];
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+      const int at = t + j;
+      x[j] = (n_ok && at < t_end) ? p.residual[static_cast<long long>(at) * p.N + n] : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+      const int at = t + j;
+      if (!(n_ok && at < t_end)) continue;
+      const float s = x[j] + fmaf(tanhf(p.norm_alpha * v[j]), w1, b1);
+      p.residual[static_cast<long long>(at) * p.N + n] = s;
+      if (p.next_mode == CACHEIR_B200_NEXT_DYT)
+        static_cast<__nv_bfloat16*>(p.next_out)[static_cast<long long>(at) * p.N + n] =
+            __float2bfloat16_rn(fmaf(tanhf(p.next_alpha * s), w2, b2));
+      else if (p.next_mode == CACHEIR_B200_NEXT_COPY)
+        static_cast<__nv_bfloat16*>(p.next_out)[static_cast<long long>(at) * p.N + n] = __float2bfloat16_rn(s);
+    }
+  } else {
+    // what the epilogue multiplies with is loaded for all tokens before anything is stored
+    float f[G];
+    if constexpr (EPI == CACHEIR_B200_DENSE_GATED) {
+#pragma unroll
+      for (int j = 0; j < G; ++j) {
+        const int at = t + j;
+        f[j] = (n_ok && at < t_end) ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.gate)[static_cast<long long>(at) * p.gate_stride + ycol]) : 0.f;
+      }
+    } else if constexpr (EPI == CACHEIR_B200_DENSE_GELU_EMBED) {
+      int64_t id[G];
+#pragma unroll
+      for (int j = 0; j < G; ++j) id[j] = p.ids[min(t + j, t_end - 1)];
+#pragma unroll
+      for (int j = 0; j < G; ++j) {
+        id[j] = min(max(id[j], static_cast<int64_t>(0)), static_cast<int64_t>(p.vocab - 1));
+        f[j] = n_ok ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.table)[id[j] * p.table_stride + p.table_col + n]) : 0.f;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+      const int row = row_of(t + j);
+      if (!n_ok || row < 0) continue;
+      float y = v[j];
+      if constexpr (!GROUPED && (EPI == CACHEIR_B200_DENSE_BF16 || EPI == CACHEIR_B200_DENSE_SILU)) {
+        if (n >= p.N - p.tail_cols) {        // plain float32 columns behind the others
+          p.tail[static_cast<long long>(row) * p.tail_stride + (n - (p.N - p.tail_cols))] = y;
+          continue;
+        }
+      }
+      if constexpr (EPI == CACHEIR_B200_DENSE_F32) {
+        static_cast<float*>(p.y)[static_cast<long long>(row) * p.y_stride + ycol] = y;
+        continue;
+      } else if constexpr (EPI == CACHEIR_B200_DENSE_SILU) {
+        if (n < p.act_cols) y = silu_exact(y);
+      } else if constexpr (EPI == CACHEIR_B200_DENSE_RELU2) {
+        y = relu_squared(y);
+      } else if constexpr (EPI == CACHEIR_B200_DENSE_GATED) {
+        y *= sigmoid_exact(f[j]);
+      } else if constexpr (EPI == CACHEIR_B200_DENSE_GELU_EMBED) {
+        y = gelu_tanh(y) * f[j];
+      }
+      static_cast<__nv_bfloat16*>(p.y)[static_cast<long long>(row) * p.y_stride + ycol] = __float2bfloat16_rn(y);
+    }
+  }
+}
+
 template <int EPI, int MT, bool GROUPED>
 __global__ void __launch_bounds__(kThreads, ctas_per_sm(MT))
 dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
@@ -216,90 +315,9 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     tc_fence_after();
     const long long ycol = GROUPED ? n : static_cast<long long>(z) * p.y_batch_cols + n;
 
+    const Column col{n, r, n_ok, ycol, bias, w1, b1, w2, b2};
     auto emit = [&](auto& v, auto count, int c0) {       // v[j] = column n of token t0 + c0 + j
-      constexpr int G = decltype(count)::value;
-#pragma unroll
-      for (int j = 0; j < G; ++j) v[j] += bias;
-      if constexpr (is_paired(EPI)) {
-        // W rows alternate gate, up: neighbouring lanes trade, the even lane finishes token j and the odd one j + 1
-        const bool odd = (r & 1) != 0, tail = n >= p.N - p.tail_cols;      // (tail: plain float32 columns behind the pairs)
-#pragma unroll
-        for (int j = 0; j < G; j += 2) {
-          const float got = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
-          const float y = odd ? paired<EPI>(got, v[j + 1], p.limit) : paired<EPI>(v[j], got, p.limit);
-          const int row = row_of(t0 + c0 + j + (odd ? 1 : 0));
-          if (n_ok && !tail && row >= 0)
-            static_cast<__nv_bfloat16*>(p.y)[static_cast<long long>(row) * p.y_stride + (n >> 1)] = __float2bfloat16_rn(y);
-          if (n_ok && tail) {
-            float* dst = p.tail + static_cast<long long>(t0 + c0 + j) * p.tail_stride + (n - (p.N - p.tail_cols));
-            if (t0 + c0 + j < t_end) dst[0] = v[j];
-            if (t0 + c0 + j + 1 < t_end) dst[p.tail_stride] = v[j + 1];
-          }
-        }
-      } else if constexpr (EPI == CACHEIR_B200_DENSE_RESIDUAL) {
-        float x[G];
-#pragma unroll
-        for (int j = 0; j < G; ++j) {
-          const int t = t0 + c0 + j;
-          x[j] = (n_ok && t < t_end) ? p.residual[static_cast<long long>(t) * p.N + n] : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < G; ++j) {
-          const int t = t0 + c0 + j;
-          if (!(n_ok && t < t_end)) continue;
-          const float s = x[j] + fmaf(tanhf(p.norm_alpha * v[j]), w1, b1);
-          p.residual[static_cast<long long>(t) * p.N + n] = s;
-          if (p.next_mode == CACHEIR_B200_NEXT_DYT)
-            static_cast<__nv_bfloat16*>(p.next_out)[static_cast<long long>(t) * p.N + n] =
-                __float2bfloat16_rn(fmaf(tanhf(p.next_alpha * s), w2, b2));
-          else if (p.next_mode == CACHEIR_B200_NEXT_COPY)
-            static_cast<__nv_bfloat16*>(p.next_out)[static_cast<long long>(t) * p.N + n] = __float2bfloat16_rn(s);
-        }
-      } else {
-        // what the epilogue multiplies with is loaded for all tokens before anything is stored
-        float f[G];
-        if constexpr (EPI == CACHEIR_B200_DENSE_GATED) {
-#pragma unroll
-          for (int j = 0; j < G; ++j) {
-            const int t = t0 + c0 + j;
-            f[j] = (n_ok && t < t_end) ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.gate)[static_cast<long long>(t) * p.gate_stride + ycol]) : 0.f;
-          }
-        } else if constexpr (EPI == CACHEIR_B200_DENSE_GELU_EMBED) {
-          int64_t id[G];
-#pragma unroll
-          for (int j = 0; j < G; ++j) id[j] = p.ids[min(t0 + c0 + j, t_end - 1)];
-#pragma unroll
-          for (int j = 0; j < G; ++j) {
-            id[j] = min(max(id[j], static_cast<int64_t>(0)), static_cast<int64_t>(p.vocab - 1));
-            f[j] = n_ok ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.table)[id[j] * p.table_stride + p.table_col + n]) : 0.f;
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < G; ++j) {
-          const int t = row_of(t0 + c0 + j);
-          if (!n_ok || t < 0) continue;
-          float y = v[j];
-          if constexpr (!GROUPED && (EPI == CACHEIR_B200_DENSE_BF16 || EPI == CACHEIR_B200_DENSE_SILU)) {
-            if (n >= p.N - p.tail_cols) {        // plain float32 columns behind the others
-              p.tail[static_cast<long long>(t) * p.tail_stride + (n - (p.N - p.tail_cols))] = y;
-              continue;
-            }
-          }
-          if constexpr (EPI == CACHEIR_B200_DENSE_F32) {
-            static_cast<float*>(p.y)[static_cast<long long>(t) * p.y_stride + ycol] = y;
-            continue;
-          } else if constexpr (EPI == CACHEIR_B200_DENSE_SILU) {
-            if (n < p.act_cols) y = silu_exact(y);
-          } else if constexpr (EPI == CACHEIR_B200_DENSE_RELU2) {
-            y = relu_squared(y);
-          } else if constexpr (EPI == CACHEIR_B200_DENSE_GATED) {
-            y *= sigmoid_exact(f[j]);
-          } else if constexpr (EPI == CACHEIR_B200_DENSE_GELU_EMBED) {
-            y = gelu_tanh(y) * f[j];
-          }
-          static_cast<__nv_bfloat16*>(p.y)[static_cast<long long>(t) * p.y_stride + ycol] = __float2bfloat16_rn(y);
-        }
-      }
+      finish_columns<EPI, GROUPED, decltype(count)::value>(p, col, v, t0 + c0, t_end, row_of);
     };
 
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(q * 32) << 16);
@@ -346,6 +364,137 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   }
 }
 
+// ---- prompts: a pair of CTAs per tile of 256 weight rows x TT tokens ------------------------------------------------------
+// By itself a CTA takes 48 KB from L2 per 512 tensor-core cycles (128 weight rows x 256 tokens, k 64), and nothing runs under its
+// epilogue: 2048 x 28672 x 4096 was 403 us, 1.19 PFLOP/s. A pair (cta_group::2) shares the token tile, 32 KB per CTA for the same
+// cycles, and its accumulator takes half of tensor memory, so that the epilogue of one tile runs under the next one's main loop. Pairs
+// walk the tiles with the tokens innermost: the weights in flight come from HBM once, the tokens stay in L2. The order of the sums is the
+// same.
+__host__ __device__ constexpr int pair_stage_bytes(int tt) { return kWBytes + tt / 2 * kBlockK * 2; }
+__host__ __device__ constexpr int pair_stages(int tt) { return tt == 256 ? 6 : 8; }
+
+__device__ __forceinline__ void mma_f16_ss_pair(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+template <int EPI, int TT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+dense_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const cacheir_b200_dense_args p) {
+  constexpr int S = pair_stages(TT);
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* s_w = smem;
+  uint8_t* s_x = smem + S * kWBytes;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * pair_stage_bytes(TT));      // [S] (even CTA) operands of both CTAs
+  uint64_t* empty = full + S;                                                          // [S]
+  uint64_t* acc_full = empty + S;                                                      // [2]
+  uint64_t* acc_empty = acc_full + 2;                                                  // [2] (even CTA)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int kblocks = (p.K + kBlockK - 1) / kBlockK;
+  const int t_tiles = (p.T + TT - 1) / TT, w_tiles = (p.N + 2 * kTileN - 1) / (2 * kTileN);
+  const int tiles = t_tiles * w_tiles * p.batch;
+  const int pairs = gridDim.x >> 1;
+
+  if (warp == 0 && lane == 0) {
+    for (int s = 0; s < S; ++s) { mbar_init(smem_u32(&full[s]), 1); mbar_init(smem_u32(&empty[s]), 1); }
+    for (int a = 0; a < 2; ++a) { mbar_init(smem_u32(&acc_full[a]), 1); mbar_init(smem_u32(&acc_empty[a]), 16); }
+    mbar_fence_init();
+  }
+  if (warp == 1) tc_alloc_pair(smem_u32(tmem_slot), 2 * TT);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_release();                         // both CTAs' barriers exist before either is signalled
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x >> 1; tile < tiles && ok; tile += pairs) {
+        const int t0 = tile % t_tiles * TT, w = tile / t_tiles % w_tiles, z = tile / t_tiles / w_tiles;
+        for (int i = 0; i < kblocks; ++i, ++it) {
+          const int s = it % S;
+          if (it >= S && !mbar_wait(smem_u32(&empty[s]), ((it / S) & 1) ^ 1, &g_dense_status, (6 << 8) | 5)) { ok = false; break; }
+          const uint32_t bar = map_to_rank(smem_u32(&full[s]), 0);
+          if (rank == 0) mbar_expect_tx(smem_u32(&full[s]), 2 * pair_stage_bytes(TT));
+          const int k = i * kBlockK;
+          tma_load_2d_pair(smem_u32(s_w + s * kWBytes), &tmap_w, bar, k, z * p.w_batch_rows + (2 * w + static_cast<int>(rank)) * kTileN);
+          tma_load_2d_pair(smem_u32(s_x + s * (TT / 2) * kBlockK * 2), &tmap_x, bar, z * p.x_batch_cols + k, t0 + static_cast<int>(rank) * (TT / 2));
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {
+      // fp32 accumulator, bf16 x bf16, both K-major, N = TT, M = 256
+      constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(TT >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);
+      int it = 0, n = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x >> 1; tile < tiles && ok; tile += pairs, ++n) {
+        const int a = n & 1;
+        if (n >= 2 && !mbar_wait(smem_u32(&acc_empty[a]), ((n >> 1) & 1) ^ 1, &g_dense_status, (6 << 8) | 6)) break;
+        tc_fence_after();
+        for (int i = 0; i < kblocks; ++i, ++it) {
+          const int s = it % S;
+          if (!mbar_wait(smem_u32(&full[s]), (it / S) & 1, &g_dense_status, (6 << 8) | 7)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t wb = smem_u32(s_w + s * kWBytes), xb = smem_u32(s_x + s * (TT / 2) * kBlockK * 2);
+#pragma unroll
+          for (int j = 0; j < kBlockK / 16; ++j)
+            mma_f16_ss_pair(tmem + a * TT, smem_desc_sw128(wb + j * 32), smem_desc_sw128(xb + j * 32), idesc, (i > 0 || j > 0) ? 1u : 0u);
+          tc_commit_pair(smem_u32(&empty[s]));
+        }
+        tc_commit_pair(smem_u32(&acc_full[a]));
+      }
+    }
+  } else {
+    const int q = warp & 3;
+    const int half = (warp - 2) >> 2;
+    const int r = q * 32 + lane;
+    int count = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x >> 1; tile < tiles; tile += pairs, ++count) {
+      const int a = count & 1;
+      const int t0 = tile % t_tiles * TT, w = tile / t_tiles % w_tiles, z = tile / t_tiles / w_tiles;
+      const int n = (2 * w + static_cast<int>(rank)) * kTileN + r;
+      const bool n_ok = n < p.N;
+      Column col{n, r, n_ok, static_cast<long long>(z) * p.y_batch_cols + n, p.bias && n_ok ? p.bias[n] : 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (EPI == CACHEIR_B200_DENSE_RESIDUAL && n_ok) {
+        col.w1 = p.norm_w[n]; col.b1 = p.norm_b[n];
+        if (p.next_mode == CACHEIR_B200_NEXT_DYT) { col.w2 = p.next_w[n]; col.b2 = p.next_b[n]; }
+      }
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&acc_full[a]), (count >> 1) & 1, &g_dense_status, (6 << 8) | 8));
+      tc_fence_after();
+      const uint32_t lane_addr = tmem + a * TT + (static_cast<uint32_t>(q * 32) << 16);
+      if (ok)
+        for (int c0 = half * 16; c0 < TT; c0 += 32) {
+          if (t0 + c0 >= p.T) break;
+          float v[16];
+          tmem_ld_x16(lane_addr + c0, v);
+          finish_columns<EPI, false, 16>(p, col, v, t0 + c0, p.T, [&](int t) { return t < p.T ? t : -1; });
+        }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&acc_empty[a]), 0));
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  cluster_sync_release();                         // nobody leaves while the other CTA may still need its barriers, operands or tensor memory
+  if (warp == 1) {
+    tc_fence_after();
+    tc_dealloc_pair(tmem, 2 * TT);
+  }
+}
+
 bool encode_bf16_rows(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t stride_elems, uint32_t box_rows) {
   EncodeTiledFn fn = tensor_map_encoder();
   if (!fn) return false;
@@ -387,6 +536,24 @@ int launch(const cacheir_b200_dense_args& p, int split, cudaStream_t stream, con
   cfg.numAttrs = split > 1 ? 1 : 0;
   e = cudaLaunchKernelEx(&cfg, kern, tw, tx, p, n_tiles, groups);
   if (e != cudaSuccess) return static_cast<int>(e);
+  return launch_status();
+}
+
+template <int EPI, int TT>
+int launch_pair(const cacheir_b200_dense_args& p, cudaStream_t stream) {
+  constexpr size_t kSmem = 1024 + static_cast<size_t>(pair_stages(TT)) * pair_stage_bytes(TT) + kTailBytes;
+  static_assert(kSmem <= 227 * 1024, "ring must fit");
+  CUtensorMap tw, tx;
+  const uint64_t w_rows = p.batch > 1 ? static_cast<uint64_t>(p.w_batch_rows) * (p.batch - 1) + p.N : p.N;
+  const uint64_t x_cols = static_cast<uint64_t>(p.x_batch_cols) * (p.batch - 1) + p.K;
+  if (!encode_bf16_rows(&tw, p.w, p.K, w_rows, p.w_stride, kTileN) || !encode_bf16_rows(&tx, p.x, x_cols, p.T, p.x_stride, TT / 2))
+    return CACHEIR_B200_EUNSUPPORTED;
+  auto kern = dense_pair_kernel<EPI, TT>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem));
+  if (e != cudaSuccess) return static_cast<int>(e);
+  const long long tiles = static_cast<long long>((p.T + TT - 1) / TT) * ((p.N + 2 * kTileN - 1) / (2 * kTileN)) * p.batch;
+  const int pairs = tiles < kNumSMs / 2 ? static_cast<int>(tiles) : kNumSMs / 2;
+  kern<<<2 * pairs, kThreads, kSmem, stream>>>(tw, tx, p);
   return launch_status();
 }
 
