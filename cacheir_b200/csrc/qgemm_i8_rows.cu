@@ -13,6 +13,10 @@
 // loop of the next. Persistent: pairs walk the tiles with the row blocks innermost, so that the weights of the few tiles
 // in flight are read from HBM once and the activation planes stay in L2.
 //
+// Few tiles leave most SMs idle, so that a tile's K range is split over the SPLIT pairs of a larger cluster (one tile per
+// cluster then): every CTA lays its partial sums out in its drained ring, and pair j adds up, through distributed shared memory, what all pairs have
+// for its share of the activation rows. Integer sums: the order cannot matter. 256 rows of 2048 x 5632: 44 k blocks on 32 SMs, or 11 on 128.
+//
 // Warps: 0 copies, 1 issues MMAs (even CTA only), 2-9 epilogue (four per half of the activation rows), with int4 codes 10-21
 // widen nibble tiles to byte tiles in three groups that take every third stage.
 #include "common.cuh"
@@ -41,6 +45,12 @@ __host__ __device__ constexpr int num_threads(int bits) { return 64 + kEpilogueT
 constexpr int kExchangeBytes = 2 * 2 * kChunk * kPairHalf * 4;
 constexpr int kTailBytes = kExchangeBytes + 2 * kRows * 16 + 512;     // SwiGLU exchange, row scales and sums of two tiles, barriers
 
+__device__ __forceinline__ uint32_t load_cluster(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+
 struct RowsParams {
   const void* scales;
   const float* zero_points;
@@ -55,8 +65,8 @@ struct RowsParams {
   int bands;          // weight tiles of 128 rows
 };
 
-template <int BITS, bool SWIGLU>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(num_threads(BITS), 1)
+template <int BITS, bool SWIGLU, int SPLIT>
+__global__ void __launch_bounds__(num_threads(BITS), 1)
 qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const RowsParams p) {
   constexpr int S = num_stages(BITS);
   extern __shared__ uint8_t smem_raw[];
@@ -73,16 +83,20 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   uint64_t* acc_full = ready + S;            // [2]
   uint64_t* acc_empty = acc_full + 2;        // [2] (even CTA) both CTAs' epilogues have read the accumulator
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  int* s_part = reinterpret_cast<int*>(smem);      // SPLIT > 1: 128 KB over the drained ring
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();
+  const uint32_t cluster_rank = cluster_ctarank();
+  const uint32_t rank = cluster_rank & 1, first = cluster_rank & ~1u;      // in the pair; the pair's even CTA
+  const int share = static_cast<int>(cluster_rank >> 1);                   // of K, and of the tile's activation rows
   const int rows = p.n_rows ? min(p.M, *p.n_rows) : p.M;
   const int row_blocks = (rows + kRows - 1) / kRows;
-  const int kblocks = p.K / kRows;
+  const int kblocks_all = p.K / kRows;
+  const int kb0 = kblocks_all * share / SPLIT, kblocks = kblocks_all * (share + 1) / SPLIT - kb0;
   const int tiles = (p.bands + 1) / 2 * row_blocks;
-  const int pairs = gridDim.x >> 1;
-  const int pair = blockIdx.x >> 1;
+  const int pairs = gridDim.x / (2 * SPLIT);
+  const int pair = blockIdx.x / (2 * SPLIT);
 
   if (warp == 0 && lane == 0) {
     for (int s = 0; s < S; ++s) {
@@ -114,18 +128,18 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         for (int kb = 0; kb < kblocks; ++kb, ++it) {
           const int s = it % S;
           if (it >= S && !mbar_wait(smem_u32(&empty[s]), ((it / S) & 1) ^ 1, &g_i8_rows_status, (6 << 8) | 1)) { ok = false; break; }
-          const uint32_t bar = map_to_rank(smem_u32(&full[s]), 0);
+          const uint32_t bar = map_to_rank(smem_u32(&full[s]), first);
           if (rank == 0) mbar_expect_tx(smem_u32(&full[s]), BITS == 8 ? 4 * kTile : 2 * kTile);
           // (a band beyond the last one, where their number is odd, reads as zero)
           if constexpr (BITS == 8) {
-            tma_load_2d_pair(smem_u32(s_w + s * kTile), &tmap_w, bar, 0, (band * kblocks + kb) * kRows);
+            tma_load_2d_pair(smem_u32(s_w + s * kTile), &tmap_w, bar, 0, (band * kblocks_all + kb0 + kb) * kRows);
           } else {
             const int b = min(band, p.bands - 1);
             mbar_expect_tx(smem_u32(&raw_full[s]), kTile / 2);
-            bulk_load(smem_u32(s_raw + s * (kTile / 2)), p.w_tiled + (static_cast<size_t>(b) * kblocks + kb) * (kTile / 2), kTile / 2,
+            bulk_load(smem_u32(s_raw + s * (kTile / 2)), p.w_tiled + (static_cast<size_t>(b) * kblocks_all + kb0 + kb) * (kTile / 2), kTile / 2,
                       smem_u32(&raw_full[s]));
           }
-          tma_load_2d_pair(smem_u32(s_x + s * kTile), &tmap_x, bar, 0, ((block * kblocks + kb) * 2 + static_cast<int>(rank)) * kRows);
+          tma_load_2d_pair(smem_u32(s_x + s * kTile), &tmap_x, bar, 0, ((block * kblocks_all + kb0 + kb) * 2 + static_cast<int>(rank)) * kRows);
         }
       }
     }
@@ -150,9 +164,9 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             tc_mma_i8_ss_pair(d, smem_desc_sw128(w + j * 32), smem_desc_sw128(x + j * 32), idesc, (kb > 0 || j > 0) ? 1u : 0u);
-          tc_commit_pair(smem_u32(&empty[s]));
+          tc_commit_pair(smem_u32(&empty[s]), first);
         }
-        tc_commit_pair(smem_u32(&acc_full[a]));
+        tc_commit_pair(smem_u32(&acc_full[a]), first);
       }
     }
   } else if (warp < 10) {
@@ -188,29 +202,59 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       col_ok = col_ok && ok;
       __syncwarp();
       tc_fence_after();
-      const uint32_t acc = tmem_base + a * kAccCols + half * (kRows / 2) + (static_cast<uint32_t>(q * 32) << 16);
+      const uint32_t lanes = tmem_base + a * kAccCols + (static_cast<uint32_t>(q * 32) << 16);
       const int real = min(kRows, rows - m0);
       __half* y = p.y + static_cast<size_t>(m0) * p.n_out + col;
       const __half* res = p.residual ? p.residual + static_cast<size_t>(m0) * p.n_out + col : nullptr;
+      if constexpr (SPLIT > 1) {       // partial sums to the drained ring: [activation row][high, low][weight row]
 #pragma unroll 1
-      for (int c0 = 0; c0 < kRows / 2; c0 += kChunk) {
+        for (int c0 = half * (kRows / 2); c0 < (half + 1) * (kRows / 2); c0 += kChunk) {
+          uint32_t hi[kChunk], lo[kChunk];
+          tc_ld_x16(lanes + c0, hi);
+          tc_ld_x16(lanes + kRows + c0, lo);
+          tc_wait_ld();
+#pragma unroll
+          for (int j = 0; j < kChunk; ++j) {
+            s_part[(2 * (c0 + j)) * kRows + r] = kblocks > 0 ? static_cast<int>(hi[j]) : 0;
+            s_part[(2 * (c0 + j) + 1) * kRows + r] = kblocks > 0 ? static_cast<int>(lo[j]) : 0;
+          }
+        }
+        __syncwarp();
+        cluster_sync_release();        // every CTA's sums are in place
+      }
+#pragma unroll 1
+      for (int c0 = 0; c0 < kRows / 2 / SPLIT; c0 += kChunk) {
+        const int first_row = (share * 2 + half) * (kRows / 2 / SPLIT) + c0;          // activation row of the tile
         uint32_t hi[kChunk], lo[kChunk];
-        tc_ld_x16(acc + c0, hi);
-        tc_ld_x16(acc + kRows + c0, lo);
-        const int first = half * (kRows / 2) + c0;          // activation row of the tile
+        if constexpr (SPLIT == 1) {
+          tc_ld_x16(lanes + first_row, hi);
+          tc_ld_x16(lanes + kRows + first_row, lo);
+        } else {
+#pragma unroll
+          for (int j = 0; j < kChunk; ++j) { hi[j] = 0u; lo[j] = 0u; }
+#pragma unroll
+          for (int k = 0; k < SPLIT; ++k) {
+            const uint32_t from = map_to_rank(smem_u32(s_part + 2 * first_row * kRows + r), 2 * k + rank);
+#pragma unroll
+            for (int j = 0; j < kChunk; ++j) {
+              hi[j] += load_cluster(from + (2 * j) * kRows * 4);
+              lo[j] += load_cluster(from + (2 * j + 1) * kRows * 4);
+            }
+          }
+        }
         float add[kChunk];
         if constexpr (!SWIGLU) {
 #pragma unroll
           for (int j = 0; j < kChunk; ++j)
-            add[j] = res && col_ok && first + j < real ? __half2float(res[static_cast<size_t>(first + j) * p.n_out]) : 0.f;
+            add[j] = res && col_ok && first_row + j < real ? __half2float(res[static_cast<size_t>(first_row + j) * p.n_out]) : 0.f;
         }
-        tc_wait_ld();
-        if (c0 + kChunk >= kRows / 2) {                     // the accumulator is in registers: the next tile may have it
+        if constexpr (SPLIT == 1) tc_wait_ld();
+        if (SPLIT == 1 && c0 + kChunk >= kRows / 2) {       // the accumulator is in registers: the next tile may have it
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&acc_empty[a]), 0));
+          if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&acc_empty[a]), first));
         }
-        const int4* row = s_row + a * kRows + first;
+        const int4* row = s_row + a * kRows + first_row;
         float v[kChunk];
         if (all_int) {
 #pragma unroll
@@ -247,13 +291,13 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
           for (int j = 0; j < H; ++j) {
             const float other = buf[(is_up ? H + j : j) * kPairHalf];
             const float g = is_up ? other : v[j], u = is_up ? v[H + j] : other;
-            const int m = first + (is_up ? H + j : j);
+            const int m = first_row + (is_up ? H + j : j);
             if (col_ok && m < real) y[static_cast<size_t>(m) * p.n_out] = __float2half_rn(silu_fast(g) * u);
           }
         } else {
 #pragma unroll
           for (int j = 0; j < kChunk; ++j)
-            if (col_ok && first + j < real) y[static_cast<size_t>(first + j) * p.n_out] = __float2half_rn(__fadd_rn(v[j], add[j]));
+            if (col_ok && first_row + j < real) y[static_cast<size_t>(first_row + j) * p.n_out] = __float2half_rn(__fadd_rn(v[j], add[j]));
         }
       }
     }
@@ -292,7 +336,13 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor core reads these bytes through the async proxy
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&ready[s]), 0));
+      if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&ready[s]), first));
+    }
+  }
+  if constexpr (SPLIT > 1) {                      // (the cluster barrier between the partial sums and their readers is everyone's)
+    if ((warp < 2 || warp >= 10) && pair < tiles) {
+      __syncwarp();
+      cluster_sync_release();
     }
   }
   // Nobody leaves while the other CTA may still signal its barriers, read its operands or use the pair's tensor memory.
@@ -305,17 +355,47 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   }
 }
 
-template <int BITS, bool SWIGLU>
-int launch_rows(const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, const RowsParams& p, cudaStream_t stream) {
+template <int BITS, bool SWIGLU, int SPLIT>
+int launch_split(const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, const RowsParams& p, int tiles, cudaStream_t stream) {
   constexpr int kSmem = 1024 + num_stages(BITS) * stage_bytes(BITS) + kTailBytes;
   static_assert((4 * num_stages(BITS) + 4) * 8 + 8 <= 512, "barriers and the tensor-memory base fit in the tail");
-  auto kern = qgemm_i8_rows_kernel<BITS, SWIGLU>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  static_assert(num_stages(BITS) * stage_bytes(BITS) >= 2 * kRows * kRows * 4, "partial sums fit in the drained ring");
+  auto kern = qgemm_i8_rows_kernel<BITS, SWIGLU, SPLIT>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (e != cudaSuccess) return static_cast<int>(e);
-  const int tiles = (p.bands + 1) / 2 * ((p.M + kRows - 1) / kRows);
-  const int pairs = tiles < kNumSMs / 2 ? tiles : kNumSMs / 2;
-  kern<<<2 * pairs, num_threads(BITS), kSmem, stream>>>(tmap_w, tmap_x, p);
+  const int clusters = SPLIT > 1 || tiles < kNumSMs / 2 ? tiles : kNumSMs / 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(2 * SPLIT * clusters, 1, 1);
+  cfg.blockDim = dim3(num_threads(BITS), 1, 1);
+  cfg.dynamicSmemBytes = kSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2 * SPLIT;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, kern, tmap_w, tmap_x, p);
+  if (e != cudaSuccess) return static_cast<int>(e);
   return launch_status();
+}
+
+// Pairs along K, with at least four k blocks each: four for up to twelve tiles (sixteen clusters of eight CTAs do not run at
+// once: 100 rows of int8 4096 x 4096 30.0 us with four, 19.5 with two, 23.5 with one; 1280 x 8192 19.6, 32.7 with one), two
+// while the CTAs have an SM each (4096 x 14336 43.6 us with four, 32.6 with two, 47.5 with one).
+int pairs_along_k(int tiles, int kblocks) {
+  if (tiles <= 12 && kblocks >= 16) return 4;
+  return tiles * 4 <= kNumSMs && kblocks >= 8 ? 2 : 1;
+}
+
+template <int BITS, bool SWIGLU>
+int launch_rows(const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, const RowsParams& p, cudaStream_t stream) {
+  const int tiles = (p.bands + 1) / 2 * ((p.M + kRows - 1) / kRows);
+  const int split = pairs_along_k(tiles, p.K / kRows);
+  if (split == 4) return launch_split<BITS, SWIGLU, 4>(tmap_w, tmap_x, p, tiles, stream);
+  if (split == 2) return launch_split<BITS, SWIGLU, 2>(tmap_w, tmap_x, p, tiles, stream);
+  return launch_split<BITS, SWIGLU, 1>(tmap_w, tmap_x, p, tiles, stream);
 }
 
 }  // namespace
@@ -330,6 +410,15 @@ bool qgemm_i8_rows_supported(const QGemvParams& q, const void* workspace, size_t
   if (!workspace || workspace_bytes < qgemm_i8_workspace_bytes(q.M, q.K) || !aligned_to(workspace, 128)) return false;
   if (!aligned_to(q.packed, 16) || !aligned_to(q.x, 16) || (q.x_stride * 2) % 16 != 0) return false;
   return tensor_map_encoder() != nullptr;
+}
+
+// Against passes of 64 rows. A pair needs about 1 us for a k block of int4 codes, so that up to 128 rows with a long K and less
+// than half of the pairs at work are faster as two passes over all SMs: 100 rows of 4096 x 14336 56.5 us here, 54.6 in passes
+// (49 for up to 96 rows); 4096 x 4096 29.6 and 36.7, 1280 x 8192 27.4 and 29.8, 14336 x 4096 38 and 61. Bytes: 20 to 45 % faster here.
+bool qgemm_i8_rows_preferred(const QGemvParams& q) {
+  if (q.bits == 8 || q.M > kRows) return true;
+  const int tiles = (q.N + 2 * kRows - 1) / (2 * kRows), kblocks = q.K / kRows, split = pairs_along_k(tiles, kblocks);
+  return tiles * split * 4 >= kNumSMs || kblocks <= 16 * split;
 }
 
 int launch_qgemm_i8_rows(const QGemvParams& q, const int* n_rows, void* workspace, cudaStream_t stream) {

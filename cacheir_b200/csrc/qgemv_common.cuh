@@ -76,6 +76,8 @@ int qgemm_i8_quantize_tall(const void* x, long long x_stride, int M, const int* 
 int qgemm_i8_rms_norm_quantize_tall(const void* x, const void* weight, int M, const int* n_rows, int hidden, float eps, void* workspace,
                                     cudaStream_t stream);
 bool qgemm_i8_rows_supported(const QGemvParams& p, const void* workspace, size_t workspace_bytes);
+// Is that faster than passes of 64 rows?
+bool qgemm_i8_rows_preferred(const QGemvParams& p);
 int launch_qgemm_i8_rows(const QGemvParams& p, const int* n_rows, void* workspace, cudaStream_t stream);
 int qgemm_i8_rows_device_status(bool reset);
 // Device-side status word of the tensor-core kernel (0 = no bounded wait ever gave up).

@@ -110,21 +110,6 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t local, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
-// A bounded wait that also acquires what the other CTA of the cluster did before its arrival.
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int* status, int code) {
-  for (uint32_t i = 0; i < kPollLimit; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    if (done) return true;
-    if (i > 64) __nanosleep(32);
-  }
-  atomicCAS(status, 0, code);
-  return false;
-}
 // Tensor copy into this CTA's shared memory whose bytes are counted on a barrier of either CTA of the pair.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t cluster_bar, int x, int y) {
   asm volatile(
@@ -138,10 +123,10 @@ __device__ __forceinline__ void tc_alloc_pair(uint32_t slot_smem, uint32_t cols)
 __device__ __forceinline__ void tc_dealloc_pair(uint32_t base, uint32_t cols) {      // one whole warp of each CTA
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
 }
-// Arrives on the barrier at offset `bar` of both CTAs once the MMAs issued so far have retired.
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+// Arrives on the barrier at offset `bar` of both CTAs (ranks `first` and `first` + 1) once the MMAs issued so far have retired.
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar, uint32_t first = 0) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
+               ::"r"(bar), "h"(static_cast<uint16_t>(3u << first)) : "memory");
 }
 __device__ __forceinline__ void tc_mma_i8_ss_pair(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(

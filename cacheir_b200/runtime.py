@@ -692,7 +692,7 @@ class _DecodePlan:
                                    workspace=ws, tiled=weight.tiled, prequantized=prequantized, paired=weight.paired)
             key = f"b200.qgemv.int{bits}" + (".swiglu" if epilogue == ops.EPI_SWIGLU else ".residual" if residual is not None else "")
             eng.gemm_plans[f"q{bits}:{(self.batch, 1, k)}x{weight.shape}"] = key
-            if ws is not None and k % 128 == 0 and k <= 32768 and not prequantized and self.batch > 8:   # activation pre-pass + integer GEMM per 64-row chunk
+            if ws is not None and k % 128 == 0 and k <= 32768 and not prequantized and (bits == 8 or self.batch > 8):   # activation pre-pass + integer GEMM per 64-row chunk
                 self._emit(fn, key, launches=2 * ((self.batch + 63) // 64))
                 return out
         else:
@@ -758,7 +758,7 @@ class _DecodePlan:
             return out, True
         self._emit(lambda: ops.paged_attention_decode_batch(q3, k_pool, v_pool, self.page_table, self.seq_lens, out=out3,
                                                             num_splits=splits, workspace=ws, kv_scales=kv_scales),
-                   "b200.paged_attention_decode_batch.persistent_shared", launches=2 if splits > 1 else 1)
+                   "b200.paged_attention_decode_batch.persistent_shared", launches=2 if splits > 8 or (splits > 1 and splits * kv_heads * self.batch > 296) else 1)
         return out, False
 
     # -- stepping --------------------------------------------------------------------

@@ -205,7 +205,9 @@ int cacheir_b200_qgemv(const void* x, const void* packed, const void* scales,
  * int4 per-row weights with fp16 activations (K % 128 == 0, K <= 32768) run on the integer
  * tensor cores: the uint8 codes are fed to the MMA as they are (int4 nibbles are widened to
  * bytes in shared memory), and x is first turned into 16-bit fixed point per row (two
- * signed bytes, 2^-15 of the row maximum) in the workspace by a pre-pass kernel. Batches above 64 rows run as
+ * signed bytes, 2^-15 of the row maximum) in the workspace by a pre-pass kernel. Batches above 64 rows of tile-ordered
+ * codes run as blocks of 128 rows in one launch, with the scratch of all rows (the bytes below grow with M above 64);
+ * other layouts, and a workspace that only holds 64 rows, as
  * 64-row chunks (128-row chunks on the fp16 tensor-core kernel, which takes 65..128 rows in
  * one launch with the activations as the 128-row operand). Other shapes ignore the
  * workspace. workspace may be NULL (then this is cacheir_b200_qgemv). The workspace is only used during the call's own kernels; two
@@ -234,7 +236,7 @@ int cacheir_b200_rmsnorm_qgemv(const void* x, const void* norm_weight, float eps
 
 /* Which kernel cacheir_b200_qgemv_ex would launch for these extents and flags (fp16 activations, aligned
  * pointers): (family << 8) | detail, family 1 = integer tensor core with detail = its split-K factor,
- * 2 = fp16 tensor core, 3 = CUDA cores, 4 = streaming int4 GEMV (up to 8 rows); epilogue 3 asks about
+ * 2 = fp16 tensor core, 3 = CUDA cores, 4 = streaming int4 GEMV (up to 32 rows); epilogue 3 asks about
  * cacheir_b200_qkv_rope_append. Negative:
  * the validation code the call would return. Launches nothing. No counterpart in the reference (its
  * kernel choice is the declarative `attrs["kernel"]`, cacheir/passes/transformer.py:391-424). */

@@ -12,10 +12,12 @@ def _status():
 
 
 # edges: one row past the 64-row kernels, whole and ragged blocks of 128, an odd number of weight tiles (half a pair), a last tile
-# that is not full, a single k block, more tiles than CTA pairs
+# that is not full, a single k block, more tiles than CTA pairs, K split over two and four pairs (evenly and not),
+# few tiles and a long K (int4: passes)
 @pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("m, n, k, epilogue", [(65, 128, 128, 0), (128, 384, 256, 1), (129, 320, 1024, 0), (300, 1280, 2048, 1), (192, 256, 640, 2),
-                                               (257, 640, 1152, 2), (1024, 4096, 512, 0)])
+                                               (257, 640, 1152, 2), (1024, 4096, 512, 0), (192, 256, 2048, 2), (200, 2304, 1024, 2), (128, 384, 1152, 1),
+                                               (129, 320, 2176, 0), (70, 512, 9216, 0)])
 def test_rows_equal_passes_of_64(bits, m, n, k, epilogue):
     from cacheir_b200 import ops
     from cacheir_b200.quantization import pack_weight_device, to_tiled
