@@ -11,11 +11,12 @@
 // serves both. That is 32 KB per CTA and 512 tensor-core cycles; a CTA by itself would need 48 KB for the same cycles (both planes), more
 // than L2 delivers. The accumulator takes 256 of the 512 tensor-memory columns, so the epilogue of one tile runs under the main
 // loop of the next. Persistent: pairs walk the tiles with the row blocks innermost, so that the weights of the few tiles
-// in flight are read from HBM once and the activation planes stay in L2.
+// in flight are read from HBM once and the activation planes stay in L2. 2048 rows, int8 28672 x 4096 with SwiGLU: 311 us, 3.1 POPS,
+// tensor pipe active 80 % of the cycles (32 passes of 64 rows take 26 us each for half of these weights).
 //
 // Few tiles leave most SMs idle, so that a tile's K range is split over the SPLIT pairs of a larger cluster (one tile per
 // cluster then): every CTA lays its partial sums out in its drained ring, and pair j adds up, through distributed shared memory, what all pairs have
-// for its share of the activation rows. Integer sums: the order cannot matter. 256 rows of 2048 x 5632: 44 k blocks on 32 SMs, or 11 on 128.
+// for its share of the activation rows. Integer sums: the order cannot matter. 256 rows of 2048 x 5632: 44 k blocks on 32 SMs, or 22 on 64.
 //
 // Warps: 0 copies, 1 issues MMAs (even CTA only), 2-9 epilogue (four per half of the activation rows), with int4 codes 10-21
 // widen nibble tiles to byte tiles in three groups that take every third stage.
