@@ -4,12 +4,17 @@
 namespace cb200 {
 namespace {
 
+// Tokens from which pairs are chosen: below, a tile of 256 weight rows leaves the last turn emptier than K split over single CTAs
+// (whole prompts of width 4096, 330 tokens: 2877 us on single CTAs, 3064 on pairs; 1944 and 1982; 230 tokens 1603 and 1574;
+// 2048 tokens 6155 and 5432, 1001 of width 2048 1773 and 1715).
+constexpr int kPairTokens = 768;
+
 struct Shape { int mt, split; };
 Shape choose_shape(int T, int N, int K, int batch) {
   const int n_tiles = (N + kTileN - 1) / kTileN * batch;
   int mt = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : 128;
   // (products per head with a short K are all epilogue: two CTAs per SM take turns. 32 heads of 128 x 512, 2048 tokens: 87 to 54 us)
-  if (T >= 256 && !(batch > 1 && K <= 1024) && n_tiles * ((T + 255) / 256) >= kNumSMs) mt = 256;
+  if (T >= 256 && !(batch > 1 && K <= 1024 && T >= kPairTokens) && n_tiles * ((T + 255) / 256) >= kNumSMs) mt = 256;
   const int tiles = n_tiles * ((T + mt - 1) / mt);
   const int kblocks = (K + kBlockK - 1) / kBlockK;
   const int slots = kNumSMs * ctas_per_sm(mt);
@@ -20,7 +25,7 @@ Shape choose_shape(int T, int N, int K, int batch) {
 
 // Tokens per tile of a CTA pair, 0: single CTAs.
 int choose_pair(int T, int N, int K, int batch) {
-  if (T < 192 || (batch > 1 && (K <= 1024 || N % (2 * kTileN) != 0))) return 0;
+  if (T < kPairTokens || (batch > 1 && (K <= 1024 || N % (2 * kTileN) != 0))) return 0;
   auto cost = [&](int tt) {          // turns of the busiest pair, in tiles of 128 tokens (a narrow tile asks more of L2)
     const long long tiles = static_cast<long long>((T + tt - 1) / tt) * ((N + 2 * kTileN - 1) / (2 * kTileN)) * batch;
     return (tiles + kNumSMs / 2 - 1) / (kNumSMs / 2) * (tt == 256 ? 16 : 10);
