@@ -389,7 +389,7 @@ bool qgemv_stream_supported(const QGemvParams& q) {
   if (!q.tiled && q.N >= 64 * kNumSMs && qgemv_mma_supported(q)) return false;
   const bool swiglu = q.epilogue == CACHEIR_B200_EPI_SWIGLU;
   if (q.epilogue == kEpiQkvRopeAppend) return false;
-  if (q.paired && !(swiglu && q.tiled && (q.N / 2) % 64 == 0)) return false;
+  if (q.paired && (q.group_size > 0 || !(swiglu && q.tiled && (q.N / 2) % 64 == 0))) return false;   // (group scales lie in logical row order)
   if (swiglu && !q.paired && (q.N / 2) % 128 != 0) return false;
   return aligned_to(q.packed, 16) && aligned_to(q.x, 16) && (q.x_stride * 2) % 16 == 0;
 }
