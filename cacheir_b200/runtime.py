@@ -124,6 +124,9 @@ class B200PrefixCache:
                 "misses": self.misses, "evictions": self.evictions}
 
 
+DECODE_PASS_ROWS = 64        # rows of a prompt pass through the decode plan
+
+
 class _Engine:
     """State shared by every fork of a runtime: weights, page pools, plans."""
 
@@ -172,8 +175,8 @@ class _Engine:
         self.tile_weights = True
         self.validated_batch: tuple[int, ...] | None = None      # identity of the last decode batch that passed the checks
         self.validated_sessions: list[Any] = []
-        # prompt tokens per pass of the chunked prefill (0: one token per step)
-        self.prefill_chunk = 2048 if self.ragged else 64
+        # prompt tokens per pass of the chunked prefill (0: one token per step); see `pass_rows`
+        self.prefill_chunk = 2048 if self.ragged else DECODE_PASS_ROWS
         self.prompt_rows = 0 if self.ragged else self._prompt_rows(kv_dtype)
         self._rope_tables: dict[tuple[int, float], torch.Tensor] = {}
         self.attention_splits = int(attention_splits)
@@ -207,8 +210,10 @@ class _Engine:
 
     @property
     def pass_rows(self) -> int:
-        """Prompt tokens that one pass takes."""
-        return self.prompt_rows if self.prompt_rows and self.prefill_chunk else self.prefill_chunk
+        """Prompt tokens that one pass takes: `prefill_chunk` where that was set, else as many as the model's prompt plans take."""
+        if not self.prompt_rows:
+            return self.prefill_chunk
+        return self.prompt_rows if self.prefill_chunk == DECODE_PASS_ROWS else min(self.prefill_chunk, self.prompt_rows)
 
     def count(self, name: str, n: int = 1) -> None:
         self.kernel_counts[name] = self.kernel_counts.get(name, 0) + n
@@ -789,6 +794,8 @@ class _DecodePlan:
         any row attends). Rows beyond the list repeat the last entry (same position, same values: harmless
         duplicates). The pages of every position must already be reserved."""
         n = len(rows)
+        if n > self.batch:
+            raise ValueError(f"a pass of {self.batch} rows cannot take {n} prompt tokens")
         self.h2d_done.synchronize()
         ids = self.host_ids.numpy()
         lens = self.host_lens.numpy()
@@ -808,10 +815,6 @@ class _DecodePlan:
         self.h2d_done.record()
         self.synced_owner_state = None
         self.repeat_left = 0            # the device rows now belong to this pass
-
-    def sync_prefill_chunk(self, cache: B200PagedKVCache, start: int, token_ids: list[int]) -> None:
-        """Rows 0..n-1 are the tokens at positions start..start+n-1 of one sequence."""
-        self.sync_prefill_rows([(cache, start + i, int(t)) for i, t in enumerate(token_ids)])
 
     def run_program(self, *, feedback: bool = False) -> None:
         """One decode step: eager launches on the first step, CUDA-graph replay afterwards."""
@@ -1266,7 +1269,7 @@ class B200DecodeRuntime:
             session.kv_cache.extend(len(tokens))
         results = []
         with torch.cuda.device(self.device):
-            passes = cut_passes(token_batches, eng.pass_rows or 64, None if eng.ragged else _PromptPlan.SEQUENCES)
+            passes = cut_passes(token_batches, eng.pass_rows or DECODE_PASS_ROWS, None if eng.ragged else _PromptPlan.SEQUENCES)
             for part in passes:                                   # (session, first token, last token + 1)
                 want = [(i, int(p)) for i, lo, hi in part for p in wanted[i] if lo <= int(p) < hi]
                 logits = self._run_rows(sessions, token_batches, starts, part, want)
@@ -1304,11 +1307,11 @@ class B200DecodeRuntime:
         rows = sum(len(tokens) for _, _, tokens in parts)
         needed = max(len(cache.pages) for cache, _, _ in parts)
         # up to 64 rows the weights are the bottleneck and the decode plan's kernels stream them best
-        if rows > 64 and eng.prompt_rows and eng.prefill_chunk:
+        if rows > DECODE_PASS_ROWS and eng.prompt_rows:
             plan = eng.prompt_plan(rows, needed)
             plan.sync_parts(parts)
         else:
-            plan = eng.prefill_plan(eng.prefill_chunk or 64, needed)
+            plan = eng.prefill_plan(eng.prefill_chunk or DECODE_PASS_ROWS, needed)
             plan.sync_prefill_rows([(cache, start + i, int(t)) for cache, start, tokens in parts for i, t in enumerate(tokens)])
         plan.run_program()
         return plan.logits[:rows]

@@ -98,10 +98,7 @@ def test_rope_append_rows_equals_rope_append():
     assert torch.equal(a[:, :q_dim], b[:, :q_dim]) and torch.equal(pools[0], pools[2]) and torch.equal(pools[1], pools[3])
 
 
-@pytest.mark.parametrize("quant", ["int8", "int4_awq", "int4_g128"])
-def test_prompt_pass_equals_passes_of_64_rows(quant):
-    """Prompts through one pass against 64-row passes of the decode plan: logits and the cached rows that later steps read. The
-    products are the same integers (int4_g128: the same fp16 products), only the attention adds in another order."""
+def _runtime(quant="int8", *, intermediate=768, **kwargs):
     import cacheir_b200 as C
 
     gen = torch.Generator(device="cuda")
@@ -110,10 +107,38 @@ def test_prompt_pass_equals_passes_of_64_rows(quant):
         gen.manual_seed(len(key) * 131 + sum(map(ord, key)))
         return torch.ones(shape, device="cuda") if len(shape) == 1 else torch.randn(shape, device="cuda", generator=gen) * 0.05
 
-    art = C.build_decoder_artifact(C.ModelConfig(architecture="LlamaForCausalLM", hidden_size=512, intermediate_size=768, num_layers=2, num_attention_heads=4,
-                                                 num_key_value_heads=2, vocab_size=640, max_position_embeddings=512, rope_theta=10000.0, dtype="float16"),
+    art = C.build_decoder_artifact(C.ModelConfig(architecture="LlamaForCausalLM", hidden_size=512, intermediate_size=intermediate, num_layers=2,
+                                                 num_attention_heads=4, num_key_value_heads=2, vocab_size=640, max_position_embeddings=512,
+                                                 rope_theta=10000.0, dtype="float16"),
                                    quant=quant, modes=("decode",))
-    rt = C.B200DecodeRuntime(art, dtype="float16", tensor_source=source, max_seq_len=512)
+    return C.B200DecodeRuntime(art, dtype="float16", tensor_source=source, max_seq_len=512, **kwargs)
+
+
+@pytest.mark.parametrize("chunk", [16, 32, 100, 512])
+def test_passes_keep_to_the_prefill_chunk(chunk):
+    """A chunk that was set bounds every pass, above 64 rows and below: all tokens reach the cache and have their logits."""
+    rt = _runtime()
+    want = rt.fork().run([list(range(200))], mode="prefill")
+    rt._engine.prefill_chunk = chunk
+    assert rt._engine.pass_rows == chunk
+    one, many = rt.fork(), [rt.fork(), rt.fork()]
+    got = one.run([list(range(200))], mode="prefill")
+    assert float((got.float() - want.float()).norm() / want.float().norm()) <= 2e-3
+    rt.run_prefill_batch(many, [list(range(150)), [7] * 40])
+    steps = rt.run_step_batch([one] + many, [[3] * 40, [5], [6] * 30])
+    rt._engine.prefill_chunk = 64
+    again, others = rt.fork(), [rt.fork(), rt.fork()]
+    again.run([list(range(200))], mode="prefill")
+    rt.run_prefill_batch(others, [list(range(150)), [7] * 40])
+    want = rt.run_step_batch([again] + others, [[3] * 40, [5], [6] * 30])
+    assert float((steps.float() - want.float()).norm() / want.float().norm()) <= 2e-3
+
+
+@pytest.mark.parametrize("quant", ["int8", "int4_awq", "int4_g128"])
+def test_prompt_pass_equals_passes_of_64_rows(quant):
+    """Prompts through one pass against 64-row passes of the decode plan: logits and the cached rows that later steps read. The
+    products are the same integers (int4_g128: the same fp16 products), only the attention adds in another order."""
+    rt = _runtime(quant)
     assert rt._engine.prompt_rows == 2048
     rng = np.random.default_rng(5)
     prompts = [[int(t) for t in rng.integers(0, 640, n)] for n in (5, 200, 1, 70)]
