@@ -906,20 +906,25 @@ class _PromptPlan(_DecodePlan):
         return storage[: self.batch * cols * 2].view(torch.float16).view(self.batch, cols)
 
     def _gemm_workspace(self, k: int) -> torch.Tensor:
-        widest = max(int(self.engine.config.hidden_size), int(self.engine.config.intermediate_size))
+        config = self.engine.config
+        widest = max(w for w in (int(config.hidden_size), int(config.intermediate_size)) if w <= 32768)      # (see _by_row_blocks)
         return self.engine.scratch("prompt.planes", ops.qgemv_workspace_bytes(self.engine.prompt_rows, widest))
 
-    def _i8_eligible(self, weight: Any, k: int, swiglu: bool = False) -> bool:
+    @staticmethod
+    def _by_row_blocks(weight: Any, swiglu: bool = False) -> bool:
+        """Is this a product of `ops.qgemm_rows`? (The 32-bit sums bound its K; longer ones take the general product.)"""
         return (isinstance(weight, B200PackedWeight) and weight.bits in (4, 8) and not weight.group_size and weight.tiled
-                and weight.paired == swiglu and k % 128 == 0 and k <= 8192)
+                and weight.paired == swiglu and weight.shape[1] <= 32768)
+
+    def _i8_eligible(self, weight: Any, k: int, swiglu: bool = False) -> bool:
+        return self._by_row_blocks(weight, swiglu) and k <= 8192
 
     def _norm_quantize(self, x: torch.Tensor, w: torch.Tensor, eps: float, ws: torch.Tensor) -> None:
         self._emit(lambda: ops.rms_norm_quantize_rows(x, w, eps, ws, self.n_rows), "b200.rms_norm_quantize")
 
     def _matmul(self, x: torch.Tensor, weight: B200PackedWeight | torch.Tensor, *, epilogue: int = ops.EPI_NONE,
                 residual: torch.Tensor | None = None, prequantized: bool = False, out: torch.Tensor | None = None) -> torch.Tensor:
-        if not (isinstance(weight, B200PackedWeight) and weight.tiled and not weight.group_size
-                and weight.paired == (epilogue == ops.EPI_SWIGLU)):
+        if not self._by_row_blocks(weight, epilogue == ops.EPI_SWIGLU):
             return super()._matmul(x, weight, epilogue=epilogue, residual=residual, prequantized=prequantized, out=out)
         n, k, bits = weight.shape[0], weight.shape[1], weight.bits
         epilogue = ops.EPI_RESIDUAL if residual is not None else epilogue

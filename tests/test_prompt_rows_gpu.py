@@ -158,3 +158,18 @@ def test_prompt_pass_equals_passes_of_64_rows(quant):
                 a, b = (torch.cat([pool[name][p.page_id][:, :p.length] for p in x.kv_cache.pages], dim=1).float() for x in (f, s))
                 assert float((a - b).norm() / b.norm()) <= 2e-3
     rt.check_device_status()
+
+
+@pytest.mark.parametrize("quant", ["int8", "int4_awq"])
+def test_prompt_pass_of_a_very_wide_model(quant):
+    """A down projection whose K is beyond the 32-bit sums of the integer products: the pass takes the general product for it, the same one
+    that 64-row passes take. Only the attention adds in another order."""
+    rt = _runtime(quant, intermediate=32896)
+    assert rt._engine.prompt_rows > 0
+    prompts = [list(range(100)), [9] * 45]
+    got = rt.run_prefill_batch([rt.fork(), rt.fork()], prompts)
+    assert rt.kernel_counts["b200.paged_attention_prompt"] > 0
+    rt._engine.prompt_rows = 0
+    want = rt.run_prefill_batch([rt.fork(), rt.fork()], prompts)
+    assert float((got.float() - want.float()).norm() / want.float().norm()) <= 2e-3
+    rt.check_device_status()
