@@ -196,7 +196,8 @@ class _Engine:
 
     def _prompt_rows(self, kv_dtype: str) -> int:
         """Rows of the widest prompt pass (`_PromptPlan`), 0 where prompts go through 64-row passes of the decode plan: it
-        takes packed fp16 graphs of fused ops with 16-token fp16 pages. Bounded so that the logits of a pass stay under 256 MB."""
+        takes packed fp16 graphs of fused ops with 16-token fp16 pages, whose projections rotate and append what their attention
+        reads. Bounded so that the logits of a pass stay under 256 MB."""
         ops_taken = {"token_embedding", "quantized_fused_rmsnorm_qkv_rope", "paged_attention_decode", "quantized_matmul", "add", "rms_norm",
                      "quantized_fused_swiglu"}
         c = self.config
@@ -205,8 +206,27 @@ class _Engine:
                 or int(c.hidden_size) % 128 or int(c.hidden_size) > 8192 or int(c.intermediate_size) % 128
                 or any(node.op not in ops_taken for node in self.graph.nodes)):
             return 0
+        heads, kv_heads, head_dim = int(c.num_attention_heads), int(c.num_key_value_heads), int(c.head_dim)
+        if heads * head_dim % 128:
+            return 0
+        nodes, served = list(self.graph.nodes), []
+        for idx, node in enumerate(nodes):
+            if node.op == "quantized_fused_rmsnorm_qkv_rope":
+                served.append(_DecodePlan._attention_consumer(nodes, idx, node))
+                if (served[-1] is None or int(node.attrs["head_dim"]) != head_dim
+                        or [self.weight_rows(name) for name in node.inputs[2:5]] != [heads * head_dim, kv_heads * head_dim, kv_heads * head_dim]):
+                    return 0
+        for node in nodes:
+            if node.op == "paged_attention_decode" and (not any(node is other for other in served)
+                                                        or (int(node.attrs["num_heads"]), int(node.attrs["num_kv_heads"]), int(node.attrs["head_dim"]))
+                                                        != (heads, kv_heads, head_dim)):
+                return 0
         rows = min(2048, (1 << 27) // int(c.vocab_size) // 128 * 128)
         return rows if rows >= 128 else 0
+
+    def weight_rows(self, name: str) -> int:
+        spec = self.graph.weights[name]
+        return int((getattr(spec, "shape", None) or spec.tensor_type.shape)[0])
 
     @property
     def pass_rows(self) -> int:
@@ -669,9 +689,7 @@ class _DecodePlan:
                                            theta=theta), "b200.rope_append")
 
     def _rows_of(self, weight_name: str) -> int:
-        spec = self.engine.graph.weights[weight_name]
-        shape = getattr(spec, "shape", None) or spec.tensor_type.shape
-        return int(shape[0])
+        return self.engine.weight_rows(weight_name)
 
     def _i8_eligible(self, weight: Any, k: int, swiglu: bool = False) -> bool:
         """Will this projection run on the integer tensor cores (and so accept pre-quantized activations)?"""
