@@ -431,6 +431,10 @@ dense_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           tma_load_2d_pair(smem_u32(s_x + s * (TT / 2) * kBlockK * 2), &tmap_x, bar, z * p.x_batch_cols + k, t0 + static_cast<int>(rank) * (TT / 2));
         }
       }
+      // Nothing may still be on its way when the blocks end (the even CTA sees the copies of both; a wait elsewhere may have given up)
+      if (rank == 0)
+        for (int i = it > S ? it - S : 0; i < it; ++i)
+          if (!mbar_wait(smem_u32(&full[i % S]), (i / S) & 1, &g_dense_status, (6 << 8) | 4)) break;
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {

@@ -101,6 +101,7 @@ paged_prompt_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
     const int32_t* table = p.page_table + static_cast<size_t>(tile.x) * p.max_pages;
     int next = lane < min(kStagePages, pages) ? table[lane] : 0;          // page ids one stage ahead
     bool ok = true;
+    int issued = 0;
     for (int it = 0; it < iters && ok; ++it) {
       const int s = it % kStages, first = it * kStagePages, count = min(kStagePages, pages - first);
       const int page = next;
@@ -115,8 +116,13 @@ paged_prompt_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
         const int row = (page * p.kv_heads + kvh) * kPage;
         tma_load_3d(dst, &tmap_k, smem_u32(&full[s]), 0, row, 0);
         tma_load_3d(dst + kTileBytes, &tmap_v, smem_u32(&full[s]), 0, row, 0);
+        issued = it + 1;
       }
     }
+    // nothing may still be on its way when the block ends (a consumer's wait may have given up); lane 0 copies in every stage
+    if (lane == 0)
+      for (int it = issued > kStages ? issued - kStages : 0; it < issued; ++it)
+        if (!mbar_wait(smem_u32(&full[it % kStages]), (it / kStages) & 1, &g_prompt_status, (7 << 8) | 4)) break;
     return;
   }
 

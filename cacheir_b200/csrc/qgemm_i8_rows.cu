@@ -143,6 +143,11 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
           tma_load_2d_pair(smem_u32(s_x + s * kTile), &tmap_x, bar, 0, ((block * kblocks_all + kb0 + kb) * 2 + static_cast<int>(rank)) * kRows);
         }
       }
+      // Nothing may still be on its way when the blocks end: a wait elsewhere may have given up. (The even CTA sees the copies of both.)
+      for (int i = it > S ? it - S : 0; i < it; ++i) {
+        if (rank == 0 && !mbar_wait(smem_u32(&full[i % S]), (i / S) & 1, &g_i8_rows_status, (6 << 8) | 7)) break;
+        if (BITS == 4 && !mbar_wait(smem_u32(&raw_full[i % S]), (i / S) & 1, &g_i8_rows_status, (6 << 8) | 8)) break;
+      }
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
