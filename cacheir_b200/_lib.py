@@ -21,6 +21,7 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "cacheir_b200_error_string": (c_char_p, [c_int]),
     "cacheir_b200_paged_attention_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
     "cacheir_b200_paged_attention_auto_splits": (c_int, [c_int] * 6),
+    "cacheir_b200_paged_attention_launches": (c_int, [c_int] * 9),
     "cacheir_b200_paged_attention_decode_batch": (
         c_int,
         [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,  # q k v page_table seq_lens out
@@ -201,6 +202,7 @@ GROUP_SIGNATURES: dict[str, dict[str, tuple[object, list[object]]]] = {
     "ragged": {
         "cacheir_b200_dense_supported": (c_int, [c_int, c_longlong, c_longlong, c_int, c_int]),
         "cacheir_b200_dense_gemm": (c_int, [c_void_p, c_void_p]),
+        "cacheir_b200_dense_pair_tokens": (c_int, [c_int] * 4),
         "cacheir_b200_dense_simple": (c_int, [c_void_p] * 3 + [c_int] * 7 + [c_longlong] * 3 + [c_void_p, c_int, c_int, c_void_p]),
         "cacheir_b200_scaled_embedding": (c_int, [c_void_p] * 3 + [c_int, c_int, c_int, c_float, c_int] + _NEXT + [c_int, c_void_p]),
         "cacheir_b200_dyt_rows": (c_int, [c_void_p] * 4 + [c_float, c_void_p, c_int, c_int, c_int, c_void_p]),

@@ -268,7 +268,7 @@ int launch_combine(const AttnParams& p, cudaStream_t stream) {
 
 }  // namespace
 
-void resolve_attention_splits(int batch, int heads, int kv_heads, int max_pages, int page_size,
+void resolve_attention_splits(int batch, int heads, int kv_heads, int max_pages, int page_size, long long room,
                               int requested, int* splits, int* chunk_tokens) {
   const long long max_ctx = static_cast<long long>(max_pages) * page_size;
   int s = requested;
@@ -291,7 +291,7 @@ void resolve_attention_splits(int batch, int heads, int kv_heads, int max_pages,
     long long near = (max_ctx + 63) / 64;
     if (near > want) near = want;
     if (near > kMaxClusterSplits) near = kMaxClusterSplits;
-    if (s > 1 && near > s && near * units <= 2 * kNumSMs) s = static_cast<int>(near);
+    if (s > 1 && near > s && near * units <= 2 * kNumSMs && near <= room) s = static_cast<int>(near);
   }
   if (s > kMaxAttentionSplits) s = kMaxAttentionSplits;
   if (s < 1) s = 1;
@@ -322,7 +322,7 @@ extern "C" int cacheir_b200_paged_attention_auto_splits(int batch_size, int num_
       page_size <= 0 || num_heads % num_kv_heads != 0)
     return 1;
   int s = 1, chunk = 0;
-  resolve_attention_splits(batch_size, num_heads, num_kv_heads, max_pages_per_seq, page_size, 0, &s,
+  resolve_attention_splits(batch_size, num_heads, num_kv_heads, max_pages_per_seq, page_size, kMaxAttentionSplits, 0, &s,
                            &chunk);
   return s;
 }
@@ -333,6 +333,12 @@ int i8_plane_rows(int M);
 }
 
 namespace {
+// Do the splits of the fast kernel merge inside a cluster? (All CTAs at once: a cluster's short members would otherwise hold
+// SMs that other sequences wait for.)
+bool merges_in_cluster(const AttnParams& p) {
+  return p.splits > 1 && p.splits <= kMaxClusterSplits && static_cast<long long>(p.splits) * p.kv_heads * p.batch <= 2 * kNumSMs;
+}
+
 // `gemm_workspace` non-null: the launch must also leave the output as the integer GEMM's activation planes
 // (CACHEIR_B200_EUNSUPPORTED when the fast single-split kernel cannot take the case). `probe`: decide only, launch nothing.
 int attention_dispatch(
@@ -365,8 +371,10 @@ int attention_dispatch(
   p.out_stride = out_batch_stride > 0 ? out_batch_stride : static_cast<long long>(num_heads) * head_dim;
   const float scale = softmax_scale > 0.f ? softmax_scale : 1.0f / sqrtf(static_cast<float>(head_dim));
   p.scale_log2 = scale * kLog2e;
+  // (scratch for fewer splits than the finest choice would take is still enough for the coarser one)
+  const size_t split_bytes = cacheir_b200_paged_attention_workspace_bytes(batch_size, num_heads, head_dim, 2) / 2;
   resolve_attention_splits(batch_size, num_heads, num_kv_heads, max_pages_per_seq, page_size,
-                           num_splits, &p.splits, &p.chunk_tokens);
+                           workspace ? static_cast<long long>(workspace_bytes / split_bytes) : 0, num_splits, &p.splits, &p.chunk_tokens);
   if (p.splits > 1) {
     const size_t need = cacheir_b200_paged_attention_workspace_bytes(batch_size, num_heads, head_dim, p.splits);
     if (!workspace || workspace_bytes < need) return CACHEIR_B200_EWORKSPACE;
@@ -394,8 +402,7 @@ int attention_dispatch(
                          (static_cast<long long>(head_dim) * kv_esize) % 8 == 0;
   int rc;
   if (paged_attention_fast_supported(p, dtype)) {
-    // (all CTAs at once: a cluster's short members would otherwise hold SMs that other sequences wait for)
-    p.cluster = p.splits > 1 && p.splits <= kMaxClusterSplits && static_cast<long long>(p.splits) * p.kv_heads * p.batch <= 2 * kNumSMs ? 1 : 0;
+    p.cluster = merges_in_cluster(p) ? 1 : 0;
     rc = launch_paged_attention_fast(p, dtype, st);
     if (p.cluster) return rc;
   } else if (kv8) {
@@ -453,6 +460,24 @@ extern "C" int cacheir_b200_paged_attention_quantize_supported(int batch_size, i
   return rc == 0 ? 1 : 0;
 }
 
+extern "C" int cacheir_b200_paged_attention_launches(int batch_size, int num_heads, int num_kv_heads, int max_pages_per_seq, int page_size,
+                                                     int head_dim, int dtype, int kv_dtype, int num_splits) {
+  if (batch_size <= 0 || num_heads <= 0 || num_kv_heads <= 0 || head_dim <= 0 || max_pages_per_seq <= 0 || page_size <= 0 ||
+      num_heads % num_kv_heads != 0)
+    return 0;
+  // Dummy, suitably aligned addresses: the answer depends on extents and alignment only.
+  void* aligned = reinterpret_cast<void*>(static_cast<uintptr_t>(1) << 20);
+  AttnParams p{};
+  p.q = aligned; p.k_cache = aligned; p.v_cache = aligned; p.kv_scales = aligned;
+  p.kv8 = kv_dtype == CACHEIR_B200_KV_INT8 ? 1 : 0;
+  p.batch = batch_size; p.heads = num_heads; p.kv_heads = num_kv_heads; p.group = num_heads / num_kv_heads;
+  p.max_pages = max_pages_per_seq; p.page_size = page_size; p.head_dim = head_dim;
+  p.q_stride = static_cast<long long>(num_heads) * head_dim;
+  resolve_attention_splits(batch_size, num_heads, num_kv_heads, max_pages_per_seq, page_size, kMaxAttentionSplits, num_splits, &p.splits,
+                           &p.chunk_tokens);
+  return p.splits > 1 && !(paged_attention_fast_supported(p, dtype) && merges_in_cluster(p)) ? 2 : 1;
+}
+
 extern "C" int cacheir_b200_paged_attention_decode_batch(
     const void* q, const void* k_cache, const void* v_cache, const int32_t* page_table,
     const int32_t* seq_lens, void* out, int batch_size, int num_heads, int num_kv_heads,
@@ -492,8 +517,9 @@ extern "C" int cacheir_b200_paged_attention_decode_batch_noalloc(
   if (batch_size <= 0 || num_heads <= 0 || num_kv_heads <= 0 || head_dim <= 0) return 0;
   if (max_pages_per_seq <= 0 || page_size <= 0 || num_splits < 0 || num_heads % num_kv_heads != 0) return CACHEIR_B200_EINVAL;
   int splits = 1, chunk = 0;
-  resolve_attention_splits(batch_size, num_heads, num_kv_heads, max_pages_per_seq, page_size, num_splits,
-                           &splits, &chunk);
+  const size_t split_bytes = cacheir_b200_paged_attention_workspace_bytes(batch_size, num_heads, head_dim, 2) / 2;
+  resolve_attention_splits(batch_size, num_heads, num_kv_heads, max_pages_per_seq, page_size,
+                           static_cast<long long>(CB200_NOALLOC_WORKSPACE_BYTES / split_bytes), num_splits, &splits, &chunk);
   const size_t need = cacheir_b200_paged_attention_workspace_bytes(batch_size, num_heads, head_dim, splits);
   if (need > CB200_NOALLOC_WORKSPACE_BYTES) return CACHEIR_B200_ELIMIT;
   int device = -1;

@@ -42,7 +42,8 @@ struct AttnParams {
 
 // Resolve the number of context splits (requested == 0: choose) and the number
 // of tokens each split covers (a multiple of page_size).
-void resolve_attention_splits(int batch, int heads, int kv_heads, int max_pages, int page_size,
+// `room`: splits that the caller's scratch holds (only what 0 chooses depends on it).
+void resolve_attention_splits(int batch, int heads, int kv_heads, int max_pages, int page_size, long long room,
                               int requested, int* splits, int* chunk_tokens);
 
 // Tensor-core path (fp16/bf16, head_dim 64/128, 16-token pages, GQA group <= 16).

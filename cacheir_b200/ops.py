@@ -52,6 +52,13 @@ def attention_auto_splits(batch: int, heads: int, kv_heads: int, max_pages: int,
     return int(_lib.load().cacheir_b200_paged_attention_auto_splits(batch, heads, kv_heads, max_pages, page_size, head_dim))
 
 
+def attention_launches(batch: int, heads: int, kv_heads: int, max_pages: int, page_size: int, head_dim: int, dtype: torch.dtype, *,
+                       kv8: bool = False, num_splits: int = 0) -> int:
+    """Kernels that one `paged_attention_decode_batch` launches."""
+    return int(_lib.load().cacheir_b200_paged_attention_launches(batch, heads, kv_heads, max_pages, page_size, head_dim, dtype_code(dtype),
+                                                                 1 if kv8 else 0, num_splits))
+
+
 def attention_workspace_bytes(batch: int, heads: int, head_dim: int, num_splits: int) -> int:
     return int(_lib.load().cacheir_b200_paged_attention_workspace_bytes(batch, heads, head_dim, num_splits))
 
@@ -145,7 +152,7 @@ def paged_attention_decode_batch(q: torch.Tensor, k_cache: torch.Tensor, v_cache
     check(lib.cacheir_b200_paged_attention_decode_batch_ex(
         q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), page_table.data_ptr(), seq_lens.data_ptr(),
         out.data_ptr(), batch, heads, kv_heads, max_pages, page_size, head_dim, dtype_code(q.dtype),
-        q.stride(0), out.stride(0), float(softmax_scale or 0.0), int(splits), _ptr(workspace), ws_bytes,
+        q.stride(0), out.stride(0), float(softmax_scale or 0.0), max(int(num_splits), 0), _ptr(workspace), ws_bytes,
         int(k_cache.shape[0]), 1 if kv8 else 0, _ptr(kv_scales), _stream()),
         "paged_attention_decode_batch")
     return out

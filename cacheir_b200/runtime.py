@@ -781,7 +781,9 @@ class _DecodePlan:
             return out, True
         self._emit(lambda: ops.paged_attention_decode_batch(q3, k_pool, v_pool, self.page_table, self.seq_lens, out=out3,
                                                             num_splits=splits, workspace=ws, kv_scales=kv_scales),
-                   "b200.paged_attention_decode_batch.persistent_shared", launches=2 if splits > 8 or (splits > 1 and splits * kv_heads * self.batch > 296) else 1)
+                   "b200.paged_attention_decode_batch.persistent_shared",
+                   launches=ops.attention_launches(self.batch, heads, kv_heads, self.width, eng.page_size, head_dim, q.dtype,
+                                                   kv8=kv_scales is not None, num_splits=splits))
         return out, False
 
     # -- stepping --------------------------------------------------------------------

@@ -81,7 +81,9 @@ const char* cacheir_b200_error_string(int code);
  *   k/v_cache:   [slots, num_kv_heads, page_size, head_dim], same dtype as q
  *   page_table:  int32 [batch, max_pages_per_seq]; seq_lens: int32 [batch]
  *   softmax_scale: <= 0 selects rsqrt(head_dim) (the reference's constant)
- *   num_splits:  context splits per sequence (flash-decoding); 0 = choose.
+ *   num_splits:  context splits per sequence (flash-decoding); 0 = choose
+ *                (no more than the workspace holds, where a coarser choice
+ *                fits it).
  *                Partials are merged in split order, so the result is
  *                bit-identical from run to run for a given num_splits.
  *   workspace:   fp32 scratch of at least
@@ -90,10 +92,14 @@ const char* cacheir_b200_error_string(int code);
  */
 size_t cacheir_b200_paged_attention_workspace_bytes(int batch_size, int num_heads,
                                                     int head_dim, int num_splits);
-/* The split count that num_splits == 0 resolves to for these extents. */
+/* The split count that num_splits == 0 resolves to for these extents, with enough workspace for it. */
 int cacheir_b200_paged_attention_auto_splits(int batch_size, int num_heads,
                                              int num_kv_heads, int max_pages_per_seq,
                                              int page_size, int head_dim);
+/* Kernels that one call launches for these extents (aligned, dense q): 2 where the splits are merged by a kernel of
+ * their own, 1 for a single split or splits that merge inside a thread-block cluster. */
+int cacheir_b200_paged_attention_launches(int batch_size, int num_heads, int num_kv_heads, int max_pages_per_seq,
+                                          int page_size, int head_dim, int dtype, int kv_dtype, int num_splits);
 int cacheir_b200_paged_attention_decode_batch(
     const void* q, const void* k_cache, const void* v_cache,
     const int32_t* page_table, const int32_t* seq_lens, void* out,
