@@ -337,18 +337,25 @@ int launch_epilogue(StreamParams p, bool swiglu, cudaStream_t stream) {
 
 struct Split { int rg, split; };
 // Row groups per CTA and CTAs along K: what the busiest SM has to take in, its weights and the activations that come with every
-// CTA, plus the exchange of a split (about a microsecond, 48 KB at an SM's share of the bandwidth) and the start of every further wave.
+// CTA, plus the exchange of a split and the start of every further wave. A cluster lives in one GPC, so that fewer of them run at
+// once than the SMs would hold: 33 of four CTAs and 15 of eight (sixteen take two turns: 2048 x 8192, 1 row, 13.2 us with eight
+// CTAs along K, 8.0 with four of half the rows). Four k blocks per CTA are enough to split (4096 x 2048, 32 rows: 12.5 us in one CTA
+// along K, 9.6 in four). Over 740 products of 512 to 28672 rows and 512 to 14336 columns the choice is 1.1 % behind the best
+// one, 17 % at most.
 Split choose_split(int weight_rows, int K, int m) {
+  constexpr struct { int split, at_once; } kForms[] = {{1, kNumSMs}, {2, kNumSMs / 2}, {3, 44}, {4, 32}, {6, 20}, {8, 14}};
   Split best{4, 1};
   long long best_cost = -1;
   for (int rg = 4; rg >= 1; rg /= 2)
-    for (int split = 1; split <= 8; split *= 2) {
-      if (split > 1 && K / kCols / split < 2 * k_groups(rg)) break;
-      const long long ctas = static_cast<long long>((weight_rows + 32 * rg - 1) / (32 * rg)) * split;
-      const long long bytes = static_cast<long long>(K / split) * (16 * rg + 2 * m);
-      const long long waves = (ctas + kNumSMs - 1) / kNumSMs;
-      const long long cost = waves * bytes + (waves - 1) * 96 * 1024 + (split > 1 ? 48 * 1024 : 0);
-      if (best_cost < 0 || cost < best_cost) { best = {rg, split}; best_cost = cost; }
+    for (const auto form : kForms) {
+      if (form.split > 1 && K / kCols / form.split < 4) break;
+      const int per_sm = rg == 1 ? 2 : 1;
+      const long long clusters = (weight_rows + 32 * rg - 1) / (32 * rg);
+      const long long waves = (clusters + form.at_once * per_sm - 1) / (form.at_once * per_sm);
+      const long long sharing = per_sm == 2 && clusters * form.split > kNumSMs ? 2 : 1;       // CTAs of an SM share its bandwidth
+      const long long bytes = sharing * (K / form.split) * (32 * rg + 5 * m) / 2;
+      const long long cost = waves * bytes + (waves - 1) * 96 * 1024 + (form.split > 1 ? 24 * 1024 : 0);
+      if (best_cost < 0 || cost < best_cost) { best = {rg, form.split}; best_cost = cost; }
     }
   return best;
 }
@@ -380,13 +387,18 @@ int launch_nt(const StreamParams& p, bool swiglu, cudaStream_t stream) {
 //     1280x8192 6.7 / 19, 8.7 / 19, 11.6 / 21; 2048x2048 4.5 / 8.7, 7.6 / 8.7, 10.5 / 10.1
 //   per-row int4, up to 8 rows, against the integer kernel: 1 row 14336x4096 13.6 / 17.0, 4096x4096 7.7 / 10.2, 2048x2048 4.3 / 8.1;
 //     at 16 rows 19.9 / 17.7, so no further
-// Codes in row order: the streaming int4 GEMV keeps the weights that fill all SMs with 64-row shares (14336x4096, 1 row: 17 / 15).
+// Codes in row order: the streaming int4 GEMV keeps the weights that fill all SMs with 64-row shares (14336x4096, 1 row: 17 / 15). On
+// smaller ones it is up to a tenth faster for group-wise codes of K <= 4096 in 5632 to 8192 rows (5632x2048, 1 row: 7.1 / 6.4), slower on the
+// others (4096x14336, 8 rows: 18.6 / 27.8), and its sums, which the constant 1024 of its operands leaves at the end, are a little less exact.
+// Per-row codes in tile order: more bands than SMs leave the second turn half empty, the integer kernel keeps them (28672x4096, 8 rows:
+// 27.4 / 24.1, the pre-pass included).
 bool qgemv_stream_supported(const QGemvParams& q) {
   if (q.x_dtype != CACHEIR_B200_F16 || q.x_prequantized || q.norm_weight) return false;
   if (q.M < 1 || q.M > (q.group_size > 0 ? 32 : 8) || q.K % 128 != 0 || q.K < 128) return false;
   if (q.bits != 4 || q.group_size % 128 != 0) return false;
   if (q.group_size > 0 && q.K / 128 * 128 * (q.scale_dtype == CACHEIR_B200_F16 ? 2 : 4) > kScaleLimit) return false;   // of 128 rows
   if (!q.tiled && q.N >= 64 * kNumSMs && qgemv_mma_supported(q)) return false;
+  if (q.tiled && q.group_size == 0 && q.N > 128 * kNumSMs) return false;
   const bool swiglu = q.epilogue == CACHEIR_B200_EPI_SWIGLU;
   if (q.epilogue == kEpiQkvRopeAppend) return false;
   if (q.paired && (q.group_size > 0 || !(swiglu && q.tiled && (q.N / 2) % 64 == 0))) return false;   // (group scales lie in logical row order)

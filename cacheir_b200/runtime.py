@@ -695,11 +695,15 @@ class _DecodePlan:
         """Will this projection run on the integer tensor cores (and so accept pre-quantized activations)?"""
         if swiglu and isinstance(weight, B200PackedWeight) and ((weight.shape[0] // 2) % 64 != 0 or (weight.tiled and not weight.paired)):
             return False
-        if isinstance(weight, B200PackedWeight) and weight.bits == 4 and self.batch <= 8:
-            return False                 # the streaming kernel takes fp16 rows as they are
         return (isinstance(weight, B200PackedWeight) and weight.bits in (4, 8) and not weight.group_size
                 and self.engine.dtype == torch.float16 and self.batch <= 64 and k % 128 == 0 and k <= 8192
-                and hasattr(self, "_gemm_ws"))
+                and hasattr(self, "_gemm_ws") and not self._streams(weight, ops.EPI_SWIGLU if swiglu else ops.EPI_NONE))
+
+    def _streams(self, weight: B200PackedWeight, epilogue: int) -> bool:
+        """Does the streaming kernel run this fp16 product? It takes the rows as they are, without a pre-pass."""
+        if weight.bits != 4 or weight.group_size or self.batch > 8 or weight.shape[1] % 128:
+            return False
+        return ops.qgemv_plan(self.batch, *weight.shape, bits=4, epilogue=epilogue, tiled=weight.tiled, paired=weight.paired)["family"] == "stream_int4"
 
     def _matmul(self, x: torch.Tensor, weight: B200PackedWeight | torch.Tensor, *, epilogue: int = ops.EPI_NONE,
                 residual: torch.Tensor | None = None, prequantized: bool = False, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -715,7 +719,7 @@ class _DecodePlan:
                                    workspace=ws, tiled=weight.tiled, prequantized=prequantized, paired=weight.paired)
             key = f"b200.qgemv.int{bits}" + (".swiglu" if epilogue == ops.EPI_SWIGLU else ".residual" if residual is not None else "")
             eng.gemm_plans[f"q{bits}:{(self.batch, 1, k)}x{weight.shape}"] = key
-            if ws is not None and k % 128 == 0 and k <= 32768 and not prequantized and (bits == 8 or self.batch > 8):   # activation pre-pass + integer GEMM per 64-row chunk
+            if ws is not None and k % 128 == 0 and k <= 32768 and not prequantized and not self._streams(weight, epilogue):   # activation pre-pass + integer GEMM per 64-row chunk
                 self._emit(fn, key, launches=2 * ((self.batch + 63) // 64))
                 return out
         else:
