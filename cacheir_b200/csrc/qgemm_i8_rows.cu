@@ -394,10 +394,11 @@ int launch_split(const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, const Row
 
 // Pairs along K, with at least four k blocks each: four for up to twelve tiles (sixteen clusters of eight CTAs do not run at
 // once: 100 rows of int8 4096 x 4096 30.0 us with four, 19.5 with two, 23.5 with one; 1280 x 8192 19.6, 32.7 with one), two
-// while the CTAs have an SM each (4096 x 14336 43.6 us with four, 32.6 with two, 47.5 with one).
+// for up to 33 (4096 x 14336 43.6 us with four, 32.6 with two, 47.5 with one; so many clusters of four CTAs run at once: 37 tiles
+// in two pairs each take two turns, 65 rows of int4 9344 x 4096 53.5 us, 9728 x 4096 in one pair each 36.5).
 int pairs_along_k(int tiles, int kblocks) {
   if (tiles <= 12 && kblocks >= 16) return 4;
-  return tiles * 4 <= kNumSMs && kblocks >= 8 ? 2 : 1;
+  return tiles <= 33 && kblocks >= 8 ? 2 : 1;
 }
 
 template <int BITS, bool SWIGLU>
@@ -426,10 +427,17 @@ bool qgemm_i8_rows_supported(const QGemvParams& q, const void* workspace, size_t
 // Against passes of 64 rows. A pair needs about 1 us for a k block of int4 codes, so that up to 128 rows with a long K and less
 // than half of the pairs at work are faster as two passes over all SMs: 100 rows of 4096 x 14336 56.5 us here, 54.6 in passes
 // (49 for up to 96 rows); 4096 x 4096 29.6 and 36.7, 1280 x 8192 27.4 and 29.8, 14336 x 4096 38 and 61. Bytes: 20 to 45 % faster here.
+// Up to 80 rows the second pass is a short one, and passes win from half as many k blocks on (65 rows of 1280 x 8192 27.7 and 25.1,
+// 4096 x 4096 28.9 and 27.5), unless their own clusters along K need two turns (2048 x 8192 27.9 and 35.6).
 bool qgemm_i8_rows_preferred(const QGemvParams& q) {
   if (q.bits == 8 || q.M > kRows) return true;
   const int tiles = (q.N + 2 * kRows - 1) / (2 * kRows), kblocks = q.K / kRows, split = pairs_along_k(tiles, kblocks);
-  return tiles * split * 4 >= kNumSMs || kblocks <= 16 * split;
+  if (tiles * split * 4 > kNumSMs) return true;
+  QGemvParams pass = q;
+  pass.M = 64;
+  const int bands = (q.N + kRows - 1) / kRows, along = qgemm_i8_plan(pass);
+  if (along * bands > (along == 8 ? 8 * 14 : along == 4 ? 4 * 32 : kNumSMs)) return true;
+  return q.M <= 80 ? kblocks < 8 * split || kblocks < 32 : kblocks <= 16 * split;
 }
 
 int launch_qgemm_i8_rows(const QGemvParams& q, const int* n_rows, void* workspace, cudaStream_t stream) {
