@@ -79,6 +79,16 @@ def test_prompt_attention_equals_the_rows_one_by_one(heads, kv_heads, dim):
     err = (out[:row].float() - want.float()).norm() / want.float().norm()
     assert float(err) <= 5e-4, float(err)
     assert bool((out[row:] == 7.0).all()) and _status() == 0
+    exact, at = [], 0                     # the same against 64-bit arithmetic: one such rounding less
+    for i, (a, n) in enumerate(parts):
+        slots = torch.from_numpy(table[i, :pages[i]]).long().cuda()
+        keys, values = (p[slots].transpose(1, 2).reshape(-1, kv_heads, dim)[:a + n].double().repeat_interleave(group, dim=1) for p in (k, v))
+        scores = torch.einsum("thd,shd->hts", q[at:at + n].double(), keys) * dim ** -0.5
+        later = torch.arange(a + n, device="cuda")[None, :] > a + torch.arange(n, device="cuda")[:, None]
+        exact.append(torch.einsum("hts,shd->thd", scores.masked_fill(later, -torch.inf).softmax(dim=2), values))
+        at += n
+    exact = torch.cat(exact)
+    assert float((out[:row].double() - exact).norm() / exact.norm()) <= 4e-4
 
 
 def test_rope_append_rows_equals_rope_append():
