@@ -62,6 +62,10 @@ extern "C" int cacheir_b200_dense_supported(int K, long long w_stride, long long
   return K > 0 && w_stride % 8 == 0 && x_stride % 8 == 0 && (batch <= 1 || x_batch_cols % 8 == 0) ? 1 : 0;
 }
 
+extern "C" int cacheir_b200_dense_pair_tokens(int T, int N, int K, int batch) {
+  return T > 0 && N > 0 && K > 0 && batch > 0 ? choose_pair(T, N, K, batch) : 0;
+}
+
 extern "C" int cacheir_b200_dense_gemm(const cacheir_b200_dense_args* args, void* stream) {
   if (!args) return CACHEIR_B200_EINVAL;
   cacheir_b200_dense_args p = *args;

@@ -69,6 +69,8 @@ typedef struct {
 /* Tensor-core GEMM Y = f(X W^T), bf16 operands. Strides must be multiples of 8 elements. */
 int cacheir_b200_dense_supported(int K, long long w_stride, long long x_stride, int batch, int x_batch_cols);
 int cacheir_b200_dense_gemm(const cacheir_b200_dense_args* args, void* stream);
+/* Tokens per tile of the CTA pairs that the product of these extents runs on, 0: single CTAs. Launches nothing. */
+int cacheir_b200_dense_pair_tokens(int T, int N, int K, int batch);
 
 /* The same product on the CUDA cores in true float32 arithmetic, any extents; y has type y_dtype. */
 int cacheir_b200_dense_simple(const void* x, const void* w, void* y, int T, int N, int K, int batch, int w_batch_rows,
