@@ -268,6 +268,15 @@ int launch_combine(const AttnParams& p, cudaStream_t stream) {
 
 }  // namespace
 
+namespace {
+// Do `splits` CTAs of the fast kernel merge inside a cluster, for `units` (sequence, kv head) pairs? All CTAs at once: a cluster's
+// short members would otherwise hold SMs that other sequences wait for. 33 clusters of four find an SM for every CTA, more put
+// two on some while others idle (37 requests of 3000 tokens, one kv head of 16 heads: 20.8 us, 16.9 with a merging kernel).
+bool cluster_pays(long long splits, long long units) {
+  return splits > 1 && splits <= kMaxClusterSplits && splits * units <= 2 * kNumSMs && !(splits == 4 && units > 33 && splits * units <= kNumSMs);
+}
+}  // namespace
+
 void resolve_attention_splits(int batch, int heads, int kv_heads, int max_pages, int page_size, long long room,
                               int requested, int* splits, int* chunk_tokens) {
   const long long max_ctx = static_cast<long long>(max_pages) * page_size;
@@ -287,11 +296,12 @@ void resolve_attention_splits(int batch, int heads, int kv_heads, int max_pages,
     const int cap = static_cast<int>((max_ctx + 255) / 256);
     if (s > cap) s = cap;
     // Up to eight splits that fit the GPU at once merge inside a thread-block cluster without a launch of their own, so
-    // that chunks down to one stage (64 tokens) pay. (Tables of up to 256 tokens keep one split, which can leave activation planes.)
+    // that chunks down to one stage (64 tokens) pay. They pay in the general kernel too, whose CTAs take longer over the same keys
+    // (float32, 1 request of 512 tokens, 32 heads of 128: 51.3 us in two splits, 18.5 in eight; pages of 32 in fp16 23.6 and 11.8). (Tables of up to 256 tokens keep one split, which can leave activation planes.)
     long long near = (max_ctx + 63) / 64;
     if (near > want) near = want;
     if (near > kMaxClusterSplits) near = kMaxClusterSplits;
-    if (s > 1 && near > s && near * units <= 2 * kNumSMs && near <= room) s = static_cast<int>(near);
+    if (s > 1 && near > s && cluster_pays(near, units) && near <= room) s = static_cast<int>(near);
   }
   if (s > kMaxAttentionSplits) s = kMaxAttentionSplits;
   if (s < 1) s = 1;
@@ -333,12 +343,6 @@ int i8_plane_rows(int M);
 }
 
 namespace {
-// Do the splits of the fast kernel merge inside a cluster? (All CTAs at once: a cluster's short members would otherwise hold
-// SMs that other sequences wait for.)
-bool merges_in_cluster(const AttnParams& p) {
-  return p.splits > 1 && p.splits <= kMaxClusterSplits && static_cast<long long>(p.splits) * p.kv_heads * p.batch <= 2 * kNumSMs;
-}
-
 // `gemm_workspace` non-null: the launch must also leave the output as the integer GEMM's activation planes
 // (CACHEIR_B200_EUNSUPPORTED when the fast single-split kernel cannot take the case). `probe`: decide only, launch nothing.
 int attention_dispatch(
@@ -402,7 +406,7 @@ int attention_dispatch(
                          (static_cast<long long>(head_dim) * kv_esize) % 8 == 0;
   int rc;
   if (paged_attention_fast_supported(p, dtype)) {
-    p.cluster = merges_in_cluster(p) ? 1 : 0;
+    p.cluster = cluster_pays(p.splits, static_cast<long long>(p.kv_heads) * p.batch) ? 1 : 0;
     rc = launch_paged_attention_fast(p, dtype, st);
     if (p.cluster) return rc;
   } else if (kv8) {
@@ -475,7 +479,7 @@ extern "C" int cacheir_b200_paged_attention_launches(int batch_size, int num_hea
   p.q_stride = static_cast<long long>(num_heads) * head_dim;
   resolve_attention_splits(batch_size, num_heads, num_kv_heads, max_pages_per_seq, page_size, kMaxAttentionSplits, num_splits, &p.splits,
                            &p.chunk_tokens);
-  return p.splits > 1 && !(paged_attention_fast_supported(p, dtype) && merges_in_cluster(p)) ? 2 : 1;
+  return p.splits > 1 && !(paged_attention_fast_supported(p, dtype) && cluster_pays(p.splits, static_cast<long long>(num_kv_heads) * batch_size)) ? 2 : 1;
 }
 
 extern "C" int cacheir_b200_paged_attention_decode_batch(

@@ -121,28 +121,50 @@ __device__ __forceinline__ void combine_in_cluster(const AttnParams& p, const fl
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
     return v;
   };
+  auto finish = [&](auto width) {                       // W neighbouring outputs of a head per thread
+    constexpr int W = decltype(width)::value;
+    for (int idx = W * (split * threads + static_cast<int>(threadIdx.x)); idx < p.group * D; idx += W * p.splits * threads) {
+      const int row = idx / D;
+      float m[8], l[8], part[8][W], m_tot = -INFINITY;   // all of them are requested before the first is used
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        m[s] = s < p.splits ? remote(s_max + row, s) : -INFINITY;
+        l[s] = s < p.splits ? remote(s_den + row, s) : 0.f;
+        if constexpr (W == 4) {
+          if (s < p.splits) {
+            uint32_t addr;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(s_out + idx)), "r"(s));
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(part[s][0]), "=f"(part[s][1]), "=f"(part[s][2]), "=f"(part[s][3]) : "r"(addr) : "memory");
+          } else {
+            part[s][0] = part[s][1] = part[s][2] = part[s][3] = 0.f;
+          }
+        } else {
+          part[s][0] = s < p.splits ? remote(s_out + idx, s) : 0.f;
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < 8; ++s) m_tot = fmaxf(m_tot, m[s]);
+      float l_tot = 0.f, o[W];
+#pragma unroll
+      for (int j = 0; j < W; ++j) o[j] = 0.f;
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const float w = m[s] == -INFINITY ? 0.f : exp2f(m[s] - m_tot);
+        l_tot = fmaf(l[s], w, l_tot);
+#pragma unroll
+        for (int j = 0; j < W; ++j) o[j] = fmaf(part[s][j], w, o[j]);
+      }
+      T* ob = static_cast<T*>(p.out) + static_cast<size_t>(b) * p.out_stride + static_cast<size_t>(kvh * p.group) * D + idx;
+#pragma unroll
+      for (int j = 0; j < W; ++j) Elem<T>::st(ob + j, l_tot > 0.f ? o[j] / l_tot : 0.f);
+    }
+  };
   cluster_sync_all();
-  for (int idx = split * threads + threadIdx.x; idx < p.group * D; idx += p.splits * threads) {
-    const int row = idx / D;
-    float m[8], l[8], part[8], m_tot = -INFINITY;        // all of them are requested before the first is used
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      m[s] = s < p.splits ? remote(s_max + row, s) : -INFINITY;
-      l[s] = s < p.splits ? remote(s_den + row, s) : 0.f;
-      part[s] = s < p.splits ? remote(s_out + idx, s) : 0.f;
-    }
-#pragma unroll
-    for (int s = 0; s < 8; ++s) m_tot = fmaxf(m_tot, m[s]);
-    float l_tot = 0.f, o = 0.f;
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      const float w = m[s] == -INFINITY ? 0.f : exp2f(m[s] - m_tot);
-      l_tot = fmaf(l[s], w, l_tot);
-      o = fmaf(part[s], w, o);
-    }
-    T* ob = static_cast<T*>(p.out) + static_cast<size_t>(b) * p.out_stride + static_cast<size_t>(kvh * p.group) * D;
-    Elem<T>::st(ob + idx, l_tot > 0.f ? o / l_tot : 0.f);
-  }
+  // One output per thread while that takes one round of remote loads, else four (18 requests of 270 tokens, eight heads for each of five kv
+  // heads, two splits: 10.9 us one by one, 9.4 by fours; partials in memory and a kernel that adds them up 10.3).
+  if (p.group * D <= p.splits * threads) finish(std::integral_constant<int, 1>{});
+  else finish(std::integral_constant<int, 4>{});
   cluster_sync_all();                                    // nobody's state is read any more
 }
 
