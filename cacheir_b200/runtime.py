@@ -22,7 +22,6 @@ cacheir/runtime/scheduler.py:508-577): `run`, `fork`, `run_decode_batch`,
 """
 from __future__ import annotations
 
-import gc
 import os
 
 from collections import OrderedDict
@@ -848,17 +847,12 @@ class _DecodePlan:
             graph = getattr(self, attr)
             if graph is None:
                 graph = torch.cuda.CUDAGraph()
-                collecting = gc.isenabled()
-                gc.disable()          # a collection that frees another plan's graph, event or pinned buffer would end the capture
-                try:
-                    with torch.cuda.graph(graph):
-                        for fn in self.program:
-                            fn()
-                        if feedback:
-                            self.feedback_tail()
-                finally:
-                    if collecting:
-                        gc.enable()
+                # (relaxed: a collection, here or in another thread, may free another plan's graph meanwhile; stricter modes end the capture then)
+                with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+                    for fn in self.program:
+                        fn()
+                    if feedback:
+                        self.feedback_tail()
                 setattr(self, attr, graph)
                 eng.graph_captures += 1
             graph.replay()

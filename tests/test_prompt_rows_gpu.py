@@ -1,4 +1,6 @@
 """The kernels of prompt passes (more than 64 rows of several sequences) against the 64-row kernels they extend."""
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -183,3 +185,24 @@ def test_prompt_pass_of_a_very_wide_model(quant):
     want = rt.run_prefill_batch([rt.fork(), rt.fork()], prompts)
     assert float((got.float() - want.float()).norm() / want.float().norm()) <= 2e-3
     rt.check_device_status()
+
+
+def test_a_collection_during_a_capture():
+    """Graphs of plans that nobody refers to any more are freed whenever the collector runs, which it may while a plan is captured."""
+    rt = _runtime()
+    session, other = rt.fork(), [rt.fork(), rt.fork()]
+    want = rt.run_decode_batch([session], [1]).clone()
+    for _ in range(2):                                     # the second step is captured
+        rt.run_decode_batch(other, [1, 1])
+    dropped = [rt._engine.plans.pop(("decode", 2))]        # (its launch list refers back to it: only the collector frees it)
+    enabled = []
+
+    def collect():
+        dropped.clear()
+        enabled.append(gc.isenabled())
+        gc.collect()
+    rt._engine.plans[("decode", 1)].program.insert(0, collect)
+    session.kv_cache.clear()
+    got = rt.run_decode_batch([session], [1])
+    assert torch.equal(got, want) and rt._engine.graph_captures == 2
+    assert enabled == [True] and gc.isenabled()
