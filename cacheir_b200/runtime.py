@@ -394,7 +394,7 @@ class _Engine:
             plan = make(max(needed_pages, (self.max_seq_len + self.page_size - 1) // self.page_size))
             self.plans_lowered += 1
             plans[key] = plan
-            while len(plans) > self.max_plans:
+            while len(plans) > (self.max_plans if plans is self.plans else 4 * self.max_plans):      # (prompt plans share their buffers)
                 plans.popitem(last=False)
         else:
             plans.move_to_end(key)

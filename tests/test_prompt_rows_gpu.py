@@ -206,3 +206,13 @@ def test_a_collection_during_a_capture():
     got = rt.run_decode_batch([session], [1])
     assert torch.equal(got, want) and rt._engine.graph_captures == 2
     assert enabled == [True] and gc.isenabled()
+
+
+def test_prompt_plans_of_every_size_stay():
+    """One plan per bucket of rows: lengths in turn make and capture each of them once."""
+    rt = _runtime(max_plans=3)
+    session, lengths = rt.fork(), (65, 129, 193, 257, 385)
+    for _ in range(3):
+        for n in lengths:
+            rt.run_prefill_batch([session], [[i % 640 for i in range(n)]])
+    assert (rt._engine.plans_lowered, rt._engine.graph_captures) == (len(lengths), len(lengths))
