@@ -405,6 +405,23 @@ class _Engine:
         size = min(bucket(rows), self.prompt_rows)
         return self._plan(("prompt", size), needed_pages, lambda width: _PromptPlan(self, size, width), self.prompt_plans)
 
+    def prompt_bytes(self) -> int:
+        """Device memory that the prompt plans share once the first of them is made."""
+        c = self.config
+        hidden, ff, attended = int(c.hidden_size), int(c.intermediate_size), int(c.num_attention_heads) * int(c.head_dim)
+        widths = {ff, attended, attended + 2 * int(c.num_key_value_heads) * int(c.head_dim), int(c.vocab_size)} - {hidden}
+        return self.prompt_rows * 2 * (5 * hidden + sum(widths)) + _PromptPlan.planes_bytes(self)
+
+    def release_prompt_plans(self) -> None:
+        """Give the memory of prompt passes back to the allocator (the next prompt makes its plan again)."""
+        if self.prompt_plans:
+            torch.cuda.synchronize(self.device)
+        for plan in self.prompt_plans.values():
+            plan.release()
+        self.prompt_plans.clear()
+        for role in [role for role in self._scratch if role.startswith("prompt")]:
+            del self._scratch[role]
+
     def prefill_plan(self, rows: int, needed_pages: int) -> "_DecodePlan":
         """The plan that pushes `rows` prompt tokens through the decode graph at once: row i is one (sequence,
         position) pair, reads that sequence's page table and attends to position+1 tokens."""
@@ -872,6 +889,11 @@ class _DecodePlan:
         if feedback:
             eng.count("b200.argmax_rows")
 
+    def release(self) -> None:
+        """Let go of what the launch list and its graphs hold (their closures refer back to the plan)."""
+        self.cuda_graph = self.feedback_graph = None
+        self.program, self.logits, self.feedback_tail = [], None, lambda: None
+
     def run_feedback_steps(self, steps: int) -> torch.Tensor:
         """`steps` greedy decode steps with the argmax fed back on the device (no host
         round trip between steps). Returns the generated tokens [steps, B]."""
@@ -923,10 +945,13 @@ class _PromptPlan(_DecodePlan):
         storage = self.engine.scratch(f"prompt{cols}.{turn}", self.engine.prompt_rows * cols * 2)
         return storage[: self.batch * cols * 2].view(torch.float16).view(self.batch, cols)
 
+    @staticmethod
+    def planes_bytes(engine: _Engine) -> int:
+        widest = max(w for w in (int(engine.config.hidden_size), int(engine.config.intermediate_size)) if w <= 32768)      # (see _by_row_blocks)
+        return ops.qgemv_workspace_bytes(engine.prompt_rows, widest)
+
     def _gemm_workspace(self, k: int) -> torch.Tensor:
-        config = self.engine.config
-        widest = max(w for w in (int(config.hidden_size), int(config.intermediate_size)) if w <= 32768)      # (see _by_row_blocks)
-        return self.engine.scratch("prompt.planes", ops.qgemv_workspace_bytes(self.engine.prompt_rows, widest))
+        return self.engine.scratch("prompt.planes", self.planes_bytes(self.engine))
 
     @staticmethod
     def _by_row_blocks(weight: Any, swiglu: bool = False) -> bool:
@@ -1101,6 +1126,11 @@ class B200DecodeRuntime:
         limit = float(self.memory_limit_mb)
         if float(torch.cuda.memory_allocated(self.device)) / (1024.0 * 1024.0) <= limit:
             return
+        if self._engine.prompt_plans:              # what costs nobody a token goes first
+            self._engine.release_prompt_plans()
+            torch.cuda.empty_cache()
+            if float(torch.cuda.memory_allocated(self.device)) / (1024.0 * 1024.0) <= limit:
+                return
         self._recover_from_oom()
         after = float(torch.cuda.memory_allocated(self.device)) / (1024.0 * 1024.0)
         if after > limit:
@@ -1113,7 +1143,25 @@ class B200DecodeRuntime:
         self.oom_recoveries += 1
         self.kv_cache.clear()
         self._engine.validated_batch = None
+        self._engine.release_prompt_plans()
         torch.cuda.empty_cache()
+
+    def _pass_rows(self, tokens: int) -> int:
+        """Prompt tokens that a pass of this step takes: `pass_rows`, or as many as the decode plan takes where the buffers of
+        longer passes would not fit the memory or the session's limit."""
+        eng = self._engine
+        rows = eng.pass_rows or DECODE_PASS_ROWS
+        if not eng.prompt_rows or min(rows, tokens) <= DECODE_PASS_ROWS:
+            return rows
+        try:
+            if self.memory_limit_mb is None or eng.prompt_plans or \
+                    torch.cuda.memory_allocated(self.device) + eng.prompt_bytes() <= float(self.memory_limit_mb) * 1024 * 1024:
+                eng.prompt_plan(min(rows, tokens), 0)
+                return rows
+        except torch.cuda.OutOfMemoryError:
+            eng.release_prompt_plans()
+            torch.cuda.empty_cache()
+        return DECODE_PASS_ROWS
 
     def _check_positions(self, sessions) -> None:
         """The cos/sin table and the page-table width cover `max_seq_len` positions; a longer sequence would read
@@ -1246,7 +1294,7 @@ class B200DecodeRuntime:
         if mode == "prefill" and chunk > 1 and len(tokens) > chunk // 4:
             self._enforce_memory_limit()
             try:
-                return self._prefill_chunked(tokens, self._engine.pass_rows)
+                return self._prefill_chunked(tokens)
             except (torch.cuda.OutOfMemoryError, KVPoolExhausted) as exc:
                 self._recover_from_oom()
                 raise RuntimeError("CacheIR CUDA runtime recovered from an out-of-memory condition; "
@@ -1292,7 +1340,7 @@ class B200DecodeRuntime:
             session.kv_cache.extend(len(tokens))
         results = []
         with torch.cuda.device(self.device):
-            passes = cut_passes(token_batches, eng.pass_rows or DECODE_PASS_ROWS, None if eng.ragged else _PromptPlan.SEQUENCES)
+            passes = cut_passes(token_batches, self._pass_rows(sum(map(len, token_batches))), None if eng.ragged else _PromptPlan.SEQUENCES)
             for part in passes:                                   # (session, first token, last token + 1)
                 want = [(i, int(p)) for i, lo, hi in part for p in wanted[i] if lo <= int(p) < hi]
                 logits = self._run_rows(sessions, token_batches, starts, part, want)
@@ -1334,7 +1382,8 @@ class B200DecodeRuntime:
             plan = eng.prompt_plan(rows, needed)
             plan.sync_parts(parts)
         else:
-            plan = eng.prefill_plan(eng.prefill_chunk or DECODE_PASS_ROWS, needed)
+            size = eng.prefill_chunk or DECODE_PASS_ROWS
+            plan = eng.prefill_plan(size if rows > DECODE_PASS_ROWS else min(size, DECODE_PASS_ROWS), needed)
             plan.sync_prefill_rows([(cache, start + i, int(t)) for cache, start, tokens in parts for i, t in enumerate(tokens)])
         plan.run_program()
         return plan.logits[:rows]
@@ -1356,8 +1405,8 @@ class B200DecodeRuntime:
             if free is not None and need > free:
                 raise KVPoolExhausted(f"the step needs {need} new state slots, {free} are free")
 
-    def _prefill_chunked(self, tokens: list[int], chunk: int) -> torch.Tensor:
-        """Prefill that fills the page pool directly, `chunk` prompt tokens per pass through the decode
+    def _prefill_chunked(self, tokens: list[int]) -> torch.Tensor:
+        """Prefill that fills the page pool directly, `pass_rows` prompt tokens per pass through the decode
         graph (cuda.py:584-629 computes the same thing with a causal mask over contiguous copies): the
         tokens of a chunk are the rows of one batched step -- the projections see a [chunk, hidden] matrix,
         every row appends its K/V at its own position and attends, through the sequence's own page table,
@@ -1366,14 +1415,19 @@ class B200DecodeRuntime:
         cache = self.kv_cache
         vocab = int(eng.config.vocab_size)
         out = torch.empty((1, len(tokens), vocab), device=self.device, dtype=self.dtype)
+        passes = 0
         with torch.cuda.device(self.device):
-            for c0 in range(0, len(tokens), chunk):
-                part = tokens[c0:c0 + chunk]
+            for c0 in range(0, len(tokens), eng.pass_rows):
+                part = tokens[c0:c0 + eng.pass_rows]
                 start = cache.tokens
                 cache.extend(len(part))
                 self._check_positions([self])
-                out[0, c0:c0 + len(part)] = self._run_prompt_rows([(cache, start, part)])
-        eng.count("cacheir.b200_prefill_chunk", (len(tokens) + chunk - 1) // chunk)
+                rows = self._pass_rows(len(part))
+                for lo in range(0, len(part), rows):
+                    piece = part[lo:lo + rows]
+                    out[0, c0 + lo:c0 + lo + len(piece)] = self._run_prompt_rows([(cache, start + lo, piece)])
+                    passes += 1
+        eng.count("cacheir.b200_prefill_chunk", passes)
         return out
 
     def _prefill_packed(self, sessions: list["B200DecodeRuntime"], token_id_batches: list[list[int]], out: torch.Tensor) -> None:
@@ -1387,7 +1441,7 @@ class B200DecodeRuntime:
             session.kv_cache.extend(len(ids))                  # reserves the pages of the whole prompt
         self._check_positions(sessions)
         with torch.cuda.device(self.device):
-            passes = cut_passes(token_id_batches, eng.pass_rows, _PromptPlan.SEQUENCES)
+            passes = cut_passes(token_id_batches, self._pass_rows(sum(map(len, token_id_batches))), _PromptPlan.SEQUENCES)
             for part in passes:                                # (sequence, first token, last token + 1)
                 logits = self._run_prompt_rows([(sessions[i].kv_cache, starts[i] + lo, token_id_batches[i][lo:hi]) for i, lo, hi in part])
                 for (i, lo, hi), rows in zip(part, logits.split([hi - lo for _, lo, hi in part])):

@@ -216,3 +216,56 @@ def test_prompt_plans_of_every_size_stay():
         for n in lengths:
             rt.run_prefill_batch([session], [[i % 640 for i in range(n)]])
     assert (rt._engine.plans_lowered, rt._engine.graph_captures) == (len(lengths), len(lengths))
+
+
+def _prefilled(rt, sessions=None):
+    prompts = [list(range(200)), [9] * 70]
+    sessions = sessions or [rt.fork() for _ in prompts]
+    logits = rt.run_prefill_batch(sessions, prompts)
+    return torch.cat([logits[i, :len(p)] for i, p in enumerate(prompts)]).float(), rt.run_decode_batch(sessions, [1, 2]).float().clone()
+
+
+def _near(a, b):
+    return all(float((x - y).norm() / y.norm()) <= 2e-3 for x, y in zip(a, b))
+
+
+def test_prompts_that_leave_no_room_for_long_passes(monkeypatch):
+    """Where the buffers of a long pass cannot be had, prompts go through passes of the decode plan, as they do for other models."""
+    from cacheir_b200 import runtime
+
+    rt = _runtime()
+    want = _prefilled(rt)
+    assert rt._engine.prompt_plans
+    other = _runtime()
+
+    def refuse(*args):
+        raise torch.cuda.OutOfMemoryError("no room")
+    monkeypatch.setattr(runtime._PromptPlan, "_make_buffers", refuse)
+    assert _near(_prefilled(other), want) and not other._engine.prompt_plans and other.oom_recoveries == 0
+    one = other.fork().run([list(range(200))], mode="prefill")[0].float()
+    assert float((one - want[0][:200]).norm() / want[0][:200].norm()) <= 2e-3
+
+
+def test_prompt_memory_under_a_limit():
+    """A session's limit counts the buffers of long passes: they are not made where they do not fit, and given back before any session
+    loses its tokens."""
+    rt = _runtime()
+    want = _prefilled(rt)
+    held = torch.cuda.memory_allocated()
+    rt._recover_from_oom()
+    freed = held - torch.cuda.memory_allocated()
+    assert not rt._engine.prompt_plans and freed >= 0.9 * rt._engine.prompt_bytes()
+    assert _near(_prefilled(rt), want) and rt._engine.prompt_plans          # (made again)
+    rt._engine.release_prompt_plans()
+    tight = [rt.fork() for _ in range(2)]
+    room = torch.cuda.memory_allocated() + rt._engine.prompt_bytes() / 2
+    for session in tight:
+        session.memory_limit_mb = room / 2 ** 20
+    rt.memory_limit_mb = room / 2 ** 20
+    assert _near(_prefilled(rt, tight), want) and not rt._engine.prompt_plans
+    rt.memory_limit_mb = None
+    _prefilled(rt)
+    rt.memory_limit_mb = (torch.cuda.memory_allocated() - rt._engine.prompt_bytes() / 4) / 2 ** 20
+    before, recovered = [s.kv_cache.tokens for s in tight], rt.oom_recoveries
+    rt.run_decode_batch(tight, [3, 4])
+    assert not rt._engine.prompt_plans and rt.oom_recoveries == recovered and [s.kv_cache.tokens for s in tight] == [n + 1 for n in before]
