@@ -240,7 +240,7 @@ int qgemv_dispatch(const void* x, const void* norm_weight, float norm_eps, const
   // More than 64 rows of per-row codes in tile order, with scratch for all of them: one launch over blocks of 128 rows (the same
   // bits as the 64-row passes below, which stream the weights once per 64 rows: 100 rows of 14336 x 4096 bytes 25.6 us against 45.6).
   if (M > 64 && qgemm_i8_rows_supported(p, workspace, workspace_bytes) && (p.x_prequantized || qgemm_i8_rows_preferred(p)))
-    return plan_only ? (1 << 8) | 1 : launch_qgemm_i8_rows(p, nullptr, workspace, st);
+    return plan_only ? 1 << 8 : launch_qgemm_i8_rows(p, nullptr, workspace, st);
   if (M > 64 && !p.x_prequantized && !norm_weight) {
     // The integer tensor-core kernel takes up to 64 batch rows per launch, the fp16 one up to 128. A taller
     // batch runs as chunks of that height (the weights stream once per chunk, still far cheaper than the
@@ -263,7 +263,7 @@ int qgemv_dispatch(const void* x, const void* norm_weight, float norm_eps, const
       return 0;
     }
   }
-  if (qgemv_stream_supported(p)) return plan_only ? (4 << 8) : launch_qgemv_stream(p, st);
+  if (qgemv_stream_supported(p)) return plan_only ? (4 << 8) | qgemv_stream_plan(p) : launch_qgemv_stream(p, st);
   // up to 8 batch rows of int4 codes in row order: the streaming GEMV reads every code once and needs no pre-pass
   if (qgemv_mma_supported(p)) return plan_only ? (4 << 8) : launch_qgemv_mma(p, st);
   if (qgemm_i8_supported(p, workspace, workspace_bytes))

@@ -49,6 +49,7 @@ int launch_qgemv_mma(const QGemvParams& p, cudaStream_t stream);
 // Streaming dequant-GEMV for up to 32 rows (warp MMAs on codes unpacked in registers; both code layouts).
 bool qgemv_stream_supported(const QGemvParams& p);
 int launch_qgemv_stream(const QGemvParams& p, cudaStream_t stream);
+int qgemv_stream_plan(const QGemvParams& p);   // (row groups << 4) | CTAs along K that the launcher would choose
 
 // Tensor-core (tcgen05) small-M GEMM: weights are the 128-row MMA operand.
 bool qgemm_tc_supported(const QGemvParams& p);

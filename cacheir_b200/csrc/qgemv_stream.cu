@@ -406,6 +406,11 @@ bool qgemv_stream_supported(const QGemvParams& q) {
   return aligned_to(q.packed, 16) && aligned_to(q.x, 16) && (q.x_stride * 2) % 16 == 0;
 }
 
+int qgemv_stream_plan(const QGemvParams& q) {
+  const Split s = choose_split(q.N, q.K, q.M);
+  return (s.rg << 4) | s.split;
+}
+
 int launch_qgemv_stream(const QGemvParams& q, cudaStream_t stream) {
   const bool swiglu = q.epilogue == CACHEIR_B200_EPI_SWIGLU;
   StreamParams p{};

@@ -241,8 +241,9 @@ int cacheir_b200_rmsnorm_qgemv(const void* x, const void* norm_weight, float eps
                                size_t workspace_bytes, void* stream);
 
 /* Which kernel cacheir_b200_qgemv_ex would launch for these extents and flags (fp16 activations, aligned
- * pointers): (family << 8) | detail, family 1 = integer tensor core with detail = its split-K factor,
- * 2 = fp16 tensor core, 3 = CUDA cores, 4 = streaming int4 GEMV (up to 32 rows); epilogue 3 asks about
+ * pointers): (family << 8) | detail, family 1 = integer tensor core with detail = its split-K factor (0: blocks of 128
+ * rows in one launch), 2 = fp16 tensor core, 3 = CUDA cores, 4 = streaming int4 product with detail = (row groups << 4) |
+ * CTAs along K (0: the GEMV for many weight rows in row order); epilogue 3 asks about
  * cacheir_b200_qkv_rope_append. Negative:
  * the validation code the call would return. Launches nothing. No counterpart in the reference (its
  * kernel choice is the declarative `attrs["kernel"]`, cacheir/passes/transformer.py:391-424). */
