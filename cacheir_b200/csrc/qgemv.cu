@@ -239,7 +239,8 @@ int qgemv_dispatch(const void* x, const void* norm_weight, float norm_eps, const
   cudaStream_t st = as_stream(stream);
   // More than 64 rows of per-row codes in tile order, with scratch for all of them: one launch over blocks of 128 rows (the same
   // bits as the 64-row passes below, which stream the weights once per 64 rows: 100 rows of 14336 x 4096 bytes 25.6 us against 45.6).
-  if (M > 64 && qgemm_i8_rows_supported(p, workspace, workspace_bytes) && (p.x_prequantized || qgemm_i8_rows_preferred(p)))
+  // (Rows that are in the workspace already: cacheir_b200_qgemm_rows.)
+  if (M > 64 && !p.x_prequantized && qgemm_i8_rows_supported(p, workspace, workspace_bytes) && qgemm_i8_rows_preferred(p))
     return plan_only ? 1 << 8 : launch_qgemm_i8_rows(p, nullptr, workspace, st);
   if (M > 64 && !p.x_prequantized && !norm_weight) {
     // The integer tensor-core kernel takes up to 64 batch rows per launch, the fp16 one up to 128. A taller

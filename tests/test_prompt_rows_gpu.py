@@ -269,3 +269,14 @@ def test_prompt_memory_under_a_limit():
     before, recovered = [s.kv_cache.tokens for s in tight], rt.oom_recoveries
     rt.run_decode_batch(tight, [3, 4])
     assert not rt._engine.prompt_plans and rt.oom_recoveries == recovered and [s.kv_cache.tokens for s in tight] == [n + 1 for n in before]
+
+
+def test_more_than_64_prequantized_rows_are_refused():
+    """`quantize_activations` fills a workspace for up to 64 rows; more of them are `qgemm_rows`' business, after `rms_norm_quantize_rows`."""
+    from cacheir_b200 import _lib, ops
+
+    for bits in (8, 4):
+        ops.qgemv_plan(64, 1024, 1024, bits=bits, tiled=True, prequantized=True)
+        for rows in (65, 128, 300):
+            with pytest.raises(_lib.CacheIRB200Error):
+                ops.qgemv_plan(rows, 1024, 1024, bits=bits, tiled=True, prequantized=True)
