@@ -78,7 +78,7 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   float* s_up = reinterpret_cast<float*>(s_raw + (BITS == 4 ? S * kTile / 2 : 0));    // [half][2][kChunk][64]
   int4* s_row = reinterpret_cast<int4*>(s_up + 4 * kChunk * kPairHalf);               // [2][128] (scale, sum >> 8, sum & 255, sum)
   uint64_t* full = reinterpret_cast<uint64_t*>(s_row + 2 * kRows);   // [S] (even CTA) operands of both CTAs have landed
-  uint64_t* empty = full + S;                // [S] the MMAs that read the stage have retired (int4: and the groups that pass it over have seen it)
+  uint64_t* empty = full + S;                // [S] the MMAs that read the stage have retired
   uint64_t* raw_full = empty + S;            // [S] int4: this CTA's nibble tile has landed
   uint64_t* ready = raw_full + S;            // [S] int4 (even CTA): the byte tiles of both CTAs are written
   uint64_t* acc_full = ready + S;            // [2]
@@ -102,7 +102,7 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   if (warp == 0 && lane == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(smem_u32(&full[s]), 1);
-      mbar_init(smem_u32(&empty[s]), BITS == 4 ? 1 + 4 * (kConverterGroups - 1) : 1);
+      mbar_init(smem_u32(&empty[s]), 1);
       mbar_init(smem_u32(&raw_full[s]), 1);
       mbar_init(smem_u32(&ready[s]), 8);          // four converter warps of each CTA
     }
@@ -316,16 +316,15 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     const int steps = tiles > pair ? ((tiles - pair - 1) / pairs + 1) * kblocks : 0;
     bool ok = true;
     const int group = (warp - 10) >> 2;
-    // Every group waits for every stage: a barrier's parity only tells neighbouring phases apart. The stage is filled again once
-    // its group has handed its bytes to the MMAs and the others have said that they saw it, so that no phase is missed.
-    for (int it = 0; it < steps; ++it) {
+    // A barrier's parity only tells neighbouring phases apart. A group therefore waits for its own stages alone, first until the MMAs
+    // have retired that read the place before (the copy behind which this group's last stage came had waited for the use before that one), then
+    // for the bytes. Neither barrier can move on without this group's conversion, so that no phase is missed, however late the group looks.
+    static_assert(kConverterGroups < S, "a group's last stage was copied after the place's last one");
+    for (int it = group; it < steps; it += kConverterGroups) {
       const int s = it % S;
-      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&raw_full[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 6));
+      ok = __all_sync(0xffffffffu, (it < S || mbar_wait(smem_u32(&empty[s]), ((it / S) & 1) ^ 1, &g_i8_rows_status, (6 << 8) | 9)) &&
+                                       mbar_wait(smem_u32(&raw_full[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 6));
       if (!ok) break;
-      if (it % kConverterGroups != group) {
-        if (lane == 0) mbar_arrive(smem_u32(&empty[s]));
-        continue;
-      }
       const uint8_t* raw_row = s_raw + s * (kTile / 2) + r * (kRows / 2);
       uint8_t* out_row = s_w + s * kTile + r * kRows;
       uint4 raw[4];
