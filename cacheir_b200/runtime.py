@@ -24,7 +24,7 @@ from __future__ import annotations
 
 import os
 
-from collections import OrderedDict
+from collections import Counter, OrderedDict
 from pathlib import Path
 from typing import Any, Callable, Iterable
 
@@ -220,8 +220,45 @@ class _Engine:
                                                         or (int(node.attrs["num_heads"]), int(node.attrs["num_kv_heads"]), int(node.attrs["head_dim"]))
                                                         != (heads, kv_heads, head_dim)):
                 return 0
+        if not self._operands_recent(nodes):
+            return 0
         rows = min(2048, (1 << 27) // int(c.vocab_size) // 128 * 128)
         return rows if rows >= 128 else 0
+
+    def _operands_recent(self, nodes: list[Any]) -> bool:
+        """Is every operand still in its buffer when a prompt plan reads it? Of the residual's width the plan's products take
+        `_PromptPlan.TURNS` buffers in turn, of every other width there is one (`_PromptPlan._buf`)."""
+        c = self.config
+        hidden = int(c.hidden_size)
+        taken: dict[int, int] = {}                     # buffers of a width taken so far
+        made: dict[str, tuple[int, int]] = {}          # activation -> (its width, taken[width] with its own)
+        uses = Counter([name for node in nodes for name in node.inputs] + list(self.graph.outputs))
+
+        def take(width: int) -> tuple[int, int]:
+            taken[width] = taken.get(width, 0) + 1
+            return width, taken[width]
+        prior = None
+        for node in nodes:
+            if node.op == "quantized_fused_rmsnorm_qkv_rope":
+                take(hidden)                           # the norm, where it is not part of the projection
+                out = take(sum(self.weight_rows(name) for name in node.inputs[2:5]))
+            elif node.op == "paged_attention_decode":
+                out = take(int(c.num_attention_heads) * int(c.head_dim))
+            elif node.op == "quantized_matmul":
+                out = take(self.weight_rows(node.inputs[1]))
+            elif node.op == "quantized_fused_swiglu":
+                out = take(self.weight_rows(node.inputs[1]))
+            elif (node.op == "add" and prior is not None and prior.op == "quantized_matmul" and prior.outputs[0] in node.inputs
+                  and uses[prior.outputs[0]] == 1 and node.inputs[0] != node.inputs[1]):
+                out = made[prior.outputs[0]]           # the residual epilogue of that product
+            else:
+                out = take(hidden)
+            for name in node.inputs:
+                if name in made and taken[made[name][0]] - made[name][1] >= (_PromptPlan.TURNS if made[name][0] == hidden else 1):
+                    return False
+            made.update(dict.fromkeys(node.outputs, out))
+            prior = node
+        return all(taken[made[name][0]] == made[name][1] for name in self.graph.outputs if name in made)
 
     def weight_rows(self, name: str) -> int:
         spec = self.graph.weights[name]
@@ -914,6 +951,7 @@ class _PromptPlan(_DecodePlan):
 
     decodes = False
     SEQUENCES = 256      # of one pass: the page tables' room
+    TURNS = 5            # buffers of the residual's width
 
     def __init__(self, engine: _Engine, batch: int, width: int):
         config = engine.config
@@ -939,9 +977,9 @@ class _PromptPlan(_DecodePlan):
 
     def _buf(self, cols: int) -> torch.Tensor:
         """Shared by all plans and layers. Of the residual's width five take turns (an operand is at most four products old),
-        of the other widths one value is alive at a time."""
+        of the other widths one value is alive at a time: `_Engine._operands_recent` has checked it."""
         turn = self._turn.get(cols, 0)
-        self._turn[cols] = (turn + 1) % (5 if cols == int(self.engine.config.hidden_size) else 1)
+        self._turn[cols] = (turn + 1) % (self.TURNS if cols == int(self.engine.config.hidden_size) else 1)
         storage = self.engine.scratch(f"prompt{cols}.{turn}", self.engine.prompt_rows * cols * 2)
         return storage[: self.batch * cols * 2].view(torch.float16).view(self.batch, cols)
 

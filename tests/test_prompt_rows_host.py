@@ -16,6 +16,7 @@ def _engine(edit=lambda graph: None, **changes):
     engine = SimpleNamespace(graph=artifact.graph("decode"), config=artifact.config, dtype=torch.float16, quant="int8", page_size=16,
                              tp=SimpleNamespace(enabled=False))
     engine.weight_rows = lambda name: _Engine.weight_rows(engine, name)
+    engine._operands_recent = lambda nodes: _Engine._operands_recent(engine, nodes)
     return engine
 
 
@@ -28,6 +29,28 @@ def test_models_that_take_them():
 
 def _nodes(graph, op):
     return [node for node in graph.nodes if node.op == op]
+
+
+def _late_residual(graph):      # the embedding joins again behind the last layer: the plan's buffer of it has been taken since
+    add = _nodes(graph, "add")[-1]
+    add.inputs[0] = "hidden_0"
+
+
+def _late_gate(graph):          # the second layer's down projection reads the first layer's gated values
+    _nodes(graph, "quantized_matmul")[3].inputs[0] = _nodes(graph, "quantized_fused_swiglu")[0].outputs[0]
+
+
+@pytest.mark.parametrize("edit", [_late_residual, _late_gate])
+def test_graphs_that_read_an_older_value_than_the_plan_keeps(edit):
+    """Prompt plans share a few buffers between all layers; graphs that reach further back keep passes of 64 rows, whose plan holds all values."""
+    assert _Engine._prompt_rows(_engine(edit), "same") == 0
+
+
+def test_widths_that_meet():
+    """A gated width, or the vocabulary, of the residual's width."""
+    assert _Engine._prompt_rows(_engine(intermediate_size=512), "same") == 2048
+    assert _Engine._prompt_rows(_engine(vocab_size=512), "same") == 2048
+    assert _Engine._prompt_rows(_engine(vocab_size=768, intermediate_size=768), "same") == 2048
 
 
 def _wider_values(graph):       # value heads of another width than the key heads
