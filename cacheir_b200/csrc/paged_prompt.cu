@@ -107,7 +107,7 @@ paged_prompt_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
       const int page = next;
       if (lane < kStagePages && first + kStagePages + lane < pages) next = table[first + kStagePages + lane];
       if (lane == 0) {
-        ok = it < kStages || mbar_wait(smem_u32(&empty[s]), ((it / kStages) & 1) ^ 1, &g_prompt_status, (7 << 8) | 1);
+        ok = it < kStages || mbar_wait(smem_u32(&empty[s]), ((it / kStages) & 1) ^ 1, &g_prompt_status, (13 << 8) | 1);
         if (ok) mbar_expect_tx(smem_u32(&full[s]), count * kPageBytes);
       }
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -122,7 +122,7 @@ paged_prompt_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
     // nothing may still be on its way when the block ends (a consumer's wait may have given up); lane 0 copies in every stage
     if (lane == 0)
       for (int it = issued > kStages ? issued - kStages : 0; it < issued; ++it)
-        if (!mbar_wait(smem_u32(&full[it % kStages]), (it / kStages) & 1, &g_prompt_status, (7 << 8) | 4)) break;
+        if (!mbar_wait(smem_u32(&full[it % kStages]), (it / kStages) & 1, &g_prompt_status, (13 << 8) | 4)) break;
     return;
   }
 
@@ -132,7 +132,7 @@ paged_prompt_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
   if (first_row >= tokens * p.group) {             // nothing for this warp: it only keeps the ring moving
     for (int it = 0; it < iters; ++it) {
       const int s = it % kStages;
-      const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&full[s]), (it / kStages) & 1, &g_prompt_status, (7 << 8) | 2));
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&full[s]), (it / kStages) & 1, &g_prompt_status, (13 << 8) | 2));
       if (!ok) break;
       if (lane == 0) mbar_arrive(smem_u32(&empty[s]));
     }
@@ -166,7 +166,7 @@ paged_prompt_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
   bool ok = true;
   for (int it = 0; it < iters; ++it) {
     const int s = it % kStages;
-    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&full[s]), (it / kStages) & 1, &g_prompt_status, (7 << 8) | 3));
+    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&full[s]), (it / kStages) & 1, &g_prompt_status, (13 << 8) | 3));
     if (!ok) break;
     const int count = min(kStagePages, warp_pages - it * kStagePages);     // pages of the stage this warp looks at
     if (count > 0) {

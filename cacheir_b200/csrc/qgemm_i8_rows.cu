@@ -128,7 +128,7 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         const int band = t / row_blocks * 2 + static_cast<int>(rank), block = t % row_blocks;
         for (int kb = 0; kb < kblocks; ++kb, ++it) {
           const int s = it % S;
-          if (it >= S && !mbar_wait(smem_u32(&empty[s]), ((it / S) & 1) ^ 1, &g_i8_rows_status, (6 << 8) | 1)) { ok = false; break; }
+          if (it >= S && !mbar_wait(smem_u32(&empty[s]), ((it / S) & 1) ^ 1, &g_i8_rows_status, (12 << 8) | 1)) { ok = false; break; }
           const uint32_t bar = map_to_rank(smem_u32(&full[s]), first);
           if (rank == 0) mbar_expect_tx(smem_u32(&full[s]), BITS == 8 ? 4 * kTile : 2 * kTile);
           // (a band beyond the last one, where their number is odd, reads as zero)
@@ -145,8 +145,8 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       }
       // Nothing may still be on its way when the blocks end: a wait elsewhere may have given up. (The even CTA sees the copies of both.)
       for (int i = it > S ? it - S : 0; i < it; ++i) {
-        if (rank == 0 && !mbar_wait(smem_u32(&full[i % S]), (i / S) & 1, &g_i8_rows_status, (6 << 8) | 7)) break;
-        if (BITS == 4 && !mbar_wait(smem_u32(&raw_full[i % S]), (i / S) & 1, &g_i8_rows_status, (6 << 8) | 8)) break;
+        if (rank == 0 && !mbar_wait(smem_u32(&full[i % S]), (i / S) & 1, &g_i8_rows_status, (12 << 8) | 7)) break;
+        if (BITS == 4 && !mbar_wait(smem_u32(&raw_full[i % S]), (i / S) & 1, &g_i8_rows_status, (12 << 8) | 8)) break;
       }
     }
   } else if (warp == 1) {
@@ -158,13 +158,13 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       bool ok = true;
       for (int t = pair; t < tiles && ok; t += pairs, ++n) {
         const int a = n & 1;
-        if (n >= 2 && !mbar_wait(smem_u32(&acc_empty[a]), ((n >> 1) & 1) ^ 1, &g_i8_rows_status, (6 << 8) | 2)) break;
+        if (n >= 2 && !mbar_wait(smem_u32(&acc_empty[a]), ((n >> 1) & 1) ^ 1, &g_i8_rows_status, (12 << 8) | 2)) break;
         tc_fence_after();
         const uint32_t d = tmem_base + a * kAccCols;
         for (int kb = 0; kb < kblocks; ++kb, ++it) {
           const int s = it % S;
-          if (!mbar_wait(smem_u32(&full[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 3)) { ok = false; break; }
-          if (BITS == 4 && !mbar_wait(smem_u32(&ready[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 4)) { ok = false; break; }
+          if (!mbar_wait(smem_u32(&full[s]), (it / S) & 1, &g_i8_rows_status, (12 << 8) | 3)) { ok = false; break; }
+          if (BITS == 4 && !mbar_wait(smem_u32(&ready[s]), (it / S) & 1, &g_i8_rows_status, (12 << 8) | 4)) { ok = false; break; }
           tc_fence_after();
           const uint32_t w = smem_u32(s_w + s * kTile), x = smem_u32(s_x + s * kTile);
 #pragma unroll
@@ -204,7 +204,7 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       const int zero_int = zero_is_int ? __float2int_rn(zero) : 0;
       const bool all_int = __all_sync(0xffffffffu, zero_is_int);
       asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueThreads) : "memory");
-      ok = ok && mbar_wait(smem_u32(&acc_full[a]), (n >> 1) & 1, &g_i8_rows_status, (6 << 8) | 5);
+      ok = ok && mbar_wait(smem_u32(&acc_full[a]), (n >> 1) & 1, &g_i8_rows_status, (12 << 8) | 5);
       col_ok = col_ok && ok;
       __syncwarp();
       tc_fence_after();
@@ -322,8 +322,8 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     static_assert(kConverterGroups < S, "a group's last stage was copied after the place's last one");
     for (int it = group; it < steps; it += kConverterGroups) {
       const int s = it % S;
-      ok = __all_sync(0xffffffffu, (it < S || mbar_wait(smem_u32(&empty[s]), ((it / S) & 1) ^ 1, &g_i8_rows_status, (6 << 8) | 9)) &&
-                                       mbar_wait(smem_u32(&raw_full[s]), (it / S) & 1, &g_i8_rows_status, (6 << 8) | 6));
+      ok = __all_sync(0xffffffffu, (it < S || mbar_wait(smem_u32(&empty[s]), ((it / S) & 1) ^ 1, &g_i8_rows_status, (12 << 8) | 9)) &&
+                                       mbar_wait(smem_u32(&raw_full[s]), (it / S) & 1, &g_i8_rows_status, (12 << 8) | 6));
       if (!ok) break;
       const uint8_t* raw_row = s_raw + s * (kTile / 2) + r * (kRows / 2);
       uint8_t* out_row = s_w + s * kTile + r * kRows;

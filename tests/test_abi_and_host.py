@@ -38,6 +38,15 @@ def test_library_exports_every_declared_symbol():
     assert 1 <= s <= 64
 
 
+def test_status_words_name_one_kernel_file():
+    """A status word is (class << 8) | wait: the class says whose wait gave up, so no two files share one."""
+    owners: dict[str, set[str]] = {}
+    for path in sorted((ROOT / "cacheir_b200" / "csrc").glob("*.cu*")):
+        for number in re.findall(r"&g_\w+_status, (?:0, )?\((\d+) << 8\)", path.read_text()):
+            owners.setdefault(number, set()).add(path.stem)
+    assert len(owners) >= 12 and all(len(files) == 1 for files in owners.values()), owners
+
+
 def test_ops_refuse_cpu_tensors():
     import torch
     from cacheir_b200 import ops
