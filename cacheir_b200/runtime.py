@@ -1047,7 +1047,10 @@ class _PromptPlan(_DecodePlan):
             count = len(tokens)
             at = np.arange(start, start + count, dtype=np.int32)
             table[i] = cache.page_table_row(self.width)
-            ids[row:row + count] = tokens
+            try:
+                ids[row:row + count] = tokens
+            except (TypeError, ValueError):            # (tokens that only `int` reads, such as elements of a CUDA tensor)
+                ids[row:row + count] = [int(t) for t in tokens]
             positions[row:row + count] = at
             pages[row:row + count] = table[i][at // self.engine.page_size]
             first = np.arange(0, count, step, dtype=np.int32)
@@ -1508,8 +1511,8 @@ class B200DecodeRuntime:
             return out
         chunk = self._engine.prefill_chunk
         if chunk > 1 and sum(lens) > chunk // 4:
-            # Packed prefill: the prompt tokens of all sequences are the rows of 64-row passes through the decode
-            # graph, sequence after sequence, so short prompts share a pass and a long prompt spans several.
+            # Packed prefill: the prompt tokens of all sequences are the rows of passes through the decode graph (up to
+            # `pass_rows` each), sequence after sequence, so short prompts share a pass and a long prompt spans several.
             self._enforce_memory_limit()
             try:
                 self._prefill_packed(sessions, token_id_batches, out)

@@ -280,3 +280,13 @@ def test_more_than_64_prequantized_rows_are_refused():
         for rows in (65, 128, 300):
             with pytest.raises(_lib.CacheIRB200Error):
                 ops.qgemv_plan(rows, 1024, 1024, bits=bits, tiled=True, prequantized=True)
+
+
+def test_prompts_as_tensors():
+    """Token batches may be anything whose elements `int` reads, a CUDA tensor among them."""
+    rt = _runtime()
+    prompts = [list(range(90)), [5] * 20]
+    want = rt.run_prefill_batch([rt.fork(), rt.fork()], prompts)
+    assert rt.kernel_counts["b200.paged_attention_prompt"] > 0
+    for form in (lambda p: torch.tensor(p, device="cuda"), lambda p: list(torch.tensor(p, device="cuda")), lambda p: np.array(p), tuple):
+        assert torch.equal(rt.run_prefill_batch([rt.fork(), rt.fork()], [form(p) for p in prompts]), want)
