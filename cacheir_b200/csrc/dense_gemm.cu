@@ -4,16 +4,18 @@
 namespace cb200 {
 namespace {
 
-// Tokens from which pairs are chosen: below, a tile of 256 weight rows leaves the last turn emptier than K split over single CTAs
-// (whole prompts of width 4096, 330 tokens: 2877 us on single CTAs, 3064 on pairs; 1944 and 1982; 230 tokens 1603 and 1574;
-// 2048 tokens 6155 and 5432, 1001 of width 2048 1773 and 1715).
+// Tokens from which pairs are chosen: below, a tile of 256 weight rows often leaves the last turn emptier than K split over single
+// CTAs. Measured over whole prompts of width 4096, single CTAs and pairs: 230 tokens 1603 and 1574 us, 330 tokens 2877 and 3064, another
+// family 1944 and 1982; 2048 tokens 6155 and 5432; 1001 tokens of width 2048 1773 and 1715. Nothing between 330 and 1001 tokens
+// was measured, and the line takes no account of N and K.
 constexpr int kPairTokens = 768;
 
 struct Shape { int mt, split; };
 Shape choose_shape(int T, int N, int K, int batch) {
   const int n_tiles = (N + kTileN - 1) / kTileN * batch;
   int mt = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : 128;
-  // (products per head with a short K are all epilogue: two CTAs per SM take turns. 32 heads of 128 x 512, 2048 tokens: 87 to 54 us)
+  // (products per head with a short K are all epilogue: two CTAs per SM take turns. 32 heads of 128 x 512, 2048 tokens: 87 to 54 us;
+  // fewer tokens than the line keep tiles of 256: not measured)
   if (T >= 256 && !(batch > 1 && K <= 1024 && T >= kPairTokens) && n_tiles * ((T + 255) / 256) >= kNumSMs) mt = 256;
   const int tiles = n_tiles * ((T + mt - 1) / mt);
   const int kblocks = (K + kBlockK - 1) / kBlockK;

@@ -368,8 +368,8 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 // By itself a CTA takes 48 KB from L2 per 512 tensor-core cycles (128 weight rows x 256 tokens, k 64), and nothing runs under its
 // epilogue: 2048 x 28672 x 4096 was 403 us, 1.19 PFLOP/s. A pair (cta_group::2) shares the token tile, 32 KB per CTA for the same
 // cycles, and its accumulator takes half of tensor memory, so that the epilogue of one tile runs under the next one's main loop. Pairs
-// walk the tiles with the tokens innermost: the weights in flight come from HBM once, the tokens stay in L2. The order of the sums is the
-// same.
+// walk the tiles with the tokens innermost: the weights in flight come from HBM once, the tokens stay in L2. A tile's sum is one chain
+// along K, as on single CTAs that do not split K (where those did, their parts are now one chain: still float32, other last bits).
 __host__ __device__ constexpr int pair_stage_bytes(int tt) { return kWBytes + tt / 2 * kBlockK * 2; }
 __host__ __device__ constexpr int pair_stages(int tt) { return tt == 256 ? 6 : 8; }
 

@@ -4,7 +4,7 @@
 //
 // Why not tcgen05 here: its weight operand comes through shared memory at about 37 bytes per clock and SM whatever the number
 // of activation rows, after int4 codes have been inflated to 16 (bytes) or 32 KB (fp16) per 128 x 128 tile that takes 440 or 880
-// cycles, where HBM delivers the tile's 8 KB in 350. mma.sync takes the weights from registers, where a few byte permutes
+// cycles, where HBM delivers the tile's 8 KB in 350 (bytes would need their sums scaled per k block to serve group scales). mma.sync takes the weights from registers, where a few byte permutes
 // turn codes into exact fp16 integers (code - zero), so nothing is written back to shared memory; its price, 64 MMAs per eight activation rows
 // and tile of 4 cycles each, is 256 to 1024 cycles. No activation pre-pass.
 //

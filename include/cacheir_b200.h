@@ -216,7 +216,10 @@ int cacheir_b200_qgemv(const void* x, const void* packed, const void* scales,
  * other layouts, and a workspace that only holds 64 rows, as
  * 64-row chunks (128-row chunks on the fp16 tensor-core kernel, which takes 65..128 rows in
  * one launch with the activations as the 128-row operand). Other shapes ignore the
- * workspace. workspace may be NULL (then this is cacheir_b200_qgemv). The workspace is only used during the call's own kernels; two
+ * workspace. Which kernel runs depends on the extents (cacheir_b200_qgemv_plan), and the kernels sum in different orders and
+ * forms: int4 rows of up to 8 (group-wise 32) run on exact fp16 activations with float32 sums, taller batches per row on 16-bit
+ * fixed point with exact integer sums, so the last bits of a row may change with the number of rows beside it (and, group-wise,
+ * for a last chunk of up to 32 rows behind chunks of 128). workspace may be NULL (then this is cacheir_b200_qgemv). The workspace is only used during the call's own kernels; two
  * calls that may overlap on the GPU need separate workspaces. */
 size_t cacheir_b200_qgemv_workspace_bytes(int M, int K);
 int cacheir_b200_qgemv_ex(const void* x, const void* packed, const void* scales,
@@ -453,7 +456,8 @@ int cacheir_b200_qgemm_rows(const void* x, const void* packed, const void* scale
                             int scale_dtype, long long x_stride, int epilogue, int weight_layout, void* workspace,
                             size_t workspace_bytes, void* stream);
 /* RoPE on q and k of dense fp16 rows [M][q_dim + 2*k_dim] by the table of cacheir_b200_rope_table; the rotated k and the v
- * go to pool slot pages[row] at positions[row] % page_size. Afterwards only the q columns of the rows are defined. */
+ * go to pool slot pages[row] at positions[row] % page_size. Afterwards only the q columns of the rows are defined. A row whose
+ * position lies outside the table is left as it is, and appends nothing. */
 int cacheir_b200_rope_append_rows(void* qkv, const int32_t* positions, const int32_t* pages, const int32_t* n_rows,
                                   const float* rope_table, int rope_table_positions, void* k_cache, void* v_cache, int M,
                                   int q_dim, int k_dim, int head_dim, int num_slots, int page_size, void* stream);
