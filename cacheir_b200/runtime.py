@@ -772,8 +772,10 @@ class _DecodePlan:
                                    workspace=ws, tiled=weight.tiled, prequantized=prequantized, paired=weight.paired)
             key = f"b200.qgemv.int{bits}" + (".swiglu" if epilogue == ops.EPI_SWIGLU else ".residual" if residual is not None else "")
             eng.gemm_plans[f"q{bits}:{(self.batch, 1, k)}x{weight.shape}"] = key
-            if ws is not None and k % 128 == 0 and k <= 32768 and not prequantized and not self._streams(weight, epilogue):   # activation pre-pass + integer GEMM per 64-row chunk
-                self._emit(fn, key, launches=2 * ((self.batch + 63) // 64))
+            if ws is not None and k % 128 == 0 and k <= 32768 and not prequantized and not self._streams(weight, epilogue):
+                # activation pre-pass + integer GEMM, for all rows at once or per chunk of 64
+                plan = ops.qgemv_plan(self.batch, n, k, bits=bits, epilogue=epilogue, tiled=weight.tiled, paired=weight.paired)
+                self._emit(fn, key, launches=2 if plan["kernel"] == "i8_rows" else 2 * ((self.batch + 63) // 64))
                 return out
         else:
             n, k = int(weight.shape[0]), int(weight.shape[1])

@@ -290,3 +290,19 @@ def test_prompts_as_tensors():
     assert rt.kernel_counts["b200.paged_attention_prompt"] > 0
     for form in (lambda p: torch.tensor(p, device="cuda"), lambda p: list(torch.tensor(p, device="cuda")), lambda p: np.array(p), tuple):
         assert torch.equal(rt.run_prefill_batch([rt.fork(), rt.fork()], [form(p) for p in prompts]), want)
+
+
+@pytest.mark.parametrize("quant, batch", [("int8", 3), ("int8", 70), ("int4_awq", 5), ("int4_awq", 70), ("int4_awq", 130)])
+def test_launches_of_a_decode_step(quant, batch):
+    """What a plan counts per step is what runs (a product of more than 64 rows: its pre-pass and one kernel, not one per 64 rows)."""
+    rt = _runtime(quant)
+    sessions = [rt.fork() for _ in range(batch)]
+    rt.run_decode_batch(sessions, [1] * batch)
+    plan = rt._engine.plans[("decode", batch)]
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as profile:
+        for fn in plan.program:
+            fn()
+        torch.cuda.synchronize()
+    kernels = [e.name for e in profile.events() if e.device_type == torch.autograd.DeviceType.CUDA and not e.name.startswith("Mem")]
+    assert len(kernels) == plan.launches_per_step, kernels
