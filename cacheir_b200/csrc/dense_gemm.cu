@@ -4,10 +4,9 @@
 namespace cb200 {
 namespace {
 
-// Tokens from which pairs are chosen: below, a tile of 256 weight rows often leaves the last turn emptier than K split over single
+// Tokens from which pairs are considered: below, a tile of 256 weight rows often leaves the last turn emptier than K split over single
 // CTAs. Measured over whole prompts of width 4096, single CTAs and pairs: 230 tokens 1603 and 1574 us, 330 tokens 2877 and 3064, another
-// family 1944 and 1982; 2048 tokens 6155 and 5432; 1001 tokens of width 2048 1773 and 1715. Nothing between 330 and 1001 tokens
-// was measured, and the line takes no account of N and K.
+// family 1944 and 1982; 2048 tokens 6155 and 5432. Nothing between 331 and 767 tokens was measured.
 constexpr int kPairTokens = 768;
 
 struct Shape { int mt, split; };
@@ -25,7 +24,27 @@ Shape choose_shape(int T, int N, int K, int batch) {
   return {mt, split};
 }
 
-// Tokens per tile of a CTA pair, 0: single CTAs.
+// Time of the product in nanoseconds on pairs (tiles of 256 weight rows x `tt` tokens) and on single CTAs: a turn is the k blocks of a
+// tile plus its epilogue, of which pairs show only what the next tile's main loop does not cover. Fitted to 325 plain products of
+// 768 to 2048 tokens, 512 to 22016 rows and K of 512 to 8192, timed on both forms; 3 to 7 % off (standard deviation).
+long long pair_cost(int T, int N, int K, int batch, int tt) {
+  const long long tiles = static_cast<long long>((T + tt - 1) / tt) * ((N + 2 * kTileN - 1) / (2 * kTileN)) * batch;
+  const long long turns = (tiles + kNumSMs / 2 - 1) / (kNumSMs / 2), kblocks = (K + kBlockK - 1) / kBlockK;
+  return tt == 256 ? 7300 + turns * (300 * kblocks + 4600) : 6000 + turns * (300 * kblocks + 1700);
+}
+
+long long single_cost(int T, int N, int K, int batch) {
+  const Shape s = choose_shape(T, N, K, batch);
+  const long long ctas = static_cast<long long>((T + s.mt - 1) / s.mt) * ((N + kTileN - 1) / kTileN) * batch * s.split;
+  const long long turns = (ctas + kNumSMs - 1) / kNumSMs, kblocks = ((K + kBlockK - 1) / kBlockK + s.split - 1) / s.split;
+  if (s.mt == 256) return 900 + turns * (350 * kblocks + 8900);
+  return s.split > 1 ? 2400 + turns * (195 * kblocks + 4800) : 1600 + turns * (195 * kblocks + 3100);
+}
+
+// Tokens per tile of a CTA pair, 0: single CTAs. Pairs only where they come out ahead: taken for all of those 325 products they were
+// up to 1.35 times slower (1153 x 1024 x 8192 46.2 us, on single CTAs that split K 34.3; 1001 x 4096 x 512 14.0 and 10.9, where the
+// epilogue is most of it), up to 1.6 times faster (2048 x 14336 x 2048 94.9 and 144.1). By cost the 325 take 4.9 % less time than on
+// pairs alone and 12.1 % less than on single CTAs alone (geometric means), 0.1 % more than the better form of each (9 % at most).
 int choose_pair(int T, int N, int K, int batch) {
   if (T < kPairTokens || (batch > 1 && (K <= 1024 || N % (2 * kTileN) != 0))) return 0;
   auto cost = [&](int tt) {          // turns of the busiest pair, in tiles of 128 tokens (a narrow tile asks more of L2)
@@ -34,7 +53,8 @@ int choose_pair(int T, int N, int K, int batch) {
   };
   const long long tiles = static_cast<long long>((T + 127) / 128) * ((N + 2 * kTileN - 1) / (2 * kTileN)) * batch;
   if (tiles < kNumSMs / 4) return 0;          // few tiles: single CTAs that split K
-  return cost(256) <= cost(128) ? 256 : 128;
+  const int tt = cost(256) <= cost(128) ? 256 : 128;
+  return pair_cost(T, N, K, batch, tt) <= single_cost(T, N, K, batch) ? tt : 0;
 }
 
 template <int EPI>
