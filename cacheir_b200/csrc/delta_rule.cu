@@ -36,6 +36,7 @@ __device__ __forceinline__ void delta_gates(const Args& a, size_t row, int h, fl
 template <typename T>
 __global__ void __launch_bounds__(256)
 delta_simple_kernel(const Args a) {
+  chain_enter();
   extern __shared__ float sm[];
   float* s_state = sm;                       // [dim][32]
   float* s_k = s_state + a.dim * 32;         // [dim]
@@ -106,6 +107,7 @@ delta_simple_kernel(const Args a) {
 template <typename T, int THREADS, int HELD>
 __global__ void __launch_bounds__(THREADS)
 delta_step_kernel(const Args a, const T* __restrict__ gate, long long gate_stride, const float* __restrict__ w, float eps) {
+  chain_enter();
   __shared__ float4 s_red[2][THREADS];
   __shared__ float s_sum[32];
   extern __shared__ float s_kq[];           // [2][dim] unit key, unit query
@@ -216,6 +218,7 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t* hi, uint3
 
 __global__ void __launch_bounds__(128)
 delta_local_kernel(const Args a, const ChunkSpace ws) {
+  chain_enter();
   extern __shared__ __align__(16) uint8_t raw[];
   constexpr int kPitch = kChunk + 4;
   const int dim = a.dim, pitch = dim + 8;
@@ -406,6 +409,7 @@ constexpr int kChainThreads = 256;
 template <int NT>
 __global__ void __launch_bounds__(kChainThreads)
 delta_chain_kernel(const Args a, const ChunkSpace ws) {
+  chain_enter();
   constexpr int kCols = NT * 8, kPitchC = kCols + 8;
   extern __shared__ __align__(16) uint8_t raw[];
   const int dim = a.dim, pitch = dim + 8;
@@ -652,7 +656,7 @@ int launch_simple(const Args& a, cudaStream_t st) {
   if (smem > 200 * 1024) return CACHEIR_B200_ELIMIT;
   const cudaError_t e = cudaFuncSetAttribute(delta_simple_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  delta_simple_kernel<T><<<dim3(a.segments, a.heads, (a.vdim + 31) / 32), 256, smem, st>>>(a);
+  launch_chained(delta_simple_kernel<T>, dim3(a.segments, a.heads, (a.vdim + 31) / 32), 256, smem, st, a);
   return launch_status();
 }
 
@@ -662,7 +666,7 @@ int launch_step(const Args& a, const void* gate, long long gate_stride, const fl
   const size_t smem = static_cast<size_t>(a.dim) * 8;
   const int per_row = a.vdim / 4;
 #define CB200_DELTA_STEP(THREADS, HELD) \
-  delta_step_kernel<T, THREADS, HELD><<<grid, THREADS, smem, st>>>(a, static_cast<const T*>(gate), gate_stride, w, eps)
+  launch_chained(delta_step_kernel<T, THREADS, HELD>, grid, THREADS, smem, st, a, static_cast<const T*>(gate), gate_stride, w, eps)
   if (a.dim <= 256 / per_row * 4) CB200_DELTA_STEP(256, 4);
   else if (a.dim <= 256 / per_row * 16) CB200_DELTA_STEP(256, 16);
   else CB200_DELTA_STEP(512, 16);
@@ -677,7 +681,7 @@ int launch_chain(const Args& a, const ChunkSpace& ws, cudaStream_t st) {
   const size_t smem = (static_cast<size_t>(4) * kChunk * (a.dim + 8) + static_cast<size_t>(2) * (a.dim + 3 * kChunk) * kPitchC) * 2 + 2 * kChunk * 16;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  kern<<<dim3(a.segments, a.heads, (a.vdim + kCols - 1) / kCols), kChainThreads, smem, st>>>(a, ws);
+  launch_chained(kern, dim3(a.segments, a.heads, (a.vdim + kCols - 1) / kCols), kChainThreads, smem, st, a, ws);
   return launch_status();
 }
 
@@ -734,7 +738,7 @@ extern "C" int cacheir_b200_delta_chunked(const cacheir_b200_delta_args* args, v
   const size_t smem = static_cast<size_t>(2) * kChunk * (a.dim + 8) * 2 + (static_cast<size_t>(2) * kChunk * (kChunk + 4) + 32 * 36) * 4;
   const cudaError_t e = cudaFuncSetAttribute(delta_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  delta_local_kernel<<<dim3(items, a.heads), 128, smem, st>>>(a, ws);
+  launch_chained(delta_local_kernel, dim3(items, a.heads), 128, smem, st, a, ws);
   const int rc = launch_status();
   if (rc != 0) return rc;
   // narrow column blocks while all of them still run at once

@@ -35,6 +35,7 @@ constexpr int kTileN = 128;
 constexpr int kBlockK = 64;               // elements of k per stage: one 128-byte swizzle span
 constexpr int kWBytes = kTileN * kBlockK * 2;
 constexpr int kThreads = 320;
+constexpr int kAhead = 8;                 // weight tiles a CTA asks for before its turn
 constexpr int kTailBytes = 512;                    // barriers; from byte 128 on the places of up to 64 rows
 
 __device__ int g_dense_status = 0;
@@ -213,6 +214,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const int krank = static_cast<int>(blockIdx.y);      // the cluster spans the whole y extent
   int t0 = blockIdx.x * MT, t_end = p.T, z = blockIdx.z / n_tiles;
   if constexpr (GROUPED) {
+    chain_wait();
     const RaggedItem it = find_item(groups.cu, p.batch, groups.place_of ? 1 << 30 : MT, blockIdx.x);
     if (it.seg < 0) return;                // (the whole cluster)
     z = it.seg; t0 = it.row0; t_end = it.row0 + it.count;
@@ -224,15 +226,24 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const int total = kblocks_all * (krank + 1) / split - kb_begin;
 
   if (warp == 0 && lane == 0) {
+    if constexpr (!GROUPED) {              // the weights set out for L2 while the kernel before this one is at work
+      if (blockIdx.x == 0)
+        for (int i = 0; i < min(total, kAhead); ++i) tma_prefetch_2d(&tmap_w, (kb_begin + i) * kBlockK, z * p.w_batch_rows + n0);
+    }
     for (int s = 0; s < kStages; ++s) { mbar_init(smem_u32(&full[s]), 1); mbar_init(smem_u32(&empty[s]), 1); }
     mbar_init(smem_u32(acc_full), 1);
     mbar_fence_init();
   }
-  if (warp == 1) tc_alloc(smem_u32(tmem_slot), tmem_cols(MT));
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  __syncthreads();                         // the barriers exist
+  if constexpr (!GROUPED) chain_wait();
+  chain_next();
+  if (warp > 0) {                          // (the copies do not wait for tensor memory)
+    if (warp == 1) tc_alloc(smem_u32(tmem_slot), tmem_cols(MT));
+    tc_fence_before();
+    asm volatile("bar.sync 3, %0;" ::"n"(kThreads - 32) : "memory");
+    tc_fence_after();
+  }
+  const uint32_t tmem = warp > 0 ? *tmem_slot : 0u;
 
   // epilogue thread: output column n of this batch entry, tokens `half`-interleaved
   const int q = warp & 3;
@@ -408,6 +419,7 @@ dense_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     for (int a = 0; a < 2; ++a) { mbar_init(smem_u32(&acc_full[a]), 1); mbar_init(smem_u32(&acc_empty[a]), 16); }
     mbar_fence_init();
   }
+  chain_enter();
   if (warp == 1) tc_alloc_pair(smem_u32(tmem_slot), 2 * TT);
   tc_fence_before();
   __syncthreads();
@@ -526,19 +538,8 @@ int launch(const cacheir_b200_dense_args& p, int split, cudaStream_t stream, con
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem));
   if (e != cudaSuccess) return static_cast<int>(e);
   const int n_tiles = (p.N + kTileN - 1) / kTileN;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = GROUPED ? dim3((groups.place_of ? 0 : p.T / MT) + (p.T < p.batch ? p.T : p.batch), split, n_tiles) : dim3((p.T + MT - 1) / MT, split, n_tiles * p.batch);
-  cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = kSmem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = split;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = split > 1 ? 1 : 0;
-  e = cudaLaunchKernelEx(&cfg, kern, tw, tx, p, n_tiles, groups);
+  const dim3 grid = GROUPED ? dim3((groups.place_of ? 0 : p.T / MT) + (p.T < p.batch ? p.T : p.batch), split, n_tiles) : dim3((p.T + MT - 1) / MT, split, n_tiles * p.batch);
+  e = launch_clusters(kern, grid, kThreads, kSmem, stream, dim3(1, split, 1), tw, tx, p, n_tiles, groups);
   if (e != cudaSuccess) return static_cast<int>(e);
   return launch_status();
 }
@@ -557,7 +558,7 @@ int launch_pair(const cacheir_b200_dense_args& p, cudaStream_t stream) {
   if (e != cudaSuccess) return static_cast<int>(e);
   const long long tiles = static_cast<long long>((p.T + TT - 1) / TT) * ((p.N + 2 * kTileN - 1) / (2 * kTileN)) * p.batch;
   const int pairs = tiles < kNumSMs / 2 ? static_cast<int>(tiles) : kNumSMs / 2;
-  kern<<<2 * pairs, kThreads, kSmem, stream>>>(tw, tx, p);
+  launch_chained(kern, 2 * pairs, kThreads, kSmem, stream, tw, tx, p);
   return launch_status();
 }
 

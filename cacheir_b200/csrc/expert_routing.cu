@@ -102,6 +102,7 @@ __global__ void __launch_bounds__(kRouteThreads)
 route_kernel(const float* __restrict__ logits, long long stride, const int32_t* __restrict__ row_seg, int rows, int experts, int top,
              const cacheir_b200_route_rule rule, int32_t* counters, int32_t* __restrict__ cu, int32_t* __restrict__ token_of, int32_t* place_of,
              float* __restrict__ weight, int32_t* chosen) {
+  chain_enter();
   extern __shared__ int s_first[];      // [experts + 1] (SOFTMAX: then a warp's choice scores, and its groups' best)
   __shared__ int s_sum[kRouteThreads / 32];
   __shared__ bool s_last;
@@ -162,6 +163,7 @@ __global__ void __launch_bounds__(kRouteThreads)
 place_kernel(int rows, int experts, int top, int32_t* counters, int32_t* __restrict__ cu, int32_t* __restrict__ token_of,
              int32_t* __restrict__ place_of, const int32_t* __restrict__ chosen, const uint4* __restrict__ x, uint4* __restrict__ placed,
              int pieces) {
+  chain_enter();
   extern __shared__ int s_count[];      // [experts], then [top] places
   __shared__ bool s_last;
   int* s_place = s_count + experts;
@@ -208,6 +210,7 @@ template <typename T, int VEC, bool SAVED>
 __global__ void __launch_bounds__(512)
 combine_kernel(float* __restrict__ x, const T* __restrict__ y, const int32_t* __restrict__ place_of, const float* __restrict__ weight, int top,
                const T* __restrict__ shared, const float* __restrict__ w, float eps, int width, T* next_out) {
+  chain_enter();
   extern __shared__ float s_m[];
   __shared__ float scratch[32];
   const size_t row = blockIdx.x;
@@ -256,6 +259,7 @@ __global__ void __launch_bounds__(512)
 combine_add_kernel(float* x, const T* __restrict__ y, const int32_t* __restrict__ place_of, const float* __restrict__ weight, int top,
                    const T* self, const T* __restrict__ shared, const float* __restrict__ shared_gate, long long shared_gate_stride, int width,
                    RowNext nx) {
+  chain_enter();
   __shared__ float scratch[32];
   const size_t row = blockIdx.x;
   float own = 0.f;                      // weight of the token itself
@@ -314,7 +318,7 @@ extern "C" int cacheir_b200_route(const float* logits, long long stride, const i
   cudaStream_t st = as_stream(stream);
   const bool held = scored <= 32 * kHeld;
 #define CB200_ROUTE(HELD, PLACE, SOFTMAX)                                                                                              \
-  route_kernel<HELD, PLACE, SOFTMAX><<<blocks, kRouteThreads, PLACE || SOFTMAX ? first + choices : 0, st>>>(                            \
+  launch_chained(route_kernel<HELD, PLACE, SOFTMAX>, blocks, kRouteThreads, PLACE || SOFTMAX ? first + choices : 0, st,                             \
       logits, stride, row_seg, rows, experts, top, *rule, counters, cu, token_of, place_of, weight, chosen)
 #define CB200_ROUTE_RULE(PLACE)                          \
   if (rule->softmax && held) CB200_ROUTE(true, PLACE, true);      \
@@ -328,7 +332,7 @@ extern "C" int cacheir_b200_route(const float* logits, long long stride, const i
   CB200_ROUTE_RULE(false);
 #undef CB200_ROUTE_RULE
 #undef CB200_ROUTE
-  place_kernel<<<rows, kRouteThreads, smem, st>>>(rows, experts, top, counters, cu, token_of, place_of, chosen, static_cast<const uint4*>(x),
+  launch_chained(place_kernel, rows, kRouteThreads, smem, st, rows, experts, top, counters, cu, token_of, place_of, chosen, static_cast<const uint4*>(x),
                                                   static_cast<uint4*>(placed), row_bytes / 16);
   return launch_status();
 }
@@ -345,7 +349,7 @@ extern "C" int cacheir_b200_combine_residual_rms(float* residual, const void* y,
   const bool saved = width <= 11 * 1024;
   const size_t smem = saved ? static_cast<size_t>(width) * 4 : 0;
 #define CB200_COMBINE(VEC, SAVED)                                                                                              \
-  combine_kernel<T, VEC, SAVED><<<rows, 512, smem, as_stream(stream)>>>(residual, static_cast<const T*>(y), place_of, weight, top, \
+  launch_chained(combine_kernel<T, VEC, SAVED>, rows, 512, smem, as_stream(stream), residual, static_cast<const T*>(y), place_of, weight, top, \
                                                                        static_cast<const T*>(shared), w, eps, width, static_cast<T*>(out))
   CB200_HYBRID_DTYPE(dtype, {
     if (vec && saved) CB200_COMBINE(4, true);
@@ -367,7 +371,7 @@ extern "C" int cacheir_b200_combine_residual(float* residual, const void* y, con
   const bool vec = width % 4 == 0 && aligned_to(residual, 16) && aligned_to(y, 16) && aligned_to(self, 16) && aligned_to(shared, 16) &&
                    row_next_aligned(next_mode, next_w, next_out);
 #define CB200_COMBINE(VEC)                                                                                                                 \
-  combine_add_kernel<T, VEC><<<rows, 512, 0, as_stream(stream)>>>(residual, static_cast<const T*>(y), place_of, weight, top,                \
+  launch_chained(combine_add_kernel<T, VEC>, rows, 512, 0, as_stream(stream), residual, static_cast<const T*>(y), place_of, weight, top,                \
                                                                  static_cast<const T*>(self), static_cast<const T*>(shared), shared_gate, \
                                                                  shared_gate_stride, width, nx)
   CB200_HYBRID_DTYPE(dtype, {

@@ -16,6 +16,7 @@ template <typename T, int VEC, int PER_THREAD>
 __global__ void __launch_bounds__(256)
 rms_norm_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ weight,
                 T* __restrict__ sum_out, T* __restrict__ out, int hidden, float eps) {
+  chain_enter();
   __shared__ float red[8];
   const size_t row = blockIdx.x;
   const T* xr = x + row * hidden;
@@ -69,6 +70,7 @@ __global__ void __launch_bounds__(256)
 rms_norm_generic_kernel(const T* __restrict__ x, const T* __restrict__ residual,
                         const T* __restrict__ weight, T* __restrict__ sum_out, T* __restrict__ out,
                         int hidden, float eps) {
+  chain_enter();
   __shared__ float red[8];
   const size_t row = blockIdx.x;
   float ss = 0.f;
@@ -105,11 +107,11 @@ int launch_rms_norm(const void* x, const void* residual, const void* weight, voi
                       aligned_to(out, 16) && (!residual || (aligned_to(residual, 16) && aligned_to(sum_out, 16)));
   const int nvec = hidden / VEC;
   if (vec_ok && nvec <= 256 * 2) {
-    rms_norm_kernel<T, VEC, 2><<<rows, 256, 0, st>>>(xp, rp, wp, sp, op, hidden, eps);
+    launch_chained(rms_norm_kernel<T, VEC, 2>, rows, 256, 0, st, xp, rp, wp, sp, op, hidden, eps);
   } else if (vec_ok && nvec <= 256 * 8) {
-    rms_norm_kernel<T, VEC, 8><<<rows, 256, 0, st>>>(xp, rp, wp, sp, op, hidden, eps);
+    launch_chained(rms_norm_kernel<T, VEC, 8>, rows, 256, 0, st, xp, rp, wp, sp, op, hidden, eps);
   } else {
-    rms_norm_generic_kernel<T><<<rows, 256, 0, st>>>(xp, rp, wp, sp, op, hidden, eps);
+    launch_chained(rms_norm_generic_kernel<T>, rows, 256, 0, st, xp, rp, wp, sp, op, hidden, eps);
   }
   return launch_status();
 }
@@ -119,6 +121,7 @@ int launch_rms_norm(const void* x, const void* residual, const void* weight, voi
 template <typename T>
 __global__ void rope_inplace_kernel(T* __restrict__ x, const int32_t* __restrict__ positions,
                                     int num_heads, int head_dim, float theta, long long stride) {
+  chain_enter();
   const int b = blockIdx.y;
   const int half = head_dim / 2;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;  // (head, pair)
@@ -150,6 +153,7 @@ __global__ void kv_append_kernel(const T* __restrict__ k, const T* __restrict__ 
                                  T* __restrict__ v_cache, const int32_t* __restrict__ page_table,
                                  const int32_t* __restrict__ positions, int num_kv_heads, int max_pages,
                                  int page_size, int head_dim, long long k_stride, long long v_stride) {
+  chain_enter();
   const int b = blockIdx.y;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;  // (kv head, dim)
   if (idx >= num_kv_heads * head_dim) return;
@@ -171,6 +175,7 @@ template <typename T>
 __global__ void rope_append_kernel(T* __restrict__ qkv, const int32_t* __restrict__ positions,
                                    const int32_t* __restrict__ page_table, T* __restrict__ k_cache, T* __restrict__ v_cache,
                                    int q_dim, int k_dim, int head_dim, float theta, int max_pages, int page_size, long long stride) {
+  chain_enter();
   const int b = blockIdx.y;
   const int pair = blockIdx.x * blockDim.x + threadIdx.x;            // pair of adjacent elements of the row
   if (pair >= (q_dim + 2 * k_dim) / 2) return;
@@ -206,6 +211,7 @@ rope_append_rows_kernel(__half* __restrict__ qkv, const int32_t* __restrict__ po
                         const int* __restrict__ n_rows, const float2* __restrict__ table, int table_positions,
                         __half* __restrict__ k_cache, __half* __restrict__ v_cache, int q_dim, int k_dim, int head_dim, int num_slots,
                         int page_size) {
+  chain_enter();
   const int row = blockIdx.x;
   if (n_rows && row >= *n_rows) return;
   const int pos = positions[row], page = pages[row];
@@ -245,6 +251,7 @@ __global__ void __launch_bounds__(128)
 kv_append_q8_kernel(const T* __restrict__ k, const T* __restrict__ v, uint8_t* __restrict__ k_cache, uint8_t* __restrict__ v_cache,
                     __half* __restrict__ kv_scales, const int32_t* __restrict__ page_table, const int32_t* __restrict__ positions,
                     int num_kv_heads, int max_pages, int page_size, int head_dim, long long k_stride, long long v_stride) {
+  chain_enter();
   __shared__ float s_max[2][4];
   const int kvh = blockIdx.x, b = blockIdx.y;
   const int pos = positions[b];
@@ -293,6 +300,7 @@ kv_append_q8_kernel(const T* __restrict__ k, const T* __restrict__ v, uint8_t* _
 // ---- elementwise ------------------------------------------------------------------
 template <typename T, bool SILU_MUL>
 __global__ void binary_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out, size_t total) {
+  chain_enter();
   const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const float x = Elem<T>::ld(a + i);
@@ -303,6 +311,7 @@ __global__ void binary_kernel(const T* __restrict__ a, const T* __restrict__ b, 
 template <typename T>
 __global__ void embedding_gather_kernel(const T* __restrict__ table, const int64_t* __restrict__ ids,
                                         T* __restrict__ out, int hidden, int vocab) {
+  chain_enter();
   const int r = blockIdx.x;
   long long id = ids[r];
   id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);  // clamp instead of faulting on a bad id
@@ -322,6 +331,7 @@ __global__ void embedding_gather_kernel(const T* __restrict__ table, const int64
 template <typename T>
 __global__ void __launch_bounds__(1024)
 argmax_rows_kernel(const T* __restrict__ logits, int64_t* __restrict__ out_ids, int vocab) {
+  chain_enter();
   __shared__ float s_val[32];
   __shared__ int s_idx[32];
   const T* row = logits + static_cast<size_t>(blockIdx.x) * vocab;
@@ -366,6 +376,7 @@ argmax_rows_kernel(const T* __restrict__ logits, int64_t* __restrict__ out_ids, 
 }
 
 __global__ void advance_positions_kernel(int32_t* positions, int32_t* seq_lens, int batch) {
+  chain_enter();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b < batch) {
     const int32_t len = seq_lens[b];
@@ -410,7 +421,7 @@ extern "C" int cacheir_b200_rope_inplace(void* x, const int32_t* positions, int 
   const long long stride = x_batch_stride > 0 ? x_batch_stride : static_cast<long long>(num_heads) * head_dim;
   const int pairs = num_heads * (head_dim / 2);
   const dim3 grid((pairs + 127) / 128, batch_size);
-  CB200_DISPATCH_DTYPE(dtype, (rope_inplace_kernel<T><<<grid, 128, 0, as_stream(stream)>>>(
+  CB200_DISPATCH_DTYPE(dtype, (launch_chained(rope_inplace_kernel<T>, grid, 128, 0, as_stream(stream),
                                   static_cast<T*>(x), positions, num_heads, head_dim, theta, stride)));
   return launch_status();
 }
@@ -433,7 +444,7 @@ extern "C" int cacheir_b200_rope_append_rows(void* qkv, const int32_t* positions
     return CACHEIR_B200_EINVAL;
   if (head_dim <= 0 || head_dim % 8 != 0 || q_dim <= 0 || k_dim <= 0 || q_dim % head_dim != 0 || k_dim % head_dim != 0) return CACHEIR_B200_EINVAL;
   if (!aligned_to(qkv, 16) || !aligned_to(rope_table, 16) || !aligned_to(k_cache, 16) || !aligned_to(v_cache, 16)) return CACHEIR_B200_EALIGN;
-  rope_append_rows_kernel<<<M, 256, 0, as_stream(stream)>>>(static_cast<__half*>(qkv), positions, pages, n_rows,
+  launch_chained(rope_append_rows_kernel, M, 256, 0, as_stream(stream), static_cast<__half*>(qkv), positions, pages, n_rows,
                                                             reinterpret_cast<const float2*>(rope_table), rope_table_positions,
                                                             static_cast<__half*>(k_cache), static_cast<__half*>(v_cache), q_dim, k_dim, head_dim,
                                                             num_slots, page_size);
@@ -451,7 +462,7 @@ extern "C" int cacheir_b200_rope_append(void* qkv, const int32_t* positions, con
   const long long stride = qkv_batch_stride > 0 ? qkv_batch_stride : static_cast<long long>(q_dim) + 2 * k_dim;
   const int pairs = (q_dim + 2 * k_dim) / 2;
   const dim3 grid((pairs + 127) / 128, batch_size);
-  CB200_DISPATCH_DTYPE(dtype, (rope_append_kernel<T><<<grid, 128, 0, as_stream(stream)>>>(
+  CB200_DISPATCH_DTYPE(dtype, (launch_chained(rope_append_kernel<T>, grid, 128, 0, as_stream(stream),
                                   static_cast<T*>(qkv), positions, page_table, static_cast<T*>(k_cache), static_cast<T*>(v_cache),
                                   q_dim, k_dim, head_dim, theta, max_pages_per_seq, page_size, stride)));
   return launch_status();
@@ -470,7 +481,7 @@ extern "C" int cacheir_b200_kv_append(const void* k, const void* v, void* k_cach
   const long long ks = k_batch_stride > 0 ? k_batch_stride : dense;
   const long long vs = v_batch_stride > 0 ? v_batch_stride : dense;
   const dim3 grid((static_cast<int>(dense) + 127) / 128, batch_size);
-  CB200_DISPATCH_DTYPE(dtype, (kv_append_kernel<T><<<grid, 128, 0, as_stream(stream)>>>(
+  CB200_DISPATCH_DTYPE(dtype, (launch_chained(kv_append_kernel<T>, grid, 128, 0, as_stream(stream),
                                   static_cast<const T*>(k), static_cast<const T*>(v), static_cast<T*>(k_cache),
                                   static_cast<T*>(v_cache), page_table, positions, num_kv_heads,
                                   max_pages_per_seq, page_size, head_dim, ks, vs)));
@@ -490,7 +501,7 @@ extern "C" int cacheir_b200_kv_append_q8(const void* k, const void* v, void* k_c
   const long long ks = k_batch_stride > 0 ? k_batch_stride : dense;
   const long long vs = v_batch_stride > 0 ? v_batch_stride : dense;
   const dim3 grid(num_kv_heads, batch_size);
-  CB200_DISPATCH_DTYPE(dtype, (kv_append_q8_kernel<T><<<grid, 128, 0, as_stream(stream)>>>(
+  CB200_DISPATCH_DTYPE(dtype, (launch_chained(kv_append_q8_kernel<T>, grid, 128, 0, as_stream(stream),
                                   static_cast<const T*>(k), static_cast<const T*>(v), static_cast<uint8_t*>(k_cache),
                                   static_cast<uint8_t*>(v_cache), static_cast<__half*>(kv_scales), page_table, positions,
                                   num_kv_heads, max_pages_per_seq, page_size, head_dim, ks, vs)));
@@ -502,7 +513,7 @@ extern "C" int cacheir_b200_silu_mul(const void* gate, const void* up, void* out
   if (total == 0) return 0;
   if (!gate || !up || !out) return CACHEIR_B200_EINVAL;
   const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
-  CB200_DISPATCH_DTYPE(dtype, (binary_kernel<T, true><<<blocks, 256, 0, as_stream(stream)>>>(
+  CB200_DISPATCH_DTYPE(dtype, (launch_chained(binary_kernel<T, true>, blocks, 256, 0, as_stream(stream),
                                   static_cast<const T*>(gate), static_cast<const T*>(up), static_cast<T*>(out), total)));
   return launch_status();
 }
@@ -512,7 +523,7 @@ extern "C" int cacheir_b200_add(const void* a, const void* b, void* out, size_t 
   if (total == 0) return 0;
   if (!a || !b || !out) return CACHEIR_B200_EINVAL;
   const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
-  CB200_DISPATCH_DTYPE(dtype, (binary_kernel<T, false><<<blocks, 256, 0, as_stream(stream)>>>(
+  CB200_DISPATCH_DTYPE(dtype, (launch_chained(binary_kernel<T, false>, blocks, 256, 0, as_stream(stream),
                                   static_cast<const T*>(a), static_cast<const T*>(b), static_cast<T*>(out), total)));
   return launch_status();
 }
@@ -521,7 +532,7 @@ extern "C" int cacheir_b200_embedding_gather(const void* table, const int64_t* i
                                              int rows, int hidden, int vocab, int dtype, void* stream) {
   if (rows <= 0 || hidden <= 0) return 0;
   if (!table || !ids || !out || vocab <= 0) return CACHEIR_B200_EINVAL;
-  CB200_DISPATCH_DTYPE(dtype, (embedding_gather_kernel<T><<<rows, 256, 0, as_stream(stream)>>>(
+  CB200_DISPATCH_DTYPE(dtype, (launch_chained(embedding_gather_kernel<T>, rows, 256, 0, as_stream(stream),
                                   static_cast<const T*>(table), ids, static_cast<T*>(out), hidden, vocab)));
   return launch_status();
 }
@@ -530,7 +541,7 @@ extern "C" int cacheir_b200_argmax_rows(const void* logits, int64_t* out_ids, in
                                         int dtype, void* stream) {
   if (rows <= 0 || vocab <= 0) return 0;
   if (!logits || !out_ids) return CACHEIR_B200_EINVAL;
-  CB200_DISPATCH_DTYPE(dtype, (argmax_rows_kernel<T><<<rows, 1024, 0, as_stream(stream)>>>(
+  CB200_DISPATCH_DTYPE(dtype, (launch_chained(argmax_rows_kernel<T>, rows, 1024, 0, as_stream(stream),
                                   static_cast<const T*>(logits), out_ids, vocab)));
   return launch_status();
 }
@@ -539,6 +550,6 @@ extern "C" int cacheir_b200_advance_positions(int32_t* positions, int32_t* seq_l
                                               void* stream) {
   if (batch_size <= 0) return 0;
   if (!positions || !seq_lens) return CACHEIR_B200_EINVAL;
-  advance_positions_kernel<<<(batch_size + 127) / 128, 128, 0, as_stream(stream)>>>(positions, seq_lens, batch_size);
+  launch_chained(advance_positions_kernel, (batch_size + 127) / 128, 128, 0, as_stream(stream), positions, seq_lens, batch_size);
   return launch_status();
 }

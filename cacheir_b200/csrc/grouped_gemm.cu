@@ -43,6 +43,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 grouped_simple_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y, const int32_t* __restrict__ cu,
                       const int32_t* __restrict__ token_of, int experts, int N, int K, long long ws, long long xs, long long ys) {
+  chain_enter();
   __shared__ float sx[kSimpleK][kSimpleRows + 1], sw[kSimpleK][kSimpleCols + 4];
   const RaggedItem it = find_item(cu, experts, kSimpleRows, blockIdx.x);
   if (it.seg < 0) return;
@@ -111,7 +112,7 @@ extern "C" int cacheir_b200_grouped_simple(const void* x, const void* w, void* y
   if (!x || !w || !y || !cu || experts < 1 || K <= 0) return CACHEIR_B200_EINVAL;
   const dim3 grid(ragged_items(places, experts, kSimpleRows), (N + kSimpleCols - 1) / kSimpleCols);
   if (grid.y > 65535) return CACHEIR_B200_ELIMIT;
-  CB200_HYBRID_DTYPE(dtype, (grouped_simple_kernel<T><<<grid, 256, 0, as_stream(stream)>>>(
+  CB200_HYBRID_DTYPE(dtype, (launch_chained(grouped_simple_kernel<T>, grid, 256, 0, as_stream(stream),
                                 static_cast<const T*>(x), static_cast<const T*>(w), static_cast<T*>(y), cu, token_of, experts, N, K,
                                 w_stride, x_stride, y_stride)));
   return launch_status();

@@ -24,6 +24,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 scaled_embedding_kernel(const T* __restrict__ table, const int64_t* __restrict__ ids, float* __restrict__ x, int width, int vocab,
                         float scale, NextArgs nx) {
+  chain_enter();
   const size_t row = blockIdx.x;
   const int64_t id = min(max(ids[row], static_cast<int64_t>(0)), static_cast<int64_t>(vocab - 1));
   for (int c = blockIdx.y * 256 + threadIdx.x; c < width; c += gridDim.y * 256) {
@@ -37,6 +38,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 dyt_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ row_index, const float* __restrict__ w,
                 const float* __restrict__ b, float alpha, T* __restrict__ out, int width) {
+  chain_enter();
   const size_t row = blockIdx.x;
   const size_t src = row_index ? static_cast<size_t>(max(row_index[row], 0)) : row;
   for (int c = blockIdx.y * 256 + threadIdx.x; c < width; c += gridDim.y * 256)
@@ -47,6 +49,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(512)
 rms_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ row_index, const float* __restrict__ w, float eps,
                 T* __restrict__ out, int width) {
+  chain_enter();
   __shared__ float scratch[32];
   const size_t row = blockIdx.x;
   const float* xr = x + (row_index ? static_cast<size_t>(max(row_index[row], 0)) : row) * width;
@@ -72,6 +75,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 residual_dyt_kernel(float* __restrict__ x, const T* __restrict__ y, const float* __restrict__ w, const float* __restrict__ b,
                     float alpha, int width, NextArgs nx) {
+  chain_enter();
   const size_t row = blockIdx.x;
   for (int c = blockIdx.y * 256 + threadIdx.x; c < width; c += gridDim.y * 256) {
     const size_t i = row * width + c;
@@ -86,6 +90,7 @@ constexpr int kRowThreads = 512;
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kRowThreads)
 residual_rms_kernel(float* __restrict__ x, const T* __restrict__ y, const float* __restrict__ w, float eps, int width, NextArgs nx) {
+  chain_enter();
   __shared__ float scratch[32];
   const size_t row = blockIdx.x;
   const T* yr = y + row * width;
@@ -121,6 +126,7 @@ residual_rms_kernel(float* __restrict__ x, const T* __restrict__ y, const float*
 template <typename T, int VEC, bool ADD>
 __global__ void __launch_bounds__(kRowThreads)
 embedding_rows_kernel(const T* __restrict__ table, const int64_t* __restrict__ ids, float* x, int width, int vocab, float scale, RowNext nx) {
+  chain_enter();
   __shared__ float scratch[32];
   const size_t row = blockIdx.x;
   const T* src = table + min(max(ids[row], static_cast<int64_t>(0)), static_cast<int64_t>(vocab - 1)) * width;
@@ -137,6 +143,7 @@ constexpr int kAddThreads = 256, kAddPieces = 8;
 template <typename T, int VEC, bool HELD>
 __global__ void __launch_bounds__(kAddThreads)
 residual_add_kernel(float* x, const T* __restrict__ y, const float* __restrict__ scale, int width, RowNext nx) {
+  chain_enter();
   __shared__ float scratch[32];
   const size_t row = blockIdx.x;
   x += row * width;
@@ -200,6 +207,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(512)
 layer_norm_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ row_index, const float* __restrict__ w, float eps,
                        T* __restrict__ out, int width) {
+  chain_enter();
   __shared__ float scratch[32];
   const size_t row = blockIdx.x;
   const float* xr = x + (row_index ? static_cast<size_t>(max(row_index[row], 0)) : row) * width;
@@ -232,6 +240,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(256)
 join_embedding_kernel(const float* __restrict__ x, const T* __restrict__ table, const int64_t* __restrict__ ids, T* __restrict__ out, int width,
                       int vocab) {
+  chain_enter();
   const size_t row = blockIdx.x;
   const T* src = table + min(max(ids[row], static_cast<int64_t>(0)), static_cast<int64_t>(vocab - 1)) * width;
   for (int c = (blockIdx.y * 256 + threadIdx.x) * VEC; c < width; c += gridDim.y * 256 * VEC) {
@@ -250,6 +259,7 @@ template <typename T, int VEC, bool HELD>
 __global__ void __launch_bounds__(kPairThreads)
 residual_rms_pair_kernel(float* x, const T* __restrict__ y1, const float* __restrict__ w1, const T* __restrict__ y2,
                          const float* __restrict__ w2, float factor, float eps, int width, RowNext nx) {
+  chain_enter();
   __shared__ float scratch[32];
   __shared__ float2 s_pair[kPairThreads / 32];
   const size_t row = blockIdx.x;
@@ -340,6 +350,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(kRowThreads)
 gated_rms_kernel(const T* __restrict__ o, const T* __restrict__ gate, long long gate_stride, const float* __restrict__ w, float eps,
                  T* __restrict__ out, int cols) {
+  chain_enter();
   __shared__ float scratch[32];
   const size_t row = blockIdx.x;
   const T* orow = o + row * cols;
@@ -368,6 +379,7 @@ template <typename T, int VEC, int WARPS>
 __global__ void __launch_bounds__(WARPS == 1 ? 256 : WARPS * 32)
 gated_parts_rms_kernel(const T* __restrict__ o, const T* __restrict__ gate, long long gate_stride, const float* __restrict__ w, int shared_weight,
                        int gate_first, float eps, T* __restrict__ out, int units, int parts, int size) {
+  chain_enter();
   __shared__ float scratch[32];
   const int unit = WARPS == 1 ? blockIdx.x * 8 + static_cast<int>(threadIdx.x >> 5) : static_cast<int>(blockIdx.x);
   const int at = WARPS == 1 ? static_cast<int>(threadIdx.x & 31) : static_cast<int>(threadIdx.x);
@@ -438,6 +450,7 @@ gated_parts_rms_kernel(const T* __restrict__ o, const T* __restrict__ gate, long
 template <typename T>
 __global__ void __launch_bounds__(256)
 glu_pairs_kernel(const T* __restrict__ y, T* __restrict__ out, int ff, int epilogue, float limit) {
+  chain_enter();
   const size_t row = blockIdx.x;
   for (int c = blockIdx.y * 256 + threadIdx.x; c < ff; c += gridDim.y * 256) {
     const T* p = y + row * 2 * ff + 2 * c;
@@ -451,6 +464,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 gelu_embed_kernel(const T* __restrict__ g, const int64_t* __restrict__ ids, const T* __restrict__ table, long long table_stride,
                   int table_col, T* __restrict__ out, int dim, int vocab) {
+  chain_enter();
   const size_t row = blockIdx.x;
   const int64_t id = min(max(ids[row], static_cast<int64_t>(0)), static_cast<int64_t>(vocab - 1));
   for (int c = threadIdx.x; c < dim; c += 256)
@@ -460,6 +474,7 @@ gelu_embed_kernel(const T* __restrict__ g, const int64_t* __restrict__ ids, cons
 template <typename T, bool RELU2>
 __global__ void __launch_bounds__(256)
 activate_cols_kernel(T* __restrict__ y, long long stride, int cols) {
+  chain_enter();
   T* yr = y + static_cast<size_t>(blockIdx.x) * stride;
   for (int c = blockIdx.y * 256 + threadIdx.x; c < cols; c += gridDim.y * 256) {
     const float z = Elem<T>::ld(yr + c);
@@ -473,6 +488,7 @@ template <typename T, typename TY>
 __global__ void __launch_bounds__(256)
 dense_simple_kernel(const T* __restrict__ x, const T* __restrict__ w, TY* __restrict__ y, int rows, int N, int K, int w_batch_rows,
                     int x_batch_cols, int y_batch_cols, long long ws, long long xs, long long ys, const float* __restrict__ bias) {
+  chain_enter();
   __shared__ float sx[kTileK][kTile + 4], sw[kTileK][kTile + 4];
   const int z = blockIdx.z;
   x += static_cast<long long>(z) * x_batch_cols;
@@ -536,7 +552,7 @@ extern "C" int cacheir_b200_scaled_embedding(const void* table, const int64_t* i
     const RowNext rn{next_mode, next_w, next_alpha, next_out};
     const bool vec = width % 4 == 0 && aligned_to(table, 16) && aligned_to(residual, 16) && row_next_aligned(next_mode, next_w, next_out);
 #define CB200_ROWS(VEC, ADD)                                                                  \
-  embedding_rows_kernel<T, VEC, ADD><<<rows, kRowThreads, 0, as_stream(stream)>>>(static_cast<const T*>(table), ids, residual, width, vocab, scale, rn)
+  launch_chained(embedding_rows_kernel<T, VEC, ADD>, rows, kRowThreads, 0, as_stream(stream), static_cast<const T*>(table), ids, residual, width, vocab, scale, rn)
     CB200_HYBRID_DTYPE(dtype, {
       if (vec && accumulate) CB200_ROWS(4, true);
       else if (vec) CB200_ROWS(4, false);
@@ -548,7 +564,7 @@ extern "C" int cacheir_b200_scaled_embedding(const void* table, const int64_t* i
   }
   if (!next_ok(next_mode, next_w, next_b, next_out)) return CACHEIR_B200_EINVAL;
   const NextArgs nx{next_mode, next_w, next_b, next_alpha, next_out};
-  CB200_HYBRID_DTYPE(dtype, (scaled_embedding_kernel<T><<<row_grid(rows, width), 256, 0, as_stream(stream)>>>(
+  CB200_HYBRID_DTYPE(dtype, (launch_chained(scaled_embedding_kernel<T>, row_grid(rows, width), 256, 0, as_stream(stream),
                                 static_cast<const T*>(table), ids, residual, width, vocab, scale, nx)));
   return launch_status();
 }
@@ -557,7 +573,7 @@ extern "C" int cacheir_b200_dyt_rows(const float* residual, const int32_t* row_i
                                      void* out, int rows, int width, int dtype, void* stream) {
   if (rows <= 0 || width <= 0) return 0;
   if (!residual || !w || !b || !out) return CACHEIR_B200_EINVAL;
-  CB200_HYBRID_DTYPE(dtype, (dyt_rows_kernel<T><<<row_grid(rows, width), 256, 0, as_stream(stream)>>>(
+  CB200_HYBRID_DTYPE(dtype, (launch_chained(dyt_rows_kernel<T>, row_grid(rows, width), 256, 0, as_stream(stream),
                                 residual, row_index, w, b, alpha, static_cast<T*>(out), width)));
   return launch_status();
 }
@@ -568,8 +584,8 @@ extern "C" int cacheir_b200_rms_rows(const float* residual, const int32_t* row_i
   if (!residual || !w || !out) return CACHEIR_B200_EINVAL;
   const bool vec = width % 4 == 0 && aligned_to(residual, 16) && aligned_to(w, 16) && aligned_to(out, 16);
   CB200_HYBRID_DTYPE(dtype, {
-    if (vec) rms_rows_kernel<T, 4><<<rows, 512, 0, as_stream(stream)>>>(residual, row_index, w, eps, static_cast<T*>(out), width);
-    else rms_rows_kernel<T, 1><<<rows, 512, 0, as_stream(stream)>>>(residual, row_index, w, eps, static_cast<T*>(out), width);
+    if (vec) launch_chained(rms_rows_kernel<T, 4>, rows, 512, 0, as_stream(stream), residual, row_index, w, eps, static_cast<T*>(out), width);
+    else launch_chained(rms_rows_kernel<T, 1>, rows, 512, 0, as_stream(stream), residual, row_index, w, eps, static_cast<T*>(out), width);
   });
   return launch_status();
 }
@@ -580,7 +596,7 @@ extern "C" int cacheir_b200_residual_dyt(float* residual, const void* y, const f
   if (rows <= 0 || width <= 0) return 0;
   if (!residual || !y || !w || !b || !next_ok(next_mode, next_w, next_b, next_out)) return CACHEIR_B200_EINVAL;
   const NextArgs nx{next_mode, next_w, next_b, next_alpha, next_out};
-  CB200_HYBRID_DTYPE(dtype, (residual_dyt_kernel<T><<<row_grid(rows, width), 256, 0, as_stream(stream)>>>(
+  CB200_HYBRID_DTYPE(dtype, (launch_chained(residual_dyt_kernel<T>, row_grid(rows, width), 256, 0, as_stream(stream),
                                 residual, static_cast<const T*>(y), w, b, alpha, width, nx)));
   return launch_status();
 }
@@ -591,8 +607,8 @@ extern "C" int cacheir_b200_layer_norm_rows(const float* residual, const int32_t
   if (!residual || !w || !out) return CACHEIR_B200_EINVAL;
   const bool vec = width % 4 == 0 && aligned_to(residual, 16) && aligned_to(w, 16) && aligned_to(out, 16);
   CB200_HYBRID_DTYPE(dtype, {
-    if (vec) layer_norm_rows_kernel<T, 4><<<rows, 512, 0, as_stream(stream)>>>(residual, row_index, w, eps, static_cast<T*>(out), width);
-    else layer_norm_rows_kernel<T, 1><<<rows, 512, 0, as_stream(stream)>>>(residual, row_index, w, eps, static_cast<T*>(out), width);
+    if (vec) launch_chained(layer_norm_rows_kernel<T, 4>, rows, 512, 0, as_stream(stream), residual, row_index, w, eps, static_cast<T*>(out), width);
+    else launch_chained(layer_norm_rows_kernel<T, 1>, rows, 512, 0, as_stream(stream), residual, row_index, w, eps, static_cast<T*>(out), width);
   });
   return launch_status();
 }
@@ -603,9 +619,9 @@ extern "C" int cacheir_b200_join_embedding(const float* residual, const void* ta
   if (!residual || !table || !ids || !out || vocab <= 0) return CACHEIR_B200_EINVAL;
   const bool vec = width % 4 == 0 && aligned_to(residual, 16) && aligned_to(table, 16) && aligned_to(out, 16);
   CB200_HYBRID_DTYPE(dtype, {
-    if (vec) join_embedding_kernel<T, 4><<<row_grid(rows, width / 4), 256, 0, as_stream(stream)>>>(
+    if (vec) launch_chained(join_embedding_kernel<T, 4>, row_grid(rows, width / 4), 256, 0, as_stream(stream),
         residual, static_cast<const T*>(table), ids, static_cast<T*>(out), width, vocab);
-    else join_embedding_kernel<T, 1><<<row_grid(rows, width), 256, 0, as_stream(stream)>>>(
+    else launch_chained(join_embedding_kernel<T, 1>, row_grid(rows, width), 256, 0, as_stream(stream),
         residual, static_cast<const T*>(table), ids, static_cast<T*>(out), width, vocab);
   });
   return launch_status();
@@ -619,7 +635,7 @@ extern "C" int cacheir_b200_residual_add(float* residual, const void* y, const f
   const bool vec = width % 4 == 0 && aligned_to(residual, 16) && aligned_to(y, 16) && (!scale || aligned_to(scale, 16)) &&
                    row_next_aligned(next_mode, next_w, next_out);
 #define CB200_ADD(VEC, HELD) \
-  residual_add_kernel<T, VEC, HELD><<<rows, kAddThreads, 0, as_stream(stream)>>>(residual, static_cast<const T*>(y), scale, width, nx)
+  launch_chained(residual_add_kernel<T, VEC, HELD>, rows, kAddThreads, 0, as_stream(stream), residual, static_cast<const T*>(y), scale, width, nx)
   CB200_HYBRID_DTYPE(dtype, {
     if (vec && width <= 4 * kAddThreads * kAddPieces) CB200_ADD(4, true);
     else if (vec) CB200_ADD(4, false);
@@ -638,7 +654,7 @@ extern "C" int cacheir_b200_residual_rms_pair(float* residual, const void* y1, c
   const bool vec = width % 4 == 0 && aligned_to(residual, 16) && aligned_to(y1, 16) && aligned_to(y2, 16) && aligned_to(w1, 16) &&
                    aligned_to(w2, 16) && row_next_aligned(next_mode, next_w, next_out);
 #define CB200_PAIR(VEC, HELD)                                                                                                        \
-  residual_rms_pair_kernel<T, VEC, HELD><<<rows, kPairThreads, 0, as_stream(stream)>>>(residual, static_cast<const T*>(y1), w1,        \
+  launch_chained(residual_rms_pair_kernel<T, VEC, HELD>, rows, kPairThreads, 0, as_stream(stream), residual, static_cast<const T*>(y1), w1,        \
                                                                                       static_cast<const T*>(y2), w2, factor, eps, width, nx)
   CB200_HYBRID_DTYPE(dtype, {
     if (vec && width <= 4 * kPairThreads * kPairPieces && next_mode != CACHEIR_B200_NEXT_LAYER) CB200_PAIR(4, true);
@@ -659,8 +675,8 @@ extern "C" int cacheir_b200_residual_rms(float* residual, const void* y, const f
                    (next_mode == CACHEIR_B200_NEXT_NONE || aligned_to(next_out, 16)) &&
                    (next_mode != CACHEIR_B200_NEXT_DYT || (aligned_to(next_w, 16) && aligned_to(next_b, 16)));
   CB200_HYBRID_DTYPE(dtype, {
-    if (vec) residual_rms_kernel<T, 4><<<rows, kRowThreads, 0, as_stream(stream)>>>(residual, static_cast<const T*>(y), w, eps, width, nx);
-    else residual_rms_kernel<T, 1><<<rows, kRowThreads, 0, as_stream(stream)>>>(residual, static_cast<const T*>(y), w, eps, width, nx);
+    if (vec) launch_chained(residual_rms_kernel<T, 4>, rows, kRowThreads, 0, as_stream(stream), residual, static_cast<const T*>(y), w, eps, width, nx);
+    else launch_chained(residual_rms_kernel<T, 1>, rows, kRowThreads, 0, as_stream(stream), residual, static_cast<const T*>(y), w, eps, width, nx);
   });
   return launch_status();
 }
@@ -671,9 +687,9 @@ extern "C" int cacheir_b200_gated_rms(const void* o, const void* gate, long long
   if (!o || !gate || !w || !out) return CACHEIR_B200_EINVAL;
   const bool vec = cols % 4 == 0 && gate_stride % 4 == 0 && aligned_to(o, 16) && aligned_to(gate, 16) && aligned_to(w, 16) && aligned_to(out, 16);
   CB200_HYBRID_DTYPE(dtype, {
-    if (vec) gated_rms_kernel<T, 4><<<rows, kRowThreads, 0, as_stream(stream)>>>(
+    if (vec) launch_chained(gated_rms_kernel<T, 4>, rows, kRowThreads, 0, as_stream(stream),
         static_cast<const T*>(o), static_cast<const T*>(gate), gate_stride, w, eps, static_cast<T*>(out), cols);
-    else gated_rms_kernel<T, 1><<<rows, kRowThreads, 0, as_stream(stream)>>>(
+    else launch_chained(gated_rms_kernel<T, 1>, rows, kRowThreads, 0, as_stream(stream),
         static_cast<const T*>(o), static_cast<const T*>(gate), gate_stride, w, eps, static_cast<T*>(out), cols);
   });
   return launch_status();
@@ -683,7 +699,7 @@ extern "C" int cacheir_b200_glu_pairs(const void* y, void* out, int rows, int ff
   if (rows <= 0 || ff <= 0) return 0;
   if (!y || !out || (epilogue != CACHEIR_B200_DENSE_GEGLU && epilogue != CACHEIR_B200_DENSE_SWIGLU && epilogue != CACHEIR_B200_DENSE_CLAMPED_GLU))
     return CACHEIR_B200_EINVAL;
-  CB200_HYBRID_DTYPE(dtype, (glu_pairs_kernel<T><<<row_grid(rows, ff), 256, 0, as_stream(stream)>>>(
+  CB200_HYBRID_DTYPE(dtype, (launch_chained(glu_pairs_kernel<T>, row_grid(rows, ff), 256, 0, as_stream(stream),
                                 static_cast<const T*>(y), static_cast<T*>(out), ff, epilogue, limit)));
   return launch_status();
 }
@@ -692,7 +708,7 @@ extern "C" int cacheir_b200_gelu_embed(const void* g, const int64_t* ids, const 
                                        void* out, int rows, int dim, int vocab, int dtype, void* stream) {
   if (rows <= 0 || dim <= 0) return 0;
   if (!g || !ids || !table || !out || vocab <= 0) return CACHEIR_B200_EINVAL;
-  CB200_HYBRID_DTYPE(dtype, (gelu_embed_kernel<T><<<rows, 256, 0, as_stream(stream)>>>(
+  CB200_HYBRID_DTYPE(dtype, (launch_chained(gelu_embed_kernel<T>, rows, 256, 0, as_stream(stream),
                                 static_cast<const T*>(g), ids, static_cast<const T*>(table), table_stride, table_col,
                                 static_cast<T*>(out), dim, vocab)));
   return launch_status();
@@ -701,14 +717,14 @@ extern "C" int cacheir_b200_gelu_embed(const void* g, const int64_t* ids, const 
 extern "C" int cacheir_b200_silu_cols(void* y, int rows, long long stride, int cols, int dtype, void* stream) {
   if (rows <= 0 || cols <= 0) return 0;
   if (!y) return CACHEIR_B200_EINVAL;
-  CB200_HYBRID_DTYPE(dtype, (activate_cols_kernel<T, false><<<row_grid(rows, cols), 256, 0, as_stream(stream)>>>(static_cast<T*>(y), stride, cols)));
+  CB200_HYBRID_DTYPE(dtype, (launch_chained(activate_cols_kernel<T, false>, row_grid(rows, cols), 256, 0, as_stream(stream), static_cast<T*>(y), stride, cols)));
   return launch_status();
 }
 
 extern "C" int cacheir_b200_relu2_cols(void* y, int rows, long long stride, int cols, int dtype, void* stream) {
   if (rows <= 0 || cols <= 0) return 0;
   if (!y) return CACHEIR_B200_EINVAL;
-  CB200_HYBRID_DTYPE(dtype, (activate_cols_kernel<T, true><<<row_grid(rows, cols), 256, 0, as_stream(stream)>>>(static_cast<T*>(y), stride, cols)));
+  CB200_HYBRID_DTYPE(dtype, (launch_chained(activate_cols_kernel<T, true>, row_grid(rows, cols), 256, 0, as_stream(stream), static_cast<T*>(y), stride, cols)));
   return launch_status();
 }
 
@@ -719,7 +735,7 @@ extern "C" int cacheir_b200_gated_parts_rms(const void* o, const void* gate, lon
   const int size = cols / parts, units = rows * parts, quad = 4 * (dtype == CACHEIR_B200_F32 ? 4 : 2);
   const bool vec = size % 4 == 0 && gate_stride % 4 == 0 && aligned_to(o, quad) && aligned_to(gate, quad) && aligned_to(w, 16) && aligned_to(out, quad);
 #define CB200_PARTS(VEC, WARPS)                                                                                                         \
-  gated_parts_rms_kernel<T, VEC, WARPS><<<WARPS == 1 ? (units + 7) / 8 : units, WARPS == 1 ? 256 : WARPS * 32, 0, as_stream(stream)>>>(                             \
+  launch_chained(gated_parts_rms_kernel<T, VEC, WARPS>, WARPS == 1 ? (units + 7) / 8 : units, WARPS == 1 ? 256 : WARPS * 32, 0, as_stream(stream), \
       static_cast<const T*>(o), static_cast<const T*>(gate), gate_stride, w, shared_weight, gate_first, eps, static_cast<T*>(out), units, parts, size)
   CB200_HYBRID_DTYPE(dtype, {
     if (vec && size <= 512) CB200_PARTS(4, 1);
@@ -741,7 +757,7 @@ extern "C" int cacheir_b200_dense_simple(const void* x, const void* w, void* y, 
   if (grid.y > 65535 || grid.z > 65535) return CACHEIR_B200_ELIMIT;
   cudaStream_t st = as_stream(stream);
 #define CB200_SIMPLE(T, TY)                                                                                              \
-  dense_simple_kernel<T, TY><<<grid, 256, 0, st>>>(static_cast<const T*>(x), static_cast<const T*>(w), static_cast<TY*>(y), rows, N, \
+  launch_chained(dense_simple_kernel<T, TY>, grid, 256, 0, st, static_cast<const T*>(x), static_cast<const T*>(w), static_cast<TY*>(y), rows, N, \
                                                    K, w_batch_rows, x_batch_cols, y_batch_cols, w_stride, x_stride, y_stride, bias)
   if (dtype == CACHEIR_B200_F32 && y_dtype == CACHEIR_B200_F32) CB200_SIMPLE(float, float);
   else if (dtype == CACHEIR_B200_BF16 && y_dtype == CACHEIR_B200_F32) CB200_SIMPLE(__nv_bfloat16, float);

@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(256)
 latent_prepare_kernel(const cacheir_b200_latent_args a, const T* __restrict__ down, long long down_stride, const float* __restrict__ norm_w,
                       float eps, const T* q, long long q_stride, T* q_rot, long long q_rot_stride, int q_rot_head_stride,
                       const float2* __restrict__ table, int table_positions, int rot_dims) {
+  chain_enter();
   __shared__ float scratch[32];
   const int row = blockIdx.x;
   const int seg = a.row_seg[row];
@@ -77,6 +78,7 @@ __global__ void __launch_bounds__(128)
 latent_simple_kernel(const cacheir_b200_latent_args a, const T* __restrict__ q, long long q_stride, const T* __restrict__ uk,
                      const T* __restrict__ uv, const float* __restrict__ sink, const T* __restrict__ gate, long long gate_stride,
                      T* __restrict__ out) {
+  chain_enter();
   extern __shared__ float sm[];
   __shared__ float scratch[32];
   const int width = a.kv_rank + a.rot_dim;
@@ -250,6 +252,7 @@ __device__ __forceinline__ void sync_softmax() { asm volatile("barrier.cta.sync 
 template <int NR>
 __global__ void __launch_bounds__(kThreads, 1)
 latent_attention_kernel(const __grid_constant__ CUtensorMap tmap_kv, const __grid_constant__ CUtensorMap tmap_q, const FastParams p) {
+  chain_enter();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   const cacheir_b200_latent_args& a = p.a;
@@ -709,19 +712,7 @@ int launch_fast(FastParams p, const void* q, dim3 grid, cudaStream_t st) {
   auto kern = latent_attention_kernel<NR>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = p.splits;
-  cfg.attrs = attr;
-  cfg.numAttrs = p.splits > 1 ? 1 : 0;
-  e = cudaLaunchKernelEx(&cfg, kern, tkv, tq, p);
+  e = launch_clusters(kern, grid, kThreads, smem, st, dim3(1, 1, p.splits), tkv, tq, p);
   if (e != cudaSuccess) return static_cast<int>(e);
   return launch_status();
 }
@@ -751,11 +742,11 @@ extern "C" int cacheir_b200_latent_prepare(const cacheir_b200_latent_args* args,
   const int parts = args->rows >= kNumSMs ? 1 : (pairs + 255) / 256 < 4 ? (pairs + 255) / 256 : 4;
   const dim3 grid(args->rows, parts + (down ? 1 : 0));
   if (args->dtype == CACHEIR_B200_F32)
-    latent_prepare_kernel<float><<<grid, 256, 0, as_stream(stream)>>>(
+    launch_chained(latent_prepare_kernel<float>, grid, 256, 0, as_stream(stream),
         *args, static_cast<const float*>(down), down_stride, norm_w, eps, static_cast<const float*>(q), q_stride, static_cast<float*>(q_rot),
         q_rot_stride, q_rot_head_stride, table, rope_positions, rot_dims);
   else if (args->dtype == CACHEIR_B200_BF16)
-    latent_prepare_kernel<__nv_bfloat16><<<grid, 256, 0, as_stream(stream)>>>(
+    launch_chained(latent_prepare_kernel<__nv_bfloat16>, grid, 256, 0, as_stream(stream),
         *args, static_cast<const __nv_bfloat16*>(down), down_stride, norm_w, eps, static_cast<const __nv_bfloat16*>(q), q_stride,
         static_cast<__nv_bfloat16*>(q_rot), q_rot_stride, q_rot_head_stride, table, rope_positions, rot_dims);
   else
@@ -773,7 +764,7 @@ extern "C" int cacheir_b200_latent_attention_simple(const cacheir_b200_latent_ar
   if (smem > 48 * 1024) return CACHEIR_B200_ELIMIT;
   const dim3 grid(args->rows, args->heads);
 #define CB200_LATENT_SIMPLE(T)                                                                                              \
-  latent_simple_kernel<T><<<grid, 128, smem, as_stream(stream)>>>(*args, static_cast<const T*>(q), q_stride, static_cast<const T*>(uk), \
+  launch_chained(latent_simple_kernel<T>, grid, 128, smem, as_stream(stream), *args, static_cast<const T*>(q), q_stride, static_cast<const T*>(uk), \
       static_cast<const T*>(uv), sink, static_cast<const T*>(gate), gate_stride, static_cast<T*>(out))
   if (args->dtype == CACHEIR_B200_F32) CB200_LATENT_SIMPLE(float);
   else if (args->dtype == CACHEIR_B200_BF16) CB200_LATENT_SIMPLE(__nv_bfloat16);

@@ -50,6 +50,7 @@ __device__ __forceinline__ int key_head(const Args& a, int h) { return a.key_hea
 template <typename T, bool GATED>
 __global__ void __launch_bounds__(256)
 recurrence_simple_kernel(const Args a) {
+  chain_enter();
   extern __shared__ float sm[];
   float* s_state = sm;                       // [dim][32]
   float* s_k = s_state + a.dim * 32;         // [dim]
@@ -119,6 +120,7 @@ recurrence_simple_kernel(const Args a) {
 template <typename T>
 __global__ void __launch_bounds__(256)
 recurrence_step_kernel(const Args a) {
+  chain_enter();
   __shared__ float4 s_red[256];
   extern __shared__ float s_kq[];           // [2][dim]
   const int seg = blockIdx.x, h = blockIdx.y;
@@ -190,6 +192,7 @@ PieceSpace piece_space(const Args& a, float* ws, int items) {
 template <int MT, int NC, bool LOCAL, bool GATED, bool AHEAD>
 __global__ void __launch_bounds__(128)
 recurrence_chunk_kernel(const Args a, const PieceSpace ws, int piece_rows) {
+  chain_enter();
   constexpr int kCols = NC * 8, kPitchV = kCols + 8;      // (rows 16 bytes over a multiple of 32: conflict-free)
   constexpr int kBuffers = AHEAD ? 2 : 1;
   extern __shared__ __align__(16) uint8_t raw[];
@@ -546,6 +549,7 @@ recurrence_chunk_kernel(const Args a, const PieceSpace ws, int piece_rows) {
 template <bool GATED>
 __global__ void __launch_bounds__(256)
 recurrence_scan_kernel(const Args a, const PieceSpace ws, int piece_rows) {
+  chain_enter();
   constexpr int kAhead = 8;
   __shared__ float s_f[256];
   const int seg = blockIdx.x, h = blockIdx.y;
@@ -619,6 +623,7 @@ __device__ __forceinline__ void log_gates(const Gates& g, int row, int heads, in
 constexpr int kGateThreads = 1024;
 __global__ void __launch_bounds__(kGateThreads)
 memory_gates_kernel(const Args a, const Gates g, float* __restrict__ log_decay, float* __restrict__ log_take, float* __restrict__ maximum) {
+  chain_enter();
   __shared__ float s_f[32], s_m[32], s_top[kGateThreads + 1];
   const int seg = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = a.cu_rows[seg], row1 = a.cu_rows[seg + 1];
@@ -672,6 +677,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(256)
 memory_norm_kernel(const T* __restrict__ o, const float* __restrict__ normaliser, const float* __restrict__ maximum, const T* __restrict__ gate,
                    long long gate_stride, const float* __restrict__ w, float eps, T* __restrict__ out, int units, int heads, int vdim) {
+  chain_enter();
   const int unit = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (unit >= units) return;
   const int row = unit / heads, h = unit % heads;
@@ -731,6 +737,7 @@ memory_norm_kernel(const T* __restrict__ o, const float* __restrict__ normaliser
 template <typename T>
 __global__ void __launch_bounds__(256, 4)
 memory_step_kernel(const Args a, const Gates g, const T* __restrict__ gate, long long gate_stride, const float* __restrict__ w, float eps) {
+  chain_enter();
   __shared__ float4 s_red[256];
   __shared__ float scratch[32];
   extern __shared__ float s_kq[];           // [2][dim]
@@ -827,6 +834,7 @@ __device__ __forceinline__ void step_gates(const Steps& s, int row, int h, float
 
 __global__ void __launch_bounds__(256)
 state_space_gates_kernel(const Steps s, int units, int heads, float* __restrict__ log_decay, float* __restrict__ log_take) {
+  chain_enter();
   const int unit = blockIdx.x * 256 + threadIdx.x;
   if (unit >= units) return;
   float dt, decay;
@@ -838,6 +846,7 @@ state_space_gates_kernel(const Steps s, int units, int heads, float* __restrict_
 template <typename T>
 __global__ void __launch_bounds__(256, 4)
 state_space_step_kernel(const Args a, const Steps s) {
+  chain_enter();
   __shared__ float4 s_red[256];
   extern __shared__ float s_kq[];           // [2][dim]
   const int seg = blockIdx.x, h = blockIdx.y, kh = key_head(a, h);
@@ -931,7 +940,7 @@ int launch_chunk(const Args& a, const PieceSpace& ws, int piece, cudaStream_t st
   const size_t smem = chunk_smem(a.dim, NC, AHEAD);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  kern<<<dim3(ragged_items(a.rows, a.segments, piece), a.heads, (a.vdim + NC * 8 - 1) / (NC * 8)), 128, smem, st>>>(a, ws, piece);
+  launch_chained(kern, dim3(ragged_items(a.rows, a.segments, piece), a.heads, (a.vdim + NC * 8 - 1) / (NC * 8)), 128, smem, st, a, ws, piece);
   return launch_status();
 }
 
@@ -948,7 +957,7 @@ int launch_passes(const Args& a, float* workspace, bool pieces, cudaStream_t st)
     const int rc = a.dim <= 64 ? launch_chunk<1, kWide, true, GATED, false>(a, ws, piece, st) : launch_chunk<2, kWide, true, GATED, false>(a, ws, piece, st);
     if (rc != 0) return rc;
     const int z = (a.dim * a.vdim + 1023) / 1024;
-    recurrence_scan_kernel<GATED><<<dim3(a.segments, a.heads, z), 256, 0, st>>>(a, ws, piece);
+    launch_chained(recurrence_scan_kernel<GATED>, dim3(a.segments, a.heads, z), 256, 0, st, a, ws, piece);
   }
   return a.dim <= 64 ? launch_chunk<1, kWide, false, GATED, false>(a, ws, piece, st) : launch_chunk<2, kWide, false, GATED, false>(a, ws, piece, st);
 }
@@ -960,7 +969,7 @@ int launch_simple(const Args& a, cudaStream_t st) {
   const dim3 grid(a.segments, a.heads, (a.vdim + 31) / 32);
   cudaError_t e = cudaFuncSetAttribute(recurrence_simple_kernel<T, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  recurrence_simple_kernel<T, GATED><<<grid, 256, smem, st>>>(a);
+  launch_chained(recurrence_simple_kernel<T, GATED>, grid, 256, smem, st, a);
   return launch_status();
 }
 
@@ -989,8 +998,8 @@ extern "C" int cacheir_b200_recurrence_step(const cacheir_b200_recurrence_args* 
   if (!aligned_to(a->state, 16) || a->slot_stride % 4 != 0) return CACHEIR_B200_EALIGN;
   const dim3 grid(a->segments, a->heads);
   const size_t smem = static_cast<size_t>(a->dim) * 8;
-  if (a->dtype == CACHEIR_B200_F32) recurrence_step_kernel<float><<<grid, 256, smem, as_stream(stream)>>>(*a);
-  else if (a->dtype == CACHEIR_B200_BF16) recurrence_step_kernel<__nv_bfloat16><<<grid, 256, smem, as_stream(stream)>>>(*a);
+  if (a->dtype == CACHEIR_B200_F32) launch_chained(recurrence_step_kernel<float>, grid, 256, smem, as_stream(stream), *a);
+  else if (a->dtype == CACHEIR_B200_BF16) launch_chained(recurrence_step_kernel<__nv_bfloat16>, grid, 256, smem, as_stream(stream), *a);
   else return CACHEIR_B200_EUNSUPPORTED;
   return launch_status();
 }
@@ -1024,7 +1033,7 @@ extern "C" int cacheir_b200_memory_gates(const cacheir_b200_recurrence_args* a, 
   if (a->rows <= 0) return 0;
   const Gates g{logits, stride, in_bias, forget_bias, cap};
   if (!recurrence_args_ok(*a) || !memory_slots_ok(*a) || a->decay_pow || !gates_ok(g, a->heads) || !log_decay || !log_take || !maximum) return CACHEIR_B200_EINVAL;
-  memory_gates_kernel<<<dim3(a->segments, a->heads), kGateThreads, 0, as_stream(stream)>>>(*a, g, log_decay, log_take, maximum);
+  launch_chained(memory_gates_kernel, dim3(a->segments, a->heads), kGateThreads, 0, as_stream(stream), *a, g, log_decay, log_take, maximum);
   return launch_status();
 }
 
@@ -1036,7 +1045,7 @@ extern "C" int cacheir_b200_memory_norm(const void* o, const float* normaliser, 
   const bool vec = vdim % 4 == 0 && gate_stride % 4 == 0 && aligned_to(o, quad) && aligned_to(gate, quad) && aligned_to(w, 16) && aligned_to(out, quad);
   const int grid = (units + 7) / 8;
 #define CB200_NORM(VEC)                                                                                                              \
-  memory_norm_kernel<T, VEC><<<grid, 256, 0, as_stream(stream)>>>(static_cast<const T*>(o), normaliser, maximum, static_cast<const T*>(gate), \
+  launch_chained(memory_norm_kernel<T, VEC>, grid, 256, 0, as_stream(stream), static_cast<const T*>(o), normaliser, maximum, static_cast<const T*>(gate), \
                                                                  gate_stride, w, eps, static_cast<T*>(out), units, heads, vdim)
   CB200_HYBRID_DTYPE(dtype, {
     if (vec) CB200_NORM(4);
@@ -1059,7 +1068,7 @@ extern "C" int cacheir_b200_memory_step(const cacheir_b200_recurrence_args* a, c
   if (!aligned_to(a->state, 16) || a->slot_stride % 4 != 0) return CACHEIR_B200_EALIGN;
   const dim3 grid(a->segments, a->heads);
   const size_t smem = static_cast<size_t>(a->dim) * 8;
-  CB200_HYBRID_DTYPE(a->dtype, (memory_step_kernel<T><<<grid, 256, smem, as_stream(stream)>>>(*a, g, static_cast<const T*>(gate), gate_stride, w, eps)));
+  CB200_HYBRID_DTYPE(a->dtype, (launch_chained(memory_step_kernel<T>, grid, 256, smem, as_stream(stream), *a, g, static_cast<const T*>(gate), gate_stride, w, eps)));
   return launch_status();
 }
 
@@ -1069,7 +1078,7 @@ extern "C" int cacheir_b200_state_space_gates(const cacheir_b200_recurrence_args
   if (a->rows <= 0) return 0;
   if (a->heads <= 0 || !z || stride < a->heads || !bias || !log_rate || !log_decay || !log_take) return CACHEIR_B200_EINVAL;
   const int units = a->rows * a->heads;
-  state_space_gates_kernel<<<(units + 255) / 256, 256, 0, as_stream(stream)>>>(Steps{z, stride, bias, log_rate}, units, a->heads, log_decay, log_take);
+  launch_chained(state_space_gates_kernel, (units + 255) / 256, 256, 0, as_stream(stream), Steps{z, stride, bias, log_rate}, units, a->heads, log_decay, log_take);
   return launch_status();
 }
 
@@ -1081,7 +1090,7 @@ extern "C" int cacheir_b200_state_space_step(const cacheir_b200_recurrence_args*
   if (a->vdim % 4 != 0 || a->vdim > 1024 || a->dim > 4096) return CACHEIR_B200_EUNSUPPORTED;
   if (!aligned_to(a->state, 16) || a->slot_stride % 4 != 0) return CACHEIR_B200_EALIGN;
   const size_t smem = static_cast<size_t>(a->dim) * 8;
-  CB200_HYBRID_DTYPE(a->dtype, (state_space_step_kernel<T><<<dim3(a->segments, a->heads), 256, smem, as_stream(stream)>>>(*a, Steps{z, stride, bias, log_rate})));
+  CB200_HYBRID_DTYPE(a->dtype, (launch_chained(state_space_step_kernel<T>, dim3(a->segments, a->heads), 256, smem, as_stream(stream), *a, Steps{z, stride, bias, log_rate})));
   return launch_status();
 }
 

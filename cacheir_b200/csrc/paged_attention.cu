@@ -38,6 +38,7 @@ __device__ __forceinline__ void load_cached(const void* cache, size_t elem, floa
 template <typename T, int VEC, int LPT, int R, int GC, bool KV8>
 __global__ void __launch_bounds__(kWarps * 32)
 paged_decode_general_kernel(const AttnParams p) {
+  chain_enter();
   constexpr int TPW = 32 / LPT;         // rows handled per warp instruction
   constexpr int SLOTS = kWarps * TPW;   // independent softmax streams per CTA
   extern __shared__ float smem[];
@@ -206,7 +207,7 @@ int launch_general_gc(const AttnParams& p0, cudaStream_t stream) {
                                            static_cast<int>(smem));                       \
       if (e != cudaSuccess) return static_cast<int>(e);                                   \
     }                                                                                     \
-    kern<<<grid, kWarps * 32, smem, stream>>>(p);                                         \
+    launch_chained(kern, grid, kWarps * 32, smem, stream, p);                                         \
   } while (0)
   switch (gc) {
     case 8: CB200_LAUNCH_GC(8); break;
@@ -236,6 +237,7 @@ int launch_general(const AttnParams& p, bool vector_ok, cudaStream_t stream) {
 // ---- split combine: fixed split order => bit-reproducible ------------------------
 template <typename T>
 __global__ void combine_splits_kernel(const AttnParams p) {
+  chain_enter();
   const int h = blockIdx.x;
   const int b = blockIdx.y;
   const int D = p.head_dim;
@@ -262,7 +264,7 @@ template <typename T>
 int launch_combine(const AttnParams& p, cudaStream_t stream) {
   const dim3 grid(p.heads, p.batch);
   const int threads = p.head_dim <= 32 ? 32 : (p.head_dim <= 64 ? 64 : 128);
-  combine_splits_kernel<T><<<grid, threads, 0, stream>>>(p);
+  launch_chained(combine_splits_kernel<T>, grid, threads, 0, stream, p);
   return launch_status();
 }
 

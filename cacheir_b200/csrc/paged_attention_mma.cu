@@ -175,6 +175,7 @@ template <typename T, int D, bool QUANT, bool CLUSTER>
 __global__ void __launch_bounds__(kFastThreads)
 paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                         const AttnParams p, const int stages) {
+  chain_enter();
   constexpr int kTileBytes = kPage * D * 2;       // one K or V page chunk: 4 KB at D=128
   constexpr int kPageBytes = 2 * kTileBytes;      // K + V
   constexpr int kStageBytes = kPagesPerStage * kPageBytes;
@@ -523,6 +524,7 @@ template <bool CLUSTER>
 __global__ void __launch_bounds__(kQ8Threads, 2)
 paged_decode_mma_q8_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                            const AttnParams p, const int stages) {
+  chain_enter();
   constexpr int D = 128;
   constexpr int kTileBytes = kPage * D;            // one K or V page chunk of bytes: 2 KB
   constexpr int kScaleBytes = 2 * kPage * 2;       // 16 K scales + 16 V scales, fp16
@@ -830,19 +832,7 @@ bool encode_pool(CUtensorMap* map, const void* base, int dtype, uint64_t rows, i
 template <typename Kernel>
 int launch_splits(Kernel kern, int threads, size_t smem, const CUtensorMap& tmap_k, const CUtensorMap& tmap_v, const AttnParams& p, int stages,
                   cudaStream_t stream) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(p.splits, p.kv_heads, p.batch);
-  cfg.blockDim = dim3(threads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = p.splits;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = p.cluster ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmap_k, tmap_v, p, stages);
+  const cudaError_t e = launch_clusters(kern, dim3(p.splits, p.kv_heads, p.batch), threads, smem, stream, dim3(p.cluster ? p.splits : 1, 1, 1), tmap_k, tmap_v, p, stages);
   if (e != cudaSuccess) return static_cast<int>(e);
   return launch_status();
 }
@@ -862,19 +852,7 @@ int launch_fast(const AttnParams& p, int dtype, uint64_t pool_rows, cudaStream_t
       auto kern = paged_decode_mma_kernel<T, D, true, false>;
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
       if (e != cudaSuccess) return static_cast<int>(e);
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3(1, p.kv_heads, p.quant_rows);
-      cfg.blockDim = dim3(kFastThreads, 1, 1);
-      cfg.dynamicSmemBytes = smem;
-      cfg.stream = stream;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 1;
-      attr[0].val.clusterDim.y = p.kv_heads;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      e = cudaLaunchKernelEx(&cfg, kern, tmap_k, tmap_v, p, stages);
+      e = launch_clusters(kern, dim3(1, p.kv_heads, p.quant_rows), kFastThreads, smem, stream, dim3(1, p.kv_heads, 1), tmap_k, tmap_v, p, stages);
       if (e != cudaSuccess) return static_cast<int>(e);
       return launch_status();
     }

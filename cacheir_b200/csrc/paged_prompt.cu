@@ -66,6 +66,7 @@ __device__ __forceinline__ uint32_t pack_halves(float lo, float hi) {
 template <int D>
 __global__ void __launch_bounds__(kThreads, 2)
 paged_prompt_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const PromptParams p) {
+  chain_enter();
   constexpr int kTileBytes = kPage * D * 2;        // one K or V page of one head
   constexpr int kPageBytes = 2 * kTileBytes;
   constexpr int kStageBytes = kStagePages * kPageBytes;
@@ -287,7 +288,7 @@ int launch(const PromptParams& p, const void* k_cache, const void* v_cache, uint
   auto kern = paged_prompt_kernel<D>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (e != cudaSuccess) return static_cast<int>(e);
-  kern<<<max_tiles * p.kv_heads, kThreads, kSmem, stream>>>(tmap_k, tmap_v, p);
+  launch_chained(kern, max_tiles * p.kv_heads, kThreads, kSmem, stream, tmap_k, tmap_v, p);
   return launch_status();
 }
 

@@ -64,6 +64,7 @@ __host__ __device__ constexpr int num_stages(int mp, int split, int bits = 8) {
 __global__ void __launch_bounds__(256)
 quantize_rows_kernel(const __half* __restrict__ x, long long x_stride, int M, int K, int mp,
                      int8_t* __restrict__ planes, float* __restrict__ sx, int* __restrict__ qsum) {
+  chain_enter();
   __shared__ float s_red[8];
   __shared__ int s_sum[8];
   const int m = blockIdx.x;
@@ -187,6 +188,7 @@ template <int PT>
 __global__ void __launch_bounds__(1024)
 quantize_rows_fast_kernel(const __half* __restrict__ x, long long x_stride, int M, int K, int mp,
                           int8_t* __restrict__ planes, float* __restrict__ sx, int* __restrict__ qsum) {
+  chain_enter();
   __shared__ float scratch[32];
   const int m = blockIdx.x;
   const int nvec = K / 8;
@@ -214,6 +216,7 @@ __global__ void __launch_bounds__(512)
 rms_norm_quantize_kernel(const __half* __restrict__ x, const __half* __restrict__ residual, const __half* __restrict__ weight,
                          __half* __restrict__ sum_out, __half* __restrict__ out, int M, int hidden, float eps, int mp,
                          int8_t* __restrict__ planes, float* __restrict__ sx, int* __restrict__ qsum) {
+  chain_enter();
   __shared__ float scratch[32];
   const int m = blockIdx.x;
   const int nvec = hidden / 8;
@@ -269,6 +272,7 @@ template <int PT>
 __global__ void __launch_bounds__(512)
 quantize_tall_kernel(const __half* __restrict__ x, long long x_stride, int M, const int* __restrict__ n_rows, int K,
                      int8_t* __restrict__ planes, float* __restrict__ sx, int* __restrict__ qsum) {
+  chain_enter();
   __shared__ float scratch[32];
   const int m = blockIdx.x;
   if (m >= (n_rows ? min(M, *n_rows) : M)) return;
@@ -288,6 +292,7 @@ template <int PT>
 __global__ void __launch_bounds__(512)
 rms_norm_quantize_tall_kernel(const __half* __restrict__ x, const __half* __restrict__ weight, int M, const int* __restrict__ n_rows,
                               int hidden, float eps, int8_t* __restrict__ planes, float* __restrict__ sx, int* __restrict__ qsum) {
+  chain_enter();
   __shared__ float scratch[32];
   const int m = blockIdx.x;
   if (m >= (n_rows ? min(M, *n_rows) : M)) return;
@@ -341,6 +346,7 @@ struct I8Params {
 // accumulator, and twice as many CTAs as whole-half tiles would give.
 constexpr int kPairRows = 64;
 
+constexpr int kAhead = 8;          // weight tiles a CTA asks for before its turn
 constexpr int kTailBytes = 1024;   // scratch behind the ring and the exchange buffer: barriers, TMEM base, per-row constants
 
 template <int MP, int SPLIT, bool ROPE, int BITS>
@@ -406,6 +412,16 @@ qgemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const I8Params p) {
     }
     bulk_load(smem_u32(s_x + s * kXBytes), p.x_planes + static_cast<size_t>(kb) * kXBytes, kXBytes, bar);
   };
+  auto ask_for = [&](int i) {
+    const int kb = kb_begin + i;
+    constexpr int kRowBytes = BITS == 4 ? kBlockK / 2 : kBlockK;
+    if (p.tiled) {
+      bulk_prefetch(p.w_tiled + (static_cast<size_t>(blockIdx.x) * kblocks_all + kb) * kLoadBytes, kLoadBytes);
+    } else {
+      tma_prefetch_2d(&tmap_w, kb * kRowBytes, n0);
+      if (swiglu) tma_prefetch_2d(&tmap_w, kb * kRowBytes, p.N / 2 + n0);
+    }
+  };
   const int pre = total < kStages ? total : kStages;
 
   // Set-up: thread 0 initialises the barriers and goes straight on to request the first ring of
@@ -423,12 +439,16 @@ qgemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const I8Params p) {
     __syncwarp();
     asm volatile("bar.arrive 2, %0;" ::"n"(kThreads) : "memory");
     if (clustered) cluster_arrive_relaxed();   // phase A: this CTA runs and its exchange barrier exists
+    if (lane == 0)                             // the weights set out for L2 while the kernel before this one is at work
+      for (int i = 0; i < min(total, kAhead); ++i) ask_for(i);
+    chain_wait();
     if (lane == 0) {
       for (int i = 0; i < pre; ++i) load_stage(i, i);
     }
   } else {
-    if (warp == 1) tc_alloc(smem_u32(tmem_slot), kTmemCols);
     if (clustered) cluster_arrive_relaxed();
+    chain_enter();
+    if (warp == 1) tc_alloc(smem_u32(tmem_slot), kTmemCols);
     tc_fence_before();
     asm volatile("bar.sync 2, %0;" ::"n"(kThreads) : "memory");
     tc_fence_after();
@@ -801,9 +821,9 @@ int launch_quantize(const __half* x, long long x_stride, int M, int K, int mp, v
   int8_t* planes = static_cast<int8_t*>(workspace);
   float* sx = reinterpret_cast<float*>(planes + static_cast<size_t>(2 * mp) * K);
   int* qsum = reinterpret_cast<int*>(sx + 64);
-  if (K <= 8192) quantize_rows_fast_kernel<1><<<mp, 1024, 0, stream>>>(x, x_stride, M, K, mp, planes, sx, qsum);
-  else if (K <= 16384) quantize_rows_fast_kernel<2><<<mp, 1024, 0, stream>>>(x, x_stride, M, K, mp, planes, sx, qsum);
-  else quantize_rows_kernel<<<mp, 256, 0, stream>>>(x, x_stride, M, K, mp, planes, sx, qsum);
+  if (K <= 8192) launch_chained(quantize_rows_fast_kernel<1>, mp, 1024, 0, stream, x, x_stride, M, K, mp, planes, sx, qsum);
+  else if (K <= 16384) launch_chained(quantize_rows_fast_kernel<2>, mp, 1024, 0, stream, x, x_stride, M, K, mp, planes, sx, qsum);
+  else launch_chained(quantize_rows_kernel, mp, 256, 0, stream, x, x_stride, M, K, mp, planes, sx, qsum);
   return launch_status();
 }
 
@@ -817,19 +837,7 @@ cudaError_t launch_i8_split(const CUtensorMap& tmap_w, const I8Params& p, cudaSt
   auto kern = qgemm_i8_kernel<MP, SPLIT, ROPE, BITS>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem));
   if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(p.n_tiles, SPLIT, 1);
-  cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = kSmem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = SPLIT;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, tmap_w, p);
+  return launch_clusters(kern, dim3(p.n_tiles, SPLIT, 1), kThreads, kSmem, stream, dim3(1, SPLIT, 1), tmap_w, p);
 }
 
 template <int MP, bool ROPE, int BITS>
@@ -905,11 +913,11 @@ TallPlanes tall_planes(void* workspace, int M, int K) {
 int qgemm_i8_quantize_tall(const void* x, long long x_stride, int M, const int* n_rows, int K, void* workspace, cudaStream_t stream) {
   const TallPlanes t = tall_planes(workspace, M, K);
   const __half* xp = static_cast<const __half*>(x);
-  if (K <= 2048) quantize_tall_kernel<1><<<M, 256, 0, stream>>>(xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);
-  else if (K <= 4096) quantize_tall_kernel<1><<<M, 512, 0, stream>>>(xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);
-  else if (K <= 8192) quantize_tall_kernel<2><<<M, 512, 0, stream>>>(xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);
-  else if (K <= 16384) quantize_tall_kernel<4><<<M, 512, 0, stream>>>(xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);
-  else quantize_tall_kernel<8><<<M, 512, 0, stream>>>(xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);   // K <= 32768
+  if (K <= 2048) launch_chained(quantize_tall_kernel<1>, M, 256, 0, stream, xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);
+  else if (K <= 4096) launch_chained(quantize_tall_kernel<1>, M, 512, 0, stream, xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);
+  else if (K <= 8192) launch_chained(quantize_tall_kernel<2>, M, 512, 0, stream, xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);
+  else if (K <= 16384) launch_chained(quantize_tall_kernel<4>, M, 512, 0, stream, xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);
+  else launch_chained(quantize_tall_kernel<8>, M, 512, 0, stream, xp, x_stride, M, n_rows, K, t.planes, t.sx, t.qsum);   // K <= 32768
   return launch_status();
 }
 
@@ -918,9 +926,9 @@ int qgemm_i8_rms_norm_quantize_tall(const void* x, const void* weight, int M, co
   const TallPlanes t = tall_planes(workspace, M, hidden);
   const __half* xp = static_cast<const __half*>(x);
   const __half* wp = static_cast<const __half*>(weight);
-  if (hidden <= 2048) rms_norm_quantize_tall_kernel<1><<<M, 256, 0, stream>>>(xp, wp, M, n_rows, hidden, eps, t.planes, t.sx, t.qsum);
-  else if (hidden <= 4096) rms_norm_quantize_tall_kernel<1><<<M, 512, 0, stream>>>(xp, wp, M, n_rows, hidden, eps, t.planes, t.sx, t.qsum);
-  else if (hidden <= 8192) rms_norm_quantize_tall_kernel<2><<<M, 512, 0, stream>>>(xp, wp, M, n_rows, hidden, eps, t.planes, t.sx, t.qsum);
+  if (hidden <= 2048) launch_chained(rms_norm_quantize_tall_kernel<1>, M, 256, 0, stream, xp, wp, M, n_rows, hidden, eps, t.planes, t.sx, t.qsum);
+  else if (hidden <= 4096) launch_chained(rms_norm_quantize_tall_kernel<1>, M, 512, 0, stream, xp, wp, M, n_rows, hidden, eps, t.planes, t.sx, t.qsum);
+  else if (hidden <= 8192) launch_chained(rms_norm_quantize_tall_kernel<2>, M, 512, 0, stream, xp, wp, M, n_rows, hidden, eps, t.planes, t.sx, t.qsum);
   else return CACHEIR_B200_EUNSUPPORTED;
   return launch_status();
 }
@@ -971,8 +979,8 @@ int qgemm_i8_rms_norm_quantize(const void* x, const void* residual, const void* 
   const __half* wp = static_cast<const __half*>(weight);
   __half* sp = static_cast<__half*>(sum_out);
   __half* op = static_cast<__half*>(out);
-  if (hidden <= 4096) rms_norm_quantize_kernel<1><<<mp, 512, 0, stream>>>(xp, rp, wp, sp, op, M, hidden, eps, mp, planes, sx, qsum);
-  else if (hidden <= 8192) rms_norm_quantize_kernel<2><<<mp, 512, 0, stream>>>(xp, rp, wp, sp, op, M, hidden, eps, mp, planes, sx, qsum);
+  if (hidden <= 4096) launch_chained(rms_norm_quantize_kernel<1>, mp, 512, 0, stream, xp, rp, wp, sp, op, M, hidden, eps, mp, planes, sx, qsum);
+  else if (hidden <= 8192) launch_chained(rms_norm_quantize_kernel<2>, mp, 512, 0, stream, xp, rp, wp, sp, op, M, hidden, eps, mp, planes, sx, qsum);
   else return CACHEIR_B200_EUNSUPPORTED;
   return launch_status();
 }

@@ -69,6 +69,7 @@ struct RowsParams {
 template <int BITS, bool SWIGLU, int SPLIT>
 __global__ void __launch_bounds__(num_threads(BITS), 1)
 qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const RowsParams p) {
+  chain_enter();
   constexpr int S = num_stages(BITS);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -374,19 +375,7 @@ int launch_split(const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, const Row
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (e != cudaSuccess) return static_cast<int>(e);
   const int clusters = SPLIT > 1 || tiles < kNumSMs / 2 ? tiles : kNumSMs / 2;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(2 * SPLIT * clusters, 1, 1);
-  cfg.blockDim = dim3(num_threads(BITS), 1, 1);
-  cfg.dynamicSmemBytes = kSmem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2 * SPLIT;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, kern, tmap_w, tmap_x, p);
+  e = launch_clusters(kern, dim3(2 * SPLIT * clusters, 1, 1), num_threads(BITS), kSmem, stream, dim3(2 * SPLIT, 1, 1), tmap_w, tmap_x, p);
   if (e != cudaSuccess) return static_cast<int>(e);
   return launch_status();
 }

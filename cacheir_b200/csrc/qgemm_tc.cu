@@ -232,6 +232,7 @@ __device__ __forceinline__ void unpack8_slow(const uint8_t* bytes, int first, fl
 template <int BITS, int MP, bool GROUPED>
 __global__ void __launch_bounds__(kThreads, 1)
 qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const TcParams p) {
+  chain_enter();
   constexpr int kStages = num_stages(BITS, MP);
   constexpr int kRawBytes = BITS == 8 ? kBlockN * 128 : kBlockN * 64;   // per stage
   constexpr int kXBytes = MP * kBlockK * 2;
@@ -763,19 +764,7 @@ int launch_tc(const QGemvParams& q, cudaStream_t stream) {
   auto kern = qgemm_tc_kernel<BITS, MP, GROUPED>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(n_tiles, p.split_k, 1);
-  cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = kSmem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = p.split_k;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, kern, tmap_w, tmap_x, p);
+  e = launch_clusters(kern, dim3(n_tiles, p.split_k, 1), kThreads, kSmem, stream, dim3(1, p.split_k, 1), tmap_w, tmap_x, p);
   if (e != cudaSuccess) return static_cast<int>(e);
   return launch_status();
 }

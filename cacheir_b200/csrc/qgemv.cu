@@ -48,6 +48,7 @@ __device__ __forceinline__ float scale_at(const void* scales, int scale_dtype, s
 template <typename XT, int BITS, int MT>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 qgemv_cuda_core_kernel(const QGemvParams p) {
+  chain_enter();
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int n_out = blockIdx.x * kWarpsPerBlock + warp;
@@ -159,10 +160,10 @@ int launch_mt(const QGemvParams& p, cudaStream_t stream) {
   const dim3 grid((n_out_total + kWarpsPerBlock - 1) / kWarpsPerBlock, (p.M + mt - 1) / mt);
   if (grid.y > 65535) return CACHEIR_B200_ELIMIT;
   switch (mt) {
-    case 8: qgemv_cuda_core_kernel<XT, BITS, 8><<<grid, kWarpsPerBlock * 32, 0, stream>>>(p); break;
-    case 4: qgemv_cuda_core_kernel<XT, BITS, 4><<<grid, kWarpsPerBlock * 32, 0, stream>>>(p); break;
-    case 2: qgemv_cuda_core_kernel<XT, BITS, 2><<<grid, kWarpsPerBlock * 32, 0, stream>>>(p); break;
-    default: qgemv_cuda_core_kernel<XT, BITS, 1><<<grid, kWarpsPerBlock * 32, 0, stream>>>(p); break;
+    case 8: launch_chained(qgemv_cuda_core_kernel<XT, BITS, 8>, grid, kWarpsPerBlock * 32, 0, stream, p); break;
+    case 4: launch_chained(qgemv_cuda_core_kernel<XT, BITS, 4>, grid, kWarpsPerBlock * 32, 0, stream, p); break;
+    case 2: launch_chained(qgemv_cuda_core_kernel<XT, BITS, 2>, grid, kWarpsPerBlock * 32, 0, stream, p); break;
+    default: launch_chained(qgemv_cuda_core_kernel<XT, BITS, 1>, grid, kWarpsPerBlock * 32, 0, stream, p); break;
   }
   return launch_status();
 }

@@ -92,6 +92,7 @@ constexpr uint32_t kNibLo = 0x000F000Fu, kNibHi = 0x00F000F0u, kFp16Magic = 0x64
 template <bool SWIGLU, bool GROUPED, bool F16SCALE>
 __global__ void __launch_bounds__(kThreadsMma, 1)
 qgemv_mma_int4_kernel(const __grid_constant__ CUtensorMap tmap_w, const MmaGemvParams p) {
+  chain_enter();
   using namespace ptx;
   constexpr int HALVES = SWIGLU ? 2 : 1;     // weight tiles per output tile
   using scale_t = typename std::conditional<F16SCALE, __half, float>::type;
@@ -381,7 +382,7 @@ template <bool SWIGLU, bool GROUPED, bool F16SCALE>
 int launch_mma_variant(const CUtensorMap& tmap, const MmaGemvParams& p, int grid, size_t smem, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(qgemv_mma_int4_kernel<SWIGLU, GROUPED, F16SCALE>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  qgemv_mma_int4_kernel<SWIGLU, GROUPED, F16SCALE><<<grid, kThreadsMma, smem, stream>>>(tmap, p);
+  launch_chained(qgemv_mma_int4_kernel<SWIGLU, GROUPED, F16SCALE>, grid, kThreadsMma, smem, stream, tmap, p);
   return launch_status();
 }
 

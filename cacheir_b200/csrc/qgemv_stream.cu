@@ -26,6 +26,7 @@ constexpr int kCols = 128;              // columns of a k block
 constexpr int kXRow = 2 * kCols;        // bytes of an activation row in it
 constexpr int kSmemLimit = 192 * 1024;  // rings; group scales come on top
 constexpr int kScaleLimit = 34 * 1024;
+constexpr int kAhead = 32;              // k blocks a CTA asks for before its turn
 
 struct StreamParams {
   const __half* x;
@@ -142,6 +143,21 @@ qgemv_stream_kernel(const StreamParams p) {
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  // The weights set out for L2 while the kernel before this one is at work: in tile order 1 KB per MMA tile and k block, in
+  // row order a run of each row.
+  if (p.tiled) {
+    const int items = 2 * RG * min(kblocks - kb0, kAhead);
+    for (int i = threadIdx.x; i < items; i += kThreads) {
+      const int row = tile_row(i % (2 * RG));
+      if (row < p.N) ptx::bulk_prefetch(p.packed + ((static_cast<size_t>(row >> 7) * kblocks_all + kb0 + i / (2 * RG)) * 128 + (row & 127)) * 64, 16 * 64);
+    }
+  } else {
+    for (int i = threadIdx.x; i < kRows; i += kThreads) {
+      const int row = tile_row(i >> 4) + (i & 15);
+      if (row < p.N) ptx::bulk_prefetch(p.packed + static_cast<size_t>(row) * (p.K / 2) + kb0 * 64, 64 * min(kblocks - kb0, kAhead));
+    }
+  }
+  chain_enter();
   for (int j = 0; j < S - 1; ++j) load(j);
 
   // per-row constants: scale (per row formats) and the zero point as an exact fp16 offset
@@ -307,19 +323,7 @@ int launch(const StreamParams& p, int ctas, cudaStream_t stream) {
   auto kern = qgemv_stream_kernel<NT, RG, GROUPED, SWIGLU>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return static_cast<int>(e);
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(ctas, p.split, 1);
-  cfg.blockDim = dim3(32 * RG * k_groups(RG), 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = p.split;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = p.split > 1 ? 1 : 0;
-  e = cudaLaunchKernelEx(&cfg, kern, p);
+  e = launch_clusters(kern, dim3(ctas, p.split, 1), 32 * RG * k_groups(RG), smem, stream, dim3(1, p.split, 1), p);
   if (e != cudaSuccess) return static_cast<int>(e);
   return launch_status();
 }

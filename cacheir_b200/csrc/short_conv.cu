@@ -22,6 +22,7 @@ __device__ __forceinline__ float* slot_inputs(const Args& a, int seg) {
 template <typename T, int VEC, int TAPS>
 __global__ void __launch_bounds__(kThreads)
 short_conv_kernel(const Args a) {
+  chain_enter();
   constexpr int H = TAPS - 1, U = 8;   // inputs kept; rows requested at a time
   const RaggedItem it = find_item(a.cu_rows, a.segments, kPieceRows, blockIdx.x);
   const int c = (blockIdx.y * kThreads + threadIdx.x) * VEC;
@@ -95,6 +96,7 @@ short_conv_kernel(const Args a) {
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 long_conv_kernel(const Args a) {
+  chain_enter();
   const RaggedItem it = find_item(a.cu_rows, a.segments, kPieceRows, blockIdx.x);
   const int c = blockIdx.y * kThreads + threadIdx.x, H = a.taps - 1;
   if (it.seg < 0 || c >= a.channels) return;
@@ -121,11 +123,11 @@ int launch_conv(const Args& a, cudaStream_t st) {
   const int items = ragged_items(a.rows, a.segments, kPieceRows), per_block = kThreads * VEC;
   const dim3 grid(items, (a.channels + per_block - 1) / per_block);
   switch (a.taps) {
-    case 1: short_conv_kernel<T, VEC, 1><<<grid, kThreads, 0, st>>>(a); break;
-    case 2: short_conv_kernel<T, VEC, 2><<<grid, kThreads, 0, st>>>(a); break;
-    case 3: short_conv_kernel<T, VEC, 3><<<grid, kThreads, 0, st>>>(a); break;
-    case 4: short_conv_kernel<T, VEC, 4><<<grid, kThreads, 0, st>>>(a); break;
-    default: long_conv_kernel<T><<<dim3(items, (a.channels + kThreads - 1) / kThreads), kThreads, 0, st>>>(a);
+    case 1: launch_chained(short_conv_kernel<T, VEC, 1>, grid, kThreads, 0, st, a); break;
+    case 2: launch_chained(short_conv_kernel<T, VEC, 2>, grid, kThreads, 0, st, a); break;
+    case 3: launch_chained(short_conv_kernel<T, VEC, 3>, grid, kThreads, 0, st, a); break;
+    case 4: launch_chained(short_conv_kernel<T, VEC, 4>, grid, kThreads, 0, st, a); break;
+    default: launch_chained(long_conv_kernel<T>, dim3(items, (a.channels + kThreads - 1) / kThreads), kThreads, 0, st, a);
   }
   return launch_status();
 }

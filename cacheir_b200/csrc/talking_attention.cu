@@ -42,6 +42,7 @@ constexpr int kHeldHeads = 8;
 template <typename T, int MIXED>
 __global__ void __launch_bounds__(256)
 talking_prepare_kernel(const PrepareParams p, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ q_out) {
+  chain_enter();
   extern __shared__ float sm[];                  // MIXED: [heads][dim] queries, [heads][heads] talk
   const Args& a = p.a;
   const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -136,6 +137,7 @@ constexpr int kSimpleKeys = 32;
 template <typename T>
 __global__ void __launch_bounds__(256)
 talking_simple_kernel(const Args a, const T* __restrict__ q, T* __restrict__ out) {
+  chain_enter();
   extern __shared__ float sm[];
   float* s_q = sm;                               // [heads][dim]
   float* s_o = s_q + a.heads * a.dim;            // [heads][vdim]
@@ -253,6 +255,7 @@ __device__ __forceinline__ void consumers_sync() { asm volatile("barrier.cta.syn
 template <int BANDS, int PAIRS, int TILE>
 __global__ void __launch_bounds__(kStepThreads, 1)
 talking_step_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const StepParams p) {
+  chain_enter();
   constexpr int kBox = TILE * 128, kBlocks = TILE / 16;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -590,19 +593,7 @@ int launch_step(const StepParams& p, cudaStream_t st) {
   auto kern = talking_step_kernel<BANDS, PAIRS, TILE>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(p.s.smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(p.splits, p.s.sets, a.rows);
-  cfg.blockDim = dim3(kStepThreads, 1, 1);
-  cfg.dynamicSmemBytes = p.s.smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = p.splits;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = p.splits > 1 ? 1 : 0;
-  e = cudaLaunchKernelEx(&cfg, kern, tk, tv, p);
+  e = launch_clusters(kern, dim3(p.splits, p.s.sets, a.rows), kStepThreads, p.s.smem, st, dim3(p.splits, 1, 1), tk, tv, p);
   if (e != cudaSuccess) return static_cast<int>(e);
   return launch_status();
 }
@@ -632,7 +623,7 @@ extern "C" int cacheir_b200_talking_prepare(const cacheir_b200_talking_args* arg
   if (!mixed) {
     const dim3 grid(a.rows, (a.heads + 2 * a.kv_heads + 7) / 8);
     if (grid.y > 65535) return CACHEIR_B200_ELIMIT;
-    CB200_HYBRID_DTYPE(a.dtype, (talking_prepare_kernel<T, 0><<<grid, 256, 0, st>>>(p, static_cast<const T*>(q), static_cast<const T*>(k),
+    CB200_HYBRID_DTYPE(a.dtype, (launch_chained(talking_prepare_kernel<T, 0>, grid, 256, 0, st, p, static_cast<const T*>(q), static_cast<const T*>(k),
                                                                                      static_cast<const T*>(v), static_cast<T*>(q_out))));
     return launch_status();
   }
@@ -643,7 +634,7 @@ extern "C" int cacheir_b200_talking_prepare(const cacheir_b200_talking_args* arg
   {                                                                                                                                   \
     const cudaError_t e = cudaFuncSetAttribute(talking_prepare_kernel<T, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)); \
     if (e != cudaSuccess) return static_cast<int>(e);                                                                                 \
-    talking_prepare_kernel<T, MIXED><<<dim3(a.rows, 1), 256, smem, st>>>(p, static_cast<const T*>(q), static_cast<const T*>(k),        \
+    launch_chained(talking_prepare_kernel<T, MIXED>, dim3(a.rows, 1), 256, smem, st, p, static_cast<const T*>(q), static_cast<const T*>(k),        \
                                                                          static_cast<const T*>(v), static_cast<T*>(q_out));           \
   }
   CB200_HYBRID_DTYPE(a.dtype, {
@@ -667,7 +658,7 @@ extern "C" int cacheir_b200_talking_simple(const cacheir_b200_talking_args* args
   CB200_HYBRID_DTYPE(a.dtype, {
     const cudaError_t e = cudaFuncSetAttribute(talking_simple_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
-    talking_simple_kernel<T><<<a.rows, 256, smem, as_stream(stream)>>>(a, static_cast<const T*>(q), static_cast<T*>(out));
+    launch_chained(talking_simple_kernel<T>, a.rows, 256, smem, as_stream(stream), a, static_cast<const T*>(q), static_cast<T*>(out));
   });
   return launch_status();
 }

@@ -120,6 +120,7 @@ template <int TILES>
 __global__ void __launch_bounds__(kThreads, 1)
 talking_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const PromptParams p) {
+  chain_enter();
   constexpr int kStage = TILES * kQBox + 2 * kKBox;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -385,7 +386,7 @@ int launch_prompt(const PromptParams& p, const void* q, int items, cudaStream_t 
   auto kern = talking_prompt_kernel<TILES>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  kern<<<dim3(a.kv_heads * p.subs, items), kThreads, smem, st>>>(tq, tk, tv, p);
+  launch_chained(kern, dim3(a.kv_heads * p.subs, items), kThreads, smem, st, tq, tk, tv, p);
   return launch_status();
 }
 

@@ -32,6 +32,7 @@ __device__ __forceinline__ int key_column(const PrepareParams& p, bool tied, int
 template <typename T, int VEC, bool WHOLE>
 __global__ void __launch_bounds__(WHOLE ? 512 : 256)
 tied_prepare_kernel(const PrepareParams p, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ q_out) {
+  chain_enter();
   constexpr int kWarpsHere = (WHOLE ? 512 : 256) / 32;
   __shared__ float s_part[2][kWarpsHere];
   const cacheir_b200_tied_args& a = p.a;
@@ -142,6 +143,7 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 tied_simple_kernel(const cacheir_b200_tied_args a, const T* __restrict__ q, const T* __restrict__ gate, long long gate_stride,
                    T* __restrict__ out) {
+  chain_enter();
   extern __shared__ float sm[];
   __shared__ float scratch[32];
   const int lead = tied_lead(a.key_from), width = a.width, qw = width - lead;
@@ -232,6 +234,7 @@ __device__ __forceinline__ void cluster_sync_all() {
 template <int DB, int kSteps>
 __global__ void __launch_bounds__(kStepThreads, DB <= 2 ? 2 : 1)
 tied_step_kernel(const __grid_constant__ CUtensorMap tmap, const StepParams p) {
+  chain_enter();
   constexpr int kTiles = DB * 8;                 // 8-column tiles of the output
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -496,19 +499,7 @@ int launch_step(const StepParams& p, int segments, cudaStream_t st) {
   auto kern = tied_step_kernel<DB, kSteps>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(p.splits, a.kv_heads * p.subs, segments);
-  cfg.blockDim = dim3(kStepThreads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = p.splits;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = p.splits > 1 ? 1 : 0;
-  e = cudaLaunchKernelEx(&cfg, kern, map, p);
+  e = launch_clusters(kern, dim3(p.splits, a.kv_heads * p.subs, segments), kStepThreads, smem, st, dim3(p.splits, 1, 1), map, p);
   if (e != cudaSuccess) return static_cast<int>(e);
   return launch_status();
 }
@@ -546,7 +537,7 @@ extern "C" int cacheir_b200_tied_prepare(const cacheir_b200_tied_args* args, con
   const bool vec = d % 4 == 0 && a.dim % 4 == 0 && rot_dims % 8 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && aligned_to(q, quad) &&
                    aligned_to(k, quad) && (!v || (v_stride % 4 == 0 && aligned_to(v, quad))) && aligned_to(a.pool, quad) && aligned_to(q_out, quad);
 #define CB200_PREPARE(VEC, WHOLE)                                                                                              \
-  tied_prepare_kernel<T, VEC, WHOLE><<<grid, WHOLE ? 512 : 256, 0, as_stream(stream)>>>(                                        \
+  launch_chained(tied_prepare_kernel<T, VEC, WHOLE>, grid, WHOLE ? 512 : 256, 0, as_stream(stream), \
       p, static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), static_cast<T*>(q_out))
   CB200_HYBRID_DTYPE(a.dtype, {
     if (vec && whole) CB200_PREPARE(4, true);
@@ -566,7 +557,7 @@ extern "C" int cacheir_b200_tied_attention_simple(const cacheir_b200_tied_args* 
   const size_t smem = static_cast<size_t>(args->dim + args->width - tied_lead(args->key_from) + 128) * 4;
   if (smem > 48 * 1024) return CACHEIR_B200_ELIMIT;
   const dim3 grid(args->rows, args->heads);
-  CB200_HYBRID_DTYPE(args->dtype, (tied_simple_kernel<T><<<grid, 128, smem, as_stream(stream)>>>(
+  CB200_HYBRID_DTYPE(args->dtype, (launch_chained(tied_simple_kernel<T>, grid, 128, smem, as_stream(stream),
                                       *args, static_cast<const T*>(q), static_cast<const T*>(gate), gate_stride, static_cast<T*>(out))));
   return launch_status();
 }

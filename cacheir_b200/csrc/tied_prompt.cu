@@ -109,6 +109,7 @@ __device__ __noinline__ bool wait_long(uint32_t bar, uint32_t parity, int code) 
 template <int TILES, bool FIXED, int TERMS>
 __global__ void __launch_bounds__(kThreads, 1)
 tied_prompt_kernel(const __grid_constant__ CUtensorMap tmap_kv, const __grid_constant__ CUtensorMap tmap_q, const PromptParams p) {
+  chain_enter();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   const cacheir_b200_tied_args& a = p.a;
@@ -478,7 +479,7 @@ int launch_prompt(const PromptParams& p, const void* q, int items, cudaStream_t 
   auto kern = tied_prompt_kernel<TILES, FIXED, TERMS>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  kern<<<dim3(a.kv_heads * p.subs, items), kThreads, smem, st>>>(tkv, tq, p);
+  launch_chained(kern, dim3(a.kv_heads * p.subs, items), kThreads, smem, st, tkv, tq, p);
   return launch_status();
 }
 
