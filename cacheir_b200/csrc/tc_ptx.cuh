@@ -9,8 +9,6 @@
 namespace cb200 {
 namespace ptx {
 
-constexpr uint32_t kPollLimit = 8u * 1000u * 1000u;   // bounded waits: ~1 s, then give up and flag
-
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -31,14 +29,34 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
-// Returns false, after recording `code` in *status, when the poll budget runs out.
+// The same, the hardware suspending the thread for up to `hint` ns instead of letting it poll: a polling warp takes issue slots from
+// the warps of its scheduler that feed the tensor cores.
+__device__ __forceinline__ bool mbar_try_wait_suspended(uint32_t bar, uint32_t parity, uint32_t hint) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done) : "r"(bar), "r"(parity), "r"(hint) : "memory");
+  return done != 0;
+}
+__device__ __forceinline__ uint64_t timer_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+constexpr uint64_t kWaitLimitNs = 1000u * 1000u * 1000u;   // bounded waits: 1 s, then give up and flag
+constexpr uint32_t kSuspendNs = 20u * 1000u;
+// Returns false, after recording `code` in *status, when the time is up.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status, int code) {
-  for (uint32_t i = 0; i < kPollLimit; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (i > 64) __nanosleep(32);
-  }
-  atomicCAS(status, 0, code);
-  return false;
+  if (mbar_try_wait(bar, parity)) return true;         // (56 cycles where the phase is over; with a hint 92)
+  const uint64_t begin = timer_ns();
+  while (!mbar_try_wait_suspended(bar, parity, kSuspendNs))
+    if (timer_ns() - begin > kWaitLimitNs) {
+      atomicCAS(status, 0, code);
+      return false;
+    }
+  return true;
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
   asm volatile(
