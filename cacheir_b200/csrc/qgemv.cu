@@ -238,6 +238,7 @@ int qgemv_dispatch(const void* x, const void* norm_weight, float norm_eps, const
   p.vector_ok = aligned_to(packed, 16) && row_bytes % 16 == 0 && aligned_to(x, 16) &&
                 (p.x_stride * esize) % 16 == 0;
   cudaStream_t st = as_stream(stream);
+  if (qgemm_w4_preferred(p)) return plan_only ? (4 << 8) | qgemm_w4_plan(p) : launch_qgemm_w4(p, st);
   // More than 64 rows of per-row codes in tile order, with scratch for all of them: one launch over blocks of 128 rows (the same
   // bits as the 64-row passes below, which stream the weights once per 64 rows: 100 rows of 14336 x 4096 bytes 25.6 us against 45.6).
   // (Rows that are in the workspace already: cacheir_b200_qgemm_rows.)
@@ -259,7 +260,8 @@ int qgemv_dispatch(const void* x, const void* norm_weight, float norm_eps, const
         c.x = static_cast<const char*>(x) + static_cast<size_t>(m0) * p.x_stride * esize;
         c.y = static_cast<char*>(y) + static_cast<size_t>(m0) * n_out * esize;
         c.residual = residual ? static_cast<const char*>(residual) + static_cast<size_t>(m0) * n_out * esize : nullptr;
-        const int rc = i8_ok ? launch_qgemm_i8(c, workspace, st) : qgemv_stream_supported(c) ? launch_qgemv_stream(c, st) : launch_qgemm_tc(c, st);
+        const int rc = i8_ok ? launch_qgemm_i8(c, workspace, st) : qgemm_w4_preferred(c) ? launch_qgemm_w4(c, st)
+                     : qgemv_stream_supported(c) ? launch_qgemv_stream(c, st) : launch_qgemm_tc(c, st);
         if (rc != 0) return rc;
       }
       return 0;
@@ -337,7 +339,8 @@ extern "C" int cacheir_b200_device_status(int reset) {
   const int gemv = qgemv_mma_device_status(reset != 0);
   const int rows = qgemm_i8_rows_device_status(reset != 0);
   const int prompt = paged_prompt_device_status(reset != 0);
-  for (const int status : {gemm, attn, i8, peer, gemv, rows, prompt})
+  const int w4 = qgemm_w4_device_status(reset != 0);
+  for (const int status : {gemm, attn, i8, peer, gemv, rows, prompt, w4})
     if (status != 0) return status;
   return 0;
 }

@@ -51,6 +51,13 @@ bool qgemv_stream_supported(const QGemvParams& p);
 int launch_qgemv_stream(const QGemvParams& p, cudaStream_t stream);
 int qgemv_stream_plan(const QGemvParams& p);   // (row groups << 4) | CTAs along K that the launcher would choose
 
+// int4 dequant-GEMM for up to 128 rows with the weights in tensor memory (both code layouts).
+bool qgemm_w4_supported(const QGemvParams& p);
+bool qgemm_w4_preferred(const QGemvParams& p);  // is it the fastest of the int4 products?
+int launch_qgemm_w4(const QGemvParams& p, cudaStream_t stream);
+int qgemm_w4_plan(const QGemvParams& p);        // 128 | (4 << 4) | CTAs along K
+int qgemm_w4_device_status(bool reset);
+
 // Tensor-core (tcgen05) small-M GEMM: weights are the 128-row MMA operand.
 bool qgemm_tc_supported(const QGemvParams& p);
 int launch_qgemm_tc(const QGemvParams& p, cudaStream_t stream);

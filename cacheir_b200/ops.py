@@ -224,8 +224,8 @@ def qgemv(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor | None, ze
 def qgemv_plan(m: int, n: int, k: int, *, bits: int, group_size: int = 0, epilogue: int = EPI_NONE, tiled: bool = False,
                prequantized: bool = False, paired: bool = False, workspace: bool = True) -> dict:
     """Which kernel `qgemv` launches for these extents: {"family": "i8"|"f16"|"cuda_core"|"stream_int4", "split_k", "kernel"},
-    kernel: the family or, within it, "i8_rows" (blocks of 128 rows), "stream" with its "row_groups" and "split", "stream_rows" (many
-    weight rows in row order). epilogue 3 asks about `qkv_rope_append`."""
+    kernel: the family or, within it, "i8_rows" (blocks of 128 rows), "stream" with its "row_groups", "split" and "tensor_memory"
+    (is that where the weights go?), "stream_rows" (many weight rows in row order). epilogue 3 asks about `qkv_rope_append`."""
     layout = (1 if tiled else 0) | (2 if prequantized else 0) | (4 if paired else 0)
     code = int(_lib.load().cacheir_b200_qgemv_plan(int(m), int(n), int(k), int(bits), int(group_size), int(epilogue), layout,
                                                    1 if workspace else 0))
@@ -236,7 +236,8 @@ def qgemv_plan(m: int, n: int, k: int, *, bits: int, group_size: int = 0, epilog
     if family == "i8" and detail == 0:
         plan["kernel"] = "i8_rows"
     elif family == "stream_int4":
-        plan.update({"kernel": "stream", "row_groups": detail >> 4, "split": detail & 15} if detail else {"kernel": "stream_rows"})
+        plan.update({"kernel": "stream", "row_groups": detail >> 4 & 7, "split": detail & 15, "tensor_memory": detail >= 128} if detail
+                    else {"kernel": "stream_rows"})
     return plan
 
 

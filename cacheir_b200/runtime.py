@@ -753,8 +753,8 @@ class _DecodePlan:
                 and hasattr(self, "_gemm_ws") and not self._streams(weight, ops.EPI_SWIGLU if swiglu else ops.EPI_NONE))
 
     def _streams(self, weight: B200PackedWeight, epilogue: int) -> bool:
-        """Does the streaming kernel run this fp16 product? It takes the rows as they are, without a pre-pass."""
-        if weight.bits != 4 or weight.group_size or self.batch > 8 or weight.shape[1] % 128:
+        """Does a streaming int4 kernel run this fp16 product? It takes the rows as they are, without a pre-pass."""
+        if weight.bits != 4 or weight.group_size or self.batch > 64 or weight.shape[1] % 128:
             return False
         return ops.qgemv_plan(self.batch, *weight.shape, bits=4, epilogue=epilogue, tiled=weight.tiled, paired=weight.paired)["family"] == "stream_int4"
 

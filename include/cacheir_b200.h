@@ -217,9 +217,9 @@ int cacheir_b200_qgemv(const void* x, const void* packed, const void* scales,
  * 64-row chunks (128-row chunks on the fp16 tensor-core kernel, which takes 65..128 rows in
  * one launch with the activations as the 128-row operand). Other shapes ignore the
  * workspace. Which kernel runs depends on the extents (cacheir_b200_qgemv_plan), and the kernels sum in different orders and
- * forms: int4 rows of up to 8 (group-wise 32) run on exact fp16 activations with float32 sums, taller batches per row on 16-bit
- * fixed point with exact integer sums, so the last bits of a row may change with the number of rows beside it (and, group-wise,
- * for a last chunk of up to 32 rows behind chunks of 128). workspace may be NULL (then this is cacheir_b200_qgemv). The workspace is only used during the call's own kernels; two
+ * forms: int4 rows of up to 8 (weights of three million numbers and more: 128; group-wise 32) run on exact fp16 activations with float32 sums, taller
+ * batches per row on 16-bit fixed point with exact integer sums, so the last bits of a row may change with the number of rows
+ * beside it (and, group-wise, for the last chunk behind chunks of 128). workspace may be NULL (then this is cacheir_b200_qgemv). The workspace is only used during the call's own kernels; two
  * calls that may overlap on the GPU need separate workspaces. */
 size_t cacheir_b200_qgemv_workspace_bytes(int M, int K);
 int cacheir_b200_qgemv_ex(const void* x, const void* packed, const void* scales,
@@ -246,7 +246,7 @@ int cacheir_b200_rmsnorm_qgemv(const void* x, const void* norm_weight, float eps
 /* Which kernel cacheir_b200_qgemv_ex would launch for these extents and flags (fp16 activations, aligned
  * pointers): (family << 8) | detail, family 1 = integer tensor core with detail = its split-K factor (0: blocks of 128
  * rows in one launch), 2 = fp16 tensor core, 3 = CUDA cores, 4 = streaming int4 product with detail = (row groups << 4) |
- * CTAs along K (0: the GEMV for many weight rows in row order); epilogue 3 asks about
+ * CTAs along K (0: the GEMV for many weight rows in row order; + 128: weights as the tensor-memory operand); epilogue 3 asks about
  * cacheir_b200_qkv_rope_append. Negative:
  * the validation code the call would return. Launches nothing. No counterpart in the reference (its
  * kernel choice is the declarative `attrs["kernel"]`, cacheir/passes/transformer.py:391-424). */

@@ -1,0 +1,55 @@
+"""The int4 product with the weights in tensor memory (up to 128 rows) against float64 products of the dequantised weights."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# edges: one row more and one less than each tile of activation rows, a full tile (another copy of x), fewer weight rows than the last band
+# holds, k blocks that no ring is a multiple of, every number of CTAs along K, groups of two k blocks
+@pytest.mark.parametrize("tiled", [True, False])
+@pytest.mark.parametrize("m, n, k, split", [(9, 2048, 2048, 4), (16, 5100, 640, 1), (17, 1280, 8192, 8), (31, 2048, 5632, 6), (32, 3072, 2176, 4),
+                                            (33, 5120, 1536, 3), (64, 6400, 3584, 2), (65, 3648, 896, 1), (127, 4096, 1280, 2), (128, 19200, 1152, 1)])
+def test_weights_in_tensor_memory(m, n, k, split, tiled):
+    """Products of exact fp16 integers are summed in float32 (2^-24 each) and rounded to fp16 once: 2^-11 / sqrt(3) of the result's
+    root mean square is 2.8e-4."""
+    from cacheir_b200 import _lib, ops
+    from cacheir_b200.quantization import dequantize_device, pack_weight_device, to_tiled
+
+    g = torch.Generator(device="cuda").manual_seed(m * 31 + n + k)
+    dense = torch.randn((n, k), device="cuda", generator=g) * 0.02
+    x = torch.randn((m, k + 8), device="cuda", generator=g).half()[:, :k]            # rows of a wider buffer
+    for quant in ("int4_g128", "int4_g256", "int4_awq"):
+        if quant == "int4_g256" and k % 256:
+            continue
+        for odd_zero in (False, True) if quant == "int4_awq" else (False,):
+            w = pack_weight_device(dense, quant)
+            if odd_zero:                                   # zero points that are no small integers
+                w.zero_points[::3] += 0.25
+                w.zero_points[1] = -1500.0
+            full = dequantize_device(w, torch.float32).double() if not odd_zero else \
+                (torch.stack([w.packed_values & 15, w.packed_values >> 4], dim=2).view(n, k).double() - w.zero_points.double()[:, None]) * w.scales.double()[:, None]
+            for epilogue in (0, 1, 2):
+                paired = tiled and epilogue == 2 and quant == "int4_awq"
+                if epilogue == 2 and n % 128:
+                    continue
+                v = to_tiled(w, paired=paired) if tiled else w
+                n_out = n // 2 if epilogue == 2 else n
+                res = torch.randn((m, n_out), device="cuda", generator=g).half() if epilogue == 1 else None
+                kw = dict(bits=4, group_size=v.group_size or 0, epilogue=epilogue, tiled=tiled, paired=paired)
+                plan = ops.qgemv_plan(m, n, k, workspace=False, **kw)
+                if quant != "int4_awq" and not plan.get("tensor_memory"):
+                    continue                               # (the streaming kernel's, of up to 32 rows and fewer than 6 M numbers)
+                assert plan["tensor_memory"] and (epilogue == 2 or plan["split"] == split), plan
+                y = ops.qgemv(x, v.packed_values, v.scales, v.zero_points, n=n, k=k, residual=res, **kw)
+                want = x.double() @ full.T
+                if epilogue == 2:
+                    want = torch.nn.functional.silu(want[:, :n_out]) * want[:, n_out:]
+                if epilogue == 1:
+                    want = want + res.double()
+                err = float((y.double() - want).norm() / want.norm())
+                # (a zero point of -1500 makes its row outweigh all others: then a single rounding counts, at most 2^-11)
+                assert err <= (2.0 ** -11 if odd_zero else 2.8e-4), (quant, epilogue, odd_zero, err)
+                again = ops.qgemv(x, v.packed_values, v.scales, v.zero_points, n=n, k=k, residual=res, **kw)
+                assert torch.equal(again, y)
+    assert int(_lib.load().cacheir_b200_device_status(1)) == 0
