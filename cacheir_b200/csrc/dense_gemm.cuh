@@ -6,8 +6,8 @@
 // prompt use the same kernel and the accumulator has one weight row per tensor-memory lane: an epilogue thread owns an
 // output column, keeps that column's norm constants in registers, and 32 lanes store 32 neighbouring outputs.
 //
-//   warp 0      TMA producer: a 64-column k block of W and X per ring stage (128-byte swizzle; what lies outside the
-//               tensors reads as zero, so K needs no padding beyond the 16-byte row rule)
+//   warp 0      TMA producer: a 64-column k block of W per ring stage (128-byte swizzle; what lies outside the
+//               tensors reads as zero, so K needs no padding beyond the 16-byte row rule); warp 2 does the same for X
 //   warp 1      one thread issues tcgen05.mma (M 128, N = token tile, K 16; four per stage)
 //   warps 2..9  epilogue: tensor memory -> registers -> f -> global; lane quarter = warp % 4, two warps per quarter
 //
@@ -230,14 +230,23 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       if (blockIdx.x == 0)
         for (int i = 0; i < min(total, kAhead); ++i) tma_prefetch_2d(&tmap_w, (kb_begin + i) * kBlockK, z * p.w_batch_rows + n0);
     }
-    for (int s = 0; s < kStages; ++s) { mbar_init(smem_u32(&full[s]), 1); mbar_init(smem_u32(&empty[s]), 1); }
+    for (int s = 0; s < kStages; ++s) { mbar_init(smem_u32(&full[s]), 2); mbar_init(smem_u32(&empty[s]), 1); }
     mbar_init(smem_u32(acc_full), 1);
     mbar_fence_init();
   }
   __syncthreads();                         // the barriers exist
   if constexpr (!GROUPED) chain_wait();
   chain_next();
-  if (warp > 0) {                          // (the copies do not wait for tensor memory)
+  auto load_x = [&](int i) {               // (warp 2: a thread issues a copy in 200 cycles, half of what a stage may take)
+    const uint32_t bar = smem_u32(&full[i % kStages]);
+    mbar_expect_tx(bar, MT * kBlockK * 2);
+    const int k = (kb_begin + i) * kBlockK;
+    tma_load_2d(smem_u32(s_x + i % kStages * MT * kBlockK * 2), &tmap_x, bar, GROUPED ? k : z * p.x_batch_cols + k, t0);
+  };
+  if (warp > 0) {                          // (the first copies do not wait for tensor memory)
+    if (warp == 2 && lane == 0)
+      for (int i = 0; i < min(total, kStages); ++i) load_x(i);
+    __syncwarp();
     if (warp == 1) tc_alloc(smem_u32(tmem_slot), tmem_cols(MT));
     tc_fence_before();
     asm volatile("bar.sync 3, %0;" ::"n"(kThreads - 32) : "memory");
@@ -260,10 +269,8 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         const int s = i % kStages;
         if (i >= kStages && !mbar_wait(smem_u32(&empty[s]), ((i / kStages) & 1) ^ 1, &g_dense_status, (6 << 8) | 1)) break;
         const uint32_t bar = smem_u32(&full[s]);
-        mbar_expect_tx(bar, stage_bytes(MT));
-        const int k = (kb_begin + i) * kBlockK;
-        tma_load_2d(smem_u32(s_w + s * kWBytes), &tmap_w, bar, k, z * p.w_batch_rows + n0);
-        tma_load_2d(smem_u32(s_x + s * MT * kBlockK * 2), &tmap_x, bar, GROUPED ? k : z * p.x_batch_cols + k, t0);
+        mbar_expect_tx(bar, kWBytes);
+        tma_load_2d(smem_u32(s_w + s * kWBytes), &tmap_w, bar, (kb_begin + i) * kBlockK, z * p.w_batch_rows + n0);
         issued = i + 1;
       }
       if (issued < total)          // a wait gave up: nothing may still be on its way when the block ends
@@ -272,21 +279,37 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      // fp32 accumulator, bf16 x bf16, both K-major, N = MT, M = 128
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(MT >> 3) << 17) |
-                             (static_cast<uint32_t>(kTileN >> 4) << 24);
-      for (int i = 0; i < total; ++i) {
-        const int s = i % kStages;
-        if (!mbar_wait(smem_u32(&full[s]), (i / kStages) & 1, &g_dense_status, (6 << 8) | 2)) break;
-        tc_fence_after();
-        const uint32_t wb = smem_u32(s_w + s * kWBytes), xb = smem_u32(s_x + s * MT * kBlockK * 2);
+    // fp32 accumulator, bf16 x bf16, both K-major, N = MT, M = 128
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(MT >> 3) << 17) |
+                           (static_cast<uint32_t>(kTileN >> 4) << 24);
+    const uint64_t w_desc = smem_desc_sw128(smem_u32(s_w)), x_desc = smem_desc_sw128(smem_u32(s_x));    // (offsets add to the lowest bits, by 16 bytes)
+    const bool leader = elect_one();
+    int s = 0;
+    uint32_t phase = 0;
+    for (int i = 0; i < total; ++i) {
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&full[s]), phase, &g_dense_status, (6 << 8) | 2))) break;
+      tc_fence_after();
+      if (leader) {
+        const uint64_t wd = w_desc + s * (kWBytes / 16), xd = x_desc + s * (MT * kBlockK * 2 / 16);
 #pragma unroll
-        for (int j = 0; j < kBlockK / 16; ++j)
-          mma_f16_ss(tmem, smem_desc_sw128(wb + j * 32), smem_desc_sw128(xb + j * 32), idesc, (i > 0 || j > 0) ? 1u : 0u);
+        for (int j = 0; j < kBlockK / 16; ++j) mma_f16_ss(tmem, wd + j * 2, xd + j * 2, idesc, (i > 0 || j > 0) ? 1u : 0u);
         tc_commit(smem_u32(&empty[s]));
       }
-      tc_commit(smem_u32(acc_full));
+      __syncwarp();
+      if (++s == kStages) { s = 0; phase ^= 1; }
+    }
+    if (leader) tc_commit(smem_u32(acc_full));
+    __syncwarp();
+  } else if (warp == 2) {
+    if (lane == 0) {
+      int issued = min(total, kStages);
+      for (; issued < total; ++issued) {
+        if (!mbar_wait(smem_u32(&empty[issued % kStages]), ((issued / kStages) & 1) ^ 1, &g_dense_status, (6 << 8) | 9)) break;
+        load_x(issued);
+      }
+      if (issued < total)
+        for (int i = issued > kStages ? issued - kStages : 0; i < issued; ++i)
+          mbar_wait(smem_u32(&full[i % kStages]), (i / kStages) & 1, &g_dense_status, (6 << 8) | 4);
     }
     __syncwarp();
   }
@@ -353,12 +376,15 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       const int share = MT / split;
       for (int c = krank * share + half * 2; c < (krank + 1) * share; c += 4) {
         if (t0 + c >= t_end) break;
-        float v[2] = {0.f, 0.f};
+        float v[2] = {0.f, 0.f}, got[8][2];        // (all of them are asked for before the first is added)
         const uint32_t a = smem_u32(part + c * kTileN + r);
-        for (int s = 0; s < split; ++s) {
-          v[0] += ld_peer(a, s);
-          v[1] += ld_peer(a + kTileN * 4, s);
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          got[s][0] = s < split ? ld_peer(a, s) : 0.f;
+          got[s][1] = s < split ? ld_peer(a + kTileN * 4, s) : 0.f;
         }
+#pragma unroll
+        for (int s = 0; s < 8; ++s) { v[0] += got[s][0]; v[1] += got[s][1]; }
         emit(v, std::integral_constant<int, 2>{}, c);
       }
       cluster_sync_all();                                      // nobody leaves while its partials are being read

@@ -84,11 +84,6 @@ __device__ __forceinline__ float load_peer(const float* local, uint32_t rank) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(map_to_rank(smem_u32(local), rank)) : "memory");
   return v;
 }
-__device__ __forceinline__ bool elect_one() {
-  uint32_t yes;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(yes));
-  return yes != 0;
-}
 __device__ __forceinline__ __half2 as_half2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
 __device__ __forceinline__ uint32_t as_bits(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
 // byte j of w: its two nibbles as (low - zero, high - zero). (0x6400 | n, 0x6400 | n << 4) = (1024 + n, 1024 + 16 n); one exact fma
@@ -396,9 +391,14 @@ qgemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     }
     auto product = [&](int h, int m) {
       const float* at = part + m * kPitch + h * 64 + r;
-      float v = 0.f;
-      if (p.split > 1) {
-        for (int k = 0; k < p.split; ++k) v += load_peer(at, k);
+      float v;
+      if (p.split > 1) {                             // all of them are asked for before the first is added
+        float sums[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) sums[k] = k < p.split ? load_peer(at, k) : 0.f;
+        v = sums[0];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) v += sums[k];
       } else {
         v = *at;
       }
@@ -435,18 +435,6 @@ bool encode_x(CUtensorMap* map, const void* base, uint64_t K, uint64_t M, uint64
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Codes in tile order as lines of 128 bytes: 32 of them are 64 weight rows of a k block, copied as they lie (in swizzled order).
-bool encode_lines(CUtensorMap* map, const void* base, uint64_t lines, uint32_t box_lines) {
-  EncodeTiledFn fn = tensor_map_encoder();
-  if (!fn) return false;
-  const cuuint64_t dims[2] = {128, lines};
-  const cuuint64_t strides[1] = {128};
-  const cuuint32_t box[2] = {128, box_lines};
-  const cuuint32_t elem_strides[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // CTAs along K. A cluster lives in one GPC, so that fewer of them run at once than the SMs would hold. In cycles: a k block is 500, the
 // first and the last steps of a CTA 3000, the exchange 1200.
 int choose_split(int tiles, int kblocks) {
@@ -471,8 +459,9 @@ int launch(const QGemvParams& q, cudaStream_t stream) {
   static_assert(op_stages(NT) * kACols + accumulators(NT) * NT <= tmem_cols(NT), "tiles and accumulators fit in tensor memory");
   CUtensorMap tw, tx;
   if (!encode_x(&tx, q.x, q.K, q.M, static_cast<uint64_t>(q.x_stride) * 2, NT)) return CACHEIR_B200_EUNSUPPORTED;
+  // codes in tile order: 32 lines are 64 weight rows of a k block, copied as they lie (in swizzled order)
   const uint64_t lines = static_cast<uint64_t>((q.N + 127) / 128) * (q.K / kCols) * 64;
-  if (!(q.tiled ? encode_lines(&tw, q.packed, lines, !SWIGLU || q.paired ? 64 : 32) : encode_u8_rows_sw64(&tw, q.packed, q.K / 2, q.N, q.K / 2, 64))) return CACHEIR_B200_EUNSUPPORTED;
+  if (!(q.tiled ? encode_u8_lines(&tw, q.packed, lines, !SWIGLU || q.paired ? 64 : 32) : encode_u8_rows_sw64(&tw, q.packed, q.K / 2, q.N, q.K / 2, 64))) return CACHEIR_B200_EUNSUPPORTED;
   W4Params p{};
   p.x = static_cast<const __half*>(q.x);
   p.scales = q.scales; p.zero_points = q.zero_points;

@@ -122,6 +122,12 @@ __device__ __forceinline__ void bulk_copy_to_rank(uint32_t dst, uint32_t src, ui
   asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(rdst), "r"(src), "r"(bytes), "r"(rbar) : "memory");
 }
+// One lane of a converged warp. (Under it tensor-core instructions issue every 10 cycles or so, in a branch that only one lane took every 48.)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t yes;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(yes));
+  return yes != 0;
+}
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -221,18 +227,19 @@ inline bool encode_u8_rows_sw64(CUtensorMap* map, const void* base, uint64_t inn
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Rows of 128 bytes [rows][128], box {128, 128 rows}, copied as they lie (the data is stored in swizzled order).
-inline bool encode_u8_tiles_plain(CUtensorMap* map, const void* base, uint64_t rows) {
+// Rows of 128 bytes [rows][128], box {128, box_rows}, copied as they lie (the data is stored in swizzled order).
+inline bool encode_u8_lines(CUtensorMap* map, const void* base, uint64_t rows, uint32_t box_rows) {
   EncodeTiledFn fn = tensor_map_encoder();
   if (!fn) return false;
   const cuuint64_t dims[2] = {128, rows};
   const cuuint64_t strides[1] = {128};
-  const cuuint32_t box[2] = {128, 128};
+  const cuuint32_t box[2] = {128, box_rows};
   const cuuint32_t elem_strides[2] = {1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, elem_strides,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+inline bool encode_u8_tiles_plain(CUtensorMap* map, const void* base, uint64_t rows) { return encode_u8_lines(map, base, rows, 128); }
 
 // 2-D tensor of 32-bit words [rows][inner_words], box {box_words, box_rows}, no swizzle; what lies outside reads as zero.
 inline bool encode_u32_rows_plain(CUtensorMap* map, const void* base, uint64_t inner_words, uint64_t rows,
