@@ -101,6 +101,23 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// The warps' n results in their order, eight of them asked for at a time (one by one each costs about 30 cycles).
+__device__ __forceinline__ float ordered_sum(const float* scratch, int n) {
+  float t = 0.f;
+  int w = 0;
+  for (; w + 8 <= n; w += 8) {
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = scratch[w + i];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t += v[i];
+  }
+  for (; w < n; ++w) t += scratch[w];
+  return t;
+}
+// Asks for a line to be brought into L2.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // silu(g) = g / (1 + e^-g) for the fused epilogues. The quotient uses the reciprocal unit directly:
 // when e^-g overflows (g below about -88) the denominator is infinite and a full IEEE division would
 // detour through its slow path on every such element; here the reciprocal is 0 and the result -0.

@@ -16,12 +16,17 @@ template <typename T, int VEC, int PER_THREAD>
 __global__ void __launch_bounds__(256)
 rms_norm_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ weight,
                 T* __restrict__ sum_out, T* __restrict__ out, int hidden, float eps) {
+  const int nvec = hidden / VEC;  // host guarantees hidden % VEC == 0 on this path
+  for (int c = threadIdx.x * 8; c < nvec; c += 256 * 8) prefetch_l2(weight + c * VEC);      // (not in L2 after a step's products)
   chain_enter();
   __shared__ float red[8];
   const size_t row = blockIdx.x;
   const T* xr = x + row * hidden;
   const T* rr = residual ? residual + row * hidden : nullptr;
-  const int nvec = hidden / VEC;  // host guarantees hidden % VEC == 0 on this path
+  float wv[PER_THREAD][VEC];      // asked for before the sum, not behind it
+#pragma unroll
+  for (int i = 0; i < PER_THREAD; ++i)
+    if (static_cast<int>(threadIdx.x) + i * 256 < nvec) VecIO<T, VEC>::ld(weight + (threadIdx.x + i * 256) * VEC, wv[i]);
   float cache[PER_THREAD][VEC];
   float ss = 0.f;
 #pragma unroll
@@ -55,10 +60,9 @@ rms_norm_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T
   for (int i = 0; i < PER_THREAD; ++i) {
     const int c = threadIdx.x + i * 256;
     if (c < nvec) {
-      float w[VEC], o[VEC];
-      VecIO<T, VEC>::ld(weight + c * VEC, w);
+      float o[VEC];
 #pragma unroll
-      for (int v = 0; v < VEC; ++v) o[v] = cache[i][v] * inv * w[v];
+      for (int v = 0; v < VEC; ++v) o[v] = cache[i][v] * inv * wv[i][v];
       VecIO<T, VEC>::st(out + row * hidden + c * VEC, o);
     }
   }

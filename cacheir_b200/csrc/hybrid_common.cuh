@@ -31,9 +31,7 @@ __device__ __forceinline__ float block_sum_all(float v, float* scratch) {
   __syncthreads();
   if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
   __syncthreads();
-  float t = 0.f;
-  for (int w = 0; w < static_cast<int>((blockDim.x + 31) >> 5); ++w) t += scratch[w];
-  return t;
+  return ordered_sum(scratch, static_cast<int>((blockDim.x + 31) >> 5));
 }
 
 // bf16 warp MMA pieces (16x8x16, fp32 accumulation)

@@ -90,6 +90,10 @@ constexpr int kRowThreads = 512;
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kRowThreads)
 residual_rms_kernel(float* __restrict__ x, const T* __restrict__ y, const float* __restrict__ w, float eps, int width, NextArgs nx) {
+  for (int c = threadIdx.x * 32; c < width; c += kRowThreads * 32) {      // (they are not in L2 after a step's products)
+    prefetch_l2(w + c);
+    if (nx.mode == CACHEIR_B200_NEXT_DYT) { prefetch_l2(nx.w + c); prefetch_l2(nx.b + c); }
+  }
   chain_enter();
   __shared__ float scratch[32];
   const size_t row = blockIdx.x;
@@ -143,6 +147,8 @@ constexpr int kAddThreads = 256, kAddPieces = 8;
 template <typename T, int VEC, bool HELD>
 __global__ void __launch_bounds__(kAddThreads)
 residual_add_kernel(float* x, const T* __restrict__ y, const float* __restrict__ scale, int width, RowNext nx) {
+  if (nx.w)                                   // (the norm's weights are not in L2 after a step's products)
+    for (int c = threadIdx.x * 32; c < width; c += kAddThreads * 32) prefetch_l2(nx.w + c);
   chain_enter();
   __shared__ float scratch[32];
   const size_t row = blockIdx.x;
@@ -159,9 +165,13 @@ residual_add_kernel(float* x, const T* __restrict__ y, const float* __restrict__
     float s[kAddPieces][VEC], sum = 0.f;
     const bool centred = nx.mode == CACHEIR_B200_NEXT_LAYER;
     const auto column = [](int k) { return (k * kAddThreads + static_cast<int>(threadIdx.x)) * VEC; };
+    float w[kAddPieces][VEC];                 // asked for before the sums, not behind them
 #pragma unroll
     for (int k = 0; k < kAddPieces; ++k)
-      if (column(k) < width) load_vec<float, VEC>(x + column(k), s[k]);
+      if (column(k) < width) {
+        load_vec<float, VEC>(x + column(k), s[k]);
+        if (nx.w) load_vec<float, VEC>(nx.w + column(k), w[k]);
+      }
 #pragma unroll
     for (int k = 0; k < kAddPieces; ++k)
       if (column(k) < width) {
@@ -191,11 +201,9 @@ residual_add_kernel(float* x, const T* __restrict__ y, const float* __restrict__
 #pragma unroll
     for (int k = 0; k < kAddPieces; ++k)
       if (column(k) < width) {
-        float w[VEC];
-        load_vec<float, VEC>(nx.w + column(k), w);
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) w[i] = (s[k][i] - mean) * inv * w[i];
-        store_vec<T, VEC>(out + column(k), w);
+        for (int i = 0; i < VEC; ++i) w[k][i] = (s[k][i] - mean) * inv * w[k][i];
+        store_vec<T, VEC>(out + column(k), w[k]);
       }
   } else {
     finish_row<T, VEC>(x, row, width, nx, scratch, added);

@@ -123,9 +123,7 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
   __syncthreads();
   if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
   __syncthreads();
-  float t = 0.f;
-  for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += scratch[w];
-  return t;
+  return ordered_sum(scratch, static_cast<int>(blockDim.x >> 5));
 }
 __device__ __forceinline__ float block_max(float v, float* scratch) {
   v = warp_max(v);
@@ -133,7 +131,16 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
   if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
   __syncthreads();
   float t = 0.f;
-  for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t = fmaxf(t, scratch[w]);
+  int w = 0;
+  const int n = static_cast<int>(blockDim.x >> 5);
+  for (; w + 8 <= n; w += 8) {
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = scratch[w + i];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t = fmaxf(t, v[i]);
+  }
+  for (; w < n; ++w) t = fmaxf(t, scratch[w]);
   return t;
 }
 
@@ -216,6 +223,7 @@ __global__ void __launch_bounds__(512)
 rms_norm_quantize_kernel(const __half* __restrict__ x, const __half* __restrict__ residual, const __half* __restrict__ weight,
                          __half* __restrict__ sum_out, __half* __restrict__ out, int M, int hidden, float eps, int mp,
                          int8_t* __restrict__ planes, float* __restrict__ sx, int* __restrict__ qsum) {
+  for (int c = threadIdx.x * 64; c < hidden; c += blockDim.x * 64) prefetch_l2(weight + c);      // (not in L2 after a step's products)
   chain_enter();
   __shared__ float scratch[32];
   const int m = blockIdx.x;
