@@ -15,10 +15,11 @@
 // tensor pipe active 80 % of the cycles (32 passes of 64 rows take 26 us each for half of these weights).
 //
 // Few tiles leave most SMs idle, so that a tile's K range is split over the SPLIT pairs of a larger cluster (one tile per
-// cluster then): every CTA lays its partial sums out in its drained ring, and pair j adds up, through distributed shared memory, what all pairs have
-// for its share of the activation rows. Integer sums: the order cannot matter. 256 rows of 2048 x 5632: 44 k blocks on 32 SMs, or 22 on 64.
+// cluster then): every CTA lays its partial sums for the other pairs' shares of the activation rows out in its drained ring, one bulk copy
+// each brings them there, and a pair adds what has come to its own sums in tensor memory (read one by one through distributed shared
+// memory they took 4000 cycles per 16 rows). Integer sums: the order cannot matter. 256 rows of 2048 x 5632: 44 k blocks on 32 SMs, or 22 on 64.
 //
-// Warps: 0 copies, 1 issues MMAs (even CTA only), 2-9 epilogue (four per half of the activation rows), with int4 codes 10-21
+// Warps: 0 copies, 1 issues MMAs (even CTA only), 2-9 or 2-17 epilogue (four per group of activation rows), with int4 codes 10-21
 // widen nibble tiles to byte tiles in three groups that take every third stage.
 #include "common.cuh"
 #include "qgemv_common.cuh"
@@ -40,17 +41,10 @@ __device__ int g_i8_rows_status = 0;
 
 __host__ __device__ constexpr int stage_bytes(int bits) { return 2 * kTile + (bits == 4 ? kTile / 2 : 0); }
 __host__ __device__ constexpr int num_stages(int bits) { return bits == 4 ? 5 : 6; }
-constexpr int kEpilogueThreads = 256;
 constexpr int kConverterGroups = 3;     // one group needs 1770 cycles from barrier to barrier for a stage of 512 tensor-core cycles
-__host__ __device__ constexpr int num_threads(int bits) { return 64 + kEpilogueThreads + (bits == 4 ? kConverterGroups * 128 : 0); }
-constexpr int kExchangeBytes = 2 * 2 * kChunk * kPairHalf * 4;
+__host__ __device__ constexpr int num_threads(int bits, int groups) { return 64 + groups * 128 + (bits == 4 ? kConverterGroups * 128 : 0); }
+constexpr int kExchangeBytes = 4 * kChunk * kPairHalf * 4;
 constexpr int kTailBytes = kExchangeBytes + 2 * kRows * 16 + 512;     // SwiGLU exchange, row scales and sums of two tiles, barriers
-
-__device__ __forceinline__ uint32_t load_cluster(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-  return v;
-}
 
 struct RowsParams {
   const void* scales;
@@ -66,17 +60,19 @@ struct RowsParams {
   int bands;          // weight tiles of 128 rows
 };
 
-template <int BITS, bool SWIGLU, int SPLIT>
-__global__ void __launch_bounds__(num_threads(BITS), 1)
+// G: groups of four epilogue warps, a share of the tile's activation rows each
+template <int BITS, bool SWIGLU, int SPLIT, int G>
+__global__ void __launch_bounds__(num_threads(BITS, G), 1)
 qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const RowsParams p) {
   chain_enter();
-  constexpr int S = num_stages(BITS);
+  constexpr int S = num_stages(BITS), kGroupRows = kRows / SPLIT / G;
+  constexpr int kEpilogueThreads = 128 * G, kConverters = 2 + 4 * G;      // (first converter warp)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* s_w = smem;                       // [S] byte tiles of this CTA's weight rows
   uint8_t* s_x = s_w + S * kTile;            // [S] this CTA's plane
   uint8_t* s_raw = s_x + S * kTile;          // [S] int4: nibble tiles
-  float* s_up = reinterpret_cast<float*>(s_raw + (BITS == 4 ? S * kTile / 2 : 0));    // [half][2][kChunk][64]
+  float* s_up = reinterpret_cast<float*>(s_raw + (BITS == 4 ? S * kTile / 2 : 0));    // [group][4 / G][kChunk][64]
   int4* s_row = reinterpret_cast<int4*>(s_up + 4 * kChunk * kPairHalf);               // [2][128] (scale, sum >> 8, sum & 255, sum)
   uint64_t* full = reinterpret_cast<uint64_t*>(s_row + 2 * kRows);   // [S] (even CTA) operands of both CTAs have landed
   uint64_t* empty = full + S;                // [S] the MMAs that read the stage have retired
@@ -85,7 +81,11 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   uint64_t* acc_full = ready + S;            // [2]
   uint64_t* acc_empty = acc_full + 2;        // [2] (even CTA) both CTAs' epilogues have read the accumulator
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-  int* s_part = reinterpret_cast<int*>(smem);      // SPLIT > 1: 128 KB over the drained ring
+  uint64_t* xch = reinterpret_cast<uint64_t*>(tmem_slot + 2);      // SPLIT > 1: the other pairs' sums have landed
+  // SPLIT > 1, over the drained ring: sums for the other pairs, then what they send, a slab [activation row][high, low][weight row] each
+  constexpr int kShare = kRows / SPLIT, kSlab = kShare * 2 * kRows;
+  int* s_out = reinterpret_cast<int*>(smem);
+  int* s_in = s_out + (SPLIT - 1) * kSlab;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -109,9 +109,11 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&acc_full[a]), 1);
-      mbar_init(smem_u32(&acc_empty[a]), 16);     // eight epilogue warps of each CTA
+      mbar_init(smem_u32(&acc_empty[a]), 8 * G);     // the epilogue warps of both CTAs
     }
+    if (SPLIT > 1) mbar_init(smem_u32(xch), 1);
     mbar_fence_init();
+    if (SPLIT > 1) mbar_expect_tx(smem_u32(xch), (SPLIT - 1) * kSlab * 4);
   }
   if (warp == 1) tc_alloc_pair(smem_u32(tmem_slot), 2 * kAccCols);
   tc_fence_before();
@@ -176,12 +178,12 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         tc_commit_pair(smem_u32(&acc_full[a]), first);
       }
     }
-  } else if (warp < 10) {
+  } else if (warp < kConverters) {
     // ---------------- epilogue: lane quarter = warp % 4, a thread owns one weight row and 64 of the activation rows ----------------
     // About ten instructions per output; a scheduler has two of these warps, so the loops keep 16 independent outputs going.
     const int q = warp & 3;
     const int r = q * 32 + lane;
-    const int half = (warp - 2) >> 2;
+    const int group = (warp - 2) >> 2;
     const int tid = threadIdx.x - 64;
     const bool is_up = SWIGLU && r >= kPairHalf;
     int n = 0;
@@ -213,50 +215,61 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       const int real = min(kRows, rows - m0);
       __half* y = p.y + static_cast<size_t>(m0) * p.n_out + col;
       const __half* res = p.residual ? p.residual + static_cast<size_t>(m0) * p.n_out + col : nullptr;
-      if constexpr (SPLIT > 1) {       // partial sums to the drained ring: [activation row][high, low][weight row]
+      if constexpr (SPLIT > 1) {       // sums of the other pairs' activation rows to them, one bulk copy each
 #pragma unroll 1
-        for (int c0 = half * (kRows / 2); c0 < (half + 1) * (kRows / 2); c0 += kChunk) {
-          uint32_t hi[kChunk], lo[kChunk];
-          tc_ld_x16(lanes + c0, hi);
-          tc_ld_x16(lanes + kRows + c0, lo);
-          tc_wait_ld();
-#pragma unroll
-          for (int j = 0; j < kChunk; ++j) {
-            s_part[(2 * (c0 + j)) * kRows + r] = kblocks > 0 ? static_cast<int>(hi[j]) : 0;
-            s_part[(2 * (c0 + j) + 1) * kRows + r] = kblocks > 0 ? static_cast<int>(lo[j]) : 0;
-          }
-        }
-        __syncwarp();
-        cluster_sync_release();        // every CTA's sums are in place
-      }
+        for (int e = 0; e < SPLIT - 1; ++e) {
+          const int to = e < share ? e : e + 1;
 #pragma unroll 1
-      for (int c0 = 0; c0 < kRows / 2 / SPLIT; c0 += kChunk) {
-        const int first_row = (share * 2 + half) * (kRows / 2 / SPLIT) + c0;          // activation row of the tile
-        uint32_t hi[kChunk], lo[kChunk];
-        if constexpr (SPLIT == 1) {
-          tc_ld_x16(lanes + first_row, hi);
-          tc_ld_x16(lanes + kRows + first_row, lo);
-        } else {
-#pragma unroll
-          for (int j = 0; j < kChunk; ++j) { hi[j] = 0u; lo[j] = 0u; }
-#pragma unroll
-          for (int k = 0; k < SPLIT; ++k) {
-            const uint32_t from = map_to_rank(smem_u32(s_part + 2 * first_row * kRows + r), 2 * k + rank);
+          for (int c0 = group * kGroupRows; c0 < (group + 1) * kGroupRows; c0 += kChunk) {
+            uint32_t hi[kChunk], lo[kChunk];
+            tc_ld_x16(lanes + to * kShare + c0, hi);
+            tc_ld_x16(lanes + kRows + to * kShare + c0, lo);
+            tc_wait_ld();
 #pragma unroll
             for (int j = 0; j < kChunk; ++j) {
-              hi[j] += load_cluster(from + (2 * j) * kRows * 4);
-              lo[j] += load_cluster(from + (2 * j + 1) * kRows * 4);
+              s_out[e * kSlab + (2 * (c0 + j)) * kRows + r] = kblocks > 0 ? static_cast<int>(hi[j]) : 0;
+              s_out[e * kSlab + (2 * (c0 + j) + 1) * kRows + r] = kblocks > 0 ? static_cast<int>(lo[j]) : 0;
             }
           }
         }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        cluster_sync_release();        // every CTA's sums are in place and its ring is no longer read
+        if (tid == 0)
+          for (int e = 0; e < SPLIT - 1; ++e) {
+            const int to = e < share ? e : e + 1, slot = share < to ? share : share - 1;
+            bulk_copy_to_rank(smem_u32(s_in + slot * kSlab), smem_u32(s_out + e * kSlab), kSlab * 4, smem_u32(xch), 2 * to + rank);
+          }
+        ok = ok && mbar_wait(smem_u32(xch), 0, &g_i8_rows_status, (12 << 8) | 10);
+        col_ok = col_ok && ok;
+        __syncwarp();
+      }
+#pragma unroll 1
+      for (int c0 = 0; c0 < kGroupRows; c0 += kChunk) {
+        const int first_row = (share * G + group) * kGroupRows + c0;          // activation row of the tile
+        uint32_t hi[kChunk], lo[kChunk];
+        tc_ld_x16(lanes + first_row, hi);
+        tc_ld_x16(lanes + kRows + first_row, lo);
         float add[kChunk];
         if constexpr (!SWIGLU) {
 #pragma unroll
           for (int j = 0; j < kChunk; ++j)
             add[j] = res && col_ok && first_row + j < real ? __half2float(res[static_cast<size_t>(first_row + j) * p.n_out]) : 0.f;
         }
-        if constexpr (SPLIT == 1) tc_wait_ld();
-        if (SPLIT == 1 && c0 + kChunk >= kRows / 2) {       // the accumulator is in registers: the next tile may have it
+        tc_wait_ld();
+        if constexpr (SPLIT > 1) {
+#pragma unroll
+          for (int j = 0; j < kChunk; ++j) {
+            if (kblocks == 0) { hi[j] = 0u; lo[j] = 0u; }
+            const int* in = s_in + (2 * (group * kGroupRows + c0 + j)) * kRows + r;
+#pragma unroll
+            for (int k = 0; k < SPLIT - 1; ++k) {
+              hi[j] += static_cast<uint32_t>(in[k * kSlab]);
+              lo[j] += static_cast<uint32_t>(in[k * kSlab + kRows]);
+            }
+          }
+        }
+        if (SPLIT == 1 && c0 + kChunk >= kGroupRows) {       // the accumulator is in registers: the next tile may have it
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&acc_empty[a]), first));
@@ -287,13 +300,13 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
           // gate and up of a column sit 64 lanes apart: the up side hands over the first half of the chunk and finishes
           // the second, the gate side the other way round
           constexpr int H = kChunk / 2;
-          float* buf = s_up + (half * 2 + ((c0 / kChunk) & 1)) * kChunk * kPairHalf + (r & (kPairHalf - 1));
+          float* buf = s_up + (G == 4 ? group : group * 2 + ((c0 / kChunk) & 1)) * kChunk * kPairHalf + (r & (kPairHalf - 1));
 #pragma unroll
           for (int j = 0; j < H; ++j) {
             if (is_up) buf[j * kPairHalf] = v[j];
             else buf[(H + j) * kPairHalf] = v[H + j];
           }
-          asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
+          asm volatile("bar.sync %0, 128;" ::"r"(2 + group) : "memory");
 #pragma unroll
           for (int j = 0; j < H; ++j) {
             const float other = buf[(is_up ? H + j : j) * kPairHalf];
@@ -301,6 +314,7 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             const int m = first_row + (is_up ? H + j : j);
             if (col_ok && m < real) y[static_cast<size_t>(m) * p.n_out] = __float2half_rn(silu_fast(g) * u);
           }
+          if (G == 4) asm volatile("bar.sync %0, 128;" ::"r"(2 + group) : "memory");      // (one buffer: it has been read)
         } else {
 #pragma unroll
           for (int j = 0; j < kChunk; ++j)
@@ -313,10 +327,10 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     // Thread r owns tile row r: 64 bytes of nibbles (16-byte chunk c at c ^ ((r >> 1) & 3)) become 128 bytes of codes in the
     // 128-byte swizzle order (chunk c at c ^ (r & 7)); even columns sit in the low nibbles.
     const int r = threadIdx.x & 127;
-    static_assert((64 + kEpilogueThreads) % 128 == 64, "converter warps start at a multiple of two warps");
+    static_assert((kConverters * 32) % 128 == 64, "converter warps start at a multiple of two warps");
     const int steps = tiles > pair ? ((tiles - pair - 1) / pairs + 1) * kblocks : 0;
     bool ok = true;
-    const int group = (warp - 10) >> 2;
+    const int group = (warp - kConverters) >> 2;
     // A barrier's parity only tells neighbouring phases apart. A group therefore waits for its own stages alone, first until the MMAs
     // have retired that read the place before (the copy behind which this group's last stage came had waited for the use before that one), then
     // for the bytes. Neither barrier can move on without this group's conversion, so that no phase is missed, however late the group looks.
@@ -351,7 +365,7 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     }
   }
   if constexpr (SPLIT > 1) {                      // (the cluster barrier between the partial sums and their readers is everyone's)
-    if ((warp < 2 || warp >= 10) && pair < tiles) {
+    if ((warp < 2 || warp >= kConverters) && pair < tiles) {
       __syncwarp();
       cluster_sync_release();
     }
@@ -366,16 +380,16 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   }
 }
 
-template <int BITS, bool SWIGLU, int SPLIT>
+template <int BITS, bool SWIGLU, int SPLIT, int G>
 int launch_split(const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, const RowsParams& p, int tiles, cudaStream_t stream) {
   constexpr int kSmem = 1024 + num_stages(BITS) * stage_bytes(BITS) + kTailBytes;
-  static_assert((4 * num_stages(BITS) + 4) * 8 + 8 <= 512, "barriers and the tensor-memory base fit in the tail");
-  static_assert(num_stages(BITS) * stage_bytes(BITS) >= 2 * kRows * kRows * 4, "partial sums fit in the drained ring");
-  auto kern = qgemm_i8_rows_kernel<BITS, SWIGLU, SPLIT>;
+  static_assert((4 * num_stages(BITS) + 5) * 8 + 8 <= 512, "barriers and the tensor-memory base fit in the tail");
+  static_assert(num_stages(BITS) * stage_bytes(BITS) >= 2 * (SPLIT - 1) * (kRows / SPLIT) * 2 * kRows * 4, "sums that leave and come fit in the drained ring");
+  auto kern = qgemm_i8_rows_kernel<BITS, SWIGLU, SPLIT, G>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (e != cudaSuccess) return static_cast<int>(e);
   const int clusters = SPLIT > 1 || tiles < kNumSMs / 2 ? tiles : kNumSMs / 2;
-  e = launch_clusters(kern, dim3(2 * SPLIT * clusters, 1, 1), num_threads(BITS), kSmem, stream, dim3(2 * SPLIT, 1, 1), tmap_w, tmap_x, p);
+  e = launch_clusters(kern, dim3(2 * SPLIT * clusters, 1, 1), num_threads(BITS, G), kSmem, stream, dim3(2 * SPLIT, 1, 1), tmap_w, tmap_x, p);
   if (e != cudaSuccess) return static_cast<int>(e);
   return launch_status();
 }
@@ -393,9 +407,15 @@ template <int BITS, bool SWIGLU>
 int launch_rows(const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, const RowsParams& p, cudaStream_t stream) {
   const int tiles = (p.bands + 1) / 2 * ((p.M + kRows - 1) / kRows);
   const int split = pairs_along_k(tiles, p.K / kRows);
-  if (split == 4) return launch_split<BITS, SWIGLU, 4>(tmap_w, tmap_x, p, tiles, stream);
-  if (split == 2) return launch_split<BITS, SWIGLU, 2>(tmap_w, tmap_x, p, tiles, stream);
-  return launch_split<BITS, SWIGLU, 1>(tmap_w, tmap_x, p, tiles, stream);
+  // With a split K an epilogue covers nothing, and it is latency: twice the warps and one bulk copy per pair instead of reads from its shared
+  // memory take 10 to 15 % off (256 rows of int8 2048x2048 13.0 / 11.3 us, 4096x2048 13.7 / 11.9, 4096x4096 16.4 / 14.6). Where pairs have
+  // whole tiles more warps get in the way (384 rows of 4096x14336 47.2 / 49.3), except with SwiGLU and at most two tiles (11264x2048
+  // 2 us less). With int4 codes the converters have the registers; four pairs along K leave each 32 activation rows.
+  if (split == 4) return launch_split<BITS, SWIGLU, 4, 2>(tmap_w, tmap_x, p, tiles, stream);
+  if (split == 2) return launch_split<BITS, SWIGLU, 2, BITS == 8 ? 4 : 2>(tmap_w, tmap_x, p, tiles, stream);
+  if constexpr (BITS == 8 && SWIGLU)
+    if (tiles <= kNumSMs) return launch_split<BITS, SWIGLU, 1, 4>(tmap_w, tmap_x, p, tiles, stream);
+  return launch_split<BITS, SWIGLU, 1, 2>(tmap_w, tmap_x, p, tiles, stream);
 }
 
 }  // namespace
