@@ -475,26 +475,34 @@ dense_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           if (!mbar_wait(smem_u32(&full[i % S]), (i / S) & 1, &g_dense_status, (6 << 8) | 4)) break;
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
-      // fp32 accumulator, bf16 x bf16, both K-major, N = TT, M = 256
+    if (rank == 0) {
+      // fp32 accumulator, bf16 x bf16, both K-major, N = TT, M = 256. The whole warp waits and one elected lane issues: a k block of 128 tokens is
+      // 256 tensor-core cycles, and in a branch that only one lane takes its four MMAs, waits and descriptors are 570.
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(TT >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);
-      int it = 0, n = 0;
+      const uint64_t w_desc = smem_desc_sw128(smem_u32(s_w)), x_desc = smem_desc_sw128(smem_u32(s_x));    // (offsets add to the lowest bits, by 16 bytes)
+      const bool leader = elect_one();
+      int s = 0, n = 0;
+      uint32_t phase = 0;
       bool ok = true;
       for (int tile = blockIdx.x >> 1; tile < tiles && ok; tile += pairs, ++n) {
         const int a = n & 1;
-        if (n >= 2 && !mbar_wait(smem_u32(&acc_empty[a]), ((n >> 1) & 1) ^ 1, &g_dense_status, (6 << 8) | 6)) break;
+        if (n >= 2 && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_empty[a]), ((n >> 1) & 1) ^ 1, &g_dense_status, (6 << 8) | 6))) break;
         tc_fence_after();
-        for (int i = 0; i < kblocks; ++i, ++it) {
-          const int s = it % S;
-          if (!mbar_wait(smem_u32(&full[s]), (it / S) & 1, &g_dense_status, (6 << 8) | 7)) { ok = false; break; }
+        for (int i = 0; i < kblocks; ++i) {
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&full[s]), phase, &g_dense_status, (6 << 8) | 7));
+          if (!ok) break;
           tc_fence_after();
-          const uint32_t wb = smem_u32(s_w + s * kWBytes), xb = smem_u32(s_x + s * (TT / 2) * kBlockK * 2);
+          if (leader) {
+            const uint64_t wd = w_desc + s * (kWBytes / 16), xd = x_desc + s * ((TT / 2) * kBlockK * 2 / 16);
 #pragma unroll
-          for (int j = 0; j < kBlockK / 16; ++j)
-            mma_f16_ss_pair(tmem + a * TT, smem_desc_sw128(wb + j * 32), smem_desc_sw128(xb + j * 32), idesc, (i > 0 || j > 0) ? 1u : 0u);
-          tc_commit_pair(smem_u32(&empty[s]));
+            for (int j = 0; j < kBlockK / 16; ++j) mma_f16_ss_pair(tmem + a * TT, wd + j * 2, xd + j * 2, idesc, (i > 0 || j > 0) ? 1u : 0u);
+            tc_commit_pair(smem_u32(&empty[s]));
+          }
+          __syncwarp();
+          if (++s == S) { s = 0; phase ^= 1; }
         }
-        tc_commit_pair(smem_u32(&acc_full[a]));
+        if (leader) tc_commit_pair(smem_u32(&acc_full[a]));
+        __syncwarp();
       }
     }
   } else {

@@ -153,29 +153,37 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
-      // ---------------- MMAs of the pair ----------------
+    if (rank == 0) {
+      // ---------------- MMAs of the pair: the whole warp waits, one elected lane issues ----------------
       // D = s32, A (codes) unsigned 8 bit, B (activation bytes) signed 8 bit, both K-major, N = 256, M = 256
       constexpr uint32_t idesc = (2u << 4) | (0u << 7) | (1u << 10) | (static_cast<uint32_t>(kAccCols >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);
-      int it = 0, n = 0;
+      const uint64_t w_desc = smem_desc_sw128(smem_u32(s_w)), x_desc = smem_desc_sw128(smem_u32(s_x));    // (offsets add to the lowest bits, by 16 bytes)
+      const bool leader = elect_one();
+      int s = 0, n = 0;
+      uint32_t phase = 0;
       bool ok = true;
       for (int t = pair; t < tiles && ok; t += pairs, ++n) {
         const int a = n & 1;
-        if (n >= 2 && !mbar_wait(smem_u32(&acc_empty[a]), ((n >> 1) & 1) ^ 1, &g_i8_rows_status, (12 << 8) | 2)) break;
+        if (n >= 2 && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_empty[a]), ((n >> 1) & 1) ^ 1, &g_i8_rows_status, (12 << 8) | 2))) break;
         tc_fence_after();
         const uint32_t d = tmem_base + a * kAccCols;
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const int s = it % S;
-          if (!mbar_wait(smem_u32(&full[s]), (it / S) & 1, &g_i8_rows_status, (12 << 8) | 3)) { ok = false; break; }
-          if (BITS == 4 && !mbar_wait(smem_u32(&ready[s]), (it / S) & 1, &g_i8_rows_status, (12 << 8) | 4)) { ok = false; break; }
+        for (int kb = 0; kb < kblocks; ++kb) {
+          ok = mbar_wait(smem_u32(&full[s]), phase, &g_i8_rows_status, (12 << 8) | 3);
+          if (BITS == 4) ok = ok && mbar_wait(smem_u32(&ready[s]), phase, &g_i8_rows_status, (12 << 8) | 4);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
           tc_fence_after();
-          const uint32_t w = smem_u32(s_w + s * kTile), x = smem_u32(s_x + s * kTile);
+          if (leader) {
+            const uint64_t wd = w_desc + s * (kTile / 16), xd = x_desc + s * (kTile / 16);
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            tc_mma_i8_ss_pair(d, smem_desc_sw128(w + j * 32), smem_desc_sw128(x + j * 32), idesc, (kb > 0 || j > 0) ? 1u : 0u);
-          tc_commit_pair(smem_u32(&empty[s]), first);
+            for (int j = 0; j < 4; ++j) tc_mma_i8_ss_pair(d, wd + j * 2, xd + j * 2, idesc, (kb > 0 || j > 0) ? 1u : 0u);
+            tc_commit_pair(smem_u32(&empty[s]), first);
+          }
+          __syncwarp();
+          if (++s == S) { s = 0; phase ^= 1; }
         }
-        tc_commit_pair(smem_u32(&acc_full[a]), first);
+        if (leader) tc_commit_pair(smem_u32(&acc_full[a]), first);
+        __syncwarp();
       }
     }
   } else if (warp < kConverters) {
