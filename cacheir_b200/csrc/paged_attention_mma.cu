@@ -203,14 +203,30 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       return;
     }
   }
+  // The length, the first page ids (the table has max_pages entries whatever the length) and the queries are asked for together: one after
+  // another they were a third of the microseconds in which a short context is done.
   const int seq_len = p.seq_lens[b];
   const int t_begin = split * p.chunk_tokens;
-  if (!CLUSTER && p.splits > 1 && t_begin >= seq_len) return;      // combine never reads this split
-  const int t_end = min(seq_len, t_begin + p.chunk_tokens);
   const int page_begin = t_begin / kPage;              // chunk_tokens is a multiple of the page size
-  const int n_pages = t_end > t_begin ? (t_end - t_begin + kPage - 1) / kPage : 0;
-  const int n_iters = (n_pages + kPagesPerStage - 1) / kPagesPerStage;
-
+  const int32_t* pt = p.page_table + static_cast<size_t>(b) * p.max_pages + page_begin;
+  int next_id = 0;
+  if (warp == kConsumerWarps && lane < kPagesPerStage && page_begin + lane < p.max_pages) next_id = pt[lane];
+  const int g = lane >> 2;                             // per-thread state of two rows (heads): g and g + 8
+  const int t4 = lane & 3;
+  // Q as the A operand: rows = heads of the group (zero beyond the group), 16 dims per k step
+  uint32_t qa[kKSteps][4];
+  if (warp < kConsumerWarps) {
+    const T* qb = static_cast<const T*>(p.q) + static_cast<size_t>(b) * p.q_stride + static_cast<size_t>(kvh) * p.group * D;
+#pragma unroll
+    for (int ks = 0; ks < kKSteps; ++ks) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int row = g + (r & 1) * 8;
+        const int col = ks * 16 + 2 * t4 + (r >> 1) * 8;
+        qa[ks][r] = row < p.group ? *reinterpret_cast<const uint32_t*>(qb + static_cast<size_t>(row) * D + col) : 0u;
+      }
+    }
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
       mbar_init(smem_u32(&full[s]), 1);
@@ -219,10 +235,11 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  if (!CLUSTER && p.splits > 1 && t_begin >= seq_len) return;      // combine never reads this split
+  const int t_end = min(seq_len, t_begin + p.chunk_tokens);
+  const int n_pages = t_end > t_begin ? (t_end - t_begin + kPage - 1) / kPage : 0;
+  const int n_iters = (n_pages + kPagesPerStage - 1) / kPagesPerStage;
 
-  // per-thread softmax / output state of the two rows (heads) this thread owns: g and g + 8
-  const int g = lane >> 2;
-  const int t4 = lane & 3;
   float m_run[2] = {-INFINITY, -INFINITY};
   float l_run[2] = {0.f, 0.f};
   float o[kDimTiles][4];
@@ -232,9 +249,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
 
   if (warp == kConsumerWarps) {
     // ---------------- producer warp: lane j copies page j of each stage ----------------
-    const int32_t* pt = p.page_table + static_cast<size_t>(b) * p.max_pages + page_begin;
-    int next_id = lane < min(kPagesPerStage, n_pages) ? pt[lane] : 0;   // page ids are fetched one stage ahead
-    for (int it = 0; it < n_iters && ok; ++it) {
+    for (int it = 0; it < n_iters && ok; ++it) {       // (page ids are fetched one stage ahead)
       const int s = it % stages;
       const uint32_t ph = (it / stages) & 1;
       const int first = it * kPagesPerStage;
@@ -255,20 +270,6 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     }
   } else {
     // ---------------- consumer warps ----------------
-    // Q as the A operand: rows = heads of the group (zero beyond the group), 16 dims per k step
-    uint32_t qa[kKSteps][4];
-    {
-      const T* qb = static_cast<const T*>(p.q) + static_cast<size_t>(b) * p.q_stride + static_cast<size_t>(kvh) * p.group * D;
-#pragma unroll
-      for (int ks = 0; ks < kKSteps; ++ks) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int row = g + (r & 1) * 8;
-          const int col = ks * 16 + 2 * t4 + (r >> 1) * 8;
-          qa[ks][r] = row < p.group ? *reinterpret_cast<const uint32_t*>(qb + static_cast<size_t>(row) * D + col) : 0u;
-        }
-      }
-    }
     const uint32_t lrow = lane & 7;        // row supplied by this lane to ldmatrix
     const uint32_t lmat = lane >> 3;       // which of the four 8x8 matrices
     for (int it = 0; it < n_iters && ok; ++it) {
