@@ -331,6 +331,33 @@ __global__ void embedding_gather_kernel(const T* __restrict__ table, const int64
   for (int c = threadIdx.x; c < hidden; c += blockDim.x) dst[c] = src[c];
 }
 
+// The rows of a shared pass to their places in [sequences][max_len], zeros behind a sequence's last one. Bound by memory: 251 rows of
+// 64 KB to 4 x 140 are 53 MB; as a fill of everything and a copy per sequence they were five launches of 36 MB + 33 MB.
+struct UnpackPart { int sequence, from, to, zero_to, row; };
+constexpr int kUnpackParts = 64;
+struct UnpackParts { UnpackPart part[kUnpackParts]; };
+__global__ void __launch_bounds__(256)
+unpack_rows_kernel(const uint4* __restrict__ rows, uint4* __restrict__ out, const __grid_constant__ UnpackParts parts, int max_len, long long row_vecs) {
+  chain_enter();
+  const UnpackPart p = parts.part[blockIdx.z];
+  const int at = p.from + static_cast<int>(blockIdx.x);
+  if (at >= p.zero_to) return;
+  const bool copied = at < p.to;
+  const uint4* src = rows + (p.row + (copied ? static_cast<long long>(at - p.from) : 0)) * row_vecs;
+  uint4* dst = out + (static_cast<long long>(p.sequence) * max_len + at) * row_vecs;
+  for (long long c = blockIdx.y * 2048LL + threadIdx.x; c < row_vecs && c < (blockIdx.y + 1) * 2048LL; c += 1024) {
+    uint4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (copied && c + i * 256 < row_vecs) v[i] = src[c + i * 256];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (c + i * 256 < row_vecs) dst[c + i * 256] = v[i];
+  }
+}
+
 // Row argmax; ties resolve to the lowest index like torch/numpy argmax.
 template <typename T>
 __global__ void __launch_bounds__(1024)
@@ -539,6 +566,34 @@ extern "C" int cacheir_b200_embedding_gather(const void* table, const int64_t* i
   CB200_DISPATCH_DTYPE(dtype, (launch_chained(embedding_gather_kernel<T>, rows, 256, 0, as_stream(stream),
                                   static_cast<const T*>(table), ids, static_cast<T*>(out), hidden, vocab)));
   return launch_status();
+}
+
+extern "C" int cacheir_b200_unpack_rows(const void* rows, void* out, const int32_t* parts, int n_parts, int sequences, int max_len,
+                                        long long row_bytes, void* stream) {
+  if (n_parts <= 0 || row_bytes <= 0) return 0;
+  if (!rows || !out || !parts) return CACHEIR_B200_EINVAL;
+  if (row_bytes % 16 != 0 || !aligned_to(rows, 16) || !aligned_to(out, 16)) return CACHEIR_B200_EALIGN;
+  if ((row_bytes / 16 + 2047) / 2048 > 65535) return CACHEIR_B200_ELIMIT;
+  for (int i = 0; i < n_parts; ++i) {
+    const int32_t* p = parts + 5 * i;
+    if (p[0] < 0 || p[0] >= sequences || p[1] < 0 || p[2] < p[1] || p[3] < p[2] || p[3] > max_len || p[4] < 0) return CACHEIR_B200_EINVAL;
+  }
+  for (int first = 0; first < n_parts; first += kUnpackParts) {
+    const int count = n_parts - first < kUnpackParts ? n_parts - first : kUnpackParts;
+    UnpackParts args{};
+    int most = 0;
+    for (int i = 0; i < count; ++i) {
+      const int32_t* p = parts + 5 * (first + i);
+      args.part[i] = {p[0], p[1], p[2], p[3], p[4]};
+      if (p[3] - p[1] > most) most = p[3] - p[1];
+    }
+    if (most == 0) continue;
+    launch_chained(unpack_rows_kernel, dim3(most, static_cast<unsigned>((row_bytes / 16 + 2047) / 2048), count), 256, 0, as_stream(stream),
+                   static_cast<const uint4*>(rows), static_cast<uint4*>(out), args, max_len, row_bytes / 16);
+    const int rc = launch_status();
+    if (rc != 0) return rc;
+  }
+  return 0;
 }
 
 extern "C" int cacheir_b200_argmax_rows(const void* logits, int64_t* out_ids, int rows, int vocab,

@@ -8,6 +8,7 @@ allocation, CUDA-graph friendly) or are allocated here.
 """
 from __future__ import annotations
 
+import ctypes
 import math
 
 import torch
@@ -519,6 +520,22 @@ def embedding_gather(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor |
                                                     int(table.shape[0]), dtype_code(table.dtype), _stream()),
           "embedding_gather")
     return out
+
+
+def unpack_rows(rows: torch.Tensor, out: torch.Tensor, parts: list[tuple[int, int, int, int]]) -> None:
+    """Rows of a shared prompt pass, part after part, into out [sequences, max_len, columns]: (sequence, first token, last token + 1, end of
+    the zeros behind it) of each part."""
+    _require_cuda(rows, out)
+    if rows.dtype != out.dtype or rows.dim() != 2 or out.dim() != 3 or rows.shape[1] != out.shape[2] or not rows.is_contiguous() or not out.is_contiguous():
+        raise ValueError("unpack_rows takes contiguous rows [R, columns] and out [sequences, max_len, columns] of one type")
+    if sum(hi - lo for _, lo, hi, _ in parts) > rows.shape[0]:
+        raise ValueError("the parts have more tokens than there are rows")
+    flat, row = [], 0
+    for sequence, lo, hi, end in parts:
+        flat += [sequence, lo, hi, end, row]
+        row += hi - lo
+    check(_lib.load().cacheir_b200_unpack_rows(rows.data_ptr(), out.data_ptr(), (ctypes.c_int32 * len(flat))(*flat), len(parts), int(out.shape[0]),
+                                               int(out.shape[1]), int(out.shape[2]) * out.element_size(), _stream()), "unpack_rows")
 
 
 def argmax_rows(logits: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:

@@ -1477,8 +1477,9 @@ class B200DecodeRuntime:
         """Prefill of several sequences through shared passes (cuda.py:584-629 pads every prompt to the longest and
         masks; here nothing is padded): the (sequence, position) pairs are laid out in order and cut into passes of
         `pass_rows` rows; a pass appends all its K/V rows, then every row attends to the tokens up to itself
-        through its own sequence's page table. `out[i, t]` receives the logits of token t of sequence i."""
+        through its own sequence's page table. `out[i, t]` (any contents) receives the logits of token t of sequence i, or zeros."""
         eng = self._engine
+        max_len = int(out.shape[1])
         starts = [session.kv_cache.tokens for session in sessions]
         for session, ids in zip(sessions, token_id_batches):
             session.kv_cache.extend(len(ids))                  # reserves the pages of the whole prompt
@@ -1487,8 +1488,14 @@ class B200DecodeRuntime:
             passes = cut_passes(token_id_batches, self._pass_rows(sum(map(len, token_id_batches))), _PromptPlan.SEQUENCES)
             for part in passes:                                # (sequence, first token, last token + 1)
                 logits = self._run_prompt_rows([(sessions[i].kv_cache, starts[i] + lo, token_id_batches[i][lo:hi]) for i, lo, hi in part])
-                for (i, lo, hi), rows in zip(part, logits.split([hi - lo for _, lo, hi in part])):
-                    out[i, lo:hi] = rows
+                # (zeros behind a sequence's last token come with it)
+                places = [(i, lo, hi, max_len if hi == len(token_id_batches[i]) else hi) for i, lo, hi in part]
+                if logits.dtype == out.dtype and out.shape[2] * out.element_size() % 16 == 0:
+                    ops.unpack_rows(logits, out, places)
+                else:
+                    for (i, lo, hi, end), rows in zip(places, logits.split([hi - lo for _, lo, hi in part])):
+                        out[i, lo:hi] = rows
+                        out[i, hi:end] = 0
         eng.count("cacheir.b200_prefill_chunk", len(passes))
 
     def run_prefill_batch(self, sessions: list["B200DecodeRuntime"], token_id_batches: list[list[int]]) -> torch.Tensor:
@@ -1503,16 +1510,17 @@ class B200DecodeRuntime:
         for session in sessions:
             session.kv_cache.clear()
         vocab = int(self._engine.config.vocab_size)
-        out = torch.zeros((len(sessions), max(lens), vocab), device=self.device,
-                          dtype=torch.float32 if self._engine.ragged else self.dtype)
+        chunk = self._engine.prefill_chunk
+        packed = not self._engine.ragged and chunk > 1 and sum(lens) > chunk // 4
+        out = (torch.empty if packed else torch.zeros)((len(sessions), max(lens), vocab), device=self.device,
+                                                       dtype=torch.float32 if self._engine.ragged else self.dtype)
         if self._engine.ragged:
             logits = self.run_step_batch(sessions, token_id_batches, [list(range(n)) for n in lens])
             for i, part in enumerate(logits.split(lens)):
                 out[i, : lens[i]] = part
             self._engine.count("cacheir.b200_prefill_batch_graph")
             return out
-        chunk = self._engine.prefill_chunk
-        if chunk > 1 and sum(lens) > chunk // 4:
+        if packed:
             # Packed prefill: the prompt tokens of all sequences are the rows of passes through the decode graph (up to
             # `pass_rows` each), sequence after sequence, so short prompts share a pass and a long prompt spans several.
             self._enforce_memory_limit()

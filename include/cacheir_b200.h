@@ -492,6 +492,11 @@ int cacheir_b200_add(const void* a, const void* b, void* out, size_t total, int 
 int cacheir_b200_embedding_gather(const void* table, const int64_t* ids, void* out,
                                   int rows, int hidden, int vocab, int dtype,
                                   void* stream);
+/* The rows of a shared prompt pass to zero-padded [sequences, max_len, row] (the padding of the reference's batched prefill,
+ * cuda.py:584-629). `parts` (host memory, read during the call) has five numbers for each of n_parts parts: sequence, first token, last
+ * token + 1, end of the zeros that follow it (the last token + 1: none), and the part's first row in `rows`. */
+int cacheir_b200_unpack_rows(const void* rows, void* out, const int32_t* parts, int n_parts, int sequences, int max_len,
+                             long long row_bytes, void* stream);
 /* Replaces `_argmax_tokens` (cacheir/runtime/scheduler.py:535-543) for
  * device-side greedy feedback: out_ids[r] = first index of the row maximum. */
 int cacheir_b200_argmax_rows(const void* logits, int64_t* out_ids, int rows, int vocab,
