@@ -35,6 +35,7 @@ constexpr int kTileN = 128;
 constexpr int kBlockK = 64;               // elements of k per stage: one 128-byte swizzle span
 constexpr int kWBytes = kTileN * kBlockK * 2;
 constexpr int kThreads = 320;
+constexpr int kPairThreads = kThreads + 32;       // a warp more for the copies of the tokens
 constexpr int kAhead = 8;                 // weight tiles a CTA asks for before its turn
 constexpr int kTailBytes = 512;                    // barriers; from byte 128 on the places of up to 64 rows
 
@@ -419,7 +420,7 @@ __device__ __forceinline__ void mma_f16_ss_pair(uint32_t tmem_d, uint64_t a_desc
 }
 
 template <int EPI, int TT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 dense_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const cacheir_b200_dense_args p) {
   constexpr int S = pair_stages(TT);
   extern __shared__ uint8_t smem_raw[];
@@ -458,21 +459,34 @@ dense_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       int it = 0;
       bool ok = true;
       for (int tile = blockIdx.x >> 1; tile < tiles && ok; tile += pairs) {
-        const int t0 = tile % t_tiles * TT, w = tile / t_tiles % w_tiles, z = tile / t_tiles / w_tiles;
+        const int w = tile / t_tiles % w_tiles, z = tile / t_tiles / w_tiles;
         for (int i = 0; i < kblocks; ++i, ++it) {
           const int s = it % S;
           if (it >= S && !mbar_wait(smem_u32(&empty[s]), ((it / S) & 1) ^ 1, &g_dense_status, (6 << 8) | 5)) { ok = false; break; }
           const uint32_t bar = map_to_rank(smem_u32(&full[s]), 0);
-          if (rank == 0) mbar_expect_tx(smem_u32(&full[s]), 2 * pair_stage_bytes(TT));
-          const int k = i * kBlockK;
-          tma_load_2d_pair(smem_u32(s_w + s * kWBytes), &tmap_w, bar, k, z * p.w_batch_rows + (2 * w + static_cast<int>(rank)) * kTileN);
-          tma_load_2d_pair(smem_u32(s_x + s * (TT / 2) * kBlockK * 2), &tmap_x, bar, z * p.x_batch_cols + k, t0 + static_cast<int>(rank) * (TT / 2));
+          if (rank == 0) mbar_expect_tx(smem_u32(&full[s]), 2 * pair_stage_bytes(TT));      // (of all four copies)
+          tma_load_2d_pair(smem_u32(s_w + s * kWBytes), &tmap_w, bar, i * kBlockK, z * p.w_batch_rows + (2 * w + static_cast<int>(rank)) * kTileN);
         }
       }
       // Nothing may still be on its way when the blocks end (the even CTA sees the copies of both; a wait elsewhere may have given up)
       if (rank == 0)
         for (int i = it > S ? it - S : 0; i < it; ++i)
           if (!mbar_wait(smem_u32(&full[i % S]), (i / S) & 1, &g_dense_status, (6 << 8) | 4)) break;
+    }
+  } else if (warp == kThreads / 32) {
+    // The tokens: a thread issues a copy in about 200 cycles, and a k block of 128 tokens takes the tensor cores 256.
+    if (lane == 0) {
+      int it = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x >> 1; tile < tiles && ok; tile += pairs) {
+        const int t0 = tile % t_tiles * TT, z = tile / t_tiles / w_tiles;
+        for (int i = 0; i < kblocks; ++i, ++it) {
+          const int s = it % S;
+          if (it >= S && !mbar_wait(smem_u32(&empty[s]), ((it / S) & 1) ^ 1, &g_dense_status, (6 << 8) | 10)) { ok = false; break; }
+          tma_load_2d_pair(smem_u32(s_x + s * (TT / 2) * kBlockK * 2), &tmap_x, map_to_rank(smem_u32(&full[s]), 0), z * p.x_batch_cols + i * kBlockK,
+                           t0 + static_cast<int>(rank) * (TT / 2));
+        }
+      }
     }
   } else if (warp == 1) {
     if (rank == 0) {
@@ -592,7 +606,7 @@ int launch_pair(const cacheir_b200_dense_args& p, cudaStream_t stream) {
   if (e != cudaSuccess) return static_cast<int>(e);
   const long long tiles = static_cast<long long>((p.T + TT - 1) / TT) * ((p.N + 2 * kTileN - 1) / (2 * kTileN)) * p.batch;
   const int pairs = tiles < kNumSMs / 2 ? static_cast<int>(tiles) : kNumSMs / 2;
-  launch_chained(kern, 2 * pairs, kThreads, kSmem, stream, tw, tx, p);
+  launch_chained(kern, 2 * pairs, kPairThreads, kSmem, stream, tw, tx, p);
   return launch_status();
 }
 
