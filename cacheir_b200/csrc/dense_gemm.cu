@@ -26,7 +26,8 @@ Shape choose_shape(int T, int N, int K, int batch) {
 
 // Time of the product in nanoseconds on pairs (tiles of 256 weight rows x `tt` tokens) and on single CTAs: a turn is the k blocks of a
 // tile plus its epilogue, of which pairs show only what the next tile's main loop does not cover. Fitted to 325 plain products of
-// 768 to 2048 tokens, 512 to 22016 rows and K of 512 to 8192, timed on both forms; 3 to 7 % off (standard deviation).
+// 768 to 2048 tokens, 512 to 22016 rows and K of 512 to 8192, timed on both forms; 3 to 7 % off (standard deviation). Since pairs issue and copy
+// faster their tiles of 128 tokens take up to a third less than this says (1001x6144x2048 37.7 / 25.2 us): the choice leaves some of that unused.
 long long pair_cost(int T, int N, int K, int batch, int tt) {
   const long long tiles = static_cast<long long>((T + tt - 1) / tt) * ((N + 2 * kTileN - 1) / (2 * kTileN)) * batch;
   const long long turns = (tiles + kNumSMs / 2 - 1) / (kNumSMs / 2), kblocks = (K + kBlockK - 1) / kBlockK;

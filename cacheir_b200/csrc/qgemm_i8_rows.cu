@@ -11,8 +11,8 @@
 // serves both. That is 32 KB per CTA and 512 tensor-core cycles; a CTA by itself would need 48 KB for the same cycles (both planes), more
 // than L2 delivers. The accumulator takes 256 of the 512 tensor-memory columns, so the epilogue of one tile runs under the main
 // loop of the next. Persistent: pairs walk the tiles with the row blocks innermost, so that the weights of the few tiles
-// in flight are read from HBM once and the activation planes stay in L2. 2048 rows, int8 28672 x 4096 with SwiGLU: 311 us, 3.1 POPS,
-// tensor pipe active 80 % of the cycles (32 passes of 64 rows take 26 us each for half of these weights).
+// in flight are read from HBM once and the activation planes stay in L2. 2048 rows, int8 28672 x 4096 with SwiGLU: 297 us, 3.2 POPS
+// (311 us and 80 % of the tensor cycles while a branch that one lane took issued the MMAs; 32 passes of 64 rows take 26 us each for half of these weights).
 //
 // Few tiles leave most SMs idle, so that a tile's K range is split over the SPLIT pairs of a larger cluster (one tile per
 // cluster then): every CTA lays its partial sums for the other pairs' shares of the activation rows out in its drained ring, one bulk copy
@@ -402,6 +402,7 @@ int launch_split(const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, const Row
   return launch_status();
 }
 
+// (Times from before partial sums travelled in bulk, which takes 10 to 15 % off the split forms.)
 // Pairs along K, with at least four k blocks each: four for up to twelve tiles (sixteen clusters of eight CTAs do not run at
 // once: 100 rows of int8 4096 x 4096 30.0 us with four, 19.5 with two, 23.5 with one; 1280 x 8192 19.6, 32.7 with one), two
 // for up to 33 (4096 x 14336 43.6 us with four, 32.6 with two, 47.5 with one; so many clusters of four CTAs run at once: 37 tiles
