@@ -248,7 +248,8 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
             const int to = e < share ? e : e + 1, slot = share < to ? share : share - 1;
             bulk_copy_to_rank(smem_u32(s_in + slot * kSlab), smem_u32(s_out + e * kSlab), kSlab * 4, smem_u32(xch), 2 * to + rank);
           }
-        ok = ok && mbar_wait(smem_u32(xch), 0, &g_i8_rows_status, (12 << 8) | 10);
+        // (also where an earlier wait gave up: the other pairs send all the same, and this block must not end before their sums have landed)
+        ok = mbar_wait(smem_u32(xch), 0, &g_i8_rows_status, (12 << 8) | 10) && ok;
         col_ok = col_ok && ok;
         __syncwarp();
       }

@@ -47,6 +47,21 @@ def test_status_words_name_one_kernel_file():
     assert len(owners) >= 12 and all(len(files) == 1 for files in owners.values()), owners
 
 
+def test_copies_between_blocks_are_waited_for_whatever_went_before():
+    """Where a bounded wait gave up, the other blocks of a cluster still send their sums: a kernel that then skipped the wait for them would end
+    with copies on their way into its shared memory."""
+    waits = []
+    for path in sorted((ROOT / "cacheir_b200" / "csrc").glob("*.cu")):
+        statements = re.sub(r"//.*", "", path.read_text()).split(";")
+        copies = [s for s in statements if re.search(r"bulk_copy_to_rank\((?!uint32_t)", s)]
+        bars = {re.search(r"(\w+)\)?,[^,]*\)$", s.strip()).group(1) for s in copies}          # the last argument but one
+        found = [s for s in statements if bars and re.search(r"wait\((?:smem_u32\()?(?:%s)\b" % "|".join(bars), s)]
+        assert len(found) >= len(copies), (path.name, bars)
+        waits += [(path.name, s.strip()) for s in found]
+    assert len(waits) >= 4
+    assert not [w for w in waits if "&&" in w[1].split("wait(")[0]]
+
+
 def test_ops_refuse_cpu_tensors():
     import torch
     from cacheir_b200 import ops
