@@ -367,7 +367,7 @@ extern "C" int cacheir_b200_combine_residual(float* residual, const void* y, con
                                              void* stream) {
   if (rows <= 0 || width <= 0) return 0;
   if (!residual || !y || !place_of || !weight || top < 1 || !self || next_b || !row_next_ok(next_mode, next_w, next_out)) return CACHEIR_B200_EINVAL;
-  const RowNext nx{next_mode, next_w, next_alpha, next_out};
+  const RowNext nx = row_next(next_mode, next_w, next_alpha, next_out);
   const bool vec = width % 4 == 0 && aligned_to(residual, 16) && aligned_to(y, 16) && aligned_to(self, 16) && aligned_to(shared, 16) &&
                    row_next_aligned(next_mode, next_w, next_out);
 #define CB200_COMBINE(VEC)                                                                                                                 \

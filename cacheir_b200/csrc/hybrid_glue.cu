@@ -557,7 +557,7 @@ extern "C" int cacheir_b200_scaled_embedding(const void* table, const int64_t* i
   if (!table || !ids || !residual || vocab <= 0) return CACHEIR_B200_EINVAL;
   if (accumulate || row_next_norms(next_mode)) {
     if (!row_next_ok(next_mode, next_w, next_out)) return CACHEIR_B200_EINVAL;
-    const RowNext rn{next_mode, next_w, next_alpha, next_out};
+    const RowNext rn = row_next(next_mode, next_w, next_alpha, next_out);
     const bool vec = width % 4 == 0 && aligned_to(table, 16) && aligned_to(residual, 16) && row_next_aligned(next_mode, next_w, next_out);
 #define CB200_ROWS(VEC, ADD)                                                                  \
   launch_chained(embedding_rows_kernel<T, VEC, ADD>, rows, kRowThreads, 0, as_stream(stream), static_cast<const T*>(table), ids, residual, width, vocab, scale, rn)
@@ -639,7 +639,7 @@ extern "C" int cacheir_b200_residual_add(float* residual, const void* y, const f
                                          const float* next_b, float next_alpha, void* next_out, int dtype, void* stream) {
   if (rows <= 0 || width <= 0) return 0;
   if (!residual || !y || next_b || !row_next_ok(next_mode, next_w, next_out)) return CACHEIR_B200_EINVAL;
-  const RowNext nx{next_mode, next_w, next_alpha, next_out};
+  const RowNext nx = row_next(next_mode, next_w, next_alpha, next_out);
   const bool vec = width % 4 == 0 && aligned_to(residual, 16) && aligned_to(y, 16) && (!scale || aligned_to(scale, 16)) &&
                    row_next_aligned(next_mode, next_w, next_out);
 #define CB200_ADD(VEC, HELD) \
@@ -658,7 +658,7 @@ extern "C" int cacheir_b200_residual_rms_pair(float* residual, const void* y1, c
                                               float next_alpha, void* next_out, int dtype, void* stream) {
   if (rows <= 0 || width <= 0) return 0;
   if (!residual || !y1 || !w1 || !y2 || !w2 || next_b || !row_next_ok(next_mode, next_w, next_out)) return CACHEIR_B200_EINVAL;
-  const RowNext nx{next_mode, next_w, next_alpha, next_out};
+  const RowNext nx = row_next(next_mode, next_w, next_alpha, next_out);
   const bool vec = width % 4 == 0 && aligned_to(residual, 16) && aligned_to(y1, 16) && aligned_to(y2, 16) && aligned_to(w1, 16) &&
                    aligned_to(w2, 16) && row_next_aligned(next_mode, next_w, next_out);
 #define CB200_PAIR(VEC, HELD)                                                                                                        \

@@ -8,7 +8,7 @@ namespace cb200 {
 
 struct RowNext {
   int mode;             // NEXT_NONE, NEXT_COPY, NEXT_RMS or NEXT_LAYER
-  const float* w;
+  const float* w;       // null unless a norm follows: kernels ask for it ahead, before they look at the mode
   float eps;
   void* out;
 };
@@ -17,6 +17,8 @@ inline bool row_next_norms(int mode) { return mode == CACHEIR_B200_NEXT_RMS || m
 inline bool row_next_ok(int mode, const float* w, const void* out) {
   return mode == CACHEIR_B200_NEXT_NONE || (mode == CACHEIR_B200_NEXT_COPY && out) || (row_next_norms(mode) && w && out);
 }
+// What a caller gives as `w` where no norm follows is never looked at, nor is its alignment (below).
+inline RowNext row_next(int mode, const float* w, float eps, void* out) { return {mode, row_next_norms(mode) ? w : nullptr, eps, out}; }
 inline bool row_next_aligned(int mode, const float* w, const void* out) {
   return mode == CACHEIR_B200_NEXT_NONE || (aligned_to(out, 16) && (!row_next_norms(mode) || aligned_to(w, 16)));
 }

@@ -62,6 +62,15 @@ def test_copies_between_blocks_are_waited_for_whatever_went_before():
     assert not [w for w in waits if "&&" in w[1].split("wait(")[0]]
 
 
+def test_norm_weights_that_a_mode_does_not_use_reach_no_kernel():
+    """A call whose row is only stored or copied may leave anything in `next_w`: kernels ask for it ahead wherever it is there, in 16-byte
+    pieces whose alignment only a norm's weights are checked for."""
+    built = []
+    for path in sorted((ROOT / "cacheir_b200" / "csrc").glob("*.cu*")):
+        built += [(path.name, line.strip()) for line in path.read_text().splitlines() if re.search(r"\bRowNext \w+ ?[{=]", line)]
+    assert len(built) >= 4 and all("= row_next(" in line for _, line in built), built
+
+
 def test_ops_refuse_cpu_tensors():
     import torch
     from cacheir_b200 import ops
