@@ -74,7 +74,7 @@ def build(force: bool = False, verbose: bool = False, groups: tuple[str, ...] = 
     BUILD_DIR.mkdir(parents=True, exist_ok=True)
     LIB_DIR.mkdir(parents=True, exist_ok=True)
     sources = sorted({src for group in groups for src in group_sources(group)})
-    headers = sorted(CSRC.glob("*.cuh")) + sorted(INCLUDE.glob("*.h")) + [Path(__file__)]
+    headers = sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + sorted(INCLUDE.glob("*.h")) + [Path(__file__)]
     extra = ["-Xptxas", "-v"] if verbose else []
 
     def compile_one(src: Path) -> Path:

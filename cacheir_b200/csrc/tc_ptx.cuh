@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "wait_limit.h"
+
 namespace cb200 {
 namespace ptx {
 
@@ -40,19 +42,23 @@ __device__ __forceinline__ bool mbar_try_wait_suspended(uint32_t bar, uint32_t p
       : "=r"(done) : "r"(bar), "r"(parity), "r"(hint) : "memory");
   return done != 0;
 }
-__device__ __forceinline__ uint64_t timer_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+// (the clock's lower half: four seconds)
+__device__ __forceinline__ uint32_t timer_ns() {
+  uint32_t t;
+  asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
   return t;
 }
-constexpr uint64_t kWaitLimitNs = 1000u * 1000u * 1000u;   // bounded waits: 1 s, then give up and flag
-constexpr uint32_t kSuspendNs = 20u * 1000u;
+// Where the clock has ended a wait (out of line: hardly ever).
+static __device__ __noinline__ bool mbar_wait_by_looks(uint32_t bar, uint32_t parity) {
+  return wait_by_looks([&] { return mbar_try_wait_suspended(bar, parity, kSuspendNs); }, [] { return timer_ns(); });
+}
 // Returns false, after recording `code` in *status, when the time is up.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status, int code) {
   if (mbar_try_wait(bar, parity)) return true;         // (56 cycles where the phase is over; with a hint 92)
-  const uint64_t begin = timer_ns();
+  const uint32_t begin = timer_ns();
   while (!mbar_try_wait_suspended(bar, parity, kSuspendNs))
-    if (timer_ns() - begin > kWaitLimitNs) {
+    if (timer_ns() - begin > kWaitNs) {
+      if (mbar_wait_by_looks(bar, parity)) return true;
       atomicCAS(status, 0, code);
       return false;
     }

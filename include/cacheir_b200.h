@@ -373,7 +373,7 @@ int cacheir_b200_peer_all_gather(void* const* data, void* const* flags, void* ou
                                  void* stream);
 
 /* Status word of the kernels that wait on hardware barriers (the tensor-core GEMM):
- * 0, or a non-zero code recorded by the first wait that ran out of its poll budget
+ * 0, or a non-zero code recorded by the first wait that ran out of time
  * (the kernel then drains and returns instead of hanging; its output is undefined).
  * Synchronises with the device. `reset` != 0 clears the word after reading it. */
 int cacheir_b200_device_status(int reset);

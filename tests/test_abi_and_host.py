@@ -4,6 +4,7 @@ behaves like the reference's. No GPU and no compute calls."""
 import ctypes
 import json
 import re
+import subprocess
 from pathlib import Path
 
 import numpy as np
@@ -60,6 +61,32 @@ def test_copies_between_blocks_are_waited_for_whatever_went_before():
         waits += [(path.name, s.strip()) for s in found]
     assert len(waits) >= 4
     assert not [w for w in waits if "&&" in w[1].split("wait(")[0]]
+
+
+def test_a_wait_does_not_give_up_because_the_program_was_paused(tmp_path):
+    """A host program takes the looks of a bounded wait with a clock of its own: an hour in which nothing ran, or thousands of short pauses, do
+    not end it much earlier; without pauses, or with a clock that stands still, it does end. What arrives during a pause is seen."""
+    (tmp_path / "looks.cpp").write_text("""
+#include <cstdio>
+#include "wait_limit.h"
+static long looks(unsigned long long gap, long every, unsigned long long pause, long arrives = -1) {
+  long n = 0;
+  unsigned long long now = 1ull << 33;
+  auto look = [&] { now += every && ++n % every == 0 ? pause : gap; n += !every; return n == arrives; };
+  return cb200::wait_by_looks(look, [&] { return static_cast<uint32_t>(now); }) ? -n : n;
+}
+int main() {
+  const unsigned long long look = cb200::kSuspendNs, hour = 3600ull * 1000 * 1000 * 1000;
+  std::printf("%u %ld %ld %ld %ld %ld\\n", cb200::kSuspendNs, looks(look, 0, 0), looks(look, 100, hour), looks(look, 10, 2000 * 1000), looks(0, 0, 0), looks(look, 5, hour, 5));
+}
+""")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(ROOT / "cacheir_b200" / "csrc"), "looks.cpp", "-o", "looks"], cwd=tmp_path, check=True)
+    suspend, plain, hours, slices, still, seen = map(int, subprocess.run([str(tmp_path / "looks")], capture_output=True, check=True).stdout.split())
+    assert 0.45 <= plain * suspend * 1e-9 <= 0.55
+    assert hours >= 0.9 * plain and slices >= 0.6 * plain
+    assert plain < still <= 1 << 30
+    assert seen == -5
+    assert "wait_by_looks(" in (ROOT / "cacheir_b200" / "csrc" / "tc_ptx.cuh").read_text()
 
 
 def test_norm_weights_that_a_mode_does_not_use_reach_no_kernel():
