@@ -245,15 +245,18 @@ int qgemv_dispatch(const void* x, const void* norm_weight, float norm_eps, const
   if (M > 64 && !p.x_prequantized && qgemm_i8_rows_supported(p, workspace, workspace_bytes) && qgemm_i8_rows_preferred(p))
     return plan_only ? 1 << 8 : launch_qgemm_i8_rows(p, nullptr, workspace, st);
   if (M > 64 && !p.x_prequantized && !norm_weight) {
-    // The integer tensor-core kernel takes up to 64 batch rows per launch, the fp16 one up to 128. A taller
+    // The integer tensor-core kernel takes up to 64 batch rows per launch, the fp16 ones up to 128. A taller
     // batch runs as chunks of that height (the weights stream once per chunk, still far cheaper than the
     // CUDA-core kernel at these heights) when a chunk-sized problem of the same shape is tensor-core eligible.
     QGemvParams c = p;
     c.M = 64;
     const bool i8_ok = qgemm_i8_supported(c, workspace, workspace_bytes);
     if (i8_ok || (!c.paired && qgemm_tc_supported(c))) {
-      if (plan_only) return i8_ok ? ((1 << 8) | qgemm_i8_plan(c)) : (2 << 8);
       const int rows = i8_ok ? 64 : 128;
+      if (plan_only) {                                // (of the first chunk)
+        c.M = M < rows ? M : rows;
+        return i8_ok ? (1 << 8) | qgemm_i8_plan(c) : qgemm_w4_preferred(c) ? (4 << 8) | qgemm_w4_plan(c) : 2 << 8;
+      }
       const size_t n_out = epilogue == CACHEIR_B200_EPI_SWIGLU ? static_cast<size_t>(N) / 2 : static_cast<size_t>(N);
       for (int m0 = 0; m0 < M; m0 += rows) {
         c.M = M - m0 < rows ? M - m0 : rows;

@@ -226,7 +226,7 @@ def qgemv_plan(m: int, n: int, k: int, *, bits: int, group_size: int = 0, epilog
                prequantized: bool = False, paired: bool = False, workspace: bool = True) -> dict:
     """Which kernel `qgemv` launches for these extents: {"family": "i8"|"f16"|"cuda_core"|"stream_int4", "split_k", "kernel"},
     kernel: the family or, within it, "i8_rows" (blocks of 128 rows), "stream" with its "row_groups", "split" and "tensor_memory"
-    (is that where the weights go?), "stream_rows" (many weight rows in row order). epilogue 3 asks about `qkv_rope_append`."""
+    (is that where the weights go?), "stream_rows" (many weight rows in row order). Of a batch that runs in chunks it is the first one's. epilogue 3 asks about `qkv_rope_append`."""
     layout = (1 if tiled else 0) | (2 if prequantized else 0) | (4 if paired else 0)
     code = int(_lib.load().cacheir_b200_qgemv_plan(int(m), int(n), int(k), int(bits), int(group_size), int(epilogue), layout,
                                                    1 if workspace else 0))

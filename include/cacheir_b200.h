@@ -214,9 +214,8 @@ int cacheir_b200_qgemv(const void* x, const void* packed, const void* scales,
  * signed bytes, 2^-15 of the row maximum) in the workspace by a pre-pass kernel. Batches above 64 rows of tile-ordered
  * codes run as blocks of 128 rows in one launch, with the scratch of all rows (the bytes below grow with M above 64);
  * other layouts, and a workspace that only holds 64 rows, as
- * 64-row chunks (128-row chunks on the fp16 tensor-core kernel, which takes 65..128 rows in
- * one launch with the activations as the 128-row operand). Other shapes ignore the
- * workspace. Which kernel runs depends on the extents (cacheir_b200_qgemv_plan), and the kernels sum in different orders and
+ * 64-row chunks. Other shapes ignore the workspace; they run as 128-row chunks on the fp16 tensor-core kernels (one launch for
+ * 65..128 rows), group-wise int4 of a million numbers and more on the one that takes its weights from tensor memory. Which kernel runs depends on the extents (cacheir_b200_qgemv_plan), and the kernels sum in different orders and
  * forms: int4 rows of up to 8 (weights of three million numbers and more: 128; group-wise 32) run on exact fp16 activations with float32 sums, taller
  * batches per row on 16-bit fixed point with exact integer sums, so the last bits of a row may change with the number of rows
  * beside it (and, group-wise, for the last chunk behind chunks of 128). workspace may be NULL (then this is cacheir_b200_qgemv). The workspace is only used during the call's own kernels; two
@@ -246,8 +245,8 @@ int cacheir_b200_rmsnorm_qgemv(const void* x, const void* norm_weight, float eps
 /* Which kernel cacheir_b200_qgemv_ex would launch for these extents and flags (fp16 activations, aligned
  * pointers): (family << 8) | detail, family 1 = integer tensor core with detail = its split-K factor (0: blocks of 128
  * rows in one launch), 2 = fp16 tensor core, 3 = CUDA cores, 4 = streaming int4 product with detail = (row groups << 4) |
- * CTAs along K (0: the GEMV for many weight rows in row order; + 128: weights as the tensor-memory operand); epilogue 3 asks about
- * cacheir_b200_qkv_rope_append. Negative:
+ * CTAs along K (0: the GEMV for many weight rows in row order; + 128: weights as the tensor-memory operand). Of a batch that runs in chunks
+ * it is the first chunk's. epilogue 3 asks about cacheir_b200_qkv_rope_append. Negative:
  * the validation code the call would return. Launches nothing. No counterpart in the reference (its
  * kernel choice is the declarative `attrs["kernel"]`, cacheir/passes/transformer.py:391-424). */
 int cacheir_b200_qgemv_plan(int M, int N, int K, int bits, int group_size, int epilogue,

@@ -53,3 +53,30 @@ def test_weights_in_tensor_memory(m, n, k, split, tiled):
                 again = ops.qgemv(x, v.packed_values, v.scales, v.zero_points, n=n, k=k, residual=res, **kw)
                 assert torch.equal(again, y)
     assert int(_lib.load().cacheir_b200_device_status(1)) == 0
+
+
+# batches that run as chunks of 128 rows, the last one a few rows, a share, or all of them
+@pytest.mark.parametrize("tiled", [True, False])
+@pytest.mark.parametrize("m", [129, 150, 177, 256])
+def test_taller_batches_in_chunks(m, tiled):
+    """The plan names the kernel that the first chunk takes, and every chunk has the bits of a call of its own."""
+    from cacheir_b200 import _lib, ops
+    from cacheir_b200.quantization import dequantize_device, pack_weight_device, quantized_matmul, to_tiled
+
+    n, k = 2048, 1024
+    g = torch.Generator(device="cuda").manual_seed(m)
+    w = pack_weight_device(torch.randn((n, k), device="cuda", generator=g) * 0.02, "int4_g128")
+    x, res = torch.randn((m, k), device="cuda", generator=g).half(), torch.randn((m, n), device="cuda", generator=g).half()
+    v = to_tiled(w) if tiled else w
+    kw = dict(bits=4, group_size=128, tiled=tiled, workspace=False)
+    assert ops.qgemv_plan(m, n, k, **kw) == ops.qgemv_plan(128, n, k, **kw)
+    assert ops.qgemv_plan(m, n, k, **kw)["tensor_memory"]
+    want = x.double() @ dequantize_device(w, torch.float32).double().T
+    for epilogue, residual in ((ops.EPI_NONE, None), (ops.EPI_RESIDUAL, res)):
+        y = quantized_matmul(x, v, epilogue=epilogue, residual=residual)
+        full = want if residual is None else want + residual.double()
+        assert float((y.double() - full).norm() / full.norm()) <= 2.8e-4
+        tail = quantized_matmul(x[128:], v, epilogue=epilogue, residual=None if residual is None else residual[128:])
+        assert torch.equal(y[128:], tail)
+    assert ops.qgemv_plan(150, 384, 512, **kw)["family"] == "f16"            # (fewer than a million numbers)
+    assert int(_lib.load().cacheir_b200_device_status(1)) == 0
