@@ -753,8 +753,9 @@ class _DecodePlan:
                 and hasattr(self, "_gemm_ws") and not self._streams(weight, ops.EPI_SWIGLU if swiglu else ops.EPI_NONE))
 
     def _streams(self, weight: B200PackedWeight, epilogue: int) -> bool:
-        """Does a streaming int4 kernel run this fp16 product? It takes the rows as they are, without a pre-pass."""
-        if weight.bits != 4 or weight.group_size or self.batch > 64 or weight.shape[1] % 128:
+        """Does a streaming int4 kernel run this fp16 product (of any number of rows: the plan query knows)? It takes the rows as they are,
+        without a pre-pass."""
+        if weight.bits != 4 or weight.group_size or weight.shape[1] % 128:
             return False
         return ops.qgemv_plan(self.batch, *weight.shape, bits=4, epilogue=epilogue, tiled=weight.tiled, paired=weight.paired)["family"] == "stream_int4"
 
