@@ -292,12 +292,10 @@ def test_prompts_as_tensors():
         assert torch.equal(rt.run_prefill_batch([rt.fork(), rt.fork()], [form(p) for p in prompts]), want)
 
 
-# (intermediate 3072: the gate and up rows are the three million numbers from which up to 128 rows run without a pre-pass)
-@pytest.mark.parametrize("quant, batch, intermediate", [("int8", 3, 768), ("int8", 70, 768), ("int4_awq", 5, 768), ("int4_awq", 70, 768), ("int4_awq", 130, 768),
-                                                        ("int4_awq", 20, 3072), ("int4_awq", 65, 3072), ("int4_awq", 128, 3072), ("int4_awq", 129, 3072)])
-def test_launches_of_a_decode_step(quant, batch, intermediate):
+@pytest.mark.parametrize("quant, batch", [("int8", 3), ("int8", 70), ("int4_awq", 5), ("int4_awq", 70), ("int4_awq", 130)])
+def test_launches_of_a_decode_step(quant, batch):
     """What a plan counts per step is what runs (a product of more than 64 rows: its pre-pass and one kernel, not one per 64 rows)."""
-    rt = _runtime(quant, intermediate=intermediate)
+    rt = _runtime(quant)
     sessions = [rt.fork() for _ in range(batch)]
     rt.run_decode_batch(sessions, [1] * batch)
     plan = rt._engine.plans[("decode", batch)]
@@ -308,3 +306,11 @@ def test_launches_of_a_decode_step(quant, batch, intermediate):
         torch.cuda.synchronize()
     kernels = [e.name for e in profile.events() if e.device_type == torch.autograd.DeviceType.CUDA and not e.name.startswith("Mem")]
     assert len(kernels) == plan.launches_per_step, kernels
+
+
+# (intermediate 3072: the gate and up rows are the three million numbers from which up to 128 rows run without a pre-pass)
+@pytest.mark.parametrize("batch", [20, 65, 128, 129])
+def test_launches_of_an_int4_decode_step_of_wide_products(batch, monkeypatch):
+    narrow = _runtime
+    monkeypatch.setitem(globals(), "_runtime", lambda quant: narrow(quant, intermediate=3072))
+    test_launches_of_a_decode_step("int4_awq", batch)
