@@ -80,3 +80,35 @@ def test_taller_batches_in_chunks(m, tiled):
         assert torch.equal(y[128:], tail)
     assert ops.qgemv_plan(150, 384, 512, **kw)["family"] == "f16"            # (fewer than a million numbers)
     assert int(_lib.load().cacheir_b200_device_status(1)) == 0
+
+
+# group scales at the row counts where the two-CTA tile of 16 rows starts and ends, and one row beside it: groups of one and two k blocks, scales
+# of both types, k blocks that its three accumulators do not divide, every epilogue
+@pytest.mark.parametrize("tiled", [True, False])
+@pytest.mark.parametrize("m, n, k", [(4, 6272, 1024), (5, 3328, 2048), (8, 1536, 4352), (9, 5120, 1280), (15, 5100, 1280), (16, 2176, 3072), (17, 8960, 768)])
+def test_group_scales_with_weights_in_tensor_memory(m, n, k, tiled):
+    """Exact fp16 products, float32 sums, one rounding to fp16: as above. (int4_g128 and int4_g256 differ in their scales alone.)"""
+    from cacheir_b200 import _lib, ops
+    from cacheir_b200.quantization import dequantize_device, pack_weight_device, to_tiled
+
+    g = torch.Generator(device="cuda").manual_seed(m * 31 + n + k)
+    dense = torch.randn((n, k), device="cuda", generator=g) * 0.02
+    x = torch.randn((m, k), device="cuda", generator=g).half()
+    for quant in ("int4_g128", "int4_g256"):
+        w = pack_weight_device(dense, quant)
+        full = dequantize_device(w, torch.float32).double()
+        v = to_tiled(w) if tiled else w
+        for scales in (w.scales.half(), w.scales.float()):
+            assert torch.equal(scales.double(), w.scales.double())
+            for epilogue in (0, 1, 2) if n % 128 == 0 else (0, 1):
+                res = torch.randn((m, n), device="cuda", generator=g).half() if epilogue == 1 else None
+                kw = dict(bits=4, group_size=w.group_size, epilogue=epilogue, tiled=tiled)
+                assert ops.qgemv_plan(m, n, k, workspace=False, **kw)["tensor_memory"]
+                y = ops.qgemv(x, v.packed_values, scales, None, n=n, k=k, residual=res, **kw)
+                want = x.double() @ full.T
+                if epilogue == 2:
+                    want = torch.nn.functional.silu(want[:, :n // 2]) * want[:, n // 2:]
+                if epilogue == 1:
+                    want = want + res.double()
+                assert float((y.double() - want).norm() / want.norm()) <= 2.8e-4, (quant, scales.dtype, epilogue)
+    assert int(_lib.load().cacheir_b200_device_status(1)) == 0
