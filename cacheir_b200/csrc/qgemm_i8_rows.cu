@@ -187,8 +187,8 @@ qgemm_i8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       }
     }
   } else if (warp < kConverters) {
-    // ---------------- epilogue: lane quarter = warp % 4, a thread owns one weight row and 64 of the activation rows ----------------
-    // About ten instructions per output; a scheduler has two of these warps, so the loops keep 16 independent outputs going.
+    // ---------------- epilogue: lane quarter = warp % 4, a thread owns one weight row and kGroupRows of the activation rows ----------------
+    // About ten instructions per output; a scheduler has G (two or four) of these warps, so the loops keep 16 independent outputs going.
     const int q = warp & 3;
     const int r = q * 32 + lane;
     const int group = (warp - 2) >> 2;
